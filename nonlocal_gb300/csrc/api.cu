@@ -218,8 +218,9 @@ CgResult solve_system(Ctx& c, const nlgpu_solve_options& o, nlgpu_solve_report* 
     if (o.preconditioner != NLGPU_PRECONDITIONER_IDENTITY) {
         if (!c.local_ready) build_local(c);
         timer.mark("local matrix");
-        // the exact sweeps' shared-memory plans only when this solve uses them
-        if (!keep_preconditioner) ilt_build(c, c.local, c.ilt, !(mixed && sweeps > 0), mixed && sweeps > 0);
+        // the exact sweeps' shared-memory plans only when this solve uses them (the FP64
+        // CG applies the factor by Jacobi sweeps and builds them itself where it must)
+        if (!keep_preconditioner) ilt_build(c, c.local, c.ilt, mixed && sweeps <= 0, mixed && sweeps > 0);
         timer.mark("preconditioner");
         if (c.ilt.ok) M = &c.ilt;   // identity fallback (stationary_heat_equation_solver_2d.hpp:97-101)
         if (learned && M && !(c.mp.ready && c.mp.n == c.local.rows)) mpnn_prepare(c, c.local);
@@ -913,7 +914,7 @@ int nlgpu_cg_solve(nlgpu_ctx* ctx, int64_t n, const int64_t* a_rowptr, const int
             P.rowptr.upload(prp.data(), prp.size(), c.stream);
             P.col.upload(pc.data(), pc.size(), c.stream);
             P.val.upload(p_val, size_t(P.nnz), c.stream);
-            ilt_build(c, P, ic);
+            ilt_build(c, P, ic, false);
             if (ic.ok) M = &ic;
         }
         const CgResult r = cg_solve(c, A, M, db.p, dx.p, tolerance, max_iterations, x0 != nullptr);

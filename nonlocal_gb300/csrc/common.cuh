@@ -226,6 +226,8 @@ struct JacobiSlab {
     dbuf<int32_t> col;
     dbuf<i64> src;               // entry -> factor value (-1: padding)
     dbuf<float> val;
+    dbuf<double> val64;          // the same in FP64 (pcg.cu)
+    int max_width = 0;           // entries of the widest row
 };
 
 // Level blocks of a sweep plan for one value type (FP64 or FP32).
@@ -285,6 +287,8 @@ struct IncompleteCholesky {
     dbuf<float> jc, jdinv;       // s_i / u_ii and 1 / u_ii
     dbuf<float> jt0, jt1, jy;    // Jacobi iterates and the scaled forward result
     bool ok = false;
+    dbuf<double> jc64, jdinv64;  // the FP64 Jacobi sweeps of the CG kernel (pcg.cu), filled at its first use
+    bool j64_ready = false;
     bool approximate = false;    // factor from the fixed-point sweeps (ilt_build), not the exact IC(0)
     bool exact_ready = false;    // fwd / bwd slabs and plans built and filled (ilt_exact_layouts)
     int attempts = 0;
@@ -295,6 +299,7 @@ struct IncompleteCholesky {
 struct CgWork {
     i64 n = 0;
     dbuf<double> r, z, p, q, x, tmp;
+    dbuf<double> steps, sync;    // tagged values the persistent kernel's CTAs pass on (pcg.cu)
     dbuf<double> partial;        // block partial sums
     dbuf<double> scalars;        // see solver.cu
     dbuf<int> flags;
@@ -532,6 +537,10 @@ struct CgResult {
 using CgChunkHook = std::function<void(i64 iterations, const double* x)>;
 CgResult cg_solve(Ctx& ctx, const Csr& A_full, const IncompleteCholesky* M, const double* b, double* x,
                   double tolerance, i64 max_iterations, bool x_is_initial_guess, const CgChunkHook& on_chunk = {});
+// pcg.cu: CG in one persistent kernel (identity, or the ILLT by FP64 Jacobi sweeps);
+// false when the factor needs the exact triangular solves
+bool pcg_solve(Ctx& ctx, const Csr& A_full, const IncompleteCholesky* M, const double* b, double* x, double tolerance,
+               i64 max_iterations, bool x_is_initial_guess, const CgChunkHook& on_chunk, CgResult& result);
 // sweep.cu
 bool sweep_plan_build(Ctx& ctx, const std::vector<i64>& lev_ptr, const std::vector<int32_t>& rows,
                       const std::vector<i64>& rp, const std::vector<int32_t>& col, const std::vector<i64>& val_index,

@@ -118,12 +118,13 @@ struct TriRows {
     __device__ __forceinline__ i64 last(i64 r) const { return lower ? rp[r + 1] - 1 : rp[r + 1]; }
 };
 
-__global__ void k_slice_width(i64 n, TriRows tr, i64* __restrict__ cnt) {
+__global__ void k_slice_width(i64 n, TriRows tr, i64* __restrict__ cnt, int* __restrict__ widest) {
     const i64 slices = (n + 31) / 32;
     for (i64 sl = blockIdx.x * i64(blockDim.x) + threadIdx.x; sl < slices; sl += i64(gridDim.x) * blockDim.x) {
         i64 w = 0;
         for (i64 r = sl * 32; r < min(n, sl * 32 + 32); ++r) w = max(w, tr.last(r) - tr.first(r));
         cnt[sl] = 32 * w;
+        atomicMax(widest, int(w));
     }
 }
 
@@ -147,12 +148,14 @@ __global__ void k_slice_fill(i64 n, TriRows tr, const int32_t* __restrict__ cols
     }
 }
 
-void jacobi_slab_gpu(Ctx& ctx, i64 n, TriRows tr, const int32_t* cols, const i64* src_of, JacobiSlab& s) {
+void jacobi_slab_gpu(Ctx& ctx, i64 n, TriRows tr, const int32_t* cols, const i64* src_of, JacobiSlab& s, int* widest) {
     const i64 slices = (n + 31) / 32;
     s.slice.resize(size_t(slices + 1));
     NL_CUDA(cudaMemsetAsync(s.slice.p + slices, 0, sizeof(i64), ctx.stream));
-    NL_LAUNCH(k_slice_width, grid_for(slices, IB_THREADS), IB_THREADS, 0, ctx.stream, n, tr, s.slice.p);
-    i64 total = 0;
+    NL_CUDA(cudaMemsetAsync(widest, 0, sizeof(int), ctx.stream));
+    NL_LAUNCH(k_slice_width, grid_for(slices, IB_THREADS), IB_THREADS, 0, ctx.stream, n, tr, s.slice.p, widest);
+    NL_CUDA(cudaMemcpyAsync(&s.max_width, widest, sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
+    i64 total = 0;   // the scan's read of it also completes max_width
     exclusive_scan(ctx, s.slice.p, s.slice.p, slices + 1, &total);
     s.entries = total;
     const size_t m = size_t(std::max<i64>(total, 1));
@@ -216,8 +219,8 @@ void ilt_structure_gpu(Ctx& ctx, const Csr& upper, IncompleteCholesky& ic, bool 
     NL_REQUIRE(ho[1] == n, NLGPU_ERR_STATE, "the factor's dependency graph does not reach every row");
     ic.ic_levels = levels ? ho[0] : 0;
     // Jacobi layouts of U^T (values u[l_to_u]) and U
-    jacobi_slab_gpu(ctx, n, TriRows{ic.lrp.p, true}, ic.lcol.p, ic.l_to_u.p, ic.jlo);
-    jacobi_slab_gpu(ctx, n, TriRows{ic.rp.p, false}, ic.col.p, nullptr, ic.jup);
+    jacobi_slab_gpu(ctx, n, TriRows{ic.lrp.p, true}, ic.lcol.p, ic.l_to_u.p, ic.jlo, bad.p);
+    jacobi_slab_gpu(ctx, n, TriRows{ic.rp.p, false}, ic.col.p, nullptr, ic.jup, bad.p);
     ic.jc.resize(size_t(n)); ic.jdinv.resize(size_t(n));
     ic.jt0.resize(size_t(n)); ic.jt1.resize(size_t(n)); ic.jy.resize(size_t(n));
     NL_CUDA(cudaStreamSynchronize(ctx.stream));

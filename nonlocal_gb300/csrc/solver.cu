@@ -6,7 +6,10 @@
 // NaturalOrdering> (eigen_preconditioner.hpp:57) built from p1*K_local
 // (stationary_heat_equation_solver_2d.hpp:91-101).
 //
-// GB300 form:
+// cg_solve runs the persistent kernel of pcg.cu (identity, or the ILLT applied by
+// FP64 Jacobi sweeps).  Here are the ILLT factorisation, the products the other
+// solvers share, and CG with the exact triangular solves, for the factors whose
+// Jacobi sweeps contract too slowly and for NLGPU_OPTION_GLOBAL_SWEEPS:
 //   * SpMV on full-row CSR (both triangles, rows padded to multiples of 4):
 //     one warp per row, 16-byte loads of 4 columns and 2x2 values, no atomics;
 //   * all CG scalars stay on the device: reductions write one partial per
@@ -17,12 +20,12 @@
 //     per chunk;
 //   * ILLT: Lin-More scaling S = diag(|a_j|_2)^(-1/2) and diagonal shift retry
 //     (alpha_S = 1e-3, doubled, at most 10 attempts) around IC(0) on the
-//     pattern of the upper local matrix, factored level by level in one CTA;
-//     the triangular solves run level by level in one CTA over a per-level
-//     column-major (ELL) copy of the factor, so consecutive threads read
-//     consecutive entries.  Eigen's factorisation additionally admits fill
-//     entries larger than the dropped originals; this one keeps the original
-//     pattern (the converged solution is the same to the tolerance).
+//     pattern of the upper local matrix; the exact triangular solves run level
+//     by level in one CTA over a per-level column-major (ELL) copy of the
+//     factor, so consecutive threads read consecutive entries.  Eigen's
+//     factorisation additionally admits fill entries larger than the dropped
+//     originals; this one keeps the original pattern (the converged solution is
+//     the same to the tolerance).
 #include "common.cuh"
 
 #include <algorithm>
@@ -146,15 +149,6 @@ __global__ void __launch_bounds__(RED_THREADS) k_update_xr(i64 n, double* __rest
 __device__ __forceinline__ bool converged(const double* partials, const double* flags, double tol2, double* sh) {
     const double rr = sum_partials(partials + P_RR * RED_BLOCKS, sh);
     return rr <= tol2 * flags[S_BB];
-}
-
-// z = r (identity preconditioner), skipped after convergence
-__global__ void __launch_bounds__(RED_THREADS) k_copy_if_running(i64 n, const double* __restrict__ r, double* __restrict__ z,
-                                                                 const double* __restrict__ partials,
-                                                                 const double* __restrict__ flags, double tol2) {
-    __shared__ double sh[40];
-    if (flags[S_DONE] != 0.0 || converged(partials, flags, tol2, sh)) return;
-    for (i64 i = blockIdx.x * i64(blockDim.x) + threadIdx.x; i < n; i += i64(gridDim.x) * blockDim.x) z[i] = r[i];
 }
 
 // beta = rz_new / rz_old; p = z + beta p; raises the done flag on convergence
@@ -584,11 +578,6 @@ void precondition(Ctx& ctx, const IncompleteCholesky* M, const double* r, double
         sweep_apply(ctx, const_cast<IncompleteCholesky&>(*M), r, z, partials, flags, tol2);
         return;
     }
-    if (!M) {
-        if (flags) NL_LAUNCH(k_copy_if_running, RED_BLOCKS, RED_THREADS, 0, ctx.stream, n, r, z, partials, flags, tol2);
-        else NL_LAUNCH(k_copy, grid_for(n, 256), 256, 0, ctx.stream, n, r, z);
-        return;
-    }
     // y = U^-T (S r); z = S U^-1 y
     NL_LAUNCH(k_trisolve<double>, 1, TRI_THREADS, 0, ctx.stream, n, M->fwd.n_levels, M->fwd.lev_ptr.p, M->fwd.slab_base.p,
               M->fwd.width.p, M->fwd.rows.p, M->fwd.col.p, M->fwd.val.p, M->fwd.inv_diag.p, r, M->scale.p, M->y.p,
@@ -664,6 +653,7 @@ void ilt_build(Ctx& ctx, const Csr& upper, IncompleteCholesky& ic, bool tma_plan
     ic.bwd_plan = SweepPlan{};
     for (TriSlab* sl : {&ic.fwd, &ic.bwd}) { sl->n_levels = 0; sl->entries = 0; }
     ic.exact_ready = false;
+    ic.j64_ready = false;
     ic.y.resize(size_t(n + 1)); ic.w.resize(size_t(n + 1));
     ic.y32.resize(size_t(n + 1)); ic.w32.resize(size_t(n + 1));
     // Lin-More scaling and the shifted factorisation
@@ -738,7 +728,12 @@ void ilt_apply(Ctx& ctx, const IncompleteCholesky& ic, const double* r, double* 
 
 CgResult cg_solve(Ctx& ctx, const Csr& A, const IncompleteCholesky* M, const double* b, double* x,
                   double tolerance, i64 max_iterations, bool x_is_initial_guess, const CgChunkHook& on_chunk) {
-    if (M) ilt_exact_layouts(ctx, const_cast<IncompleteCholesky&>(*M));
+    if (!(M && ctx.force_global_sweeps)) {
+        CgResult r;
+        if (pcg_solve(ctx, A, M, b, x, tolerance, max_iterations, x_is_initial_guess, on_chunk, r)) return r;
+    }
+    // exact triangular sweeps: asked for, or a factor whose Jacobi sweeps contract too slowly
+    ilt_exact_layouts(ctx, const_cast<IncompleteCholesky&>(*M));
     const i64 n = A.rows;
     CgWork& w = ctx.cg;
     w.n = n;

@@ -1,0 +1,70 @@
+"""The FP64 CG kernel (ILLT by FP64 Jacobi sweeps, or the identity) on caller matrices of the sizes where its
+row split changes: fewer rows than a CTA's minimum, partial last CTAs, one row more than the CTAs hold, and
+a system whose vectors do not fit shared memory."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from nonlocal_gb300 import _lib
+    from nonlocal_gb300 import thermal as T
+    if _lib.device_count() == 0:
+        pytest.skip("no CUDA device")
+    return T.Context()
+
+
+def banded(n, band, seed, dominance):
+    """A symmetric matrix of `band` random off-diagonals (every third one empty beyond the first) whose diagonal is
+    `dominance` times the row's absolute sum: eigenvalues within (1 -+ 1 / dominance) of the diagonal."""
+    import scipy.sparse as sp
+    rng = np.random.default_rng(seed)
+    offs = [k for k in range(1, band + 1) if k < n and (k == 1 or k % 3)]
+    U = sp.diags([-rng.uniform(0.1, 1.0, n - k) for k in offs], offs, shape=(n, n)) if offs else sp.csr_matrix((n, n))
+    A = (U + U.T).tocsr()
+    d = dominance * np.maximum(np.asarray(abs(A).sum(axis=1)).ravel(), 1.0)
+    return (A + sp.diags(d)).tocsr(), (U + sp.diags(d)).tocsr()
+
+
+@pytest.mark.parametrize("preconditioned", [True, False])
+@pytest.mark.parametrize("n, band", [(1, 1), (7, 3), (8, 2), (9, 8), (33, 40), (152 * 8, 5), (152 * 8 + 1, 17),
+                                     (152 * 16 - 3, 30), (5003, 70), (152 * 1024 + 5, 4)])
+def test_pcg_sizes(ctx, n, band, preconditioned):
+    from scipy.sparse.linalg import spsolve
+    from nonlocal_gb300 import thermal as T
+    A, U = banded(n, band, n, 1.25)
+    U.sort_indices()
+    csr = (U.indptr.astype(np.int64), U.indices.astype(np.int64), U.data)
+    b = np.random.default_rng(1).standard_normal(n)
+    x, rep = T.conjugate_gradient(ctx, csr, b, preconditioner_csr=csr if preconditioned else None, tolerance=1e-12)
+    assert np.linalg.norm(b - A @ x) <= 1.01e-12 * np.linalg.norm(b)
+    assert rep.residual <= 1e-12
+    # |x - x*| <= |r| / lambda_min, lambda_min >= 0.2 / 1.25 of the smallest diagonal
+    ref = spsolve(A.tocsc(), b)
+    lo = A.diagonal().min() * 0.2 / 1.25
+    assert np.linalg.norm(x - ref) <= 2e-12 * np.linalg.norm(b) / lo
+    # from the solution itself: nothing left to do
+    again, rep2 = T.conjugate_gradient(ctx, csr, b, x0=x, preconditioner_csr=csr if preconditioned else None,
+                                       tolerance=1e-11)
+    assert rep2.iterations == 0 and np.array_equal(again, x)
+
+
+def test_slowly_contracting_factor_takes_the_exact_sweeps(ctx):
+    """A tridiagonal matrix: IC(0) is the exact factor, whose Jacobi sweeps would need hundreds of steps, so the
+    solve goes back to the exact triangular sweeps and ends after one or two iterations."""
+    from nonlocal_gb300 import thermal as T
+    n = 700
+    rp = np.append(np.arange(0, 2 * n, 2), 2 * n - 1).astype(np.int64)
+    col = np.empty(2 * n - 1, dtype=np.int64)
+    val = np.empty(2 * n - 1)
+    col[0::2], col[1::2] = np.arange(n), np.arange(1, n)
+    val[0::2], val[1::2] = 2.0001, -1.0
+    b = np.sin(0.37 * np.arange(n))
+    x, rep = T.conjugate_gradient(ctx, (rp, col, val), b, preconditioner_csr=(rp, col, val), tolerance=1e-10)
+    assert rep.iterations <= 3 and rep.residual <= 1e-10
+    r = b - 2.0001 * x
+    r[:-1] += x[1:]
+    r[1:] += x[:-1]
+    assert np.linalg.norm(r) <= 1.01e-10 * np.linalg.norm(b)

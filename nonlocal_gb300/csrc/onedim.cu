@@ -11,8 +11,8 @@
 //     Eigen::SimplicialCholesky<..., Upper, NaturalOrdering>).
 //
 // Assembly: one thread per (element, neighbour element) pair computes the
-// (order+1)^2 block.  Factorisation: one CTA walks the diagonal; at step k
-// every thread updates part of the trailing (bandwidth x bandwidth) window.
+// (order+1)^2 block.  Factorisation: blocks of 16 rows in one cluster of 16 CTAs
+// (k_band_factor); the substitutions use the inverses of its diagonal blocks.
 //
 // 1D nonstationary (nonstationary_heat_equation_solver_1d.hpp:24-259):
 // compute() assembles A = dt K + C (C the local capacity matrix c rho int N_i N_j,
@@ -100,10 +100,25 @@ __global__ void k_assemble_1d(Problem1d P, Line L, double* __restrict__ band, do
         const i64 e = t / width, f = e - P.nb + t % width;
         if (f < 0 || f >= P.E) continue;
         const bool nonlocal = P.p1 < 0.999;
-        double xl[3], xn[3];
-        for (int q = 0; q < L.nq; ++q) {
-            xl[q] = P.h * double(e) + (L.x[q] - (-1.0)) * P.jac;
-            xn[q] = P.h * double(f) + (L.x[q] - (-1.0)) * P.jac;
+        // pairs below the diagonal keep only the node two neighbours share and the
+        // right end's bound row
+        if (f < e - 1 && !(P.fk1 && e == P.E - 1)) continue;
+        double inner[3][3];   // [qL][j]: the influence once per pair of points, not per entry
+        if (nonlocal) {
+            double xl[3], xn[3];
+            for (int q = 0; q < L.nq; ++q) {
+                xl[q] = P.h * double(e) + (L.x[q] - (-1.0)) * P.jac;
+                xn[q] = P.h * double(f) + (L.x[q] - (-1.0)) * P.jac;
+            }
+            for (int qL = 0; qL < L.nq; ++qL) {
+                double g[3];
+                for (int qNL = 0; qNL < L.nq; ++qNL) g[qNL] = influence_1d(P, xl[qL], xn[qNL]) * P.lambda * L.w[qNL];
+                for (int j = 0; j < L.nen; ++j) {
+                    double v = 0.0;
+                    for (int qNL = 0; qNL < L.nq; ++qNL) v += g[qNL] * L.qNxi[j * L.nq + qNL];
+                    inner[qL][j] = v;
+                }
+            }
         }
         for (int i = 0; i < L.nen; ++i) {
             const i64 row = e * P.order + i;
@@ -111,12 +126,7 @@ __global__ void k_assemble_1d(Problem1d P, Line L, double* __restrict__ band, do
                 const i64 col = f * P.order + j;
                 if (nonlocal) {
                     double integral = 0.0;
-                    for (int qL = 0; qL < L.nq; ++qL) {
-                        double inner = 0.0;
-                        for (int qNL = 0; qNL < L.nq; ++qNL)
-                            inner += influence_1d(P, xl[qL], xn[qNL]) * P.lambda * L.w[qNL] * L.qNxi[j * L.nq + qNL];
-                        integral += L.w[qL] * L.qNxi[i * L.nq + qL] * inner;
-                    }
+                    for (int qL = 0; qL < L.nq; ++qL) integral += L.w[qL] * L.qNxi[i * L.nq + qL] * inner[qL][j];
                     band_add(P, band, bound0, boundN, row, col, (1.0 - P.p1) * integral);
                 }
                 if (f == e) {
@@ -150,60 +160,276 @@ __global__ void k_first_kind_1d(i64 n, const double* __restrict__ bound0, double
     }
 }
 
-// In-place band LDL^T (upper band: band[i*(bw+1) + (j-i)]) in one CTA.  Step
-// k scales row k by 1/d_k after using it to update the trailing window.
-// Returns false (and raises *failed) on a zero pivot.
-__device__ bool band_ldlt(i64 n, i64 bw, double* __restrict__ band, int* __restrict__ failed) {
-    const i64 w = bw + 1;
-    __shared__ double dk;
-    for (i64 k = 0; k < n; ++k) {
-        if (threadIdx.x == 0) {
-            dk = band[k * w];
-            if (dk == 0.0) *failed = 1;
-        }
-        __syncthreads();
-        if (dk == 0.0) return false;
-        const i64 m = min(bw, n - 1 - k);   // rows k+1 .. k+m
-        for (i64 t = threadIdx.x; t < m * m; t += blockDim.x) {
-            const i64 a = t / m + 1, b = t % m + 1;   // row k+a, col k+b
-            if (b < a) continue;
-            const double uka = band[k * w + a], ukb = band[k * w + b];
-            band[(k + a) * w + (b - a)] -= uka * ukb / dk;
-        }
-        __syncthreads();
-        for (i64 t = threadIdx.x + 1; t <= m; t += blockDim.x) band[k * w + t] /= dk;
-        __syncthreads();
-    }
-    return true;
+// Band LDL^T in blocks of BF_NB rows, one cluster of BF_CTAS CTAs (upper band:
+// band[i * (bw + 1) + (j - i)]).
+//
+// A row at a time, every pivot cost three CTA barriers and bw^2 / 2 updates with a
+// division each on one SM's FP64 pipe (two lanes a clock): 33 us a pivot,
+// 66.8 ms for 2 001 rows of half bandwidth 102.  Here a block of 16 pivots is one
+// warp's work in registers: it eliminates [A_kk | I], lane j < 16 holding column
+// j of A_kk and lane 16 + j column j of I, which leaves D L^T and L^-1 at no extra
+// instructions; those 216 FP64 instructions of one warp (64 cycles each on its
+// quarter of the SM's FP64 pipe) are the critical path, and everything else is
+// spread over the cluster between two of them:
+//   W = L^-1 A(block, columns after it)                 (all CTAs)
+//   A(i, j) -= sum_k W(k, i) W(k, j) / d_k               (all CTAs but the first)
+//   next diagonal block: the same update, then its elimination   (first CTA)
+// with one cluster barrier after each phase.  The rows keep U = D^-1 W beyond
+// their block; L^-1 and 1 / d are kept per block.  The right-hand side, when there
+// is one, is one more column (its forward substitution comes for free).
+// 2 001 rows of half bandwidth 102: 66.8 -> 2.0 ms, of which the eliminations 1.1.
+constexpr int BF_NB = 16;
+constexpr int BF_CTAS = 16;
+constexpr int BF_THREADS = 256;
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
-__global__ void __launch_bounds__(1024) k_band_ldlt(i64 n, i64 bw, double* __restrict__ band, int* __restrict__ failed) {
-    band_ldlt(n, bw, band, failed);
+struct BandFactor {
+    i64 n, bw;
+    double* band;
+    double* f;                // right-hand side, becomes L^-1 f (null: none)
+    double* linv;             // [blocks][BF_NB][BF_NB]
+    double* dinv;             // [blocks * BF_NB]
+    double* w;                // [BF_NB][bw + 1] scratch
+    int* failed;
+    int in_shared;            // W is copied to shared memory
+};
+
+// 1 / d by two Newton steps from the hardware's approximation, without the
+// division's special cases (the chain of pivots waits for it).  0 gives a
+// non-finite value, as the division.
+__device__ __forceinline__ double reciprocal(double d) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    r = fma(fma(-d, r, 1.0), r, r);
+    return fma(fma(-d, r, 1.0), r, r);
 }
 
-// U^T D U x = f with the factor of k_band_ldlt (unit upper U), by one warp:
-// forward U^T y = f, y /= d, backward U x = y.  Every row's dot product is
-// spread over the lanes and reduced by shuffles; __syncwarp orders each
-// solved value before the next row reads it.
-__global__ void __launch_bounds__(32) k_band_solve_warp(i64 n, i64 bw, const double* __restrict__ band,
-                                                        double* __restrict__ f) {
-    const i64 w = bw + 1;
-    const int lane = threadIdx.x;
-    for (i64 i = 1; i < n; ++i) {
-        double s = 0.0;
-        for (i64 k = max(i64(0), i - bw) + lane; k < i; k += 32) s += band[k * w + (i - k)] * f[k];
-        s = warp_sum(s);
-        if (lane == 0) f[i] -= s;
-        __syncwarp();
+// eliminates the diagonal block in `a` (rows i of column lane), writes L^-1 and 1 / d
+__device__ __forceinline__ void eliminate_block(double (&a)[BF_NB], double* linv, double* dinv, int* failed) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < BF_NB; ++k) {
+        // row k is final; by symmetry its lane i holds the multiplier of row i, so the
+        // broadcasts do not wait for the reciprocal
+        const double t = a[k], d = __shfl_sync(0xffffffffu, t, k);
+        double u[BF_NB];
+#pragma unroll
+        for (int i = k + 1; i < BF_NB; ++i) u[i] = __shfl_sync(0xffffffffu, t, i);
+        const double inv = reciprocal(d);
+        if (lane == 0) {
+            dinv[k] = inv;
+            if (d == 0.0) *failed = 1;
+        }
+        const double s = -t * inv;
+#pragma unroll
+        for (int i = k + 1; i < BF_NB; ++i) a[i] = fma(u[i], s, a[i]);   // row k + 1, the next pivot's, first
     }
-    for (i64 i = lane; i < n; i += 32) f[i] /= band[i * w];
-    __syncwarp();
-    for (i64 i = n - 2; i >= 0; --i) {
-        double s = 0.0;
-        for (i64 j = i + 1 + lane; j <= min(n - 1, i + bw); j += 32) s += band[i * w + (j - i)] * f[j];
-        s = warp_sum(s);
-        if (lane == 0) f[i] -= s;
-        __syncwarp();
+    if (lane >= BF_NB)
+#pragma unroll
+        for (int i = 0; i < BF_NB; ++i) linv[i * BF_NB + lane - BF_NB] = a[i];
+}
+
+__global__ void __launch_bounds__(BF_THREADS) k_band_factor(BandFactor p) {
+    extern __shared__ double bf_w[];
+    __shared__ double diag[BF_NB][BF_NB + 1], scaled[BF_NB][BF_NB], dk[BF_NB], lk[BF_NB * BF_NB];
+    const i64 w = p.bw + 1, blocks = (p.n + BF_NB - 1) / BF_NB;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x;
+    // entry (i, j >= i) of the matrix, rows past the end an identity
+    auto entry = [&](i64 i, i64 j) {
+        if (i >= p.n || j >= p.n) return i == j ? 1.0 : 0.0;
+        return j - i <= p.bw ? p.band[i * w + (j - i)] : 0.0;
+    };
+    auto eliminate = [&](i64 kb) {   // warp 0 of the first CTA, the block in `diag` (upper)
+        double a[BF_NB];
+#pragma unroll
+        for (int i = 0; i < BF_NB; ++i)
+            a[i] = lane < BF_NB ? diag[min(i, lane)][max(i, lane)] : (i == lane - BF_NB ? 1.0 : 0.0);
+        eliminate_block(a, p.linv + kb * BF_NB * BF_NB, p.dinv + kb * BF_NB, p.failed);
+    };
+    if (rank == 0) {
+        diag[tid >> 4][tid & 15] = (tid >> 4) <= (tid & 15) ? entry(tid >> 4, tid & 15) : 0.0;
+        __syncthreads();
+        if (warp == 0) eliminate(0);
+    }
+    for (i64 kb = 0; kb < blocks; ++kb) {
+        cluster_barrier();
+        const i64 k0 = kb * BF_NB, next = k0 + BF_NB;
+        const int m = int(max(i64(0), min(p.bw, p.n - next)));   // columns after the block that it reaches
+        const int cols = m + (p.f ? 1 : 0);
+        if (tid < BF_NB) dk[tid] = p.dinv[k0 + tid];
+        lk[tid] = p.linv[kb * BF_NB * BF_NB + tid];
+        __syncthreads();
+        for (int t = tid * BF_CTAS + rank; t < BF_NB * cols; t += BF_CTAS * BF_THREADS) {
+            const int r = t / cols, c = t % cols;
+            double v = 0.0, v2 = 0.0;
+#pragma unroll
+            for (int s = 0; s < BF_NB; s += 2) {
+                const double x = c < m ? entry(k0 + s, next + c) : (k0 + s < p.n ? p.f[k0 + s] : 0.0);
+                const double y = c < m ? entry(k0 + s + 1, next + c) : (k0 + s + 1 < p.n ? p.f[k0 + s + 1] : 0.0);
+                if (s <= r) v = fma(lk[r * BF_NB + s], x, v);
+                if (s + 1 <= r) v2 = fma(lk[r * BF_NB + s + 1], y, v2);
+            }
+            p.w[i64(r) * w + c] = v + v2;
+        }
+        cluster_barrier();
+        const double* W = p.w;
+        if (p.in_shared) {
+            for (int t = tid; t < BF_NB * cols; t += BF_THREADS) bf_w[i64(t / cols) * w + t % cols] = p.w[i64(t / cols) * w + t % cols];
+            W = bf_w;
+            __syncthreads();
+        }
+        if (rank == 0) {
+            if (kb + 1 < blocks) {
+                const int r = tid >> 4, c = tid & 15;
+                scaled[r][c] = c < m ? W[r * w + c] * dk[r] : 0.0;
+                __syncthreads();
+                double v = 0.0;
+                if (r <= c) {
+                    v = entry(next + r, next + c);
+                    if (c < m) {
+                        double u = 0.0, u2 = 0.0;
+#pragma unroll
+                        for (int k = 0; k < BF_NB; k += 2) {
+                            u = fma(scaled[k][r], W[k * w + c], u);
+                            u2 = fma(scaled[k + 1][r], W[(k + 1) * w + c], u2);
+                        }
+                        v -= u + u2;
+                    }
+                }
+                diag[r][c] = v;
+                __syncthreads();
+                if (warp == 0) eliminate(kb + 1);
+            }
+            // the block's rows: U = D^-1 W, and L^-1 f
+            if (warp > 0)
+                for (int t = tid - 32; t < BF_NB * cols; t += BF_THREADS - 32) {
+                    const int r = t / cols, c = t % cols;
+                    if (k0 + r >= p.n) continue;
+                    if (c == m) p.f[k0 + r] = W[r * w + c];
+                    else if (BF_NB + c - r <= p.bw) p.band[(k0 + r) * w + (BF_NB + c - r)] = W[r * w + c] * dk[r];
+                }
+        } else {
+            // a warp per row a, rows dealt out over the other CTAs
+            for (int a = (rank - 1) + (BF_CTAS - 1) * warp; a < m; a += (BF_CTAS - 1) * (BF_THREADS / 32)) {
+                double wa[BF_NB];
+#pragma unroll
+                for (int k = 0; k < BF_NB; ++k) wa[k] = W[k * w + a] * dk[k];
+                // the next diagonal block is the first CTA's
+                for (int b = (a < BF_NB ? BF_NB : a) + lane; b < cols; b += 32) {
+                    double v = 0.0, v2 = 0.0;
+#pragma unroll
+                    for (int k = 0; k < BF_NB; k += 2) {
+                        v = fma(wa[k], W[k * w + b], v);
+                        v2 = fma(wa[k + 1], W[(k + 1) * w + b], v2);
+                    }
+                    if (b < m) p.band[(next + a) * w + (b - a)] -= v + v2;
+                    else p.f[next + a] -= v + v2;
+                }
+                // the right-hand side's entry of a short window (m < 16)
+                if (p.f && m < BF_NB && lane == 0) {
+                    double v = 0.0;
+#pragma unroll
+                    for (int k = 0; k < BF_NB; ++k) v = fma(wa[k], W[k * w + m], v);
+                    p.f[next + a] -= v;
+                }
+            }
+        }
+    }
+}
+
+// The substitutions with the factor of k_band_factor in one CTA, a block at a
+// time: forward y = L^-1 f (skipped when the factorisation carried f along), then
+// x = L^-T (D^-1 y - U x beyond the block).  The factor's entries of the next
+// block are loaded while the current one is worked on, the vector stays in shared
+// memory.  667 rows of half bandwidth 48: both substitutions 147 us a step, a row
+// at a time in one warp about 460.
+__global__ void __launch_bounds__(BF_THREADS) k_band_solve(i64 n, i64 bw, const double* __restrict__ band,
+                                                           const double* __restrict__ linv,
+                                                           const double* __restrict__ dinv, double* fg, bool forward,
+                                                           bool in_shared) {
+    extern __shared__ double bs_f[];
+    __shared__ double blk[BF_NB];
+    double* f = in_shared ? bs_f : fg;
+    if (in_shared) {
+        for (i64 i = threadIdx.x; i < n; i += BF_THREADS) f[i] = fg[i];
+        __syncthreads();
+    }
+    const i64 w = bw + 1, blocks = (n + BF_NB - 1) / BF_NB;
+    const int tid = threadIdx.x, r = tid >> 4, l = tid & 15;   // 16 lanes per row of a block
+    auto sum16 = [](double v) {
+        for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        return v;
+    };
+    if (forward) {
+        double u[BF_NB], lv = 0.0;
+        auto load = [&](i64 kb) {
+            const i64 k0 = kb * BF_NB;
+            lv = linv[kb * BF_NB * BF_NB + tid];
+            const i64 j = k0 + BF_NB + tid;
+#pragma unroll
+            for (int s = 0; s < BF_NB; ++s) u[s] = j < n && BF_NB + tid - s <= bw ? band[(k0 + s) * w + (BF_NB + tid - s)] : 0.0;
+        };
+        load(0);
+        for (i64 kb = 0; kb < blocks; ++kb) {
+            const i64 k0 = kb * BF_NB;
+            const double y = sum16(l <= r && k0 + l < n ? lv * f[k0 + l] : 0.0);
+            if (l == 0) blk[r] = y;
+            __syncthreads();
+            if (tid < BF_NB && k0 + tid < n) f[k0 + tid] = blk[tid];
+            const i64 j = k0 + BF_NB + tid;
+            if (j < n && tid < bw) {
+                double v = 0.0, v2 = 0.0;
+#pragma unroll
+                for (int s = 0; s < BF_NB; s += 2) { v = fma(u[s], blk[s], v); v2 = fma(u[s + 1], blk[s + 1], v2); }
+                f[j] -= v + v2;
+            }
+            for (i64 c = tid + BF_THREADS; c < bw && k0 + BF_NB + c < n; c += BF_THREADS) {   // wide bands
+                double v = 0.0;
+                for (int s = 0; s < BF_NB; ++s)
+                    if (BF_NB + c - s <= bw) v = fma(band[(k0 + s) * w + (BF_NB + c - s)], blk[s], v);
+                f[k0 + BF_NB + c] -= v;
+            }
+            if (kb + 1 < blocks) load(kb + 1);
+            __syncthreads();
+        }
+    }
+    constexpr int PER = 8;   // entries of U per lane kept ahead: half bandwidths up to 128
+    double u[PER], lv = 0.0, di = 0.0;
+    auto load = [&](i64 kb) {
+        const i64 i = kb * BF_NB + r;
+        lv = linv[kb * BF_NB * BF_NB + l * BF_NB + r];
+        di = dinv[i];
+#pragma unroll
+        for (int s = 0; s < PER; ++s) {
+            const int c = l + 16 * s;
+            u[s] = i < n && kb * BF_NB + BF_NB + c < n && BF_NB + c - r <= bw ? band[i * w + (BF_NB + c - r)] : 0.0;
+        }
+    };
+    load(blocks - 1);
+    for (i64 kb = blocks - 1; kb >= 0; --kb) {
+        const i64 k0 = kb * BF_NB, i = k0 + r, j0 = k0 + BF_NB;
+        double v = 0.0, v2 = 0.0;
+#pragma unroll
+        for (int s = 0; s < PER; ++s) {
+            const i64 j = j0 + l + 16 * s;
+            if (j < n && l + 16 * s < bw) (s & 1 ? v2 : v) = fma(u[s], f[j], s & 1 ? v2 : v);
+        }
+        v += v2;
+        for (i64 c = l + 16 * PER; i < n && c < bw && j0 + c < n && BF_NB + c - r <= bw; c += 16)
+            v = fma(band[i * w + (BF_NB + c - r)], f[j0 + c], v);
+        v = sum16(v);
+        if (l == 0) blk[r] = i < n ? fma(f[i], di, -v) : 0.0;
+        __syncthreads();
+        const double x = sum16(l >= r ? lv * blk[l] : 0.0);
+        if (kb > 0) load(kb - 1);
+        if (l == 0 && i < n) {
+            f[i] = x;
+            if (in_shared) fg[i] = x;
+        }
+        __syncthreads();
     }
 }
 
@@ -279,34 +505,45 @@ __global__ void k_step_rhs_1d(Problem1d P, double dt, const double* __restrict__
     }
 }
 
-// One CTA: band LDL^T and both triangular solves (the stationary solve).
-__global__ void __launch_bounds__(1024) k_band_ldlt_solve(i64 n, i64 bw, double* __restrict__ band, double* __restrict__ f,
-                                                          int* __restrict__ failed) {
-    const i64 w = bw + 1;
-    if (!band_ldlt(n, bw, band, failed)) return;
-    // U^T D U x = f with unit upper U: forward U^T y = f
-    for (i64 i = 1; i < n; ++i) {
-        double s = 0.0;
-        for (i64 k = max(i64(0), i - bw) + threadIdx.x; k < i; k += blockDim.x) s += band[k * w + (i - k)] * f[k];
-        s = warp_sum(s);
-        __shared__ double red[32];
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-        __syncthreads();
-        if (threadIdx.x == 0) { double tsum = 0.0; for (int q = 0; q < int(blockDim.x >> 5); ++q) tsum += red[q]; f[i] -= tsum; }
-        __syncthreads();
+// L^-1 and 1 / d of the blocks, and the factorisation's scratch
+struct BandWork {
+    dbuf<double> linv, dinv, w;
+    void resize(i64 n, i64 bw) {
+        const size_t blocks = size_t((n + BF_NB - 1) / BF_NB);
+        linv.resize(blocks * BF_NB * BF_NB);
+        dinv.resize(blocks * BF_NB);
+        w.resize(size_t(BF_NB) * size_t(bw + 1));
     }
-    for (i64 i = threadIdx.x; i < n; i += blockDim.x) f[i] /= band[i * w];
-    __syncthreads();
-    for (i64 i = n - 2; i >= 0; --i) {
-        double s = 0.0;
-        for (i64 j = i + 1 + threadIdx.x; j <= min(n - 1, i + bw); j += blockDim.x) s += band[i * w + (j - i)] * f[j];
-        s = warp_sum(s);
-        __shared__ double red2[32];
-        if ((threadIdx.x & 31) == 0) red2[threadIdx.x >> 5] = s;
-        __syncthreads();
-        if (threadIdx.x == 0) { double tsum = 0.0; for (int q = 0; q < int(blockDim.x >> 5); ++q) tsum += red2[q]; f[i] -= tsum; }
-        __syncthreads();
-    }
+};
+
+void band_factor(Ctx& ctx, i64 n, i64 bw, double* band, double* f, BandWork& work, int* failed) {
+    work.resize(n, bw);
+    BandFactor p{n, bw, band, f, work.linv.p, work.dinv.p, work.w.p, failed, 0};
+    const size_t bytes = size_t(BF_NB) * size_t(bw + 1) * sizeof(double);
+    p.in_shared = bytes <= 200 * 1024;
+    const size_t smem = p.in_shared ? bytes : 0;
+    NL_CUDA(cudaFuncSetAttribute(k_band_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    NL_CUDA(cudaFuncSetAttribute(k_band_factor, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = BF_CTAS;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(BF_CTAS);
+    cfg.blockDim = dim3(BF_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx.stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    NL_CUDA(cudaLaunchKernelEx(&cfg, k_band_factor, p));
+    count_launch();
+}
+
+void band_solve(Ctx& ctx, i64 n, i64 bw, const double* band, const BandWork& work, double* f, bool forward) {
+    const bool in_shared = n <= 24 * 1024;   // the vector in shared memory
+    const size_t smem = in_shared ? size_t(n) * sizeof(double) : 0;
+    NL_CUDA(cudaFuncSetAttribute(k_band_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    NL_LAUNCH(k_band_solve, 1, BF_THREADS, smem, ctx.stream, n, bw, band, work.linv.p, work.dinv.p, f, forward, in_shared);
 }
 
 // mesh, model and band geometry of one segment [0, length]
@@ -338,6 +575,7 @@ struct OneDimState {
     Line L{};
     double dt = 0.0;
     dbuf<double> a, c, bound0, boundN, t, f;
+    BandWork factor;
 };
 
 void nonstationary_1d_compute(Ctx& ctx, i64 elements, int order, double length, double radius, double local_weight,
@@ -376,7 +614,7 @@ void nonstationary_1d_compute(Ctx& ctx, i64 elements, int order, double length, 
               capacity * density, st->c.p);
     NL_LAUNCH(k_combine_1d, grid_for(i64(nb), 256), 256, 0, ctx.stream, P, time_step, st->a.p, st->c.p, st->bound0.p,
               st->boundN.p);
-    NL_LAUNCH(k_band_ldlt, 1, 1024, 0, ctx.stream, P.n, P.bw, st->a.p, failed.p);
+    band_factor(ctx, P.n, P.bw, st->a.p, nullptr, st->factor, failed.p);
     int hf = 0;
     NL_CUDA(cudaMemcpyAsync(&hf, failed.p, sizeof hf, cudaMemcpyDeviceToHost, ctx.stream));
     NL_CUDA(cudaStreamSynchronize(ctx.stream));
@@ -394,7 +632,7 @@ void nonstationary_1d_step(Ctx& ctx, double left_value, double right_value, bool
               sin_source, st.f.p);
     NL_LAUNCH(k_step_rhs_1d, grid_for(P.n, 256), 256, 0, ctx.stream, P, st.dt, st.c.p, st.t.p, st.bound0.p,
               st.boundN.p, left_value, right_value, st.f.p);
-    NL_LAUNCH(k_band_solve_warp, 1, 32, 0, ctx.stream, P.n, P.bw, st.a.p, st.f.p);
+    band_solve(ctx, P.n, P.bw, st.a.p, st.factor, st.f.p, true);
     std::swap(st.t, st.f);
     if (temperature) st.t.download(temperature, n, ctx.stream);
     NL_CUDA(cudaStreamSynchronize(ctx.stream));
@@ -423,7 +661,9 @@ void stationary_1d(Ctx& ctx, i64 elements, int order, double length, double radi
               static_cast<double*>(nullptr));
     NL_LAUNCH(k_rhs_1d, grid_for(P.E * L.nen, 256), 256, 0, ctx.stream, P, L, q_right, sin_source, f.p);
     NL_LAUNCH(k_first_kind_1d, grid_for(P.n, 256), 256, 0, ctx.stream, P.n, bound0.p, t_left, f.p, band.p);
-    NL_LAUNCH(k_band_ldlt_solve, 1, 1024, 0, ctx.stream, P.n, P.bw, band.p, f.p, failed.p);
+    BandWork factor;
+    band_factor(ctx, P.n, P.bw, band.p, f.p, factor, failed.p);
+    band_solve(ctx, P.n, P.bw, band.p, factor, f.p, false);
     int hf = 0;
     NL_CUDA(cudaMemcpyAsync(&hf, failed.p, sizeof hf, cudaMemcpyDeviceToHost, ctx.stream));
     f.download(temperature, size_t(P.n), ctx.stream);

@@ -67,3 +67,50 @@ def test_nonstationary_1d_rejects_other_ends(lib):
                                                           None))
     with pytest.raises(L.NlgpuError):   # no compute yet
         s.calc_step(0.0, 0.0)
+
+
+@pytest.mark.parametrize("order", [1, 2])
+@pytest.mark.parametrize("elements, radius, p1", [(1, 0.1, 1.0), (7, 0.3, 0.5), (15, 0.1, 1.0), (16, 0.2, 0.5), (33, 0.06, 0.4),
+                                                  (120, 0.9, 0.5), (500, 0.3, 0.5)])
+def test_band_factor_sizes(elements, radius, p1, order):
+    """The blocked band factorisation where its blocks and bands meet edges: fewer rows than a block, a band
+    narrower than a block, wider than the whole matrix and wider than the substitutions' prefetch, the last
+    block partial; the stationary solve and the first implicit Euler step (temperature left, flux right) of the
+    matrices restated densely."""
+    from nonlocal_gb300 import thermal as T
+    g, w = ((np.array([-1.0, 1.0]) / np.sqrt(3.0), np.ones(2)) if order == 1 else
+            (np.array([-1.0, 0.0, 1.0]) * np.sqrt(0.6), np.array([5.0, 8.0, 5.0]) / 9.0))
+    if order == 1:
+        N, D = np.array([(1 - g) / 2, (1 + g) / 2]), np.array([-0.5 + 0 * g, 0.5 + 0 * g])
+    else:
+        N, D = np.array([g * (g - 1) / 2, 1 - g * g, g * (g + 1) / 2]), np.array([g - 0.5, -2 * g, g + 0.5])
+    E, n, h = elements, elements * order + 1, 1.0 / elements
+    x = (np.arange(E)[:, None] + (g + 1) / 2) * h
+    K, C = np.zeros((n, n)), np.zeros((n, n))
+    reach = int(np.floor(radius / h + 0.5)) if p1 < 0.999 else 0
+    for e in range(E):
+        ie = e * order + np.arange(order + 1)
+        K[np.ix_(ie, ie)] += p1 * np.einsum("iq,jq,q->ij", D, D, w) / (h / 2)
+        C[np.ix_(ie, ie)] += np.einsum("iq,jq,q->ij", N, N, w) * (h / 2)
+        for f in range(max(0, e - reach), min(E, e + reach + 1)) if p1 < 0.999 else ():
+            d = np.abs(x[e][:, None] - x[f][None, :])
+            phi = np.where(d < radius, 0.75 / radius * (1 - (d / radius) ** 2), 0.0)
+            K[np.ix_(ie, f * order + np.arange(order + 1))] += (1 - p1) * (D * w) @ phi @ (D * w).T
+    b = np.zeros(n)
+    for e in range(E):
+        b[e * order:e * order + order + 1] += (N * w) @ np.sin(np.pi * x[e]) * (h / 2)
+    b[-1] += 0.7
+    t = T.stationary_heat_equation_solver_1d(elements=E, order=order, radius=radius, local_weight=p1, t_left=0.3,
+                                             q_right=0.7)
+    A, rhs = K[1:, 1:], b[1:] - K[1:, 0] * 0.3
+    # both are backward stable: the residual of the solution, in units of its terms
+    bound = 64 * n * np.finfo(float).eps * (np.abs(A) @ np.abs(t[1:]) + np.abs(rhs))
+    assert t[0] == 0.3 and np.all(np.abs(A @ t[1:] - rhs) <= bound.max())
+    s = T.NonstationaryHeatEquationSolver1D(elements=E, order=order, radius=radius, local_weight=p1, time_step=1e-3)
+    s.compute(("temperature", 0.3), ("flux", 0.7), np.full(n, 0.5))
+    u = s.calc_step()
+    A = (C + 1e-3 * K)[1:, 1:]
+    rhs = C[1:, 1:] @ np.full(n - 1, 0.5) - 1e-3 * K[1:, 0] * 0.3
+    rhs[-1] += 1e-3 * 0.7
+    bound = 64 * n * np.finfo(float).eps * (np.abs(A) @ np.abs(u[1:]) + np.abs(rhs))
+    assert u[0] == 0.3 and np.all(np.abs(A @ u[1:] - rhs) <= bound.max())

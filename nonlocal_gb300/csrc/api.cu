@@ -220,7 +220,10 @@ CgResult solve_system(Ctx& c, const nlgpu_solve_options& o, nlgpu_solve_report* 
         timer.mark("local matrix");
         // the exact sweeps' shared-memory plans only when this solve uses them (the FP64
         // CG applies the factor by Jacobi sweeps and builds them itself where it must)
-        if (!keep_preconditioner) ilt_build(c, c.local, c.ilt, mixed && sweeps <= 0, mixed && sweeps > 0);
+        if (!keep_preconditioner) {
+            const int factor_sweeps = !mixed ? IC_SWEEPS_FP64 : sweeps > 0 ? IC_SWEEPS_FP32 : 0;
+            ilt_build(c, c.local, c.ilt, mixed && sweeps <= 0, factor_sweeps, !mixed);
+        }
         timer.mark("preconditioner");
         if (c.ilt.ok) M = &c.ilt;   // identity fallback (stationary_heat_equation_solver_2d.hpp:97-101)
         if (learned && M && !(c.mp.ready && c.mp.n == c.local.rows)) mpnn_prepare(c, c.local);
@@ -914,7 +917,7 @@ int nlgpu_cg_solve(nlgpu_ctx* ctx, int64_t n, const int64_t* a_rowptr, const int
             P.rowptr.upload(prp.data(), prp.size(), c.stream);
             P.col.upload(pc.data(), pc.size(), c.stream);
             P.val.upload(p_val, size_t(P.nnz), c.stream);
-            ilt_build(c, P, ic, false);
+            ilt_build(c, P, ic, false, IC_SWEEPS_FP64, true);
             if (ic.ok) M = &ic;
         }
         const CgResult r = cg_solve(c, A, M, db.p, dx.p, tolerance, max_iterations, x0 != nullptr);

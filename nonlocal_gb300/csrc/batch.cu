@@ -448,7 +448,7 @@ void batch_prepare_mixed(Batch& bt) {
     bt.solver.n_nodes = bt.N;
     // the exact IC(0): factored once for every step (the fixed-point factor,
     // cheaper to build, took 41 instead of 31 to 41 FCG iterations a step)
-    ilt_build(bt.solver, bt.M, bt.ic, false, false);
+    ilt_build(bt.solver, bt.M, bt.ic, false);
     NL_REQUIRE(bt.ic.ok, NLGPU_ERR_NUMERICAL, "the ILLT of the batched local matrix failed");
     matrix_to_f32(bt.solver, bt.A, nullptr);
     NL_REQUIRE(bt.A.col16_ok, NLGPU_ERR_UNSUPPORTED, "an instance's band is wider than 16-bit column offsets");
@@ -829,7 +829,7 @@ std::vector<CgResult> batch_bicgstab(const std::vector<Ctx*>& instances, double 
         }, false);
         bt.solver.stream = bt.stream;
         bt.solver.n_nodes = N;
-        ilt_build(bt.solver, bt.M, bt.ic, false, true);
+        ilt_build(bt.solver, bt.M, bt.ic, false, IC_SWEEPS_FP32);
         illt = bt.ic.ok;   // the diagonal otherwise (as the reference)
         timer.mark("local matrices, ILLT");
     }

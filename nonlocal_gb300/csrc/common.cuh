@@ -292,7 +292,7 @@ struct IncompleteCholesky {
     bool approximate = false;    // factor from the fixed-point sweeps (ilt_build), not the exact IC(0)
     bool exact_ready = false;    // fwd / bwd slabs and plans built and filled (ilt_exact_layouts)
     int attempts = 0;
-    double shift = 0.0;
+    double shift = 0.0, first_shift = 0.0;
 };
 
 // Persistent device state of CG.
@@ -521,8 +521,14 @@ void nonstationary_rhs(Ctx& ctx, double dirichlet_value, bool per_node_values, c
 void spmv_full(Ctx& ctx, const Csr& A, const double* x, double* y);
 // tma_plans: also build the TMA-fed shared-memory sweep plans of the exact
 // triangular solves (without them exact solves use the global-memory sweeps)
-// approximate: the factor from a few fixed-point sweeps (for the FP32 Jacobi-sweep application)
-void ilt_build(Ctx& ctx, const Csr& upper, IncompleteCholesky& ic, bool tma_plans = true, bool approximate = false);
+// factor_sweeps > 0: the factor from that many fixed-point sweeps (for the Jacobi-sweep
+// applications); exact_on_failure: a pivot that fails in them sends the factorisation
+// to the exact form and its shift retries
+constexpr int IC_SWEEPS_FP32 = 3, IC_SWEEPS_FP64 = 8;
+void ilt_build(Ctx& ctx, const Csr& upper, IncompleteCholesky& ic, bool tma_plans = true, int factor_sweeps = 0,
+               bool exact_on_failure = false);
+// the exact factor in place of the fixed-point sweeps' one
+void ilt_make_exact(Ctx& ctx, IncompleteCholesky& ic);
 void ilt_apply(Ctx& ctx, const IncompleteCholesky& ic, const double* r, double* z);
 // the exact sweeps' layouts of a factorised ILLT (once; before any stream capture)
 void ilt_exact_layouts(Ctx& ctx, IncompleteCholesky& ic);
@@ -576,6 +582,8 @@ void add_constant(Ctx& ctx, double a, double* y);
 // iltbuild.cu: U pattern copies, U^T, the factorisation's levels (offsets on the
 // host too) and the Jacobi sweeps' layouts, built on the device
 void ilt_structure_gpu(Ctx& ctx, const Csr& upper, IncompleteCholesky& ic, bool levels = true);
+// the rows in dependency-level order, from the structure
+void ilt_levels_gpu(Ctx& ctx, IncompleteCholesky& ic);
 // jacobi.cu: the factor applied by Jacobi sweeps on its two triangles
 void jacobi_fill(Ctx& ctx, IncompleteCholesky& ic);
 void jacobi_apply32(Ctx& ctx, IncompleteCholesky& ic, int sweeps, const float* r, float* z, const double* flags);

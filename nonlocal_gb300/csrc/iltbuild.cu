@@ -172,6 +172,24 @@ void jacobi_slab_gpu(Ctx& ctx, i64 n, TriRows tr, const int32_t* cols, const i64
 
 }  // namespace
 
+// the levels of the exact factorisation's schedule
+void ilt_levels_gpu(Ctx& ctx, IncompleteCholesky& ic) {
+    const i64 n = ic.n;
+    dbuf<int> indeg;
+    dbuf<i64> out;
+    indeg.resize(size_t(n));
+    ic.ic_rows.resize(size_t(n));
+    ic.ic_lev_ptr.resize(size_t(n + 1));
+    out.resize(2);
+    NL_LAUNCH(k_levels, 1, IB_LEVEL_THREADS, 0, ctx.stream, n, ic.lrp.p, ic.rp.p, ic.col.p, indeg.p, ic.ic_rows.p,
+              ic.ic_lev_ptr.p, out.p);
+    i64 ho[2] = {0, 0};
+    out.download(ho, 2, ctx.stream);
+    NL_CUDA(cudaStreamSynchronize(ctx.stream));
+    NL_REQUIRE(ho[1] == n, NLGPU_ERR_STATE, "the factor's dependency graph does not reach every row");
+    ic.ic_levels = ho[0];
+}
+
 // U pattern copies, U^T, the factorisation's rows in level order and the
 // Jacobi layouts, all on the device
 void ilt_structure_gpu(Ctx& ctx, const Csr& upper, IncompleteCholesky& ic, bool levels) {
@@ -199,25 +217,12 @@ void ilt_structure_gpu(Ctx& ctx, const Csr& upper, IncompleteCholesky& ic, bool 
     NL_LAUNCH(k_transpose_place, grid_for(n, IB_THREADS), IB_THREADS, 0, ctx.stream, n, upper.rowptr.p, upper.col.p,
               ic.lrp.p, cursor.p, ic.lcol.p, ic.l_to_u.p);
     NL_LAUNCH(k_sort_rows, grid_for(n, IB_THREADS), IB_THREADS, 0, ctx.stream, n, ic.lrp.p, ic.lcol.p, ic.l_to_u.p);
-    // levels of the exact factorisation's schedule
-    i64 ho[2] = {0, n};
     int hbad = 0;
-    dbuf<int> indeg;
-    dbuf<i64> out;
-    if (levels) {
-        indeg.resize(size_t(n));
-        ic.ic_rows.resize(size_t(n));
-        ic.ic_lev_ptr.resize(size_t(n + 1));
-        out.resize(2);
-        NL_LAUNCH(k_levels, 1, IB_LEVEL_THREADS, 0, ctx.stream, n, ic.lrp.p, upper.rowptr.p, upper.col.p, indeg.p,
-                  ic.ic_rows.p, ic.ic_lev_ptr.p, out.p);
-        out.download(ho, 2, ctx.stream);
-    }
     NL_CUDA(cudaMemcpyAsync(&hbad, bad.p, sizeof hbad, cudaMemcpyDeviceToHost, ctx.stream));
     NL_CUDA(cudaStreamSynchronize(ctx.stream));
     NL_REQUIRE(!hbad, NLGPU_ERR_ARG, "every row of the preconditioner matrix needs its diagonal first");
-    NL_REQUIRE(ho[1] == n, NLGPU_ERR_STATE, "the factor's dependency graph does not reach every row");
-    ic.ic_levels = levels ? ho[0] : 0;
+    ic.ic_levels = 0;
+    if (levels) ilt_levels_gpu(ctx, ic);
     // Jacobi layouts of U^T (values u[l_to_u]) and U
     jacobi_slab_gpu(ctx, n, TriRows{ic.lrp.p, true}, ic.lcol.p, ic.l_to_u.p, ic.jlo, bad.p);
     jacobi_slab_gpu(ctx, n, TriRows{ic.rp.p, false}, ic.col.p, nullptr, ic.jup, bad.p);

@@ -237,11 +237,14 @@ __global__ void k_scaled(i64 n, const i64* __restrict__ rp, const int32_t* __res
 // row at once, reading the other rows' values of the previous sweep (uin) and
 // writing its own (u), with no order and no waits.  Started from the scaled
 // matrix's rows divided by the root of their diagonal, a few sweeps give a
-// factor that serves the FP32 Jacobi-sweep application as well as the exact
-// one, without the exact form's dependency chain (2 401 levels on the
-// 300x300 serendipity mesh, at a few microseconds each).
+// factor that serves the Jacobi-sweep applications as well as the exact one,
+// without the exact form's dependency chain (2 401 levels on the 300x300
+// serendipity mesh, at a few microseconds each): IC_SWEEPS_FP32 of them for the
+// FP32 application, IC_SWEEPS_FP64 for the FP64 CG, whose iteration counts are then
+// those of the exact factor (48 / 49 / 36 on 8-node heat, 8-node local and
+// elasticity meshes; 3 sweeps 51 / 53 / 40).  Exact factor and levels against 8
+// sweeps: 2.5 -> 0.2 ms (71x53 8-node), 3.9 -> 0.2 (33x26 8-node elasticity).
 constexpr int IC_WARPS = 8;
-constexpr int IC_SWEEPS = 3;
 constexpr int IC_MAXS = 16;
 constexpr unsigned long long IC_WAIT_LIMIT_NS = 2000000000ull;
 
@@ -303,10 +306,14 @@ __global__ void __launch_bounds__(IC_WARPS * 32) k_ic0_rows(i64 n, const int32_t
     __shared__ int32_t rowcol[IC_WARPS][32];
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
-    for (;;) {
-        int t = 0;
-        if (lane == 0) t = atomicAdd(ticket, 1);
-        t = __shfl_sync(full, t, 0);
+    // a sweep's rows depend on nothing of this launch: warps take them in turn
+    i64 t = i64(blockIdx.x) * IC_WARPS + wb;
+    for (;; t += i64(gridDim.x) * IC_WARPS) {
+        if constexpr (!SWEEP) {
+            int k = 0;
+            if (lane == 0) k = atomicAdd(ticket, 1);
+            t = __shfl_sync(full, k, 0);
+        }
         if (t >= n) break;
         const int32_t i = SWEEP ? int32_t(t) : order[t];
         const i64 b = rp[i], e = rp[i + 1];
@@ -639,13 +646,71 @@ void ilt_exact_layouts(Ctx& ctx, IncompleteCholesky& ic) {
     timer.mark("value fills");
 }
 
-void ilt_build(Ctx& ctx, const Csr& upper, IncompleteCholesky& ic, bool tma_plans, bool approximate) {
+namespace {
+
+// IC(0) of the scaled matrix with the shift retries, from `first_shift`: exact, or by
+// `sweeps` fixed-point sweeps.  one_attempt: no retry.  Sets ic.ok, attempts and shift.
+void ilt_factor(Ctx& ctx, IncompleteCholesky& ic, int sweeps, double first_shift, bool one_attempt) {
+    const i64 n = ic.n;
+    dbuf<int> failed, sync;   // failed: [pivot, timeout]; sync: [ticket, done flags per row]
+    failed.resize(2);
+    if (sweeps == 0) sync.resize(size_t(n + 1));
+    // resident warps well above the widest level, so the rows of the next
+    // levels are taken while the current one finishes
+    const unsigned ic_grid = unsigned(std::max<i64>(1, std::min<i64>((n + IC_WARPS - 1) / IC_WARPS, 152 * 2)));
+    const unsigned sweep_grid = unsigned(std::max<i64>(1, std::min<i64>((n + IC_WARPS - 1) / IC_WARPS, 152 * 16)));
+    const double initial_shift = 1e-3;
+    double shift = first_shift;
+    ic.ok = false;
+    dbuf<double> u_prev;
+    if (sweeps > 0) u_prev.resize(size_t(ic.nnz));
+    for (ic.attempts = 1; ic.attempts <= 10; ++ic.attempts) {
+        failed.zero(ctx.stream);
+        if (sweeps > 0) {
+            // the sweeps alternate between the two buffers and end in ic.u
+            double* buf[2] = {sweeps % 2 ? u_prev.p : ic.u.p, sweeps % 2 ? ic.u.p : u_prev.p};
+            NL_LAUNCH(k_ic0_start, grid_for(n, 256), 256, 0, ctx.stream, n, ic.rp.p, ic.a_scaled.p, shift, buf[0],
+                      failed.p);
+            for (int sw = 0; sw < sweeps; ++sw)
+                NL_LAUNCH(k_ic0_rows<true>, sweep_grid, IC_WARPS * 32, 0, ctx.stream, n,
+                          static_cast<const int32_t*>(nullptr), ic.rp.p, ic.col.p, ic.a_scaled.p, shift, ic.lrp.p,
+                          ic.lcol.p, ic.l_to_u.p, buf[sw & 1], buf[(sw + 1) & 1], static_cast<int*>(nullptr),
+                          static_cast<int*>(nullptr), failed.p, failed.p + 1);
+        } else {
+            sync.zero(ctx.stream);
+            NL_LAUNCH(k_ic0_rows<false>, ic_grid, IC_WARPS * 32, 0, ctx.stream, n, ic.ic_rows.p, ic.rp.p, ic.col.p,
+                      ic.a_scaled.p, shift, ic.lrp.p, ic.lcol.p, ic.l_to_u.p, ic.u.p, ic.u.p, sync.p, sync.p + 1,
+                      failed.p, failed.p + 1);
+        }
+        int hf[2] = {0, 0};
+        NL_CUDA(cudaMemcpyAsync(hf, failed.p, sizeof hf, cudaMemcpyDeviceToHost, ctx.stream));
+        NL_CUDA(cudaStreamSynchronize(ctx.stream));
+        NL_REQUIRE(!hf[1], NLGPU_ERR_TIMEOUT, "the factorisation's wait for a dependency row timed out");
+        if (!hf[0]) { ic.ok = true; break; }
+        if (one_attempt) break;
+        shift = std::max(initial_shift, 2.0 * shift);
+    }
+    ic.shift = shift;
+}
+
+}  // namespace
+
+void ilt_make_exact(Ctx& ctx, IncompleteCholesky& ic) {
+    if (!ic.approximate || !ic.ok) return;
+    ilt_levels_gpu(ctx, ic);
+    ilt_factor(ctx, ic, 0, ic.first_shift, false);
+    ic.approximate = false;
+    ic.exact_ready = ic.j64_ready = false;
+    if (ic.ok) jacobi_fill(ctx, ic);
+}
+
+void ilt_build(Ctx& ctx, const Csr& upper, IncompleteCholesky& ic, bool tma_plans, int factor_sweeps, bool exact_on_failure) {
     const i64 n = upper.rows, nnz = upper.nnz;
     ic.n = n; ic.nnz = nnz;
-    ic.approximate = approximate;
+    ic.approximate = factor_sweeps > 0;
     PhaseTimer timer(ctx.stream, "ilt_build");
     // U^T, the factorisation's levels (exact form) and the Jacobi layouts on the device
-    ilt_structure_gpu(ctx, upper, ic, !approximate);
+    ilt_structure_gpu(ctx, upper, ic, !ic.approximate);
     timer.mark("structure");
     ctx.sweep_error.resize(1);
     ctx.sweep_error.zero(ctx.stream);
@@ -664,11 +729,7 @@ void ilt_build(Ctx& ctx, const Csr& upper, IncompleteCholesky& ic, bool tma_plan
     NL_LAUNCH(k_to_float, grid_for(n, 256), 256, 0, ctx.stream, n, ic.scale.p, ic.scale32.p);
     ic.a_scaled.resize(size_t(nnz)); ic.u.resize(size_t(nnz));
     dbuf<unsigned long long> mind;
-    dbuf<int> failed, sync;   // failed: [pivot, timeout]; sync: [ticket, done flags per row]
-    mind.resize(1); failed.resize(2); sync.resize(size_t(n + 1));
-    // resident warps well above the widest level, so the rows of the next
-    // levels are taken while the current one finishes
-    const unsigned ic_grid = unsigned(std::max<i64>(1, std::min<i64>((n + IC_WARPS - 1) / IC_WARPS, 152 * 2)));
+    mind.resize(1);
     const unsigned long long init = ~0ull;
     NL_CUDA(cudaMemcpyAsync(mind.p, &init, sizeof init, cudaMemcpyHostToDevice, ctx.stream));
     NL_LAUNCH(k_scaled, grid_for(n, 256), 256, 0, ctx.stream, n, upper.rowptr.p, upper.col.p, upper.val.p, ic.scale.p,
@@ -679,40 +740,13 @@ void ilt_build(Ctx& ctx, const Csr& upper, IncompleteCholesky& ic, bool tma_plan
     const unsigned long long raw = (mbits & 0x8000000000000000ull) ? (mbits & 0x7fffffffffffffffull) : ~mbits;
     double mindiag;
     std::memcpy(&mindiag, &raw, sizeof mindiag);
-    const double initial_shift = 1e-3;
-    double shift = mindiag <= 0.0 ? initial_shift - mindiag : 0.0;
-    ic.ok = false;
-    dbuf<double> u_prev;
-    if (approximate) u_prev.resize(size_t(nnz));
-    for (ic.attempts = 1; ic.attempts <= 10; ++ic.attempts) {
-        failed.zero(ctx.stream);
-        if (approximate) {
-            // the sweeps alternate between the two buffers and end in ic.u
-            double* buf[2] = {IC_SWEEPS % 2 ? u_prev.p : ic.u.p, IC_SWEEPS % 2 ? ic.u.p : u_prev.p};
-            NL_LAUNCH(k_ic0_start, grid_for(n, 256), 256, 0, ctx.stream, n, ic.rp.p, ic.a_scaled.p, shift, buf[0],
-                      failed.p);
-            const unsigned sweep_grid = unsigned(std::max<i64>(1, std::min<i64>((n + IC_WARPS - 1) / IC_WARPS, 152 * 16)));
-            for (int sw = 0; sw < IC_SWEEPS; ++sw) {
-                sync.zero(ctx.stream);   // the sweep's row ticket
-                NL_LAUNCH(k_ic0_rows<true>, sweep_grid, IC_WARPS * 32, 0, ctx.stream, n,
-                          static_cast<const int32_t*>(nullptr), ic.rp.p, ic.col.p, ic.a_scaled.p, shift, ic.lrp.p,
-                          ic.lcol.p, ic.l_to_u.p, buf[sw & 1], buf[(sw + 1) & 1], sync.p, sync.p + 1, failed.p,
-                          failed.p + 1);
-            }
-        } else {
-            sync.zero(ctx.stream);
-            NL_LAUNCH(k_ic0_rows<false>, ic_grid, IC_WARPS * 32, 0, ctx.stream, n, ic.ic_rows.p, ic.rp.p, ic.col.p,
-                      ic.a_scaled.p, shift, ic.lrp.p, ic.lcol.p, ic.l_to_u.p, ic.u.p, ic.u.p, sync.p, sync.p + 1,
-                      failed.p, failed.p + 1);
-        }
-        int hf[2] = {0, 0};
-        NL_CUDA(cudaMemcpyAsync(hf, failed.p, sizeof hf, cudaMemcpyDeviceToHost, ctx.stream));
-        NL_CUDA(cudaStreamSynchronize(ctx.stream));
-        NL_REQUIRE(!hf[1], NLGPU_ERR_TIMEOUT, "the factorisation's wait for a dependency row timed out");
-        if (!hf[0]) { ic.ok = true; break; }
-        shift = std::max(initial_shift, 2.0 * shift);
+    ic.first_shift = mindiag <= 0.0 ? 1e-3 - mindiag : 0.0;
+    ilt_factor(ctx, ic, factor_sweeps, ic.first_shift, exact_on_failure);
+    if (!ic.ok && ic.approximate && exact_on_failure) {
+        ilt_levels_gpu(ctx, ic);
+        ilt_factor(ctx, ic, 0, ic.first_shift, false);
+        ic.approximate = false;
     }
-    ic.shift = shift;
     timer.mark("scaling, factorisation");
     if (!ic.ok) return;
     jacobi_fill(ctx, ic);
@@ -732,7 +766,14 @@ CgResult cg_solve(Ctx& ctx, const Csr& A, const IncompleteCholesky* M, const dou
         CgResult r;
         if (pcg_solve(ctx, A, M, b, x, tolerance, max_iterations, x_is_initial_guess, on_chunk, r)) return r;
     }
-    // exact triangular sweeps: asked for, or a factor whose Jacobi sweeps contract too slowly
+    // exact triangular sweeps and the exact factor: asked for, or a factor whose Jacobi
+    // sweeps contract too slowly
+    ilt_make_exact(ctx, const_cast<IncompleteCholesky&>(*M));
+    if (!M->ok) {
+        CgResult r;   // the identity when the exact factorisation breaks down
+        pcg_solve(ctx, A, nullptr, b, x, tolerance, max_iterations, x_is_initial_guess, on_chunk, r);
+        return r;
+    }
     ilt_exact_layouts(ctx, const_cast<IncompleteCholesky&>(*M));
     const i64 n = A.rows;
     CgWork& w = ctx.cg;

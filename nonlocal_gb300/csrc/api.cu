@@ -875,30 +875,9 @@ int nlgpu_cg_solve(nlgpu_ctx* ctx, int64_t n, const int64_t* a_rowptr, const int
         Ctx& c = *ctx;
         const auto t0 = std::chrono::steady_clock::now();
         // full padded rows from the upper storage (both triangles)
-        std::vector<std::vector<std::pair<int32_t, double>>> rows(static_cast<size_t>(n));
-        for (int64_t r = 0; r < n; ++r)
-            for (int64_t k = a_rowptr[r]; k < a_rowptr[r + 1]; ++k) {
-                const int64_t cc = a_col[k];
-                NL_REQUIRE(cc >= r && cc < n, NLGPU_ERR_ARG, "A must be the upper triangle with columns in range");
-                rows[size_t(r)].push_back({int32_t(cc), a_val[k]});
-                if (cc != r) rows[size_t(cc)].push_back({int32_t(r), a_val[k]});
-            }
-        std::vector<i64> rp(size_t(n + 1), 0);
-        std::vector<int32_t> col;
-        std::vector<double> val;
-        for (int64_t r = 0; r < n; ++r) {
-            auto& row = rows[size_t(r)];
-            std::sort(row.begin(), row.end(), [](const auto& u, const auto& v) { return u.first < v.first; });
-            for (const auto& [cc, v] : row) { col.push_back(cc); val.push_back(v); }
-            while (col.size() % 4) { col.push_back(int32_t(r)); val.push_back(0.0); }
-            rp[size_t(r) + 1] = i64(col.size());
-        }
-        rows.clear();
+        NL_REQUIRE(n < (int64_t(1) << 31), NLGPU_ERR_UNSUPPORTED, "more than 2^31 rows");
         Csr A;
-        A.rows = n; A.nnz = i64(col.size());
-        A.rowptr.upload(rp.data(), rp.size(), c.stream);
-        A.col.upload(col.data(), col.size(), c.stream);
-        A.val.upload(val.data(), val.size(), c.stream);
+        full_rows_from_caller(c, n, a_rowptr, a_col, a_val, A);
         dbuf<double> db, dx;
         db.upload(b, size_t(n), c.stream);
         dx.resize(size_t(n));

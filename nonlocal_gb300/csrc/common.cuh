@@ -517,6 +517,8 @@ void set_dirichlet_diagonal(Ctx& ctx, Csr& m, double value);
 void combine_nonstationary(Ctx& ctx, double dt);
 // f = dt (flux + source [+ radiation]) + C T_prev, then the first kind
 void nonstationary_rhs(Ctx& ctx, double dirichlet_value, bool per_node_values, const double* radiation = nullptr);
+// callercsr.cu: the solver's padded full rows of a caller's upper-stored matrix
+void full_rows_from_caller(Ctx& ctx, i64 n, const int64_t* rowptr, const int64_t* col, const double* val, Csr& A);
 // solver.cu
 void spmv_full(Ctx& ctx, const Csr& A, const double* x, double* y);
 // tma_plans: also build the TMA-fed shared-memory sweep plans of the exact

@@ -68,3 +68,35 @@ def test_slowly_contracting_factor_takes_the_exact_sweeps(ctx):
     r[:-1] += x[1:]
     r[1:] += x[:-1]
     assert np.linalg.norm(r) <= 1.01e-10 * np.linalg.norm(b)
+
+
+def test_caller_rows_in_any_order(ctx):
+    """The caller's upper rows unsorted, with entries given in two parts, rows without a diagonal, the arrays starting
+    at an offset: the solve is that of the same matrix sorted and summed; a column below the diagonal or out of range
+    is refused."""
+    import scipy.sparse as sp
+    from nonlocal_gb300 import _lib
+    from nonlocal_gb300 import thermal as T
+    rng = np.random.default_rng(7)
+    n = 301
+    A, U = banded(n, 45, 3, 1.25)
+    U = U.tocoo()
+    r, c, v = U.row, U.col, U.data
+    split = rng.random(r.size) < 0.2                       # a fifth of the entries in two parts
+    r, c, v = np.concatenate([r, r[split]]), np.concatenate([c, c[split]]), np.concatenate([v, 0.25 * v[split]])
+    v[:split.size][split] *= 0.75
+    order = rng.permutation(r.size)
+    order = order[np.argsort(r[order], kind="stable")]     # by row, any order inside
+    off = 5
+    rp = off + np.concatenate([[0], np.cumsum(np.bincount(r, minlength=n))]).astype(np.int64)
+    col = np.concatenate([np.full(off, -9), c[order]]).astype(np.int64)
+    val = np.concatenate([np.full(off, np.nan), v[order]])
+    b = rng.standard_normal(n)
+    x, rep = T.conjugate_gradient(ctx, (rp, col, val), b, tolerance=1e-12)
+    assert rep.nnz_solver == sum((k + 3) // 4 * 4 for k in np.bincount(r, minlength=n) + np.bincount(c[r != c], minlength=n))
+    assert np.linalg.norm(b - A @ x) <= 1.01e-12 * np.linalg.norm(b)
+    for wrong in (0, n):
+        bad = col.copy()
+        bad[rp[n - 1]] = wrong
+        with pytest.raises(_lib.NlgpuError):
+            T.conjugate_gradient(ctx, (rp, bad, val), b)

@@ -286,6 +286,9 @@ struct IncompleteCholesky {
     JacobiSlab jlo, jup;         // U^T and U for Jacobi sweeps, rows scaled by 1 / u_ii
     dbuf<float> jc, jdinv;       // s_i / u_ii and 1 / u_ii
     dbuf<float> jt0, jt1, jy;    // Jacobi iterates and the scaled forward result
+    dbuf<unsigned long long> jsteps;   // one-launch application: tagged sweep values, each CTA's last number
+    dbuf<unsigned> jtags;
+    i64 jsplit_n = 0, jsplit_rows = 0;
     bool ok = false;
     dbuf<double> jc64, jdinv64;  // the FP64 Jacobi sweeps of the CG kernel (pcg.cu), filled at its first use
     bool j64_ready = false;
@@ -660,6 +663,35 @@ void stationary_1d(Ctx& ctx, i64 elements, int order, double length, double radi
                    double conductivity, double t_left, double q_right, bool sin_source, double* temperature);
 
 // device helpers --------------------------------------------------------
+// This lane's part of one row of y = A x: entries k, k + g, ... below `end`, so
+// that the g lanes of a row read neighbouring columns and values and gather runs of
+// x.  Two FMA chains, four entries in flight.
+__device__ __forceinline__ double row_part(const int32_t* __restrict__ col, const double* __restrict__ val,
+                                           const double* x, i64 k, i64 end, int g) {
+    double s = 0.0, s2 = 0.0;
+    for (; k + 3 * g < end; k += 4 * g) {
+        const int32_t j0 = __ldg(col + k), j1 = __ldg(col + k + g), j2 = __ldg(col + k + 2 * g), j3 = __ldg(col + k + 3 * g);
+        const double v0 = __ldg(val + k), v1 = __ldg(val + k + g), v2 = __ldg(val + k + 2 * g), v3 = __ldg(val + k + 3 * g);
+        s = fma(v0, x[j0], s);
+        s2 = fma(v1, x[j1], s2);
+        s = fma(v2, x[j2], s);
+        s2 = fma(v3, x[j3], s2);
+    }
+    for (; k < end; k += g) s = fma(__ldg(val + k), x[__ldg(col + k)], s);
+    return s + s2;
+}
+
+// log2 of the lanes per row of an FP64 product with rows of `mean` entries: about
+// twelve entries a lane (each reduction step costs as much of the FP64 pipe as an
+// entry per lane), at most 16 lanes unless the rows are few (`threads`: what the
+// launch can run at once)
+inline int spmv_lanes(double mean, double rows, double threads) {
+    int lg = 1;
+    while (lg < 4 && double(1 << lg) * 12.0 < mean) ++lg;
+    while (lg < 5 && rows * double(2 << lg) <= threads && double(2 << lg) <= mean) ++lg;
+    return lg;
+}
+
 __device__ __forceinline__ double warp_sum(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;

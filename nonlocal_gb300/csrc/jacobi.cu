@@ -18,10 +18,14 @@
 // solve.  The truncated operator is S F^T F S with F lower triangular and
 // nonsingular: symmetric positive definite, so it is a valid CG
 // preconditioner; FP32 rounding makes it slightly non-symmetric, which the
-// flexible CG of mixed.cu absorbs.  Every sweep is one fully parallel pass
-// over one triangle (thread per row, sliced ELL), so a preconditioner
-// application costs 2 k short bandwidth-bound launches instead of two chains
-// of per-level barriers.
+// flexible CG of mixed.cu absorbs.
+//
+// Two forms.  k_jacobi_all runs the whole application as one cooperative launch:
+// a CTA owns consecutive rows, and a sweep's values are stored as 64-bit words of
+// the float and the step's number, which a reader polls until the number is
+// there: no barrier, no launch between sweeps, and a row waits only for the rows
+// of its band.  k_jacobi32 is one sweep per launch (thread per row), for systems
+// whose sweeps are bound by bandwidth (JA_MAX_ROWS).
 #include "common.cuh"
 
 #include <algorithm>
@@ -89,6 +93,147 @@ __global__ void __launch_bounds__(JB_THREADS) k_jacobi32(i64 n, const i64* __res
     out[r] = v;
 }
 
+// The application in one launch (see the top).  Bound by the 2 k dependent steps,
+// each a store and a load through L2 (a message between SMs of different dies
+// takes about 0.45 us) and the row's sum.  Microseconds an application of twelve
+// sweeps, the kernels of one launch per sweep (without the gaps between them) ->
+// this: 40 401 rows of 4 (200x200 bilinear) 21 -> 16; 163 000 rows of 4 (a dozen
+// systems) 24 -> 23; 56 454 rows of 4 28 -> 18; 271 201 rows of 10 (300x300 8-node)
+// 48 -> 50.
+constexpr int JA_THREADS = 1024;
+constexpr int JA_MIN_ROWS = 64;
+constexpr i64 JA_MAX_ROWS = 400000;
+constexpr int JA_MAX_SWEEPS = 32;
+constexpr int JA_BATCH = 4;       // gathers in flight per lane
+constexpr unsigned long long JA_WAIT_LIMIT_NS = 2000000000ull;
+
+__device__ __forceinline__ unsigned long long ja_globaltimer() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+__device__ __forceinline__ void ja_put(unsigned long long* p, float v, unsigned tag) {
+    const unsigned long long w = (static_cast<unsigned long long>(tag) << 32) | __float_as_uint(v);
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+}
+
+__device__ __forceinline__ unsigned long long ja_get(const unsigned long long* p) {
+    unsigned long long w;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
+    return w;
+}
+
+// a wait that runs out marks the CTA, which then waits no more; the host sees *error
+__device__ __noinline__ unsigned long long ja_wait_long(const unsigned long long* p, unsigned tag, volatile int* gave_up,
+                                                        int* error) {
+    const unsigned long long t0 = ja_globaltimer();
+    unsigned long long w = ja_get(p);
+    while (unsigned(w >> 32) != tag && !*gave_up) {
+        if (ja_globaltimer() - t0 > JA_WAIT_LIMIT_NS) {
+            atomicExch(error, 1);
+            *gave_up = 1;
+        }
+        w = ja_get(p);
+    }
+    return w;
+}
+
+struct JacobiAll {
+    i64 n;
+    int rows;                 // per CTA, a multiple of 32
+    int sweeps, lg;           // sweeps per triangle, log2 of the lanes per row
+    const i64 *slo, *sup;     // slices, columns and values of both triangles
+    const int32_t *clo, *cup;
+    const float *vlo, *vup;
+    const float *r, *c, *dinv, *scale;
+    float* z;
+    unsigned long long* steps;   // [sweeps + 1][n]
+    unsigned* tags;              // [gridDim.x] last number each CTA used
+    int* error;
+};
+
+__global__ void __launch_bounds__(JA_THREADS) k_jacobi_all(JacobiAll a, const double* __restrict__ flags) {
+    extern __shared__ float ja_base[];
+    __shared__ int gave_up;
+    if (flags && flags[S_DONE] != 0.0) return;
+    const i64 r0 = i64(blockIdx.x) * a.rows;
+    const int rows = int(min(a.n, r0 + a.rows) - r0);
+    const int lane = threadIdx.x & 31, g = 1 << a.lg, sub = lane & (g - 1), per = 32 >> a.lg;
+    unsigned tag = a.tags[blockIdx.x] + 1;
+    if (threadIdx.x == 0) gave_up = 0;
+    for (int i = threadIdx.x; i < rows; i += JA_THREADS) {
+        const float y = a.c[r0 + i] * a.r[r0 + i];
+        ja_base[i] = y;
+        ja_put(a.steps + r0 + i, y, tag);
+    }
+    __syncthreads();
+    // the rows a warp takes are the same in every sweep, and a row's own values pass
+    // between them in its lanes' warp: no barrier
+    for (int s = 1; s <= 2 * a.sweeps; ++s) {
+        const bool upper = s > a.sweeps;
+        const int t = upper ? s - a.sweeps : s;           // sweep of this triangle
+        const bool last = t == a.sweeps;
+        const i64* slice = upper ? a.sup : a.slo;
+        const int32_t* cols = upper ? a.cup : a.clo;
+        const float* vals = upper ? a.vup : a.vlo;
+        // backward sweep t writes step t again: a row has read the forward results of every
+        // row above it by then, and those are the rows that read its forward values
+        const unsigned long long* in = a.steps + size_t(upper && t == 1 ? a.sweeps : t - 1) * size_t(a.n);
+        unsigned long long* out = a.steps + size_t(t) * size_t(a.n);
+        for (int i0 = int(threadIdx.x >> 5) * per; i0 < rows; i0 += (JA_THREADS / 32) * per) {
+            const int i = i0 + (lane >> a.lg);
+            const i64 row = r0 + i;
+            float acc = 0.0f;
+            if (i < rows) {
+                const i64 b = __ldg(slice + (row >> 5));
+                const int w = int((__ldg(slice + (row >> 5) + 1) - b) >> 5);
+                const int32_t* col = cols + b + (row & 31);
+                const float* val = vals + b + (row & 31);
+                for (int k = sub; k < w; k += JA_BATCH * g) {
+                    unsigned long long y[JA_BATCH];
+                    int32_t j[JA_BATCH];
+                    float v[JA_BATCH];
+#pragma unroll
+                    for (int u = 0; u < JA_BATCH; ++u)
+                        if (k + u * g < w) {
+                            j[u] = __ldg(col + 32 * (k + u * g));
+                            v[u] = __ldg(val + 32 * (k + u * g));
+                            y[u] = ja_get(in + j[u]);
+                        }
+#pragma unroll
+                    for (int u = 0; u < JA_BATCH; ++u)
+                        if (k + u * g < w) {
+                            for (int tries = 0; unsigned(y[u] >> 32) != tag; ++tries) {
+                                if (tries == 4096) {
+                                    y[u] = ja_wait_long(in + j[u], tag, &gave_up, a.error);
+                                    break;
+                                }
+                                y[u] = ja_get(in + j[u]);
+                            }
+                            acc += v[u] * __uint_as_float(unsigned(y[u]));
+                        }
+                }
+            }
+            for (int o = g >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (i < rows && sub == 0) {
+                float v = ja_base[i] - acc;
+                if (!last) {
+                    ja_put(out + row, v, tag + 1);
+                } else if (!upper) {
+                    v *= a.dinv[row];
+                    ja_base[i] = v;   // the backward sweeps' base, read by this lane only
+                    ja_put(out + row, v, tag + 1);
+                } else {
+                    a.z[row] = v * a.scale[row];
+                }
+            }
+        }
+        ++tag;
+    }
+    if (threadIdx.x == 0) a.tags[blockIdx.x] = tag;
+}
+
 void sweep(Ctx& ctx, i64 n, const JacobiSlab& s, const float* base, const float* bs, const float* y, const float* ys,
            const float* o, float* out, const double* flags) {
     NL_LAUNCH(k_jacobi32, unsigned((n + JB_THREADS - 1) / JB_THREADS), JB_THREADS, 0, ctx.stream, n, s.slice.p,
@@ -108,6 +253,47 @@ void jacobi_fill(Ctx& ctx, IncompleteCholesky& ic) {
 void jacobi_apply32(Ctx& ctx, IncompleteCholesky& ic, int sweeps, const float* r, float* z, const double* flags) {
     NL_REQUIRE(sweeps >= 1, NLGPU_ERR_ARG, "at least one Jacobi sweep per triangle");
     const i64 n = ic.n;
+    // one launch for the whole application unless bandwidth bounds the sweeps, or a
+    // row's neighbours are too many or too far apart to be worth polling
+    if (n <= JA_MAX_ROWS && sweeps <= JA_MAX_SWEEPS) {
+        int dev = 0, sms = 0;
+        NL_CUDA(cudaGetDevice(&dev));
+        NL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        const i64 rows = std::max<i64>(JA_MIN_ROWS, ((n + sms - 1) / sms + 31) / 32 * 32);
+        const unsigned grid = unsigned((n + rows - 1) / rows);
+        const size_t words = size_t(sweeps + 1) * size_t(n);
+        // the CTAs' numbers go on from application to application; another split starts
+        // afresh (outside any capture: a solve's first application is eager)
+        if (ic.jsteps.n < words || ic.jsplit_n != n || ic.jsplit_rows != rows) {
+            ic.jsteps.reserve(words);
+            ic.jtags.reserve(size_t(sms));
+            ic.jsteps.zero(ctx.stream);
+            ic.jtags.zero(ctx.stream);
+            ic.jsplit_n = n;
+            ic.jsplit_rows = rows;
+        }
+        ctx.sweep_error.reserve(1);
+        JacobiAll a{};
+        a.n = n; a.rows = int(rows); a.sweeps = sweeps;
+        while (a.lg < 2 && (rows << (a.lg + 1)) <= JA_THREADS && (2 << a.lg) <= ic.jlo.max_width) ++a.lg;
+        a.slo = ic.jlo.slice.p; a.clo = ic.jlo.col.p; a.vlo = ic.jlo.val.p;
+        a.sup = ic.jup.slice.p; a.cup = ic.jup.col.p; a.vup = ic.jup.val.p;
+        a.r = r; a.c = ic.jc.p; a.dinv = ic.jdinv.p; a.scale = ic.scale32.p; a.z = z;
+        a.steps = ic.jsteps.p; a.tags = ic.jtags.p; a.error = ctx.sweep_error.p;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = dim3(JA_THREADS);
+        cfg.dynamicSmemBytes = size_t(rows) * sizeof(float);
+        cfg.stream = ctx.stream;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        NL_CUDA(cudaLaunchKernelEx(&cfg, k_jacobi_all, a, flags));
+        count_launch();
+        return;
+    }
     float* t[2] = {ic.jt0.p, ic.jt1.p};
     // forward: y_t+1 = c r - L y_t from y_0 = c r; the last sweep scales by 1 / u_ii
     const float* prev = r;

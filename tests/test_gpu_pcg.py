@@ -100,3 +100,22 @@ def test_caller_rows_in_any_order(ctx):
         bad[rp[n - 1]] = wrong
         with pytest.raises(_lib.NlgpuError):
             T.conjugate_gradient(ctx, (rp, bad, val), b)
+
+
+@pytest.mark.parametrize("n, band", [(1, 1), (31, 3), (64, 2), (65, 70), (152 * 64, 5), (152 * 64 + 1, 9), (152 * 96 + 40, 33),
+                                     (400001, 3)])
+def test_jacobi_application_sizes(ctx, n, band):
+    """The FP32 ILLT application at the edges of its row split (and past the size of the one-launch form): on a
+    strongly dominant matrix a sweep contracts by at least 2.5, so 24 sweeps per triangle are the exact application to FP32
+    rounding, and 32 and 33 sweeps (one launch, one per sweep) agree."""
+    from nonlocal_gb300 import thermal as T
+    _, U = banded(n, band, 11, 4.0)
+    U.sort_indices()
+    pre = T.EigenILLTPreconditioner(ctx)
+    assert pre.compute((U.indptr.astype(np.int64), U.indices.astype(np.int64), U.data)).computation_info() == pre.SUCCESS
+    x = np.random.default_rng(2).standard_normal(n)
+    exact = pre.solve(x)
+    # an entry's sum has at most `band` terms of FP32 products, twice; the sweeps' remainder is 2.5^-24
+    tol = (2 * (band + 4) * np.finfo(np.float32).eps + 2.5 ** -24) * np.abs(exact).max()
+    for sweeps in (24, 32, 33):
+        assert np.abs(pre.solve_f32(x, sweeps) - exact).max() <= tol, sweeps

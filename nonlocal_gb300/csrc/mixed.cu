@@ -36,7 +36,7 @@ namespace nlgpu {
 namespace {
 
 constexpr int MX_THREADS = 256;
-constexpr int MX_ITERS = 16;
+constexpr int MX_ITERS = 8;   // a reliable update comes every six or seven iterations: what a chunk holds beyond one is skipped launches
 constexpr int MX_M = 4;   // directions kept for the A-orthogonalisation (flexible CG truncation)
 constexpr i64 MX_UPDATE_MAX = 64;   // iterations between reliable updates at most
 // partial slots: P_RR as in the FP64 solver (the exact sweeps' early exit reads
@@ -71,27 +71,26 @@ __device__ __forceinline__ double mx_partials(const double* part, double* sh) {
     return s;
 }
 
-// N block sums in one pass (sh: at least 33 N doubles); every thread gets them
+// N block sums in one pass (sh: at least MX_THREADS N + N doubles); every thread
+// gets them.  The threads' values meet in shared memory and warp s adds slot s,
+// eight values a lane: a warp-wide FP64 add holds GB300's FP64 pipe for 16 cycles,
+// and shuffles in every warp are five of them per slot and warp.
 template<int N>
 __device__ __forceinline__ void mx_block_sums(double (&v)[N], double* sh) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = int(blockDim.x >> 5);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int s = 0; s < N; ++s) v[s] = warp_sum(v[s]);
-    if (lane == 0) {
-#pragma unroll
-        for (int s = 0; s < N; ++s) sh[s * 32 + warp] = v[s];
-    }
+    for (int s = 0; s < N; ++s) sh[s * MX_THREADS + threadIdx.x] = v[s];
     __syncthreads();
-    if (warp == 0) {
+    if (warp < N) {
+        double t = 0.0;
 #pragma unroll
-        for (int s = 0; s < N; ++s) {
-            const double t = warp_sum(lane < nw ? sh[s * 32 + lane] : 0.0);
-            if (lane == 0) sh[32 * N + s] = t;
-        }
+        for (int k = 0; k < MX_THREADS; k += 32) t += sh[warp * MX_THREADS + k + lane];
+        t = warp_sum(t);
+        if (lane == 0) sh[MX_THREADS * N + warp] = t;
     }
     __syncthreads();
 #pragma unroll
-    for (int s = 0; s < N; ++s) v[s] = sh[32 * N + s];
+    for (int s = 0; s < N; ++s) v[s] = sh[MX_THREADS * N + s];
     __syncthreads();
 }
 
@@ -141,7 +140,7 @@ __global__ void __launch_bounds__(MX_THREADS) k_spmv32(i64 n, const i64* __restr
                                                        const float* __restrict__ rowsum, const float* __restrict__ x,
                                                        float* __restrict__ y, double* __restrict__ dot_partial,
                                                        double* __restrict__ flags, i64 ring, unsigned* ticket) {
-    __shared__ double sh[40];
+    __shared__ double sh[MX_THREADS + 1];
     if (flags && flags[S_DONE] != 0.0) return;
     i64 slot = 0;
     if (ring) {   // direction slot of the current iteration in the rings of x and y
@@ -256,7 +255,7 @@ __global__ void __launch_bounds__(UP_THREADS, 1) k_spmv32_up(const i64* __restri
 __global__ void __launch_bounds__(MX_THREADS) k_pq32(i64 n, const float* __restrict__ pring,
                                                      const float* __restrict__ qring, double* __restrict__ part,
                                                      double* __restrict__ flags, unsigned* ticket) {
-    __shared__ double sh[40];
+    __shared__ double sh[MX_THREADS + 1];
     if (flags[S_DONE] != 0.0) return;
     const i64 slot = i64(flags[S_ITERS]) % MX_M;
     const float* p = pring + slot * n;
@@ -463,7 +462,7 @@ __global__ void __launch_bounds__(MX_THREADS) k_update_dr32(i64 n, float* __rest
                                                             const float* __restrict__ p, const float* __restrict__ q,
                                                             double* __restrict__ part, double* __restrict__ flags,
                                                             unsigned* ticket, double tol2, double max_iterations) {
-    __shared__ double sh[40];
+    __shared__ double sh[MX_THREADS + 1];
     if (flags[S_DONE] != 0.0) return;
     const i64 slot = i64(flags[S_ITERS]) % MX_M;
     p += slot * n;
@@ -492,7 +491,7 @@ __global__ void __launch_bounds__(MX_THREADS) k_update_dr32(i64 n, float* __rest
 __global__ void __launch_bounds__(MX_THREADS) k_dotm32(i64 n, const float* __restrict__ z, const float* __restrict__ qring,
                                                        double* __restrict__ part, double* __restrict__ flags,
                                                        unsigned* ticket) {
-    __shared__ double sh[33 * MX_M];
+    __shared__ double sh[(MX_THREADS + 1) * MX_M];
     if (flags[S_DONE] != 0.0) return;
     const int count = mx_count(flags);
     float zq32[MX_M] = {};
@@ -516,7 +515,7 @@ __global__ void __launch_bounds__(MX_THREADS) k_update_pm32(i64 n, float* __rest
                                                             const float* __restrict__ r, double* __restrict__ part,
                                                             double* __restrict__ flags, unsigned* ticket,
                                                             float* __restrict__ qring_clear) {
-    __shared__ double sh[40];
+    __shared__ double sh[MX_THREADS + 1];
     if (flags[S_DONE] != 0.0) return;
     const i64 k = i64(flags[S_ITERS]);
     const int count = mx_count(flags), next = int(k % MX_M);

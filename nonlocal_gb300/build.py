@@ -24,7 +24,7 @@ UNITS = ["util.cu", "mesh.cu", "neighbours.cu", "boundary.cu", "pattern.cu", "as
          "bicgstab.cu", "elastic.cu", "coarse.cu", "iltbuild.cu",
          "batch.cu", "tc_gemm.cu",
          "mpnn.cu", "noalloc.cu", "api.cu"]
-HEADERS = ["common.cuh", "ff.cuh", "influence.cuh"]
+HEADERS = ["common.cuh", "ff.cuh", "influence.cuh", "influence_ff.cuh"]
 NO_FMA = {"mesh.cu", "neighbours.cu"}
 
 

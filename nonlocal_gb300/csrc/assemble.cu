@@ -27,6 +27,7 @@
 #include "common.cuh"
 #include "ff.cuh"
 #include "influence.cuh"
+#include "influence_ff.cuh"
 
 #include <cmath>
 
@@ -279,26 +280,6 @@ struct PairFF {
     int32_t nodes[NEN];
     int32_t inner[NEN];   // whether each of eNL's nodes is inner (read once per pair, not per entry)
 };
-
-// shape<INF> in float-float (fast polynomial, polynomial and exponential with
-// p divisible by n; the host sends the other kinds to the FP64 kernel)
-// z0, z1: the coordinate differences in units of the radii
-template<int INF>
-__device__ __forceinline__ ff shape_ff(const Model& m, ff z0, ff z1, ff q, const ff* exp_table) {
-    ff d;
-    if (m.n == 2) d = ff_add(ff_mul(z0, z0), ff_mul(z1, z1));
-    else if (m.n == 1) d = ff_add(ff_abs(z0), ff_abs(z1));
-    else d = ff_add(ff_ipow(ff_abs(z0), m.n), ff_ipow(ff_abs(z1), m.n));
-    if constexpr (INF == NLGPU_INFLUENCE_FAST_POLYNOMIAL) {
-        return ff_lt(d, 1.0f) ? ff_sub(ff_make(1.0f), d) : ff_make(0.0f);
-    } else {
-        const ff dp = ff_ipow(d, m.p / m.n);
-        if constexpr (INF == NLGPU_INFLUENCE_POLYNOMIAL)
-            return ff_lt(d, 1.0f) ? ff_ipow(ff_sub(ff_make(1.0f), dp), int(m.q)) : ff_make(0.0f);
-        else
-            return ff_exp_nonpositive(ff_neg(ff_mul(q, dp)), exp_table);
-    }
-}
 
 template<int NEN, int NQ, int INF, bool SYM, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_assemble_pairs_ff(AssembleArgs a, FFArgs f, Model m, Basis b) {
@@ -649,17 +630,6 @@ void dispatch_influence_ff(Ctx& ctx, const AssembleArgs& a, const FFArgs& f, boo
     }
 }
 
-// float-float covers the continuous influence kinds with an integral power
-// p / n and constant conductivity; the rest runs the FP64 kernel
-bool ff_supported(const Ctx& ctx) {
-    const Model& m = ctx.model;
-    if (m.n < 1) return false;
-    if (m.influence == NLGPU_INFLUENCE_FAST_POLYNOMIAL) return true;
-    if (m.influence == NLGPU_INFLUENCE_POLYNOMIAL || m.influence == NLGPU_INFLUENCE_EXPONENTIAL)
-        return m.p >= 0 && m.p % m.n == 0;
-    return false;
-}
-
 }  // namespace
 
 // Assembles p1*K_local + (1-p1)*K_nonlocal (or p1*K_local for a local model)
@@ -685,7 +655,7 @@ void assemble_full(Ctx& ctx) {
     a.error = err.p;
     // unordered pairs need a symmetric influence and constant conductivity
     const bool sym = ctx.symmetric && !ctx.cond_field.n && !ctx.ordered_pairs;
-    ctx.ff_assembled = ctx.ff_assembly && ff_supported(ctx);
+    ctx.ff_assembled = ctx.ff_assembly && ff_supported(ctx.model);
     if (ctx.ff_assembled) {
         const int nen = ctx.basis.nen, nq = ctx.basis.nq;
         ctx.deriv_ff.reserve(size_t(ctx.n_elems * nen * nq));
@@ -695,11 +665,7 @@ void assemble_full(Ctx& ctx) {
                   ctx.deriv.p, ctx.qcoord.p, a.cond_field, ctx.model, ctx.basis, ctx.deriv_ff.p, ctx.qcoord_ff.p,
                   ctx.cw_ff.p);
         FFArgs f{ctx.deriv_ff.p, ctx.qcoord_ff.p, ctx.cw_ff.p, {}};
-        for (int k = -FF_EXP_K; k <= FF_EXP_K; ++k) {
-            const double x = std::exp(double(k) / double(FF_EXP_STEPS));
-            const float hi = float(x);
-            f.exp_table.v[k + FF_EXP_K] = make_float2(hi, float(x - double(hi)));
-        }
+        fill_exp_table(f.exp_table);
         if (nen == 4) dispatch_influence_ff<4, 4>(ctx, a, f, sym);
         else dispatch_influence_ff<8, 9>(ctx, a, f, sym);
     } else if (ctx.basis.nen == 4) {

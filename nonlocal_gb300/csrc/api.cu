@@ -34,6 +34,13 @@ int guarded(F&& f) {
     }
 }
 
+// the same with the context's arena for the call's buffers
+template<class F>
+int guarded(Ctx* ctx, F&& f) {
+    const ArenaScope scope{ctx->arena};
+    return guarded(std::forward<F>(f));
+}
+
 // the status of a solve entry: its error, else NLGPU_ERR_NO_CONVERGENCE (with a
 // message) when the solve ended before the tolerance
 int solve_status(int rc, int conv_status) {
@@ -404,7 +411,7 @@ int nlgpu_create(nlgpu_ctx** ctx, void* stream) {
 
 int nlgpu_destroy(nlgpu_ctx* ctx) {
     if (!ctx) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         cudaStreamSynchronize(ctx->stream);
         const bool own = ctx->own_stream;
         cudaStream_t s = ctx->stream;
@@ -415,13 +422,13 @@ int nlgpu_destroy(nlgpu_ctx* ctx) {
 
 int nlgpu_synchronize(nlgpu_ctx* ctx) {
     if (!ctx) return NLGPU_ERR_ARG;
-    return guarded([&] { NL_CUDA(cudaStreamSynchronize(ctx->stream)); });
+    return guarded(ctx, [&] { NL_CUDA(cudaStreamSynchronize(ctx->stream)); });
 }
 
 int nlgpu_mesh_2d(nlgpu_ctx* ctx, int element_type, int64_t n_nodes, const double* nodes, int64_t n_elements,
                   const int64_t* elements) {
     if (!ctx || !nodes || !elements || n_nodes <= 0 || n_elements <= 0) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         c.basis = make_basis(element_type);
         NL_REQUIRE(n_nodes < (int64_t(1) << 31) && n_elements * c.basis.nen < (int64_t(1) << 40), NLGPU_ERR_UNSUPPORTED,
@@ -446,7 +453,7 @@ int nlgpu_mesh_2d(nlgpu_ctx* ctx, int element_type, int64_t n_nodes, const doubl
 
 int nlgpu_cuthill_mckee(nlgpu_ctx* ctx, int only_local, int reverse, int64_t* permutation) {
     if (!ctx || !permutation) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.mesh_ready, NLGPU_ERR_STATE, "no mesh");
         const bool local_graph = only_local || !(c.model_ready && c.model.nonlocal());
@@ -464,7 +471,7 @@ int nlgpu_cuthill_mckee(nlgpu_ctx* ctx, int only_local, int reverse, int64_t* pe
 
 int nlgpu_renumbering(nlgpu_ctx* ctx, const int64_t* permutation) {
     if (!ctx || !permutation) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.mesh_ready, NLGPU_ERR_STATE, "no mesh");
         const size_t n = size_t(c.n_nodes);
@@ -484,7 +491,7 @@ int nlgpu_renumbering(nlgpu_ctx* ctx, const int64_t* permutation) {
 
 int nlgpu_get_quadrature(nlgpu_ctx* ctx, double* qcoords, double* jacobians, double* derivatives) {
     if (!ctx) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.mesh_ready, NLGPU_ERR_STATE, "no mesh");
         if (qcoords) c.qcoord.download(qcoords, c.qcoord.n, c.stream);
@@ -497,7 +504,7 @@ int nlgpu_get_quadrature(nlgpu_ctx* ctx, double* qcoords, double* jacobians, dou
 int nlgpu_get_basis(nlgpu_ctx* ctx, int* nodes_per_element, int* qnodes, double* qN, double* qNxi, double* qNeta,
                     double* weights, double* centre) {
     if (!ctx) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         const Basis& b = ctx->basis;
         NL_REQUIRE(ctx->mesh_ready, NLGPU_ERR_STATE, "no mesh");
         if (nodes_per_element) *nodes_per_element = b.nen;
@@ -513,7 +520,7 @@ int nlgpu_get_basis(nlgpu_ctx* ctx, int* nodes_per_element, int* qnodes, double*
 
 int nlgpu_set_model_2d(nlgpu_ctx* ctx, const nlgpu_model_2d* model) {
     if (!ctx || !model) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         ctx->model = make_model(*model);
         ctx->model_ready = true;
         reset_from_model(*ctx);
@@ -522,7 +529,7 @@ int nlgpu_set_model_2d(nlgpu_ctx* ctx, const nlgpu_model_2d* model) {
 
 int nlgpu_set_conductivity_field(nlgpu_ctx* ctx, const double* values) {
     if (!ctx) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.mesh_ready, NLGPU_ERR_STATE, "no mesh");
         if (values) c.cond_field.upload(values, size_t(c.n_elems * c.basis.nq), c.stream);
@@ -539,7 +546,7 @@ int nlgpu_set_capacity(nlgpu_ctx* ctx, double capacity, double density) {
 
 int nlgpu_find_neighbours(nlgpu_ctx* ctx, int strategy, double* search_radius, int64_t* pairs) {
     if (!ctx) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         find_neighbours(*ctx, strategy);
         if (search_radius) { search_radius[0] = ctx->search_r[0]; search_radius[1] = ctx->search_r[1]; }
         if (pairs) *pairs = ctx->pairs;
@@ -549,7 +556,7 @@ int nlgpu_find_neighbours(nlgpu_ctx* ctx, int strategy, double* search_radius, i
 
 int nlgpu_get_neighbours(nlgpu_ctx* ctx, int64_t* offsets, int64_t* list) {
     if (!ctx) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.neighbours_ready, NLGPU_ERR_STATE, "no neighbour search yet");
         if (offsets) c.noff.download(offsets, size_t(c.n_elems + 1), c.stream);
@@ -588,7 +595,7 @@ void add_group(Ctx& c, int kind, int64_t n_edges, int nodes_per_edge, const int6
 int nlgpu_add_boundary_2d(nlgpu_ctx* ctx, int kind, int64_t n_edges, int nodes_per_edge, const int64_t* edges,
                           double value, const double* node_values) {
     if (!ctx || !edges || n_edges < 0) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         NL_REQUIRE(kind == NLGPU_BC_TEMPERATURE || kind == NLGPU_BC_FLUX, NLGPU_ERR_ARG,
                    "unknown boundary kind (convection and radiation: nlgpu_add_flux_boundary_2d)");
         add_group(*ctx, kind, n_edges, nodes_per_edge, edges, value, node_values, 0.0, 0.0);
@@ -598,7 +605,7 @@ int nlgpu_add_boundary_2d(nlgpu_ctx* ctx, int kind, int64_t n_edges, int nodes_p
 int nlgpu_add_flux_boundary_2d(nlgpu_ctx* ctx, int kind, int64_t n_edges, int nodes_per_edge, const int64_t* edges,
                                double flux, double heat_transfer, double ambient_temperature, double emissivity) {
     if (!ctx || !edges || n_edges < 0) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         double value = 0.0;
         switch (kind) {
         case NLGPU_BC_FLUX: value = flux; heat_transfer = emissivity = 0.0; break;
@@ -616,7 +623,7 @@ int nlgpu_add_flux_boundary_2d(nlgpu_ctx* ctx, int kind, int64_t n_edges, int no
 int nlgpu_set_stationary_parameters(nlgpu_ctx* ctx, double tolerance, int64_t max_iterations, double energy,
                                     const double* initial_temperature) {
     if (!ctx || max_iterations < 0 || !std::isfinite(energy)) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.mesh_ready, NLGPU_ERR_STATE, "no mesh");
         c.nl_tolerance = tolerance;
@@ -630,7 +637,7 @@ int nlgpu_set_stationary_parameters(nlgpu_ctx* ctx, double tolerance, int64_t ma
 
 int nlgpu_get_system_rows(nlgpu_ctx* ctx, int64_t* rows) {
     if (!ctx || !rows) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         NL_REQUIRE(ctx->inner_ready, NLGPU_ERR_STATE, "FULL part not assembled");
         *rows = ctx->n_nodes + (ctx->neumann ? 1 : 0);
     });
@@ -638,7 +645,7 @@ int nlgpu_get_system_rows(nlgpu_ctx* ctx, int64_t* rows) {
 
 int nlgpu_set_source(nlgpu_ctx* ctx, double value, const double* per_qnode) {
     if (!ctx) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.mesh_ready, NLGPU_ERR_STATE, "no mesh");
         c.source = value;
@@ -650,7 +657,7 @@ int nlgpu_set_source(nlgpu_ctx* ctx, double value, const double* per_qnode) {
 
 int nlgpu_set_dirichlet_values(nlgpu_ctx* ctx, const double* values) {
     if (!ctx) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.mesh_ready, NLGPU_ERR_STATE, "no mesh");
         if (values) c.dirichlet_override.upload(values, size_t(c.n_nodes), c.stream);
@@ -671,7 +678,7 @@ int nlgpu_clear_boundaries(nlgpu_ctx* ctx) {
 
 int nlgpu_conductivity_matrix_2d(nlgpu_ctx* ctx, int part, int64_t* nnz_inner, int64_t* nnz_bound) {
     if (!ctx) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(part == NLGPU_PART_FULL || part == NLGPU_PART_LOCAL, NLGPU_ERR_ARG, "part is LOCAL or FULL");
         NL_REQUIRE(c.mesh_ready && c.model_ready, NLGPU_ERR_STATE, "mesh and model must be set before assembly");
@@ -691,7 +698,7 @@ int nlgpu_conductivity_matrix_2d(nlgpu_ctx* ctx, int part, int64_t* nnz_inner, i
 
 int nlgpu_get_matrix(nlgpu_ctx* ctx, int which, int64_t* rowptr, int64_t* col, double* val) {
     if (!ctx) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         if (which == NLGPU_MATRIX_INNER || which == NLGPU_MATRIX_BOUND) {
             NL_REQUIRE(c.inner_ready, NLGPU_ERR_STATE, "FULL part not assembled");
@@ -714,7 +721,7 @@ int nlgpu_get_matrix(nlgpu_ctx* ctx, int which, int64_t* rowptr, int64_t* col, d
 
 int nlgpu_get_rhs(nlgpu_ctx* ctx, double* rhs, double* rhs_init) {
     if (!ctx) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.inner_ready, NLGPU_ERR_STATE, "FULL part not assembled");
         if (rhs_init) c.rhs_init.download(rhs_init, size_t(c.n_nodes), c.stream);
@@ -731,7 +738,7 @@ int nlgpu_get_rhs(nlgpu_ctx* ctx, double* rhs, double* rhs_init) {
 
 int nlgpu_calc_flux(nlgpu_ctx* ctx, const double* temperature, double* flux_x, double* flux_y) {
     if (!ctx || !temperature || !flux_x || !flux_y) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.mesh_ready && c.model_ready, NLGPU_ERR_STATE, "mesh and model must be set");
         if (c.model.nonlocal()) ensure_neighbours(c);
@@ -751,7 +758,7 @@ int nlgpu_solve_assembled(nlgpu_ctx* ctx, const nlgpu_solve_options* options, do
                           nlgpu_solve_report* report) {
     if (!ctx || !options || !temperature) return NLGPU_ERR_ARG;
     int conv_status = NLGPU_OK;
-    const int rc = guarded([&] {
+    const int rc = guarded(ctx, [&] {
         Ctx& c = *ctx;
         const auto t0 = std::chrono::steady_clock::now();
         const CgResult r = stationary_solve(c, *options, report);
@@ -789,6 +796,7 @@ int nlgpu_solve_assembled_batch(int64_t count, nlgpu_ctx* const* instances, cons
         size_t next = 0;
         for (int64_t k = 0; k < count; ++k) {
             Ctx& c = *instances[k];
+            const ArenaScope own{c.arena};
             nlgpu_solve_report* rep = reports ? reports + k : nullptr;
             if (rep) std::memset(rep, 0, sizeof *rep);
             CgResult r;
@@ -813,7 +821,7 @@ int nlgpu_stationary_2d(nlgpu_ctx* ctx, const nlgpu_solve_options* options, doub
                         nlgpu_solve_report* report) {
     if (!ctx || !options || !temperature) return NLGPU_ERR_ARG;
     int conv_status = NLGPU_OK;
-    const int rc = guarded([&] {
+    const int rc = guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.mesh_ready && c.model_ready, NLGPU_ERR_STATE, "mesh and model must be set");
         nlgpu_solve_report local_rep{};
@@ -871,7 +879,7 @@ int nlgpu_cg_solve(nlgpu_ctx* ctx, int64_t n, const int64_t* a_rowptr, const int
                    double tolerance, int64_t max_iterations, double* x, nlgpu_solve_report* report) {
     if (!ctx || n <= 0 || !a_rowptr || !a_col || !a_val || !b || !x) return NLGPU_ERR_ARG;
     int conv_status = NLGPU_OK;
-    const int rc = guarded([&] {
+    const int rc = guarded(ctx, [&] {
         Ctx& c = *ctx;
         const auto t0 = std::chrono::steady_clock::now();
         // full padded rows from the upper storage (both triangles)
@@ -920,7 +928,7 @@ int nlgpu_cg_solve(nlgpu_ctx* ctx, int64_t n, const int64_t* a_rowptr, const int
 int nlgpu_illt_compute(nlgpu_ctx* ctx, int64_t n, const int64_t* rowptr, const int64_t* col, const double* val,
                        int* computation_info) {
     if (!ctx || n <= 0 || n >= (int64_t(1) << 31) || !rowptr || !col || !val || !computation_info) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         c.plugin_ilt_ready = false;
         NL_REQUIRE(rowptr[0] == 0 && rowptr[n] >= n, NLGPU_ERR_ARG, "row pointers must start at 0 and hold a diagonal per row");
@@ -947,7 +955,7 @@ int nlgpu_illt_compute(nlgpu_ctx* ctx, int64_t n, const int64_t* rowptr, const i
 
 int nlgpu_illt_solve(nlgpu_ctx* ctx, int64_t n, const double* x, double* y) {
     if (!ctx || !x || !y) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.plugin_ilt_ready, NLGPU_ERR_STATE, "nlgpu_illt_compute has not succeeded on this context");
         NL_REQUIRE(n == c.plugin_ilt.n, NLGPU_ERR_ARG, "vector size differs from the factorised matrix");
@@ -966,7 +974,7 @@ int nlgpu_illt_solve(nlgpu_ctx* ctx, int64_t n, const double* x, double* y) {
 
 int nlgpu_illt_solve_f32(nlgpu_ctx* ctx, int64_t n, int sweeps, const float* x, float* y) {
     if (!ctx || !x || !y || sweeps == 0 || sweeps > 4096) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.plugin_ilt_ready, NLGPU_ERR_STATE, "nlgpu_illt_compute has not succeeded on this context");
         NL_REQUIRE(n == c.plugin_ilt.n, NLGPU_ERR_ARG, "vector size differs from the factorised matrix");
@@ -999,7 +1007,7 @@ void ensure_learning_state(Ctx& c) {
 
 int nlgpu_mpnn_set_weights(nlgpu_ctx* ctx, const float* params) {
     if (!ctx || !params) return NLGPU_ERR_ARG;
-    return guarded([&] { mpnn_set_weights(*ctx, params); NL_CUDA(cudaStreamSynchronize(ctx->stream)); });
+    return guarded(ctx, [&] { mpnn_set_weights(*ctx, params); NL_CUDA(cudaStreamSynchronize(ctx->stream)); });
 }
 
 int nlgpu_mpnn_set_enabled(nlgpu_ctx* ctx, int enabled) {
@@ -1010,7 +1018,7 @@ int nlgpu_mpnn_set_enabled(nlgpu_ctx* ctx, int enabled) {
 
 int nlgpu_mpnn_get_weights(nlgpu_ctx* ctx, float* params) {
     if (!ctx || !params) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         NL_REQUIRE(ctx->mp.params.n == size_t(MPNN_PARAMS), NLGPU_ERR_STATE, "no weights yet");
         mpnn_get_weights(*ctx, params);
     });
@@ -1018,7 +1026,7 @@ int nlgpu_mpnn_get_weights(nlgpu_ctx* ctx, float* params) {
 
 int nlgpu_mpnn_train(nlgpu_ctx* ctx, const nlgpu_train_options* options, nlgpu_train_report* report) {
     if (!ctx || !options) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         ensure_learning_state(c);
         MpnnTrainOptions o;
@@ -1046,7 +1054,7 @@ int nlgpu_mpnn_train(nlgpu_ctx* ctx, const nlgpu_train_options* options, nlgpu_t
 int nlgpu_mpnn_loss_grad(nlgpu_ctx* ctx, const float* r, const float* e, float* z, float* p, double* loss,
                          float* grad) {
     if (!ctx || !r || !e) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         ensure_learning_state(c);
         const i64 n = c.full.rows;
@@ -1072,7 +1080,7 @@ int nlgpu_mpnn_loss_grad(nlgpu_ctx* ctx, const float* r, const float* e, float* 
 
 int nlgpu_nonstationary_2d_compute(nlgpu_ctx* ctx, double time_step, const double* initial) {
     if (!ctx || !(time_step > 0.0)) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.mesh_ready && c.model_ready, NLGPU_ERR_STATE, "mesh and model must be set");
         // nonstationary_heat_equation_solver_2d::compute (nonstationary_heat_equation_solver_2d.hpp:63-88)
@@ -1107,7 +1115,7 @@ int nlgpu_nonstationary_2d_step(nlgpu_ctx* ctx, double dirichlet_value, const do
                                 double tolerance, int64_t max_iterations, double* temperature, int64_t* iterations) {
     if (!ctx) return NLGPU_ERR_ARG;
     int conv_status = NLGPU_OK;
-    const int rc = guarded([&] {
+    const int rc = guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.nonstationary_ready, NLGPU_ERR_STATE, "nonstationary_2d_compute must run first");
         // calc_step (nonstationary_heat_equation_solver_2d.hpp:90-106):
@@ -1200,7 +1208,7 @@ int nlgpu_stationary_1d(nlgpu_ctx* ctx, int64_t elements, int order, double leng
                         int influence, double conductivity, double t_left, double q_right, int sin_source,
                         double* temperature) {
     if (!ctx || elements <= 0 || (order != 1 && order != 2) || !(length > 0.0) || !temperature) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         stationary_1d(*ctx, elements, order, length, radius, local_weight, influence, conductivity, t_left, q_right,
                       sin_source != 0, temperature);
     });
@@ -1212,7 +1220,7 @@ int nlgpu_nonstationary_1d_compute(nlgpu_ctx* ctx, int64_t elements, int order, 
                                    const double* initial_temperature, int64_t* nodes) {
     if (!ctx || elements <= 0 || (order != 1 && order != 2) || !(length > 0.0) || !(time_step > 0.0))
         return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         nonstationary_1d_compute(*ctx, elements, order, length, radius, local_weight, influence, conductivity,
                                  capacity, density, time_step, left_kind, right_kind, initial_temperature);
         if (nodes) *nodes = nonstationary_1d_nodes(*ctx);
@@ -1229,17 +1237,17 @@ int nlgpu_nonstationary_1d_convection(nlgpu_ctx* ctx, double heat_transfer_left,
 int nlgpu_nonstationary_1d_step(nlgpu_ctx* ctx, double left_value, double right_value, int sin_source,
                                 double* temperature) {
     if (!ctx) return NLGPU_ERR_ARG;
-    return guarded([&] { nonstationary_1d_step(*ctx, left_value, right_value, sin_source != 0, temperature); });
+    return guarded(ctx, [&] { nonstationary_1d_step(*ctx, left_value, right_value, sin_source != 0, temperature); });
 }
 
 int nlgpu_nonstationary_1d_temperature(nlgpu_ctx* ctx, double* temperature) {
     if (!ctx || !temperature) return NLGPU_ERR_ARG;
-    return guarded([&] { nonstationary_1d_temperature(*ctx, temperature); });
+    return guarded(ctx, [&] { nonstationary_1d_temperature(*ctx, temperature); });
 }
 
 int nlgpu_set_elastic_2d(nlgpu_ctx* ctx, int kind, const double* prm, double* hooke_out) {
     if (!ctx || !prm) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Elastic& el = ctx->el;
         double h[6] = {0, 0, 0, 0, 0, 0};   // h11 h12 h66 h22 h16 h26
         if (kind == NLGPU_ELASTIC_ISOTROPIC) {
@@ -1287,7 +1295,7 @@ int nlgpu_set_elastic_2d(nlgpu_ctx* ctx, int kind, const double* prm, double* ho
 int nlgpu_add_mechanical_boundary_2d(nlgpu_ctx* ctx, int64_t n_edges, int nodes_per_edge, const int64_t* edges,
                                      int kind_x, double value_x, int kind_y, double value_y) {
     if (!ctx || !edges || n_edges < 0) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.mesh_ready, NLGPU_ERR_STATE, "no mesh");
         NL_REQUIRE(nodes_per_edge == 2 || nodes_per_edge == 3, NLGPU_ERR_UNSUPPORTED, "boundary edges have 2 or 3 nodes");
@@ -1319,7 +1327,7 @@ int nlgpu_clear_mechanical_boundaries(nlgpu_ctx* ctx) {
 
 int nlgpu_stiffness_matrix_2d(nlgpu_ctx* ctx, int part, int64_t* nnz_inner, int64_t* nnz_bound) {
     if (!ctx) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(part == NLGPU_PART_FULL || part == NLGPU_PART_LOCAL, NLGPU_ERR_ARG, "part FULL or LOCAL");
         if (part == NLGPU_PART_FULL && c.model.nonlocal()) ensure_neighbours(c);
@@ -1332,7 +1340,7 @@ int nlgpu_stiffness_matrix_2d(nlgpu_ctx* ctx, int part, int64_t* nnz_inner, int6
 
 int nlgpu_get_stiffness_matrix(nlgpu_ctx* ctx, int which, int64_t* rowptr, int64_t* col, double* val) {
     if (!ctx) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(which >= NLGPU_MATRIX_INNER && which <= NLGPU_MATRIX_LOCAL, NLGPU_ERR_ARG, "unknown matrix");
         if (which == NLGPU_MATRIX_LOCAL) {
@@ -1347,7 +1355,7 @@ int nlgpu_get_stiffness_matrix(nlgpu_ctx* ctx, int which, int64_t* rowptr, int64
 
 int nlgpu_get_mechanical_rhs(nlgpu_ctx* ctx, double* rhs, double* rhs_init) {
     if (!ctx) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.el.assembled, NLGPU_ERR_STATE, "FULL stiffness not assembled");
         const size_t rows = size_t(2 * c.n_nodes);
@@ -1361,7 +1369,7 @@ int nlgpu_equilibrium_equation_2d(nlgpu_ctx* ctx, const nlgpu_solve_options* opt
                                   nlgpu_solve_report* report) {
     if (!ctx || !options || !displacement) return NLGPU_ERR_ARG;
     int conv_status = NLGPU_OK;
-    const int rc = guarded([&] {
+    const int rc = guarded(ctx, [&] {
         Ctx& c = *ctx;
         const auto t0 = std::chrono::steady_clock::now();
         if (report) *report = nlgpu_solve_report{};
@@ -1424,7 +1432,7 @@ int nlgpu_assembly_tuning(nlgpu_ctx* ctx, int* warps, double* sample_ms) {
 
 int nlgpu_event_record(nlgpu_ctx* ctx, int slot) {
     if (!ctx || slot < 0 || slot >= 64) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         if (!c.events[slot]) NL_CUDA(cudaEventCreate(&c.events[slot]));
         NL_CUDA(cudaEventRecord(c.events[slot], c.stream));
@@ -1433,7 +1441,7 @@ int nlgpu_event_record(nlgpu_ctx* ctx, int slot) {
 
 int nlgpu_event_elapsed(nlgpu_ctx* ctx, int a, int b, double* ms) {
     if (!ctx || !ms || a < 0 || b < 0 || a >= 64 || b >= 64) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         NL_REQUIRE(c.events[a] && c.events[b], NLGPU_ERR_STATE, "event slot not recorded");
         NL_CUDA(cudaEventSynchronize(c.events[b]));
@@ -1445,7 +1453,7 @@ int nlgpu_event_elapsed(nlgpu_ctx* ctx, int a, int b, double* ms) {
 
 int nlgpu_flush_l2(nlgpu_ctx* ctx, int64_t bytes) {
     if (!ctx || bytes <= 0) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         c.flush.reserve(size_t(bytes));
         NL_CUDA(cudaMemsetAsync(c.flush.p, int(c.flush_value++ & 0xff), size_t(bytes), c.stream));
@@ -1454,7 +1462,7 @@ int nlgpu_flush_l2(nlgpu_ctx* ctx, int64_t bytes) {
 
 int nlgpu_time_stage(nlgpu_ctx* ctx, int stage, int reps, double* ms) {
     if (!ctx || !ms || reps <= 0) return NLGPU_ERR_ARG;
-    return guarded([&] {
+    return guarded(ctx, [&] {
         Ctx& c = *ctx;
         cudaEvent_t e0, e1;
         NL_CUDA(cudaEventCreate(&e0));

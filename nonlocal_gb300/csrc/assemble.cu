@@ -233,92 +233,161 @@ __global__ void __launch_bounds__(AS_THREADS) k_assemble_pairs(AssembleArgs a, M
 }
 
 // ---------------------------------------------------------------- float-float
-// The same pair blocks with the influence values and both contractions in
-// float-float arithmetic (ff.cuh) on the FP32 pipes -- the mixed-precision
-// form's FP32 nonlocal blocks, carried to about 48 bits so that the matrix
-// stays within the FP64 entries' tolerance and the FP64 refinement converges
-// to the FP64 solution.  Only the rows' accumulators, the rare self term and
-// the index work stay FP64 / integer.  Element data is staged once per
-// assembly as float-float (k_ff_stage), so the pair loop converts nothing.
-// 16 or 32 warps per CTA (the FP64 kernel's 8 leave the FP32 pipes idle),
-// chosen per problem by timing both on a sample of elements (ff_warps).
+// The same pair blocks with the influence values in float-float arithmetic
+// (ff.cuh, about 48 bits) on the FP32 pipes and both contractions in fixed point
+// on the integer multipliers.  Everything a block multiplies lies within a few
+// binary orders of its largest factor, so eNL's gradients carry one exponent per
+// element and the influence values one per pair; a number is then 53 to 57 bits in
+// two signed words (hi 2^28 + lo), a multiply-add three 32 x 32 + 64-bit ones
+// (hi hi, and hi lo + lo hi into a second accumulator; lo lo lies below the result's
+// last bit), and the sums are exact.  Against the compensated float-float dot
+// product (12 FP32 instructions a term, errors of order 2^-48) that is a quarter of
+// the instructions, half the pipe time (64 lanes a clock against 128) and an error
+// of 2^-51 of the block's scale: the float-float influence values remain the only
+// rounding.  Weights, Lambda and the constant factors are folded into the two staged
+// copies of the gradients (k_ff_stage), the pairs this element owns are listed once
+// per element, and a pair whose influence is zero everywhere ends there.
+// 8-node 300 x 300 elements, exponential influence: 116.9 ms with the compensated
+// dots, 76.5 with fixed point; 4-node 200 x 200: 7.4 and 4.2; 17.9 million listed
+// 8-node pairs: 24.1 and 13.2 G instructions, 28.0 and 18.6 ms.  What bounds it
+// now: issue (57 % of the slots, FMA-heavy pipe 55 %, shared-memory wavefronts
+// 52 %), the influence values being the largest part.
+// 16 or 32 warps per CTA (the FP64 kernel's 8 leave the pipes idle), chosen per
+// problem by timing both on a sample of elements; a warp takes one 8-node pair or
+// two 4-node pairs at a time (16 lanes cover a 4 x 4 block).
+
+constexpr int FF_BAD = 1 << 20;   // exponent of an element with a non-finite value
+constexpr int FF_LIST = 1024;     // candidates listed at a time
 
 struct FFArgs {
-    const float4* deriv;    // [e][i][q]: (gx.h, gx.l, gy.h, gy.l)
     const float4* qcoord;   // [e][q]: (x/r0 .h, .l, y/r1 .h, .l), coordinates in units of the radii
-    const float2* cw;       // [e][q]: c_q = w_q norm (1 - p1) [lambda_q]
+    const int2* g;          // [e][q][x, y][j]: w_q norm (1 - p1) [lambda_q] Lambda G_j 2^(56 - exps.x) as hi 2^28 + lo
+    const int4* w;          // [e][i][q]: w_q G_i 2^(56 - exps.y), (x hi, lo, y hi, lo)
+    const int2* exps;       // [e]: the exponents of the largest |g| and |w|
+    const int32_t* nodes;   // [e][j]: the node, its complement where it is not inner
     FFExpTable exp_table;   // exp(k / 256), copied to shared memory by each CTA
 };
 
-__global__ void k_ff_stage(i64 E, int nen, int nq, const double* __restrict__ deriv, const double* __restrict__ qcoord,
-                           const double* __restrict__ cond_field, Model m, Basis b, float4* __restrict__ dff,
-                           float4* __restrict__ qff, float2* __restrict__ cw) {
+__device__ __forceinline__ int2 ff_fixed(double x, int e) {
+    const long long z = __double2ll_rn(scalbn(x, 56 - e));   // |z| < 2^57
+    const long long hi = (z + (1 << 27)) >> 28;
+    return make_int2(int(hi), int(z - hi * (1 << 28)));
+}
+
+// one warp per element
+__global__ void k_ff_stage(i64 E, int nen, int nq, const int32_t* __restrict__ elems, const uint8_t* __restrict__ is_inner,
+                           const double* __restrict__ deriv, const double* __restrict__ qcoord,
+                           const double* __restrict__ cond_field, Model m, Basis b, float4* __restrict__ qff,
+                           int2* __restrict__ g, int4* __restrict__ w, int2* __restrict__ exps,
+                           int32_t* __restrict__ nodes) {
     const double cnl = m.norm * (1.0 - m.p1);
     const bool iso = m.cond_kind == NLGPU_CONDUCTIVITY_ISOTROPIC;
-    for (i64 t = blockIdx.x * i64(blockDim.x) + threadIdx.x; t < E * nen * nq; t += i64(gridDim.x) * blockDim.x) {
-        const ff gx = ff_from(deriv[2 * t]), gy = ff_from(deriv[2 * t + 1]);
-        dff[t] = make_float4(gx.h, gx.l, gy.h, gy.l);
-        if (t < E * nq) {
-            const ff x = ff_from(qcoord[2 * t] * m.inv_r[0]), y = ff_from(qcoord[2 * t + 1] * m.inv_r[1]);
-            qff[t] = make_float4(x.h, x.l, y.h, y.l);
-            const double lam = cond_field ? cond_field[t] : m.cond[0];
-            const ff c = ff_from(b.w[t % nq] * cnl * (iso ? lam : 1.0));
-            cw[t] = make_float2(c.h, c.l);
+    const int lane = threadIdx.x & 31;
+    auto values = [&](i64 e, int t, double (&v)[4]) {   // (Lambda G scaled, w G) of (i, q) = (t / nq, t % nq)
+        const double gx = deriv[2 * (e * nen * nq + t)], gy = deriv[2 * (e * nen * nq + t) + 1];
+        const int q = t % nq;
+        const double lam = cond_field ? cond_field[e * nq + q] : m.cond[0];
+        const double c = b.w[q] * cnl * (iso ? lam : 1.0);
+        v[0] = c * gx; v[1] = c * gy;
+        if (m.cond_kind == NLGPU_CONDUCTIVITY_ORTHOTROPIC) { v[0] *= m.cond[0]; v[1] *= m.cond[1]; }
+        else if (!iso) {
+            v[0] = c * (m.cond[0] * gx + m.cond[2] * gy);
+            v[1] = c * (m.cond[2] * gx + m.cond[1] * gy);
+        }
+        v[2] = b.w[q] * gx; v[3] = b.w[q] * gy;
+    };
+    for (i64 e = (blockIdx.x * i64(blockDim.x) + threadIdx.x) / 32; e < E; e += i64(gridDim.x) * blockDim.x / 32) {
+        double mg = 0.0, mw = 0.0;
+        bool bad_g = false, bad_w = false;
+        for (int t = lane; t < nen * nq; t += 32) {
+            double v[4];
+            values(e, t, v);
+            mg = fmax(mg, fmax(fabs(v[0]), fabs(v[1])));
+            mw = fmax(mw, fmax(fabs(v[2]), fabs(v[3])));
+            bad_g = bad_g || !isfinite(v[0]) || !isfinite(v[1]);
+            bad_w = bad_w || !isfinite(v[2]) || !isfinite(v[3]);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            mg = fmax(mg, __shfl_xor_sync(0xffffffffu, mg, o));
+            mw = fmax(mw, __shfl_xor_sync(0xffffffffu, mw, o));
+        }
+        bad_g = __any_sync(0xffffffffu, bad_g);
+        bad_w = __any_sync(0xffffffffu, bad_w);
+        const int eg = bad_g ? FF_BAD : mg > 0.0 ? ilogb(mg) : 0, ew = bad_w ? FF_BAD : mw > 0.0 ? ilogb(mw) : 0;
+        if (lane == 0) exps[e] = make_int2(eg, ew);
+        for (int t = lane; t < nen * nq; t += 32) {
+            double v[4];
+            values(e, t, v);
+            if (bad_g) v[0] = v[1] = 0.0;
+            if (bad_w) v[2] = v[3] = 0.0;
+            const int i = t / nq, q = t % nq;
+            g[((e * nq + q) * 2 + 0) * nen + i] = ff_fixed(v[0], eg);
+            g[((e * nq + q) * 2 + 1) * nen + i] = ff_fixed(v[1], eg);
+            const int2 x = ff_fixed(v[2], ew), y = ff_fixed(v[3], ew);
+            w[e * nen * nq + t] = make_int4(x.x, x.y, y.x, y.y);
+        }
+        if (lane < nq) {
+            const ff x = ff_from(qcoord[2 * (e * nq + lane)] * m.inv_r[0]);
+            const ff y = ff_from(qcoord[2 * (e * nq + lane) + 1] * m.inv_r[1]);
+            qff[e * nq + lane] = make_float4(x.h, x.l, y.h, y.l);
+        }
+        if (lane < nen) {
+            const int32_t r = elems[e * nen + lane];
+            nodes[e * nen + lane] = is_inner[r] ? r : ~r;
         }
     }
 }
 
-// per warp: eNL's data; g holds eNL's gradients (x then y) for H = Phi (Lambda
-// G) and then H itself (x then y), which the lanes keep in registers until
-// every lane has read G
+// one pair's data
 template<int NEN, int NQ>
 struct PairFF {
-    ff qx[NQ], qy[NQ];
-    ff g[2 * NEN * NQ];
-    ff phi[NQ * NQ];
-    ff c[NQ];
+    static constexpr int PS = (NQ + 1) / 2 * 2;   // influence values per row, padded to whole 16 bytes
+    float4 q[NQ];         // eNL's points
+    int2 phi[NQ * PS];    // shape(qL, qNL) 2^(51 - ep), ep the exponent of the pair's largest
+    int4 h[NQ * NEN];     // H(qL, j): (x hi, lo, y hi, lo)
     int32_t nodes[NEN];
-    int32_t inner[NEN];   // whether each of eNL's nodes is inner (read once per pair, not per entry)
 };
 
 template<int NEN, int NQ, int INF, bool SYM, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_assemble_pairs_ff(AssembleArgs a, FFArgs f, Model m, Basis b) {
     constexpr int THREADS = WARPS * 32;
-    constexpr int HN = 2 * NQ * NEN, HR = (HN + 31) / 32;   // H outputs and lane rounds
+    constexpr int LANES = NQ * NQ <= 16 ? 16 : 32, GROUPS = 32 / LANES;   // lanes per pair, pairs per warp
+    constexpr int PR = (NQ * NQ + LANES - 1) / LANES;                     // influence values per lane
+    constexpr int HL = 2 * NEN, HG = LANES / HL;                          // H: one lane per (direction, j), HG rows at a time
+    constexpr int OUT = NEN * NEN / LANES;                                // block entries per lane
+    constexpr int PS = PairFF<NEN, NQ>::PS;
+    static_assert(NEN * NEN % LANES == 0 && LANES % HL == 0 && NEN % 4 == 0 && NEN * NEN / 4 / OUT * 4 == LANES, "lane layout");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ ff eqx[NQ], eqy[NQ], ewx[NEN * NQ], ewy[NEN * NQ];
+    __shared__ float4 eq[NQ];
+    __shared__ int4 ew[NEN * NQ];
     __shared__ double egx[NEN * NQ], egy[NEN * NQ], ejac[NQ], elam[NQ];   // the self term stays FP64
     __shared__ int32_t enodes[NEN], einner[NEN];   // eL's nodes and whether each is inner
     __shared__ i64 row_start[NEN];
     __shared__ int row_len[NEN], row_off[NEN + 1];
-    __shared__ int use_smem;
+    __shared__ int use_smem, listed;
+    __shared__ int32_t list[FF_LIST];
     __shared__ ff etab[2 * FF_EXP_K + 1];
     for (int t = threadIdx.x; t < 2 * FF_EXP_K + 1; t += blockDim.x)
         etab[t] = ff{f.exp_table.v[t].x, f.exp_table.v[t].y};
 
     auto* pairs = reinterpret_cast<PairFF<NEN, NQ>*>(smem_raw);
-    double* acc = reinterpret_cast<double*>(smem_raw + sizeof(PairFF<NEN, NQ>) * WARPS);
+    double* acc = reinterpret_cast<double*>(smem_raw + sizeof(PairFF<NEN, NQ>) * WARPS * GROUPS);
     int32_t* cols = reinterpret_cast<int32_t*>(acc + a.cap);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    PairFF<NEN, NQ>& ps = pairs[warp];
+    const int group = lane / LANES, gl = lane % LANES;
+    PairFF<NEN, NQ>& ps = pairs[warp * GROUPS + group];
     const bool iso = m.cond_kind == NLGPU_CONDUCTIVITY_ISOTROPIC;
     const ff qf = ff_from(m.q);
-    const ff k0 = ff_from(m.cond[0]), k1 = ff_from(m.cond[1]), k2 = ff_from(m.cond[2]);
 
     for (i64 eL = a.e0 + blockIdx.x; eL < a.E; eL += gridDim.x) {
         // ---- element eL: quadrature data, weighted gradients and its node rows
         for (int t = threadIdx.x; t < NEN * NQ; t += THREADS) {
             egx[t] = a.deriv[2 * (eL * NEN * NQ + t)];
             egy[t] = a.deriv[2 * (eL * NEN * NQ + t) + 1];
-            const float4 g = f.deriv[eL * NEN * NQ + t];
-            const ff w = ff_from(b.w[t % NQ]);
-            ewx[t] = ff_mul(w, ff{g.x, g.y});
-            ewy[t] = ff_mul(w, ff{g.z, g.w});
+            ew[t] = f.w[eL * NEN * NQ + t];
         }
         for (int t = threadIdx.x; t < NQ; t += THREADS) {
-            const float4 q = f.qcoord[eL * NQ + t];
-            eqx[t] = ff{q.x, q.y};
-            eqy[t] = ff{q.z, q.w};
+            eq[t] = f.qcoord[eL * NQ + t];
             ejac[t] = a.jac[eL * NQ + t];
             elam[t] = a.cond_field ? a.cond_field[eL * NQ + t] : m.cond[0];
         }
@@ -336,6 +405,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_assemble_pairs_ff(AssembleArgs a
             for (int i = 0; i < NEN; ++i) { row_off[i] = off; off += row_len[i]; }
             row_off[NEN] = off;
             use_smem = off <= a.cap;
+            listed = 0;
         }
         __syncthreads();
         const bool smem_rows = use_smem;
@@ -346,121 +416,161 @@ __global__ void __launch_bounds__(WARPS * 32) k_assemble_pairs_ff(AssembleArgs a
                     acc[row_off[i] + t] = 0.0;
                 }
         }
-        __syncthreads();
         const int32_t key_l = SYM ? a.minnode[eL] : 0;
+        const int e_w = f.exps[eL].y;
 
-        // ---- pairs (eL, eNL): one warp each
         const i64 kb = a.noff[eL], ke = a.noff[eL + 1];
-        for (i64 k = kb + warp; k < ke; k += WARPS) {
-            const int32_t eNL = a.nlist[k];
-            if constexpr (SYM) {   // the pair belongs to the element with the smaller key
-                const int32_t key_n = a.minnode[eNL];
-                if (key_n < key_l || (key_n == key_l && eNL < int32_t(eL))) continue;
-            }
-            for (int t = lane; t < NEN * NQ; t += 32) {
-                const float4 g = f.deriv[i64(eNL) * NEN * NQ + t];
-                ps.g[t] = ff{g.x, g.y};
-                ps.g[NEN * NQ + t] = ff{g.z, g.w};
-            }
-            if (lane < NQ) {
-                const float4 q = f.qcoord[i64(eNL) * NQ + lane];
-                ps.qx[lane] = ff{q.x, q.y};
-                ps.qy[lane] = ff{q.z, q.w};
-                const float2 c = f.cw[i64(eNL) * NQ + lane];
-                ps.c[lane] = ff{c.x, c.y};
-            }
-            if (lane < NEN) {
-                const int32_t c = a.elems[i64(eNL) * NEN + lane];
-                ps.nodes[lane] = c;
-                ps.inner[lane] = a.is_inner[c];
-            }
-            __syncwarp();
-            for (int t = lane; t < NQ * NQ; t += 32) {
-                const int qL = t / NQ, qNL = t % NQ;
-                ps.phi[t] = ff_mul(ps.c[qNL], shape_ff<INF>(m, ff_sub(eqx[qL], ps.qx[qNL]), ff_sub(eqy[qL], ps.qy[qNL]),
-                                                             qf, etab));
-            }
-            __syncwarp();
-            // one lane per (direction, qL, j): 2 NQ NEN dots of NQ terms fill
-            // the lanes better than NQ NEN pairs of dots (144 = 4.5 rounds of
-            // 32 against 72 = 2.25 rounds of double work for the 8-node element)
-            ff hv[HR];
-#pragma unroll
-            for (int rnd = 0; rnd < HR; ++rnd) {
-                const int t = lane + 32 * rnd;
-                if (t < HN) {
-                    const int dir = t >= NQ * NEN, u = dir ? t - NQ * NEN : t;
-                    const int qL = u / NEN, j = u % NEN;
-                    const ff* gd = ps.g + dir * NEN * NQ;
-                    ffdot d;
-#pragma unroll
-                    for (int qNL = 0; qNL < NQ; ++qNL) {
-                        const ff fq = ps.phi[qL * NQ + qNL];
-                        if (m.cond_kind != NLGPU_CONDUCTIVITY_ANISOTROPIC) {
-                            ffdot_add(d, fq, gd[j * NQ + qNL]);
-                        } else {
-                            const ff gx = ps.g[j * NQ + qNL], gy = ps.g[NEN * NQ + j * NQ + qNL];
-                            ffdot_add(d, fq, dir ? ff_add(ff_mul(k2, gx), ff_mul(k1, gy))
-                                                 : ff_add(ff_mul(k0, gx), ff_mul(k2, gy)));
-                        }
+        for (i64 k0 = kb; k0 < ke; k0 += FF_LIST) {
+            // ---- the pairs of this element: with unordered pairs, those whose key is not the smaller one's
+            for (int t = warp * 32; t < FF_LIST && k0 + t < ke; t += THREADS) {
+                const i64 k = k0 + t + lane;
+                int32_t eNL = -1;
+                bool own = k < ke;
+                if (own) {
+                    eNL = a.nlist[k];
+                    if constexpr (SYM) {   // the pair belongs to the element with the smaller key
+                        const int32_t key_n = a.minnode[eNL];
+                        own = !(key_n < key_l || (key_n == key_l && eNL < int32_t(eL)));
                     }
-                    hv[rnd] = ffdot_value(d);
-                    if (m.cond_kind == NLGPU_CONDUCTIVITY_ORTHOTROPIC) hv[rnd] = ff_mul(hv[rnd], dir ? k1 : k0);
                 }
+                const unsigned votes = __ballot_sync(0xffffffffu, own);
+                int at = 0;
+                if (lane == 0 && votes) at = atomicAdd(&listed, __popc(votes));
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (own) list[at + __popc(votes & ((1u << lane) - 1u))] = eNL;
             }
-            __syncwarp();   // every lane has read G: H (x then y, [qL][j]) replaces it
+            __syncthreads();
+            const int count = listed;
+            // ---- one group of lanes each
+            for (int n0 = warp * GROUPS; n0 < count; n0 += WARPS * GROUPS) {
+                bool active = n0 + group < count;
+                const int32_t eNL = list[min(n0 + group, count - 1)];
+                // eNL's gradients of this lane's (direction, j): used after the influence values
+                int2 g[NQ];
 #pragma unroll
-            for (int rnd = 0; rnd < HR; ++rnd)
-                if (lane + 32 * rnd < HN) ps.g[lane + 32 * rnd] = hv[rnd];
-            __syncwarp();
-            const bool self = eNL == int32_t(eL);
-            for (int t = lane; t < NEN * NEN; t += 32) {
-                const int i = t / NEN, j = t % NEN;
-                const int32_t r = enodes[i], c = ps.nodes[j];
-                const bool r_in = einner[i] != 0, c_in = ps.inner[j] != 0;
-                const bool fwd_inner = c_in && r_in && (!a.symmetric || r <= c);
-                const bool fwd_bound = !c_in && r != c;
-                const bool tr = SYM && !self;
-                const bool bwd_inner = tr && c_in && r_in && c <= r;
-                const bool bwd_bound = tr && !r_in && c != r;
-                if (!fwd_inner && !fwd_bound && !bwd_inner && !bwd_bound) continue;
-                ffdot dv;
+                for (int q = 0; q < NQ; ++q) g[q] = f.g[(i64(eNL) * NQ + q) * HL + gl % HL];
+                const int e_g = f.exps[eNL].x;
+                if (gl < NQ) ps.q[gl] = f.qcoord[i64(eNL) * NQ + gl];
+                if (gl < NEN) ps.nodes[gl] = f.nodes[i64(eNL) * NEN + gl];
+                __syncwarp();
+                ff v[PR];
+                unsigned largest = 0;
 #pragma unroll
-                for (int qL = 0; qL < NQ; ++qL) {
-                    ffdot_add(dv, ewx[i * NQ + qL], ps.g[qL * NEN + j]);
-                    ffdot_add(dv, ewy[i * NQ + qL], ps.g[NQ * NEN + qL * NEN + j]);
+                for (int rnd = 0; rnd < PR; ++rnd) {
+                    const int t = min(gl + LANES * rnd, NQ * NQ - 1);
+                    const float4 xl = eq[t / NQ], xn = ps.q[t % NQ];
+                    v[rnd] = shape_ff<INF>(m, ff_sub(ff{xl.x, xl.y}, ff{xn.x, xn.y}), ff_sub(ff{xl.z, xl.w}, ff{xn.z, xn.w}),
+                                           qf, etab);
+                    largest = max(largest, __float_as_uint(v[rnd].h) & 0x7fffffffu);
                 }
-                double v = ff_to(ffdot_value(dv));
-                if (self) {
-                    double loc = 0.0;
+#pragma unroll
+                for (int o = LANES / 2; o > 0; o >>= 1) largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, o));
+                const bool self = eNL == int32_t(eL);
+                active = active && (largest != 0 || self || e_w + e_g >= FF_BAD / 2);
+                if (!__any_sync(0xffffffffu, active)) continue;
+                const int e_p = max(int(largest >> 23) - 127, -100);
+                const float up = __int_as_float((127 + 23 - e_p) << 23);
+#pragma unroll
+                for (int rnd = 0; rnd < PR; ++rnd) {
+                    const int t = gl + LANES * rnd;
+                    const float s = __fmul_rn(v[rnd].h, up);
+                    const int hi = __float2int_rn(s);
+                    const float rest = __fmaf_rn(v[rnd].l, up, __fsub_rn(s, __int2float_rn(hi)));
+                    const int lo = __float2int_rn(__fmul_rn(rest, 268435456.0f));   // 2^28
+                    if (PR * LANES == NQ * NQ || t < NQ * NQ) ps.phi[t / NQ * PS + t % NQ] = make_int2(hi, lo);
+                }
+                __syncwarp();
+                // H(qL, j) = sum_qNL shape G: unit 2^(e_p + e_g - 55)
+#pragma unroll 1
+                for (int qL = gl / HL; qL < NQ; qL += HG) {
+                    long long s0 = 0, s1 = 1 << 23;
 #pragma unroll
                     for (int q = 0; q < NQ; ++q) {
-                        const double ax = egx[i * NQ + q], ay = egy[i * NQ + q];
-                        const double bx = egx[j * NQ + q], by = egy[j * NQ + q];
-                        double val;
-                        if (iso) val = elam[q] * (ax * bx + ay * by);
-                        else if (m.cond_kind == NLGPU_CONDUCTIVITY_ORTHOTROPIC) val = m.cond[0] * ax * bx + m.cond[1] * ay * by;
-                        else val = ax * (m.cond[0] * bx + m.cond[2] * by) + ay * (m.cond[2] * bx + m.cond[1] * by);
-                        loc += b.w[q] * val / ejac[q];
+                        const int2 p = ps.phi[qL * PS + q];
+                        s0 += (long long)p.x * g[q].x;
+                        s1 += (long long)p.x * g[q].y;
+                        s1 += (long long)p.y * g[q].x;
                     }
-                    v += m.p1 * loc;
+                    const long long h = s0 * 16 + (s1 >> 24);   // |h| < 2^61
+                    const int lo = int(h), hi = int(h >> 32) + (lo < 0 ? 1 : 0);
+                    // the low word to 28 bits, so that both cross products below have one unit
+                    reinterpret_cast<int2*>(ps.h)[(qL * NEN + gl % NEN) * 2 + gl % HL / NEN] = make_int2(hi, ((lo >> 3) + 1) >> 1);
                 }
-                if (fwd_inner) {
-                    if (smem_rows) {
-                        const i64 pos = find_col(cols, row_off[i], row_off[i + 1], c);
-                        if (pos < row_off[i + 1] && cols[pos] == c) atomicAdd(acc + pos, v);
-                        else atomicExch(a.error, 1);
-                    } else {
-                        add_global(a.in_rp, a.in_col, a.in_val, r, c, v, a.error);
+                __syncwarp();
+                // K(i, j) = sum_qL (w G_i) . H(qL, j): unit 2^(e_w + e_g + e_p - 51)
+                const int i = gl >> 2, j0 = gl & 3;
+                long long s0[OUT], s1[OUT];
+#pragma unroll
+                for (int o = 0; o < OUT; ++o) { s0[o] = 0; s1[o] = 1 << 27; }
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) {
+                    const int4 w = ew[i * NQ + q];
+#pragma unroll
+                    for (int o = 0; o < OUT; ++o) {
+                        const int4 h = ps.h[q * NEN + j0 + 4 * o];
+                        s0[o] += (long long)w.x * h.x;
+                        s0[o] += (long long)w.z * h.z;
+                        s1[o] += (long long)w.x * h.y;
+                        s1[o] += (long long)w.y * h.x;
+                        s1[o] += (long long)w.z * h.w;
+                        s1[o] += (long long)w.w * h.z;
                     }
                 }
-                if (fwd_bound) add_global(a.bd_rp, a.bd_col, a.bd_val, r, c, v, a.error);
-                if (bwd_inner) add_global(a.in_rp, a.in_col, a.in_val, c, r, v, a.error);
-                if (bwd_bound) add_global(a.bd_rp, a.bd_col, a.bd_val, c, r, v, a.error);
+                const int e_k = e_w + e_g + e_p - 51;
+                double unit = __hiloint2double((1023 + e_k) << 20, 0);
+                if (abs(e_k) > 1000 || largest >= 0x7f800000u)   // a non-finite factor, or far out of range
+                    unit = e_w + e_g >= FF_BAD / 2 || largest >= 0x7f800000u ? nan("") : scalbn(1.0, e_k);
+                const int32_t r = enodes[i];
+                const bool r_in = einner[i] != 0;
+#pragma unroll
+                for (int o = 0; o < OUT; ++o) {
+                    const int j = j0 + 4 * o;
+                    const int32_t cn = ps.nodes[j], c = cn < 0 ? ~cn : cn;
+                    const bool c_in = cn >= 0;
+                    const bool fwd_inner = active && c_in && r_in && (!a.symmetric || r <= c);
+                    const bool fwd_bound = active && !c_in && r != c;
+                    const bool tr = SYM && active && !self;
+                    const bool bwd_inner = tr && c_in && r_in && c <= r;
+                    const bool bwd_bound = tr && !r_in && c != r;
+                    double val = __ll2double_rn(s0[o] + (s1[o] >> 28)) * unit;
+                    if (self) {
+                        double loc = 0.0;
+#pragma unroll 1
+                        for (int q = 0; q < NQ; ++q) {
+                            const double ax = egx[i * NQ + q], ay = egy[i * NQ + q];
+                            const double bx = egx[j * NQ + q], by = egy[j * NQ + q];
+                            double u;
+                            if (iso) u = elam[q] * (ax * bx + ay * by);
+                            else if (m.cond_kind == NLGPU_CONDUCTIVITY_ORTHOTROPIC) u = m.cond[0] * ax * bx + m.cond[1] * ay * by;
+                            else u = ax * (m.cond[0] * bx + m.cond[2] * by) + ay * (m.cond[2] * bx + m.cond[1] * by);
+                            loc += b.w[q] * u / ejac[q];
+                        }
+                        val += m.p1 * loc;
+                    }
+                    if (fwd_inner) {
+                        if (smem_rows) {
+                            int lo = row_off[i], n = row_len[i];
+                            while (n > 1) {   // the last column <= c
+                                const int half = n >> 1;
+                                if (cols[lo + half] <= c) lo += half;
+                                n -= half;
+                            }
+                            if (n && cols[lo] == c) atomicAdd(acc + lo, val);
+                            else atomicExch(a.error, 1);
+                        } else {
+                            add_global(a.in_rp, a.in_col, a.in_val, r, c, val, a.error);
+                        }
+                    }
+                    if (fwd_bound) add_global(a.bd_rp, a.bd_col, a.bd_val, r, c, val, a.error);
+                    if (bwd_inner) add_global(a.in_rp, a.in_col, a.in_val, c, r, val, a.error);
+                    if (bwd_bound) add_global(a.bd_rp, a.bd_col, a.bd_val, c, r, val, a.error);
+                }
+                __syncwarp();
             }
-            __syncwarp();
+            __syncthreads();
+            if (threadIdx.x == 0) listed = 0;
+            __syncthreads();
         }
-        __syncthreads();
         if (smem_rows)
             for (int i = 0; i < NEN; ++i)
                 for (int t = threadIdx.x; t < row_len[i]; t += THREADS) {
@@ -564,7 +674,7 @@ void launch_pairs_ff_w(Ctx& ctx, AssembleArgs a, const FFArgs& f, bool sym) {
     NL_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     cudaFuncAttributes fa{};
     NL_CUDA(cudaFuncGetAttributes(&fa, kernel));
-    const size_t fixed = sizeof(PairFF<NEN, NQ>) * WARPS;
+    const size_t fixed = sizeof(PairFF<NEN, NQ>) * WARPS * (NQ * NQ <= 16 ? 2 : 1);
     const size_t avail = size_t(optin) - fa.sharedSizeBytes;
     NL_REQUIRE(avail > fixed + 4096, NLGPU_ERR_UNSUPPORTED, "not enough shared memory for the pair assembly");
     a.cap = int((avail - fixed) / 12);
@@ -658,13 +768,15 @@ void assemble_full(Ctx& ctx) {
     ctx.ff_assembled = ctx.ff_assembly && ff_supported(ctx.model);
     if (ctx.ff_assembled) {
         const int nen = ctx.basis.nen, nq = ctx.basis.nq;
-        ctx.deriv_ff.reserve(size_t(ctx.n_elems * nen * nq));
-        ctx.qcoord_ff.reserve(size_t(ctx.n_elems * nq));
-        ctx.cw_ff.reserve(size_t(ctx.n_elems * nq));
-        NL_LAUNCH(k_ff_stage, grid_for(ctx.n_elems * nen * nq, 256), 256, 0, ctx.stream, ctx.n_elems, nen, nq,
-                  ctx.deriv.p, ctx.qcoord.p, a.cond_field, ctx.model, ctx.basis, ctx.deriv_ff.p, ctx.qcoord_ff.p,
-                  ctx.cw_ff.p);
-        FFArgs f{ctx.deriv_ff.p, ctx.qcoord_ff.p, ctx.cw_ff.p, {}};
+        ctx.ff_qcoord.reserve(size_t(ctx.n_elems * nq));
+        ctx.ff_g.reserve(size_t(ctx.n_elems * nen * nq * 2));
+        ctx.ff_w.reserve(size_t(ctx.n_elems * nen * nq));
+        ctx.ff_exps.reserve(size_t(ctx.n_elems));
+        ctx.ff_nodes.reserve(size_t(ctx.n_elems * nen));
+        NL_LAUNCH(k_ff_stage, grid_for(ctx.n_elems * 32, 256), 256, 0, ctx.stream, ctx.n_elems, nen, nq, ctx.elems.p,
+                  ctx.is_inner.p, ctx.deriv.p, ctx.qcoord.p, a.cond_field, ctx.model, ctx.basis, ctx.ff_qcoord.p,
+                  ctx.ff_g.p, ctx.ff_w.p, ctx.ff_exps.p, ctx.ff_nodes.p);
+        FFArgs f{ctx.ff_qcoord.p, ctx.ff_g.p, ctx.ff_w.p, ctx.ff_exps.p, ctx.ff_nodes.p, {}};
         fill_exp_table(f.exp_table);
         if (nen == 4) dispatch_influence_ff<4, 4>(ctx, a, f, sym);
         else dispatch_influence_ff<8, 9>(ctx, a, f, sym);

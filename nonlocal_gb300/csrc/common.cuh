@@ -539,8 +539,11 @@ struct Ctx {
     int ff_warps_used = 0;              // ... of its last launch
     double ff_tune_ms[2] = {0.0, 0.0};  // the last tuning's sample times with 16 and 32 warps
     std::map<int, int> ff_warps_tuned;  // tuned choice per (element type, influence kind, pair mode)
-    dbuf<float4> deriv_ff, qcoord_ff;   // float-float copies: (gx, gy) / (x, y) as (hi, lo, hi, lo)
-    dbuf<float2> cw_ff;                 // w_q norm (1 - p1) [lambda_q] per element and point
+    // the float-float pair assembly's copies of the element data (FFArgs)
+    dbuf<float4> ff_qcoord;
+    dbuf<int2> ff_g, ff_exps;
+    dbuf<int4> ff_w;
+    dbuf<int32_t> ff_nodes;
     // measurement
     cudaEvent_t events[64] = {};
     dbuf<unsigned char> flush;

@@ -98,6 +98,7 @@ __device__ __forceinline__ ff ff_abs(ff a) { return a.h < 0.0f ? ff_neg(a) : a; 
 
 // x^n, n >= 0, by repeated squaring
 __device__ __forceinline__ ff ff_ipow(ff x, int n) {
+    if (n == 1) return x;
     ff r = ff_make(1.0f);
     while (n > 0) {
         if (n & 1) { r = ff_mul(r, x); --n; } else { x = ff_mul(x, x); n >>= 1; }

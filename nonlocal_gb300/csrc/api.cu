@@ -108,17 +108,25 @@ void neumann_prepare(Ctx& c) {
     add_scaled(c, -sf / sb, c.node_integral.p, c.rhs.p);
 }
 
+// the patterns of the system; the full -> upper map only where every radiation
+// step fills the full rows again
+void build_system_patterns(Ctx& c) {
+    c.full_from_upper.release();
+    build_patterns(c, !c.model.nonlocal(), c.symmetric, c.inner, &c.bound, &c.full,
+                   has_radiation(c) ? &c.full_from_upper : nullptr);
+}
+
 // conductivity_matrix_2d::compute(FULL) into inner/bound, and the solver's full rows
 void build_inner(Ctx& c) {
     NL_REQUIRE(c.mesh_ready && c.model_ready, NLGPU_ERR_STATE, "mesh and model must be set before assembly");
     ensure_boundary(c);
     c.symmetric = !(c.model.nonlocal() && c.cond_field.n);   // problem_settings::is_symmetric (problem_settings.hpp:32-34)
     if (c.model.nonlocal()) ensure_neighbours(c);
-    build_patterns(c, !c.model.nonlocal(), c.symmetric, c.inner, &c.bound, &c.full, &c.full_from_upper);
+    build_system_patterns(c);
     c.ff_assembly = c.assembly_precision == NLGPU_ASSEMBLY_FF;
     assemble_full(c);
     boundary_matrix_terms(c);
-    fill_full_from_upper(c, c.inner, c.full, c.full_from_upper);
+    fill_full_from_upper(c, c.inner, c.full, c.full_from_upper, c.symmetric);
     c.rhs.resize(size_t(c.n_nodes));
     apply_first_kind(c, c.bound, c.rhs_init.p, c.rhs.p, c.x_dirichlet.p);
     neumann_prepare(c);
@@ -309,11 +317,11 @@ CgResult radiation_loop(Ctx& c, const nlgpu_solve_options& o, nlgpu_solve_report
     while (it < c.nl_max_iterations && c.nl_tolerance < difference && c.nl_tolerance < norm) {
         NL_CUDA(cudaMemcpyAsync(c.inner.val.p, c.upper_base.p, size_t(c.inner.nnz) * sizeof(double),
                                 cudaMemcpyDeviceToDevice, c.stream));
-        fill_full_from_upper(c, c.inner, c.full, c.full_from_upper);
+        fill_full_from_upper(c, c.inner, c.full, c.full_from_upper, c.symmetric);
         spmv_full(c, c.full, prev, kt);
         NL_CUDA(cudaMemsetAsync(rad, 0, size_t(n) * sizeof(double), c.stream));
         add_radiation(c, prev, rad, -4.0, -1.0);
-        fill_full_from_upper(c, c.inner, c.full, c.full_from_upper);
+        fill_full_from_upper(c, c.inner, c.full, c.full_from_upper, c.symmetric);
         subtract3(c, kt, rad, c.rhs.p, residual);
         const CgResult r = solve_system(c, o, rep, residual, it > 0);
         total.iterations += r.iterations;
@@ -331,7 +339,7 @@ CgResult radiation_loop(Ctx& c, const nlgpu_solve_options& o, nlgpu_solve_report
     // leave the assembled matrix (conductivity and convection) in place
     NL_CUDA(cudaMemcpyAsync(c.inner.val.p, c.upper_base.p, size_t(c.inner.nnz) * sizeof(double),
                             cudaMemcpyDeviceToDevice, c.stream));
-    fill_full_from_upper(c, c.inner, c.full, c.full_from_upper);
+    fill_full_from_upper(c, c.inner, c.full, c.full_from_upper, c.symmetric);
     NL_CUDA(cudaStreamSynchronize(c.stream));
     fill_report(c, rep, total);
     if (rep) rep->nonlinear_iterations = it;
@@ -838,7 +846,7 @@ int nlgpu_stationary_2d(nlgpu_ctx* ctx, const nlgpu_solve_options* options, doub
         rep->seconds_neighbours = seconds(t0);
         t0 = std::chrono::steady_clock::now();
         c.symmetric = !(c.model.nonlocal() && c.cond_field.n);
-        build_patterns(c, !c.model.nonlocal(), c.symmetric, c.inner, &c.bound, &c.full, &c.full_from_upper);
+        build_system_patterns(c);
         // the local matrix feeds the ILLT; the non-symmetric systems' BiCGSTAB uses the diagonal
         if (c.symmetric) build_patterns(c, true, true, c.local, nullptr, nullptr, nullptr);
         NL_CUDA(cudaStreamSynchronize(c.stream));
@@ -851,7 +859,7 @@ int nlgpu_stationary_2d(nlgpu_ctx* ctx, const nlgpu_solve_options* options, doub
                         (c.assembly_precision == NLGPU_ASSEMBLY_AUTO && mixed);
         assemble_full(c);
         boundary_matrix_terms(c);
-        fill_full_from_upper(c, c.inner, c.full, c.full_from_upper);
+        fill_full_from_upper(c, c.inner, c.full, c.full_from_upper, c.symmetric);
         if (c.symmetric) {
             assemble_local(c, c.local, c.model.p1, 0);
             c.local_ready = true;
@@ -1088,17 +1096,17 @@ int nlgpu_nonstationary_2d_compute(nlgpu_ctx* ctx, double time_step, const doubl
         ensure_boundary(c);
         c.symmetric = true;
         if (c.model.nonlocal()) ensure_neighbours(c);
-        build_patterns(c, !c.model.nonlocal(), true, c.inner, &c.bound, &c.full, &c.full_from_upper);
+        build_system_patterns(c);
         c.ff_assembly = c.assembly_precision == NLGPU_ASSEMBLY_FF;
         assemble_full(c);
         boundary_matrix_terms(c);   // convection before the time-step scaling (nonstationary_heat_equation_solver_2d.hpp:74)
         c.neumann = false;
-        build_patterns(c, true, true, c.capacity_m, nullptr, &c.capacity_full, &c.capacity_map);
+        build_patterns(c, true, true, c.capacity_m, nullptr, &c.capacity_full, nullptr);
         assemble_local(c, c.capacity_m, c.capacity * c.density, 1);
-        fill_full_from_upper(c, c.capacity_m, c.capacity_full, c.capacity_map);
+        fill_full_from_upper(c, c.capacity_m, c.capacity_full, dbuf<i64>{}, true);
         c.time_step = time_step;
         combine_nonstationary(c, time_step);   // K <- dt K + C, unit Dirichlet diagonal, bound <- dt bound
-        fill_full_from_upper(c, c.inner, c.full, c.full_from_upper);
+        fill_full_from_upper(c, c.inner, c.full, c.full_from_upper, c.symmetric);
         c.temperature.resize(size_t(c.n_nodes));
         if (initial) c.temperature.upload(initial, size_t(c.n_nodes), c.stream);
         else c.temperature.zero(c.stream);
@@ -1130,7 +1138,7 @@ int nlgpu_nonstationary_2d_step(nlgpu_ctx* ctx, double dirichlet_value, const do
             c.nl_work.resize(size_t(c.n_nodes));
             c.nl_work.zero(c.stream);
             add_radiation(c, c.temperature.p, c.nl_work.p, 4.0 * c.time_step, 3.0);
-            fill_full_from_upper(c, c.inner, c.full, c.full_from_upper);
+            fill_full_from_upper(c, c.inner, c.full, c.full_from_upper, c.symmetric);
             radiation = c.nl_work.p;
         }
         nonstationary_rhs(c, dirichlet_value, dirichlet_values != nullptr, radiation);

@@ -811,10 +811,8 @@ void set_dirichlet_diagonal(Ctx& ctx, Csr& mtx, double value) {
               mtx.rowptr.p, mtx.val.p, value);
 }
 
-void fill_full_from_upper(Ctx& ctx, const Csr& upper, Csr& full, const dbuf<i64>& map) {
-    full.val.resize(size_t(full.nnz));
-    NL_LAUNCH(k_gather_full, grid_for(full.nnz, 256), 256, 0, ctx.stream, full.nnz, map.p, upper.val.p, full.val.p,
-              full.val32.n ? full.val32.p : nullptr);
+void gather_full(Ctx& ctx, Csr& full, const dbuf<i64>& map, const double* upper, float* full32) {
+    NL_LAUNCH(k_gather_full, grid_for(full.nnz, 256), 256, 0, ctx.stream, full.nnz, map.p, upper, full.val.p, full32);
 }
 
 // ---------------------------------------------------------------- nonstationary

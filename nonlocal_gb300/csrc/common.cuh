@@ -507,7 +507,7 @@ struct Ctx {
     // matrices (reference storage) and the solver's full-row copy
     bool symmetric = true;
     Csr inner, bound, local, full;
-    dbuf<i64> full_from_upper;   // full entry -> upper entry (lower part via transpose)
+    dbuf<i64> full_from_upper;   // full entry -> upper entry (lower part via transpose); kept with radiation only
     bool inner_ready = false, local_ready = false;
     IncompleteCholesky ilt;
     IncompleteCholesky plugin_ilt;   // nlgpu_illt_compute / nlgpu_illt_solve
@@ -522,7 +522,6 @@ struct Ctx {
     Mpnn mp;
     // nonstationary
     Csr capacity_m, capacity_full;
-    dbuf<i64> capacity_map;
     dbuf<double> step_tmp, step_xd;
     double time_step = 0.0;
     dbuf<double> temperature;
@@ -579,7 +578,8 @@ void full_map(Ctx& ctx, const Csr& upper, const Csr& full, dbuf<i64>& map, bool 
 // assemble.cu
 void assemble_full(Ctx& ctx);
 void assemble_local(Ctx& ctx, Csr& m, double weight, int integrand);   // integrand 0 conductivity, 1 capacity
-void fill_full_from_upper(Ctx& ctx, const Csr& upper, Csr& full, const dbuf<i64>& map);
+void fill_full_from_upper(Ctx& ctx, const Csr& upper, Csr& full, const dbuf<i64>& map, bool symmetric);
+void gather_full(Ctx& ctx, Csr& full, const dbuf<i64>& map, const double* upper, float* full32);
 void set_dirichlet_diagonal(Ctx& ctx, Csr& m, double value);
 void combine_nonstationary(Ctx& ctx, double dt);
 // f = dt (flux + source [+ radiation]) + C T_prev, then the first kind

@@ -437,7 +437,7 @@ void elastic_assemble(Ctx& ctx, bool local_part) {
                "neighbour search must run before a nonlocal assembly");
     dof_patterns(ctx, !ctx.model.nonlocal(), el.inner, &el.bound, &el.full, &el.full_from_upper);
     assemble_values(ctx, false, el.inner, &el.bound);
-    fill_full_from_upper(ctx, el.inner, el.full, el.full_from_upper);
+    fill_full_from_upper(ctx, el.inner, el.full, el.full_from_upper, true);
     // f = pressure integrals; f -= K_bound x_D, f[D] = x_D (equilibrium_equation_2d.hpp:28-33)
     el.rhs.resize(size_t(2 * ctx.n_nodes));
     apply_first_kind(ctx, el.bound, el.rhs_init.p, el.rhs.p, el.x_dirichlet.p, el.is_inner.p);

@@ -123,7 +123,8 @@ __device__ __forceinline__ void load_nodes(const int32_t* __restrict__ elems, in
 // beyond that window are expanded every time).  The set bits are then
 // classified a word at a time against the inner-node bitmap and emitted in
 // increasing order, 32 words per round with a warp scan of the counts: the
-// reference's sorted column list without a sort.
+// reference's sorted column list without a sort.  (Writing each lane's own word bit by bit, scattered stores: 300x300
+// 8-node elements, count and fill, 12.6 ms instead of 11.3.)
 template<int NEN>
 __global__ void __launch_bounds__(PW_WARPS * 32) k_pattern(PatternArgs a) {
     extern __shared__ uint32_t pw_smem[];
@@ -159,10 +160,12 @@ __global__ void __launch_bounds__(PW_WARPS * 32) k_pattern(PatternArgs a) {
             ehi = max(ehi, __shfl_xor_sync(full, ehi, o));
         }
         const bool row_inner = a.is_inner[r];
+        i64 to_inner = 0, to_bound = 0, to_full = 0;
+        if (fill) { to_inner = a.rp_inner[r]; to_bound = a.rp_bound[r]; to_full = a.rp_full[r]; }
         i64 n_inner = 0, n_bound = 0, n_full = 0;
         if (!row_inner) {   // Dirichlet row: unit diagonal only in the inner parts
             n_inner = 1; n_full = 1;
-            if (fill && lane == 0) { a.col_inner[a.rp_inner[r]] = int32_t(r); a.col_full[a.rp_full[r]] = int32_t(r); }
+            if (fill && lane == 0) { a.col_inner[to_inner] = int32_t(r); a.col_full[to_full] = int32_t(r); }
         }
         const bool dedupe = !a.local_only && ne > 1;
         const i64 elem_span = min(i64(ehi) - elo, i64(PW_EWORDS) * 32 - 1);
@@ -234,14 +237,19 @@ __global__ void __launch_bounds__(PW_WARPS * 32) k_pattern(PatternArgs a) {
                 }
                 const unsigned long long tot = __shfl_sync(full, incl, 31);
                 if (fill) {
+                    // a word at a time, a lane per bit: the stores of a word are contiguous
                     const unsigned long long ex = incl - c;
                     const unsigned long long f21 = (1ull << 21) - 1;
-                    i64 pi = a.rp_inner[r] + n_inner + i64(ex & f21);
-                    i64 pb = a.rp_bound[r] + n_bound + i64((ex >> 21) & f21);
-                    i64 pf = a.rp_full[r] + n_full + i64(ex >> 42);
-                    for (uint32_t t = mi; t; t &= t - 1) a.col_inner[pi++] = int32_t(nb + __ffs(t) - 1);
-                    for (uint32_t t = mb; t; t &= t - 1) a.col_bound[pb++] = int32_t(nb + __ffs(t) - 1);
-                    for (uint32_t t = mf; t; t &= t - 1) a.col_full[pf++] = int32_t(nb + __ffs(t) - 1);
+                    const uint32_t before = (1u << lane) - 1u;
+                    for (unsigned words = __ballot_sync(full, (mi | mb | mf) != 0u); words; words &= words - 1) {
+                        const int s = __ffs(words) - 1;
+                        const uint32_t wi = __shfl_sync(full, mi, s), wb = __shfl_sync(full, mb, s), wf = __shfl_sync(full, mf, s);
+                        const unsigned long long at = __shfl_sync(full, ex, s);
+                        const int32_t node = int32_t(base + i64(w0 + s) * 32 + lane);
+                        if (wi >> lane & 1u) a.col_inner[to_inner + n_inner + i64(at & f21) + __popc(wi & before)] = node;
+                        if (wb >> lane & 1u) a.col_bound[to_bound + n_bound + i64((at >> 21) & f21) + __popc(wb & before)] = node;
+                        if (wf >> lane & 1u) a.col_full[to_full + n_full + i64(at >> 42) + __popc(wf & before)] = node;
+                    }
                 }
                 n_inner += i64(tot & ((1ull << 21) - 1));
                 n_bound += i64((tot >> 21) & ((1ull << 21) - 1));
@@ -253,7 +261,7 @@ __global__ void __launch_bounds__(PW_WARPS * 32) k_pattern(PatternArgs a) {
             if (lane == 0) { a.cnt_inner[r] = n_inner; a.cnt_bound[r] = n_bound; a.cnt_full[r] = (n_full + 3) & ~i64(3); }
         } else {   // pad the solver row to a multiple of 4 with (r, 0) entries
             const i64 end = a.rp_full[r + 1];
-            for (i64 k = a.rp_full[r] + n_full + lane; k < end; k += 32) a.col_full[k] = int32_t(r);
+            for (i64 k = to_full + n_full + lane; k < end; k += 32) a.col_full[k] = int32_t(r);
         }
     }
 }
@@ -270,32 +278,149 @@ void launch_pattern(Ctx& ctx, int nen, unsigned grid, const PatternArgs& a) {
     }
 }
 
+// the index in the upper storage of entry k of full row r (-1 for padding)
+__device__ __forceinline__ i64 upper_entry(const i64* __restrict__ up_rp, const int32_t* __restrict__ up_col, i64 fb,
+                                           const int32_t* __restrict__ full_col, i64 r, i64 k, bool symmetric) {
+    const int32_t c = full_col[k];
+    // real entries are strictly increasing; padding (col r) breaks the order
+    if (k > fb && c <= full_col[k - 1]) return -1;
+    const bool own = !symmetric || c >= int32_t(r);   // c in row r, or (transpose) r in row c
+    const i64 b = own ? up_rp[r] : up_rp[c], e = own ? up_rp[r + 1] : up_rp[c + 1];
+    const int32_t want = own ? c : int32_t(r);
+    i64 lo = b, hi = e;
+    while (lo < hi) { const i64 mid = (lo + hi) >> 1; if (up_col[mid] < want) lo = mid + 1; else hi = mid; }
+    return (lo < e && up_col[lo] == want) ? lo : -1;
+}
+
 // full-row entry -> index of the same value in the upper storage (or -1 for padding)
 __global__ void k_full_map(i64 n, const i64* __restrict__ up_rp, const int32_t* __restrict__ up_col,
-                           const i64* __restrict__ full_rp, const int32_t* __restrict__ full_col,
-                           const uint8_t* __restrict__ is_inner, bool symmetric, i64* __restrict__ map) {
+                           const i64* __restrict__ full_rp, const int32_t* __restrict__ full_col, bool symmetric,
+                           i64* __restrict__ map) {
+    const int lane = threadIdx.x & 31;
+    const i64 warps = i64(gridDim.x) * (blockDim.x >> 5);
+    for (i64 r = (blockIdx.x * i64(blockDim.x) + threadIdx.x) >> 5; r < n; r += warps)
+        for (i64 k = full_rp[r] + lane; k < full_rp[r + 1]; k += 32)
+            map[k] = upper_entry(up_rp, up_col, full_rp[r], full_col, r, k, symmetric);
+}
+
+// The full rows' values straight from the upper storage, where no map is kept:
+// a search per entry (short rows) ...
+__global__ void k_full_search(i64 n, const i64* __restrict__ up_rp, const int32_t* __restrict__ up_col,
+                              const double* __restrict__ up_val, const i64* __restrict__ full_rp,
+                              const int32_t* __restrict__ full_col, double* __restrict__ full_val,
+                              float* __restrict__ full32) {
+    const int lane = threadIdx.x & 31;
+    const i64 warps = i64(gridDim.x) * (blockDim.x >> 5);
+    for (i64 r = (blockIdx.x * i64(blockDim.x) + threadIdx.x) >> 5; r < n; r += warps)
+        for (i64 k = full_rp[r] + lane; k < full_rp[r + 1]; k += 32) {
+            const i64 at = upper_entry(up_rp, up_col, full_rp[r], full_col, r, k, true);
+            const double v = at >= 0 ? up_val[at] : 0.0;
+            full_val[k] = v;
+            if (full32) full32[k] = float(v);
+        }
+}
+
+// ... or the entries right of the diagonal copied as they lie and the padding after
+// them cleared (a warp per row; without symmetry the whole row) ...
+__global__ void k_full_upper(i64 n, const i64* __restrict__ up_rp, const double* __restrict__ up_val,
+                             const i64* __restrict__ full_rp, const int32_t* __restrict__ full_col, bool symmetric,
+                             double* __restrict__ full_val, float* __restrict__ full32) {
     const int lane = threadIdx.x & 31;
     const i64 warps = i64(gridDim.x) * (blockDim.x >> 5);
     for (i64 r = (blockIdx.x * i64(blockDim.x) + threadIdx.x) >> 5; r < n; r += warps) {
-        const i64 fb = full_rp[r], fe = full_rp[r + 1];
-        const i64 ub = up_rp[r], ue = up_rp[r + 1];
-        for (i64 k = fb + lane; k < fe; k += 32) {
-            const int32_t c = full_col[k];
-            i64 target = -1;
-            // real entries are strictly increasing; padding (col r) breaks the order
-            if (k > fb && c <= full_col[k - 1]) target = -1;
-            else if (!symmetric || c >= int32_t(r)) {
-                i64 lo = ub, hi = ue;   // search c in row r
-                while (lo < hi) { const i64 mid = (lo + hi) >> 1; if (up_col[mid] < c) lo = mid + 1; else hi = mid; }
-                target = (lo < ue && up_col[lo] == c) ? lo : -1;
-            } else {
-                i64 lo = up_rp[c], hi = up_rp[c + 1];   // transpose: search r in row c
-                while (lo < hi) { const i64 mid = (lo + hi) >> 1; if (up_col[mid] < int32_t(r)) lo = mid + 1; else hi = mid; }
-                target = (lo < up_rp[c + 1] && up_col[lo] == int32_t(r)) ? lo : -1;
-            }
-            map[k] = target;
+        const i64 ub = up_rp[r], fe = full_rp[r + 1];
+        const i64 len = up_rp[r + 1] - ub;
+        i64 lo = full_rp[r];
+        if (symmetric) {   // the diagonal: the first column not left of it
+            i64 hi = fe;
+            while (lo < hi) { const i64 mid = (lo + hi) >> 1; if (full_col[mid] < int32_t(r)) lo = mid + 1; else hi = mid; }
         }
-        (void)is_inner;
+        for (i64 k = lane; lo + k < fe; k += 32) {
+            const double v = k < len ? up_val[ub + k] : 0.0;
+            full_val[lo + k] = v;
+            if (full32) full32[lo + k] = float(v);
+        }
+    }
+}
+
+// ... and the transposed ones left of it: a warp takes `rows` consecutive rows c of the
+// upper storage and moves along them a tile of 32 columns r at a time, lane r keeping
+// its place in full row r.  A row's entries in the tile are read together
+// (FL_AHEAD rows in flight) and reach their lanes by shuffles; no entry is searched
+// for, a tile costs one search per lane.  A search per entry, a map of 8 bytes each
+// and a gather through it took 15.7 ms on 745 million entries; this takes 8.0 (9.4
+// with four rows in flight, 9.2 through a tile of shared memory written
+// row by row), clearing and k_full_upper 3.  What bounds it is the
+// 8-byte stores, one line each.  Full entries that no upper entry matches stay
+// 0 (the caller has cleared them).
+constexpr int FL_AHEAD = 8;
+__global__ void __launch_bounds__(256) k_full_lower(i64 n, int rows, const i64* __restrict__ up_rp,
+                                                    const int32_t* __restrict__ up_col,
+                                                    const double* __restrict__ up_val, const i64* __restrict__ full_rp,
+                                                    const int32_t* __restrict__ full_col, double* __restrict__ full_val,
+                                                    float* __restrict__ full32) {
+    const unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const i64 warps = i64(gridDim.x) * (blockDim.x >> 5);
+    for (i64 c0 = ((blockIdx.x * i64(blockDim.x) + threadIdx.x) >> 5) * rows; c0 < n; c0 += warps * rows) {
+        const i64 base = up_rp[c0];
+        // row c0 + lane: its next entry's place (from `base`), its end, and that entry's column
+        int at = 0, end = 0, next = 0x7fffffff;
+        if (lane < rows && c0 + lane < n) {
+            at = int(up_rp[c0 + lane] - base);
+            end = int(up_rp[c0 + lane + 1] - base);
+            if (at < end && up_col[base + at] == int32_t(c0 + lane)) ++at;   // the diagonal
+            if (at < end) next = up_col[base + at];
+        }
+        for (;;) {
+            const int r0 = __reduce_min_sync(all, next);
+            if (r0 == 0x7fffffff) break;
+            const i64 r = i64(r0) + lane;
+            i64 pos = 0;
+            int32_t cur = 0x7fffffff;
+            if (r < n) {   // the first entry of full row r from column c0 on (c0 < r: left of the diagonal or at it)
+                i64 lo = full_rp[r], hi = full_rp[r + 1];
+                const i64 row_end = hi;
+                while (lo < hi) { const i64 mid = (lo + hi) >> 1; if (full_col[mid] < int32_t(c0)) lo = mid + 1; else hi = mid; }
+                pos = lo;
+                if (lo < row_end) cur = full_col[lo];
+            }
+            for (unsigned todo = __ballot_sync(all, next - r0 < 32); todo;) {
+                int b[FL_AHEAD];
+                int32_t col[FL_AHEAD];
+                double v[FL_AHEAD];
+#pragma unroll
+                for (int u = 0; u < FL_AHEAD; ++u) {
+                    b[u] = todo ? __ffs(todo) - 1 : -1;
+                    todo &= todo - 1;
+                    const int from = __shfl_sync(all, at, b[u] & 31), to = __shfl_sync(all, end, b[u] & 31);
+                    const bool in = b[u] >= 0 && from + lane < to;
+                    col[u] = in ? up_col[base + from + lane] : 0x7fffffff;
+                    v[u] = in ? up_val[base + from + lane] : 0.0;
+                }
+#pragma unroll
+                for (int u = 0; u < FL_AHEAD; ++u) {
+                    if (b[u] < 0) break;
+                    const unsigned present = __reduce_or_sync(all, col[u] - r0 < 32 ? 1u << (col[u] - r0) : 0u);
+                    const int count = __popc(present);
+                    const double mine = __shfl_sync(all, v[u], __popc(present & ((1u << lane) - 1u)) & 31);
+                    if (present >> lane & 1u) {
+                        const int32_t c = int32_t(c0) + b[u];
+                        while (cur < c) cur = full_col[++pos];   // ends at the diagonal at the latest
+                        if (cur == c) {
+                            full_val[pos] = mine;
+                            if (full32) full32[pos] = float(mine);
+                            cur = full_col[++pos];
+                        }
+                    }
+                    const int32_t after = __shfl_sync(all, col[u], count & 31);
+                    if (lane == b[u]) {
+                        at += count;
+                        next = count < 32 ? after : at < end ? up_col[base + at] : 0x7fffffff;
+                    }
+                }
+            }
+        }
     }
 }
 
@@ -304,7 +429,36 @@ __global__ void k_full_map(i64 n, const i64* __restrict__ up_rp, const int32_t* 
 void full_map(Ctx& ctx, const Csr& upper, const Csr& full, dbuf<i64>& map, bool symmetric) {
     map.resize(size_t(full.nnz));
     NL_LAUNCH(k_full_map, grid_for(full.rows * 32, 256, 152 * 64), 256, 0, ctx.stream, full.rows, upper.rowptr.p,
-              upper.col.p, full.rowptr.p, full.col.p, static_cast<const uint8_t*>(nullptr), symmetric, map.p);
+              upper.col.p, full.rowptr.p, full.col.p, symmetric, map.p);
+}
+
+// The values of the full rows from the upper storage: through the map where one
+// was built (matrices that are filled again and again: radiation, the elasticity
+// systems), straight otherwise; rows of a non-symmetric system are copied.  Below 1024 entries a row on average a search per
+// entry is as fast as the tiles of k_full_lower (200 x 200 4-node, 350 entries: 0.22 ms
+// both; 71 x 53 8-node: 0.10) and faster on the smallest; the rows per warp are
+// as many as leave every SM 32 warps.
+void fill_full_from_upper(Ctx& ctx, const Csr& upper, Csr& full, const dbuf<i64>& map, bool symmetric) {
+    full.val.resize(size_t(full.nnz));
+    float* val32 = full.val32.n == size_t(full.nnz) ? full.val32.p : nullptr;
+    const i64 n = full.rows;
+    if (map.n == size_t(full.nnz)) {
+        gather_full(ctx, full, map, upper.val.p, val32);
+    } else if (!symmetric) {
+        NL_LAUNCH(k_full_upper, grid_for(n * 32, 256, 152 * 64), 256, 0, ctx.stream, n, upper.rowptr.p, upper.val.p,
+                  full.rowptr.p, full.col.p, false, full.val.p, val32);
+    } else if (full.nnz < 1024 * n) {
+        NL_LAUNCH(k_full_search, grid_for(n * 32, 256, 152 * 64), 256, 0, ctx.stream, n, upper.rowptr.p, upper.col.p,
+                  upper.val.p, full.rowptr.p, full.col.p, full.val.p, val32);
+    } else {
+        full.val.zero(ctx.stream);
+        if (val32) full.val32.zero(ctx.stream);
+        NL_LAUNCH(k_full_upper, grid_for(n * 32, 256, 152 * 64), 256, 0, ctx.stream, n, upper.rowptr.p, upper.val.p,
+                  full.rowptr.p, full.col.p, true, full.val.p, val32);
+        const int rows = int(std::max<i64>(1, std::min<i64>(32, n / (152 * 32))));
+        NL_LAUNCH(k_full_lower, grid_for((n + rows - 1) / rows * 32, 256, 152 * 64), 256, 0, ctx.stream, n, rows,
+                  upper.rowptr.p, upper.col.p, upper.val.p, full.rowptr.p, full.col.p, full.val.p, val32);
+    }
 }
 
 void build_patterns(Ctx& ctx, bool local_only, bool symmetric, Csr& inner, Csr* bound, Csr* full,
@@ -362,9 +516,7 @@ void build_patterns(Ctx& ctx, bool local_only, bool symmetric, Csr& inner, Csr* 
     inner.val.resize(size_t(nnz_i)); inner.val.zero(ctx.stream);
     B.val.resize(size_t(nnz_b)); B.val.zero(ctx.stream);
     if (full && full_from_upper) {
-        full_from_upper->resize(size_t(nnz_f));
-        NL_LAUNCH(k_full_map, grid_for(n * 32, 256, 152 * 64), 256, 0, ctx.stream, n, inner.rowptr.p, inner.col.p,
-                  F.rowptr.p, F.col.p, a.is_inner, symmetric, full_from_upper->p);
+        full_map(ctx, inner, F, *full_from_upper, symmetric);
         F.val.resize(size_t(nnz_f));
     }
     NL_CUDA(cudaStreamSynchronize(ctx.stream));

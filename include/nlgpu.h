@@ -553,25 +553,30 @@ int nlgpu_nonstationary_1d_temperature(nlgpu_ctx* ctx, double* temperature);
  * sweeps, 6 FP32 ILLT application with the Jacobi sweeps of the last mixed
  * solve (NLGPU_DEFAULT_TRIANGULAR_SWEEPS before any), 7 pair assembly in
  * float-float (stage 1 is the FP64 one), 8 nodal flux of the last solution. */
-/* Options of a context: NLGPU_OPTION_GLOBAL_SWEEPS = 1 makes the ILLT
- * triangular sweeps read and write their values in global memory instead of
- * the TMA-fed shared-memory ring (same arithmetic); NLGPU_OPTION_ORDERED_PAIRS
+/* Options of a context: NLGPU_OPTION_GLOBAL_SWEEPS = 1 makes the FP64 CG run
+ * launch by launch with exact ILLT triangular sweeps, whose values are in
+ * global memory, instead of as one kernel with Jacobi sweeps; NLGPU_OPTION_ORDERED_PAIRS
  * = 1 makes a symmetric assembly evaluate every ordered element pair instead
  * of each unordered pair once (both for comparison).
  * NLGPU_OPTION_ASSEMBLY_PRECISION selects how the nonlocal pair blocks are
- * computed: NLGPU_ASSEMBLY_AUTO (default) in float-float on the FP32 pipes for
- * a mixed-precision stationary solve and in FP64 otherwise, NLGPU_ASSEMBLY_FF
- * always in float-float, NLGPU_ASSEMBLY_FP64 always in FP64.  Float-float
- * (about 48 significant bits) applies to the fast-polynomial, polynomial and
- * exponential influence with constant conductivity; other models use FP64.
+ * computed: NLGPU_ASSEMBLY_AUTO (default) in float-float or fixed point on the
+ * FP32 and integer pipes for a mixed-precision stationary solve and to FP64's
+ * accuracy otherwise (58 to 60-bit fixed point where it covers the model, else
+ * FP64), NLGPU_ASSEMBLY_FF always as for a mixed-precision solve,
+ * NLGPU_ASSEMBLY_FP64 always in FP64 operations.  Float-float (about 48
+ * significant bits) covers the fast-polynomial, polynomial and exponential
+ * influence with integral p / n, fixed point those with n = 2 (polynomials of
+ * even p and q <= 16, exponentials of p = 2 and 0.333 <= q <= 16); other models
+ * use FP64.
  * NLGPU_OPTION_FP32_SYMMETRIC = 1 makes the mixed solve's FP32 SpMV read only
  * the strictly upper part of a symmetric solver matrix (half the entries,
  * transposed contributions added with shared-memory atomics) instead of its
  * full rows (the default; for comparison).
  * NLGPU_OPTION_ASSEMBLY_WARPS sets the warps per CTA of the float-float pair
  * assembly: 16 or 32, or 0 (default) to time both on a sample of elements at
- * the first float-float assembly of each (element type, influence kind, pair
- * mode) and keep the faster; nlgpu_assembly_tuning reports the choice. */
+ * the first such assembly of each (element type, influence kind, pair mode)
+ * and keep the faster (32 without timing below 9 728 elements);
+ * nlgpu_assembly_tuning reports the choice. */
 enum { NLGPU_OPTION_GLOBAL_SWEEPS = 0, NLGPU_OPTION_ORDERED_PAIRS = 1, NLGPU_OPTION_ASSEMBLY_PRECISION = 2,
        NLGPU_OPTION_FP32_SYMMETRIC = 3, NLGPU_OPTION_ASSEMBLY_WARPS = 4 };
 enum { NLGPU_ASSEMBLY_AUTO = 0, NLGPU_ASSEMBLY_FF = 1, NLGPU_ASSEMBLY_FP64 = 2 };

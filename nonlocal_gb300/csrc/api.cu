@@ -124,6 +124,7 @@ void build_inner(Ctx& c) {
     if (c.model.nonlocal()) ensure_neighbours(c);
     build_system_patterns(c);
     c.ff_assembly = c.assembly_precision == NLGPU_ASSEMBLY_FF;
+    c.fx_assembly = c.assembly_precision != NLGPU_ASSEMBLY_FP64;
     assemble_full(c);
     boundary_matrix_terms(c);
     fill_full_from_upper(c, c.inner, c.full, c.full_from_upper, c.symmetric);
@@ -857,6 +858,7 @@ int nlgpu_stationary_2d(nlgpu_ctx* ctx, const nlgpu_solve_options* options, doub
                            options->preconditioner == NLGPU_PRECONDITIONER_ILLT_LEARNED;
         c.ff_assembly = c.assembly_precision == NLGPU_ASSEMBLY_FF ||
                         (c.assembly_precision == NLGPU_ASSEMBLY_AUTO && mixed);
+        c.fx_assembly = c.assembly_precision != NLGPU_ASSEMBLY_FP64;
         assemble_full(c);
         boundary_matrix_terms(c);
         fill_full_from_upper(c, c.inner, c.full, c.full_from_upper, c.symmetric);
@@ -1098,6 +1100,7 @@ int nlgpu_nonstationary_2d_compute(nlgpu_ctx* ctx, double time_step, const doubl
         if (c.model.nonlocal()) ensure_neighbours(c);
         build_system_patterns(c);
         c.ff_assembly = c.assembly_precision == NLGPU_ASSEMBLY_FF;
+        c.fx_assembly = c.assembly_precision != NLGPU_ASSEMBLY_FP64;
         assemble_full(c);
         boundary_matrix_terms(c);   // convection before the time-step scaling (nonstationary_heat_equation_solver_2d.hpp:74)
         c.neumann = false;
@@ -1484,8 +1487,8 @@ int nlgpu_time_stage(nlgpu_ctx* ctx, int stage, int reps, double* ms) {
             if (c.model.nonlocal()) ensure_neighbours(c);
             flux_x.resize(size_t(c.n_nodes)); flux_y.resize(size_t(c.n_nodes));
         }
-        const bool ff_before = c.ff_assembly;
-        if (stage == 1 || stage == 7) c.ff_assembly = stage == 7;
+        const bool ff_before = c.ff_assembly, fx_before = c.fx_assembly;
+        if (stage == 1 || stage == 7) { c.ff_assembly = stage == 7; c.fx_assembly = false; }
         if (stage == 0 || stage == 2 || (stage >= 4 && stage <= 6)) {
             NL_REQUIRE(c.full.nnz > 0, NLGPU_ERR_STATE, "assemble the system first");
             x.resize(size_t(c.n_nodes)); y.resize(size_t(c.n_nodes));
@@ -1517,6 +1520,7 @@ int nlgpu_time_stage(nlgpu_ctx* ctx, int stage, int reps, double* ms) {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         c.ff_assembly = ff_before;
+        c.fx_assembly = fx_before;
         *ms = double(f) / reps;
     });
 }

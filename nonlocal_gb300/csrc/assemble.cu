@@ -232,26 +232,29 @@ __global__ void __launch_bounds__(AS_THREADS) k_assemble_pairs(AssembleArgs a, M
     }
 }
 
-// ---------------------------------------------------------------- float-float
-// The same pair blocks with the influence values in float-float arithmetic
-// (ff.cuh, about 48 bits) on the FP32 pipes and both contractions in fixed point
-// on the integer multipliers.  Everything a block multiplies lies within a few
-// binary orders of its largest factor, so eNL's gradients carry one exponent per
-// element and the influence values one per pair; a number is then 53 to 57 bits in
-// two signed words (hi 2^28 + lo), a multiply-add three 32 x 32 + 64-bit ones
-// (hi hi, and hi lo + lo hi into a second accumulator; lo lo lies below the result's
-// last bit), and the sums are exact.  Against the compensated float-float dot
-// product (12 FP32 instructions a term, errors of order 2^-48) that is a quarter of
-// the instructions, half the pipe time (64 lanes a clock against 128) and an error
-// of 2^-51 of the block's scale: the float-float influence values remain the only
-// rounding.  Weights, Lambda and the constant factors are folded into the two staged
-// copies of the gradients (k_ff_stage), the pairs this element owns are listed once
-// per element, and a pair whose influence is zero everywhere ends there.
+// ---------------------------------------------------- float-float, fixed point
+// The same pair blocks off the FP64 pipe: the influence values in fixed point
+// (influence_ff.cuh, 60 bits) or float-float (ff.cuh, about 48 bits, for exponents that
+// the former does not cover), both contractions in fixed point on the integer
+// multipliers.  Everything a block multiplies lies within a few binary orders of its
+// largest factor, so eNL's gradients carry one exponent per element and the
+// exponential's values one per pair; a number is then up to 61 bits in two signed
+// words (hi 2^30 + lo), a multiply-add three 32 x 32 + 64-bit ones (hi hi, and
+// hi lo + lo hi into a second accumulator; lo lo lies below the result's last bit),
+// and the sums are exact.  Against the compensated float-float dot product (12
+// FP32 instructions a term, errors of order 2^-48) that is a quarter of the
+// instructions and half the pipe time (64 lanes a clock against 128); the gradients'
+// 58 bits leave an error below FP64's (against extended precision, entries' median
+// 2.4e-14 for the FP64 kernel's 3.4e-14 on 8-node meshes, with cancellation).
+// Weights, Lambda and the constant factors are folded into the two staged copies
+// of the gradients (k_ff_stage), the pairs this element owns are listed once per
+// element, and a pair whose influence is zero everywhere ends there.
 // 8-node 300 x 300 elements, exponential influence: 116.9 ms with the compensated
 // dots, 76.5 with fixed point; 4-node 200 x 200: 7.4 and 4.2; 17.9 million listed
 // 8-node pairs: 24.1 and 13.2 G instructions, 28.0 and 18.6 ms.  What bounds it
-// now: issue (57 % of the slots, FMA-heavy pipe 55 %, shared-memory wavefronts
-// 52 %), the influence values being the largest part.
+// now: issue, with no part that stands out (the scatter 15 %, the influence values
+// 20, H 4, K 10, a CTA's rows 7); a column bitmap instead of the scatter's binary
+// search costs as much as it saves.
 // 16 or 32 warps per CTA (the FP64 kernel's 8 leave the pipes idle), chosen per
 // problem by timing both on a sample of elements; a warp takes one 8-node pair or
 // two 4-node pairs at a time (16 lanes cover a 4 x 4 block).
@@ -260,24 +263,52 @@ constexpr int FF_BAD = 1 << 20;   // exponent of an element with a non-finite va
 constexpr int FF_LIST = 1024;     // candidates listed at a time
 
 struct FFArgs {
-    const float4* qcoord;   // [e][q]: (x/r0 .h, .l, y/r1 .h, .l), coordinates in units of the radii
-    const int2* g;          // [e][q][x, y][j]: w_q norm (1 - p1) [lambda_q] Lambda G_j 2^(56 - exps.x) as hi 2^28 + lo
-    const int4* w;          // [e][i][q]: w_q G_i 2^(56 - exps.y), (x hi, lo, y hi, lo)
+    const int4* qcoord;     // [e][q]: coordinates in units of the radii, (x/r0 .h, .l, y/r1 .h, .l) or fixed point
+    const unsigned long long* extent;   // fixed point: the largest |coordinate|, as the bits of a double
+    const int2* g;          // [e][q][x, y][j]: w_q norm (1 - p1) [lambda_q] Lambda G_j 2^(57 - exps.x) as hi 2^30 + lo
+    const int4* w;          // [e][i][q]: w_q G_i 2^(57 - exps.y), (x hi, lo, y hi, lo)
     const int2* exps;       // [e]: the exponents of the largest |g| and |w|
     const int32_t* nodes;   // [e][j]: the node, its complement where it is not inner
-    FFExpTable exp_table;   // exp(k / 256), copied to shared memory by each CTA
+    // the exponential's tables, copied to shared memory by each CTA
+    FFExpTable ff_table;    // exp(k / 256)
+    FXExpTable fx_table;    // 2^(-k / 256)
+    FXExp fx_exp;
 };
 
+__device__ __forceinline__ int fx_exponent(const unsigned long long* extent) {
+    const double x = __longlong_as_double((long long)*extent);
+    return x >= 8.0 ? ilogb(x) : 2;
+}
+
+// the largest finite |coordinate| in units of the radii
+__global__ void k_fx_extent(i64 n, const double* __restrict__ qcoord, double ix, double iy,
+                            unsigned long long* __restrict__ extent) {
+    unsigned long long m = 0ull;
+    for (i64 t = blockIdx.x * i64(blockDim.x) + threadIdx.x; t < n; t += i64(gridDim.x) * blockDim.x) {
+        const double x = fabs(qcoord[2 * t] * ix), y = fabs(qcoord[2 * t + 1] * iy);
+        if (isfinite(x)) m = max(m, (unsigned long long)__double_as_longlong(x));
+        if (isfinite(y)) m = max(m, (unsigned long long)__double_as_longlong(y));
+    }
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(extent, m);
+}
+
+// x 2^(57 - e), |x| < 2^(e + 1), by integer operations (the FP64 pipe's conversions made the staging 0.19 ms
+// on 200 x 200 elements)
 __device__ __forceinline__ int2 ff_fixed(double x, int e) {
-    const long long z = __double2ll_rn(scalbn(x, 56 - e));   // |z| < 2^57
-    const long long hi = (z + (1 << 27)) >> 28;
-    return make_int2(int(hi), int(z - hi * (1 << 28)));
+    const long long b = __double_as_longlong(x);
+    const int ex = int(b >> 52 & 0x7ff);
+    const long long m = (b & 0xfffffffffffffll) | (1ll << 52);
+    const int s = ex - 1018 - e;
+    const long long z = ex == 0 || s < -53 ? 0 : s >= 0 ? m << min(s, 5) : (m + (1ll << (-s - 1))) >> -s;
+    return fx_split(b < 0 ? -z : z);
 }
 
 // one warp per element
 __global__ void k_ff_stage(i64 E, int nen, int nq, const int32_t* __restrict__ elems, const uint8_t* __restrict__ is_inner,
                            const double* __restrict__ deriv, const double* __restrict__ qcoord,
-                           const double* __restrict__ cond_field, Model m, Basis b, float4* __restrict__ qff,
+                           const double* __restrict__ cond_field, Model m, Basis b,
+                           const unsigned long long* __restrict__ extent, int4* __restrict__ qff,
                            int2* __restrict__ g, int4* __restrict__ w, int2* __restrict__ exps,
                            int32_t* __restrict__ nodes) {
     const double cnl = m.norm * (1.0 - m.p1);
@@ -297,23 +328,37 @@ __global__ void k_ff_stage(i64 E, int nen, int nq, const int32_t* __restrict__ e
         v[2] = b.w[q] * gx; v[3] = b.w[q] * gy;
     };
     for (i64 e = (blockIdx.x * i64(blockDim.x) + threadIdx.x) / 32; e < E; e += i64(gridDim.x) * blockDim.x / 32) {
-        double mg = 0.0, mw = 0.0;
-        bool bad_g = false, bad_w = false;
+        // the high words of the largest magnitudes
+        unsigned mg = 0u, mw = 0u;
         for (int t = lane; t < nen * nq; t += 32) {
             double v[4];
             values(e, t, v);
-            mg = fmax(mg, fmax(fabs(v[0]), fabs(v[1])));
-            mw = fmax(mw, fmax(fabs(v[2]), fabs(v[3])));
-            bad_g = bad_g || !isfinite(v[0]) || !isfinite(v[1]);
-            bad_w = bad_w || !isfinite(v[2]) || !isfinite(v[3]);
+            auto high = [](double x) { return unsigned(__double2hiint(x)) & 0x7fffffffu; };
+            mg = max(mg, max(high(v[0]), high(v[1])));
+            mw = max(mw, max(high(v[2]), high(v[3])));
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            mg = fmax(mg, __shfl_xor_sync(0xffffffffu, mg, o));
-            mw = fmax(mw, __shfl_xor_sync(0xffffffffu, mw, o));
+        mg = __reduce_max_sync(0xffffffffu, mg);
+        mw = __reduce_max_sync(0xffffffffu, mw);
+        bool bad_g = mg >= 0x7ff00000u, bad_w = mw >= 0x7ff00000u;
+        if (lane < nq) {
+            const double x = qcoord[2 * (e * nq + lane)], y = qcoord[2 * (e * nq + lane) + 1];
+            if (extent) {   // fixed point has no NaN: the element's blocks become one
+                const bool finite = isfinite(x * m.inv_r[0]) && isfinite(y * m.inv_r[1]);
+                const int ex = fx_exponent(extent);
+                const int2 fx = fx_coordinate(finite ? x : 0.0, m.inv_r[0], ex);
+                const int2 fy = fx_coordinate(finite ? y : 0.0, m.inv_r[1], ex);
+                qff[e * nq + lane] = make_int4(fx.x, fx.y, fy.x, fy.y);
+                bad_g = bad_g || !finite;
+                bad_w = bad_w || !finite;
+            } else {
+                const ff fx = ff_from(x * m.inv_r[0]), fy = ff_from(y * m.inv_r[1]);
+                qff[e * nq + lane] = make_int4(__float_as_int(fx.h), __float_as_int(fx.l), __float_as_int(fy.h),
+                                               __float_as_int(fy.l));
+            }
         }
         bad_g = __any_sync(0xffffffffu, bad_g);
         bad_w = __any_sync(0xffffffffu, bad_w);
-        const int eg = bad_g ? FF_BAD : mg > 0.0 ? ilogb(mg) : 0, ew = bad_w ? FF_BAD : mw > 0.0 ? ilogb(mw) : 0;
+        const int eg = bad_g ? FF_BAD : mg ? int(mg >> 20) - 1023 : 0, ew = bad_w ? FF_BAD : mw ? int(mw >> 20) - 1023 : 0;
         if (lane == 0) exps[e] = make_int2(eg, ew);
         for (int t = lane; t < nen * nq; t += 32) {
             double v[4];
@@ -326,11 +371,6 @@ __global__ void k_ff_stage(i64 E, int nen, int nq, const int32_t* __restrict__ e
             const int2 x = ff_fixed(v[2], ew), y = ff_fixed(v[3], ew);
             w[e * nen * nq + t] = make_int4(x.x, x.y, y.x, y.y);
         }
-        if (lane < nq) {
-            const ff x = ff_from(qcoord[2 * (e * nq + lane)] * m.inv_r[0]);
-            const ff y = ff_from(qcoord[2 * (e * nq + lane) + 1] * m.inv_r[1]);
-            qff[e * nq + lane] = make_float4(x.h, x.l, y.h, y.l);
-        }
         if (lane < nen) {
             const int32_t r = elems[e * nen + lane];
             nodes[e * nen + lane] = is_inner[r] ? r : ~r;
@@ -342,13 +382,13 @@ __global__ void k_ff_stage(i64 E, int nen, int nq, const int32_t* __restrict__ e
 template<int NEN, int NQ>
 struct PairFF {
     static constexpr int PS = (NQ + 1) / 2 * 2;   // influence values per row, padded to whole 16 bytes
-    float4 q[NQ];         // eNL's points
-    int2 phi[NQ * PS];    // shape(qL, qNL) 2^(51 - ep), ep the exponent of the pair's largest
+    int4 q[NQ];           // eNL's points
+    int2 phi[NQ * PS];    // shape(qL, qNL) 2^(60 - e_p), e_p an exponent of the pair
     int4 h[NQ * NEN];     // H(qL, j): (x hi, lo, y hi, lo)
     int32_t nodes[NEN];
 };
 
-template<int NEN, int NQ, int INF, bool SYM, int WARPS>
+template<int NEN, int NQ, int INF, bool SYM, int WARPS, bool FIX>
 __global__ void __launch_bounds__(WARPS * 32) k_assemble_pairs_ff(AssembleArgs a, FFArgs f, Model m, Basis b) {
     constexpr int THREADS = WARPS * 32;
     constexpr int LANES = NQ * NQ <= 16 ? 16 : 32, GROUPS = 32 / LANES;   // lanes per pair, pairs per warp
@@ -358,7 +398,8 @@ __global__ void __launch_bounds__(WARPS * 32) k_assemble_pairs_ff(AssembleArgs a
     constexpr int PS = PairFF<NEN, NQ>::PS;
     static_assert(NEN * NEN % LANES == 0 && LANES % HL == 0 && NEN % 4 == 0 && NEN * NEN / 4 / OUT * 4 == LANES, "lane layout");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ float4 eq[NQ];
+    constexpr bool EXP = INF == NLGPU_INFLUENCE_EXPONENTIAL;
+    __shared__ int4 eq[NQ];
     __shared__ int4 ew[NEN * NQ];
     __shared__ double egx[NEN * NQ], egy[NEN * NQ], ejac[NQ], elam[NQ];   // the self term stays FP64
     __shared__ int32_t enodes[NEN], einner[NEN];   // eL's nodes and whether each is inner
@@ -366,9 +407,13 @@ __global__ void __launch_bounds__(WARPS * 32) k_assemble_pairs_ff(AssembleArgs a
     __shared__ int row_len[NEN], row_off[NEN + 1];
     __shared__ int use_smem, listed;
     __shared__ int32_t list[FF_LIST];
-    __shared__ ff etab[2 * FF_EXP_K + 1];
-    for (int t = threadIdx.x; t < 2 * FF_EXP_K + 1; t += blockDim.x)
-        etab[t] = ff{f.exp_table.v[t].x, f.exp_table.v[t].y};
+    __shared__ ff etab[EXP && !FIX ? 2 * FF_EXP_K + 1 : 1];
+    __shared__ unsigned long long xtab[EXP && FIX ? FX_EXP_K : 1];
+    if constexpr (EXP && !FIX)
+        for (int t = threadIdx.x; t < 2 * FF_EXP_K + 1; t += blockDim.x) etab[t] = ff{f.ff_table.v[t].x, f.ff_table.v[t].y};
+    if constexpr (EXP && FIX)
+        for (int t = threadIdx.x; t < FX_EXP_K; t += blockDim.x) xtab[t] = f.fx_table.v[t];
+    const int ex = FIX ? fx_exponent(f.extent) : 0;
 
     auto* pairs = reinterpret_cast<PairFF<NEN, NQ>*>(smem_raw);
     double* acc = reinterpret_cast<double*>(smem_raw + sizeof(PairFF<NEN, NQ>) * WARPS * GROUPS);
@@ -453,37 +498,84 @@ __global__ void __launch_bounds__(WARPS * 32) k_assemble_pairs_ff(AssembleArgs a
                 if (gl < NQ) ps.q[gl] = f.qcoord[i64(eNL) * NQ + gl];
                 if (gl < NEN) ps.nodes[gl] = f.nodes[i64(eNL) * NEN + gl];
                 __syncwarp();
-                ff v[PR];
-                unsigned largest = 0;
-#pragma unroll
-                for (int rnd = 0; rnd < PR; ++rnd) {
-                    const int t = min(gl + LANES * rnd, NQ * NQ - 1);
-                    const float4 xl = eq[t / NQ], xn = ps.q[t % NQ];
-                    v[rnd] = shape_ff<INF>(m, ff_sub(ff{xl.x, xl.y}, ff{xn.x, xn.y}), ff_sub(ff{xl.z, xl.w}, ff{xn.z, xn.w}),
-                                           qf, etab);
-                    largest = max(largest, __float_as_uint(v[rnd].h) & 0x7fffffffu);
-                }
-#pragma unroll
-                for (int o = LANES / 2; o > 0; o >>= 1) largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, o));
                 const bool self = eNL == int32_t(eL);
-                active = active && (largest != 0 || self || e_w + e_g >= FF_BAD / 2);
-                if (!__any_sync(0xffffffffu, active)) continue;
-                const int e_p = max(int(largest >> 23) - 127, -100);
-                const float up = __int_as_float((127 + 23 - e_p) << 23);
+                const bool bad = e_w + e_g >= FF_BAD / 2;
+                int e_p = 0;
+                bool finite = !bad;
+                if constexpr (FIX) {
+                    long long v[PR];
+                    if constexpr (EXP) {
+                        int mv[PR], smallest = FX_EXP_ZERO;
 #pragma unroll
-                for (int rnd = 0; rnd < PR; ++rnd) {
-                    const int t = gl + LANES * rnd;
-                    const float s = __fmul_rn(v[rnd].h, up);
-                    const int hi = __float2int_rn(s);
-                    const float rest = __fmaf_rn(v[rnd].l, up, __fsub_rn(s, __int2float_rn(hi)));
-                    const int lo = __float2int_rn(__fmul_rn(rest, 268435456.0f));   // 2^28
-                    if (PR * LANES == NQ * NQ || t < NQ * NQ) ps.phi[t / NQ * PS + t % NQ] = make_int2(hi, lo);
+                        for (int rnd = 0; rnd < PR; ++rnd) {
+                            const int t = min(gl + LANES * rnd, NQ * NQ - 1);
+                            v[rnd] = (long long)(fx_exp(fx_distance<FX_EXP_UNIT>(eq[t / NQ], ps.q[t % NQ], ex), f.fx_exp, xtab,
+                                                    mv[rnd]) >> 3);
+                            smallest = min(smallest, mv[rnd]);
+                        }
+#pragma unroll
+                        for (int o = LANES / 2; o > 0; o >>= 1) smallest = min(smallest, __shfl_xor_sync(0xffffffffu, smallest, o));
+                        active = active && (smallest != FX_EXP_ZERO || self || bad);
+                        if (smallest != FX_EXP_ZERO) e_p = -smallest;
+#pragma unroll
+                        for (int rnd = 0; rnd < PR; ++rnd) v[rnd] >>= min(mv[rnd] - smallest, 63);
+                    } else {
+                        bool some = false;
+#pragma unroll
+                        for (int rnd = 0; rnd < PR; ++rnd) {
+                            const int t = min(gl + LANES * rnd, NQ * NQ - 1);
+                            const long long d = fx_distance<60>(eq[t / NQ], ps.q[t % NQ], ex);
+                            if constexpr (INF == NLGPU_INFLUENCE_POLYNOMIAL)
+                                v[rnd] = d < FX_ONE ? fx_ipow(FX_ONE - fx_ipow(d, m.p / 2), int(m.q)) : 0;
+                            else
+                                v[rnd] = d < FX_ONE ? FX_ONE - d : 0;
+                            some = some || v[rnd] != 0;
+                        }
+                        const unsigned any = __ballot_sync(0xffffffffu, some) >> (LANES * group) & (0xffffffffu >> (32 - LANES));
+                        active = active && (any != 0 || self || bad);
+                    }
+                    if (!__any_sync(0xffffffffu, active)) continue;
+#pragma unroll
+                    for (int rnd = 0; rnd < PR; ++rnd) {
+                        const int t = gl + LANES * rnd;
+                        if (PR * LANES == NQ * NQ || t < NQ * NQ)
+                            ps.phi[t / NQ * PS + t % NQ] = fx_split(v[rnd]);
+                    }
+                } else {
+                    ff v[PR];
+                    unsigned largest = 0;
+#pragma unroll
+                    for (int rnd = 0; rnd < PR; ++rnd) {
+                        const int t = min(gl + LANES * rnd, NQ * NQ - 1);
+                        const int4 xl = eq[t / NQ], xn = ps.q[t % NQ];
+                        auto coord = [](int h, int l) { return ff{__int_as_float(h), __int_as_float(l)}; };
+                        v[rnd] = shape_ff<INF>(m, ff_sub(coord(xl.x, xl.y), coord(xn.x, xn.y)),
+                                               ff_sub(coord(xl.z, xl.w), coord(xn.z, xn.w)), qf, etab);
+                        largest = max(largest, __float_as_uint(v[rnd].h) & 0x7fffffffu);
+                    }
+#pragma unroll
+                    for (int o = LANES / 2; o > 0; o >>= 1) largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, o));
+                    active = active && (largest != 0 || self || bad);
+                    if (!__any_sync(0xffffffffu, active)) continue;
+                    finite = finite && largest < 0x7f800000u;
+                    const int e = max(int(largest >> 23) - 127, -100);
+                    e_p = e + 7;
+                    const float up = __int_as_float((127 + 23 - e) << 23);
+#pragma unroll
+                    for (int rnd = 0; rnd < PR; ++rnd) {
+                        const int t = gl + LANES * rnd;
+                        const float s = __fmul_rn(v[rnd].h, up);
+                        const int hi = __float2int_rn(s);
+                        const float rest = __fmaf_rn(v[rnd].l, up, __fsub_rn(s, __int2float_rn(hi)));
+                        const int lo = __float2int_rn(__fmul_rn(rest, 1073741824.0f));   // 2^30
+                        if (PR * LANES == NQ * NQ || t < NQ * NQ) ps.phi[t / NQ * PS + t % NQ] = make_int2(hi, lo);
+                    }
                 }
                 __syncwarp();
-                // H(qL, j) = sum_qNL shape G: unit 2^(e_p + e_g - 55)
+                // H(qL, j) = sum_qNL shape G: unit 2^(e_p + e_g - 56)
 #pragma unroll 1
                 for (int qL = gl / HL; qL < NQ; qL += HG) {
-                    long long s0 = 0, s1 = 1 << 23;
+                    long long s0 = 0, s1 = (1ll << 30) + (1 << 29);   // the two shifts below round
 #pragma unroll
                     for (int q = 0; q < NQ; ++q) {
                         const int2 p = ps.phi[qL * PS + q];
@@ -491,17 +583,17 @@ __global__ void __launch_bounds__(WARPS * 32) k_assemble_pairs_ff(AssembleArgs a
                         s1 += (long long)p.x * g[q].y;
                         s1 += (long long)p.y * g[q].x;
                     }
-                    const long long h = s0 * 16 + (s1 >> 24);   // |h| < 2^61
+                    const long long h = (s0 + (s1 >> 30)) >> 1;   // |h| < 2^60.4
                     const int lo = int(h), hi = int(h >> 32) + (lo < 0 ? 1 : 0);
-                    // the low word to 28 bits, so that both cross products below have one unit
-                    reinterpret_cast<int2*>(ps.h)[(qL * NEN + gl % NEN) * 2 + gl % HL / NEN] = make_int2(hi, ((lo >> 3) + 1) >> 1);
+                    // the low word to 30 bits, so that both cross products below have one unit
+                    reinterpret_cast<int2*>(ps.h)[(qL * NEN + gl % NEN) * 2 + gl % HL / NEN] = make_int2(hi, ((lo >> 1) + 1) >> 1);
                 }
                 __syncwarp();
                 // K(i, j) = sum_qL (w G_i) . H(qL, j): unit 2^(e_w + e_g + e_p - 51)
                 const int i = gl >> 2, j0 = gl & 3;
                 long long s0[OUT], s1[OUT];
 #pragma unroll
-                for (int o = 0; o < OUT; ++o) { s0[o] = 0; s1[o] = 1 << 27; }
+                for (int o = 0; o < OUT; ++o) { s0[o] = 0; s1[o] = 1 << 29; }
 #pragma unroll
                 for (int q = 0; q < NQ; ++q) {
                     const int4 w = ew[i * NQ + q];
@@ -518,8 +610,8 @@ __global__ void __launch_bounds__(WARPS * 32) k_assemble_pairs_ff(AssembleArgs a
                 }
                 const int e_k = e_w + e_g + e_p - 51;
                 double unit = __hiloint2double((1023 + e_k) << 20, 0);
-                if (abs(e_k) > 1000 || largest >= 0x7f800000u)   // a non-finite factor, or far out of range
-                    unit = e_w + e_g >= FF_BAD / 2 || largest >= 0x7f800000u ? nan("") : scalbn(1.0, e_k);
+                if (!finite || abs(e_k) > 1000)   // a non-finite factor, or far out of range
+                    unit = finite ? scalbn(1.0, e_k) : nan("");
                 const int32_t r = enodes[i];
                 const bool r_in = einner[i] != 0;
 #pragma unroll
@@ -532,7 +624,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_assemble_pairs_ff(AssembleArgs a
                     const bool tr = SYM && active && !self;
                     const bool bwd_inner = tr && c_in && r_in && c <= r;
                     const bool bwd_bound = tr && !r_in && c != r;
-                    double val = __ll2double_rn(s0[o] + (s1[o] >> 28)) * unit;
+                    double val = __ll2double_rn(s0[o] + (s1[o] >> 30)) * unit;
                     if (self) {
                         double loc = 0.0;
 #pragma unroll 1
@@ -667,7 +759,10 @@ void dispatch_influence(Ctx& ctx, const AssembleArgs& a, bool sym) {
 
 template<int NEN, int NQ, int INF, int WARPS>
 void launch_pairs_ff_w(Ctx& ctx, AssembleArgs a, const FFArgs& f, bool sym) {
-    auto kernel = sym ? k_assemble_pairs_ff<NEN, NQ, INF, true, WARPS> : k_assemble_pairs_ff<NEN, NQ, INF, false, WARPS>;
+    auto kernel = f.extent ? (sym ? k_assemble_pairs_ff<NEN, NQ, INF, true, WARPS, true>
+                                  : k_assemble_pairs_ff<NEN, NQ, INF, false, WARPS, true>)
+                           : (sym ? k_assemble_pairs_ff<NEN, NQ, INF, true, WARPS, false>
+                                  : k_assemble_pairs_ff<NEN, NQ, INF, false, WARPS, false>);
     // the row accumulators take what shared memory the per-warp blocks leave
     int dev = 0, optin = 0;
     NL_CUDA(cudaGetDevice(&dev));
@@ -686,18 +781,19 @@ void launch_pairs_ff_w(Ctx& ctx, AssembleArgs a, const FFArgs& f, bool sym) {
 
 // Warps per CTA: forced by NLGPU_OPTION_ASSEMBLY_WARPS, else tuned once per
 // (element type, influence kind, pair mode) and context by timing both forms
-// on the same sample of elements from the middle of the mesh (their
+// on the same sample of elements from the middle of the mesh, three per SM (their
 // contributions are cleared afterwards: the matrices are zeroed again).
 template<int NEN, int NQ, int INF>
 void launch_pairs_ff(Ctx& ctx, AssembleArgs a, const FFArgs& f, bool sym) {
     int warps = ctx.ff_warps_option;
+    if (warps == 0 && a.E < 152 * 64) warps = 32;   // the four samples would cost as much as the assembly
     if (warps == 0) {
-        const int key = NEN * 1000 + INF * 10 + (sym ? 1 : 0);
+        const int key = NEN * 1000 + INF * 10 + (sym ? 1 : 0) + (f.extent ? 2 : 0);
         auto it = ctx.ff_warps_tuned.find(key);
         if (it != ctx.ff_warps_tuned.end()) {
             warps = it->second;
         } else {
-            const i64 sample = std::min<i64>(a.E, 152 * 8);
+            const i64 sample = std::min<i64>(a.E, 152 * 3);
             AssembleArgs s = a;
             s.e0 = (a.E - sample) / 2;
             s.E = s.e0 + sample;
@@ -763,21 +859,40 @@ void assemble_full(Ctx& ctx) {
     err.resize(1);
     err.zero(ctx.stream);
     a.error = err.p;
+    dbuf<unsigned long long> extent;
     // unordered pairs need a symmetric influence and constant conductivity
     const bool sym = ctx.symmetric && !ctx.cond_field.n && !ctx.ordered_pairs;
+    // The pair blocks in fixed point: the FP64 kernel's accuracy at a quarter of its
+    // time (71 x 53 8-node elements, polynomial: 3.73 and 0.93 ms), so also for FP64 solves unless
+    // that kernel is asked for.  The mixed-precision form takes the exponential in
+    // float-float, 4 % faster (150 x 150 8-node: 18.6 against 19.3 ms) and accurate
+    // enough for it; polynomials are as fast in fixed point (16.3 and 16.0).
+    const bool fx = fx_supported(ctx.model);
+    const bool fixed = fx && (ctx.ff_assembly ? ctx.model.influence != NLGPU_INFLUENCE_EXPONENTIAL : ctx.fx_assembly);
     ctx.ff_assembled = ctx.ff_assembly && ff_supported(ctx.model);
-    if (ctx.ff_assembled) {
+    if (ctx.ff_assembled || fixed) {
         const int nen = ctx.basis.nen, nq = ctx.basis.nq;
         ctx.ff_qcoord.reserve(size_t(ctx.n_elems * nq));
         ctx.ff_g.reserve(size_t(ctx.n_elems * nen * nq * 2));
         ctx.ff_w.reserve(size_t(ctx.n_elems * nen * nq));
         ctx.ff_exps.reserve(size_t(ctx.n_elems));
         ctx.ff_nodes.reserve(size_t(ctx.n_elems * nen));
+        if (fixed) {
+            extent.resize(1);
+            extent.zero(ctx.stream);
+            NL_LAUNCH(k_fx_extent, grid_for(ctx.n_elems * nq, 256, 152 * 4), 256, 0, ctx.stream, ctx.n_elems * nq,
+                      ctx.qcoord.p, ctx.model.inv_r[0], ctx.model.inv_r[1], extent.p);
+        }
         NL_LAUNCH(k_ff_stage, grid_for(ctx.n_elems * 32, 256), 256, 0, ctx.stream, ctx.n_elems, nen, nq, ctx.elems.p,
-                  ctx.is_inner.p, ctx.deriv.p, ctx.qcoord.p, a.cond_field, ctx.model, ctx.basis, ctx.ff_qcoord.p,
-                  ctx.ff_g.p, ctx.ff_w.p, ctx.ff_exps.p, ctx.ff_nodes.p);
-        FFArgs f{ctx.ff_qcoord.p, ctx.ff_g.p, ctx.ff_w.p, ctx.ff_exps.p, ctx.ff_nodes.p, {}};
-        fill_exp_table(f.exp_table);
+                  ctx.is_inner.p, ctx.deriv.p, ctx.qcoord.p, a.cond_field, ctx.model, ctx.basis, extent.p,
+                  ctx.ff_qcoord.p, ctx.ff_g.p, ctx.ff_w.p, ctx.ff_exps.p, ctx.ff_nodes.p);
+        FFArgs f{ctx.ff_qcoord.p, extent.p, ctx.ff_g.p, ctx.ff_w.p, ctx.ff_exps.p, ctx.ff_nodes.p, {}, {}, {}};
+        if (ctx.model.influence == NLGPU_INFLUENCE_EXPONENTIAL && fixed) {
+            f.fx_table = fx_exp_table();
+            f.fx_exp = fx_exp_setup(ctx.model.q);
+        } else if (ctx.model.influence == NLGPU_INFLUENCE_EXPONENTIAL) {
+            fill_exp_table(f.ff_table);
+        }
         if (nen == 4) dispatch_influence_ff<4, 4>(ctx, a, f, sym);
         else dispatch_influence_ff<8, 9>(ctx, a, f, sym);
     } else if (ctx.basis.nen == 4) {

@@ -534,14 +534,14 @@ struct Ctx {
     int assembly_precision = NLGPU_ASSEMBLY_AUTO;
     bool ff_assembly = false;           // pair blocks in float-float on the FP32 pipes (mixed precision)
     bool ff_assembled = false;          // the last assembly ran in float-float
+    bool fx_assembly = true;            // else: pair blocks in fixed point instead of FP64 (where it covers the model)
     int ff_warps_option = 0;            // warps per CTA of the float-float pair assembly (0: tuned)
     int ff_warps_used = 0;              // ... of its last launch
     double ff_tune_ms[2] = {0.0, 0.0};  // the last tuning's sample times with 16 and 32 warps
     std::map<int, int> ff_warps_tuned;  // tuned choice per (element type, influence kind, pair mode)
     // the float-float pair assembly's copies of the element data (FFArgs)
-    dbuf<float4> ff_qcoord;
     dbuf<int2> ff_g, ff_exps;
-    dbuf<int4> ff_w;
+    dbuf<int4> ff_qcoord, ff_w;
     dbuf<int32_t> ff_nodes;
     // measurement
     cudaEvent_t events[64] = {};

@@ -47,4 +47,119 @@ inline bool ff_supported(const Model& m) {
     return false;
 }
 
+// ---------------------------------------------------------------- fixed point
+// The influence functions of the usual exponents (n = 2) in 64-bit integers, for the
+// pair assembly, whose contractions want fixed-point operands.  Coordinates in
+// units of the radii are 59-bit integers with one exponent per mesh, values have 60
+// bits: as accurate as FP64 (whose squared distance and exponential round to 53 bits
+// each), on pipes that have 32 times the FP64 rate.
+
+// floor-like a b 2^-64 of unsigned numbers, up to 2 below (the low halves' product is left out)
+__device__ __forceinline__ unsigned long long fx_mulhi(unsigned long long a, unsigned long long b) {
+    const unsigned ah = unsigned(a >> 32), al = unsigned(a), bh = unsigned(b >> 32), bl = unsigned(b);
+    return (unsigned long long)ah * bh + __umulhi(ah, bl) + __umulhi(al, bh);
+}
+
+constexpr int FX_SPLIT = 30;              // a number is hi 2^30 + lo
+constexpr long long FX_ONE = 1ll << 60;   // influence values, and the polynomials' squared distance
+constexpr int FX_EXP_UNIT = 54;           // the exponential's squared distance, in 2^-54
+constexpr long long FX_FAR = 1ll << 62;   // any squared distance beyond 2^62 units
+
+__device__ __forceinline__ int2 fx_split(long long z) {
+    const long long hi = (z + (1 << (FX_SPLIT - 1))) >> FX_SPLIT;
+    return make_int2(int(hi), int(z - (hi << FX_SPLIT)));
+}
+
+// x inv as an integer in 2^(ex - 58), ex >= 2 the exponent of the mesh's largest: the product to 106 bits
+__device__ __forceinline__ int2 fx_coordinate(double x, double inv, int ex) {
+    const double p = x * inv, r = fma(x, inv, -p);
+    return fx_split(__double2ll_rn(scalbn(p, 58 - ex)) + __double2ll_rn(scalbn(r, 58 - ex)));
+}
+
+__device__ __forceinline__ long long fx_shift(long long v, int left) {
+    return left >= 0 ? v << min(left, 63) : v >> min(-left, 63);
+}
+
+// the squared distance of two points (x hi, x lo, y hi, y lo) in 2^-UNIT
+template<int UNIT>
+__device__ __forceinline__ long long fx_distance(int4 a, int4 b, int ex) {
+    const int xh = a.x - b.x, xl = a.y - b.y, yh = a.z - b.z, yl = a.w - b.w;
+    const long long hh = (long long)xh * xh + (long long)yh * yh;
+    const long long hl = (long long)xh * xl + (long long)yh * yl;
+    const long long ll = (long long)xl * xl + (long long)yl * yl;
+    const int s = 2 * ex + UNIT;   // hh 2^(s - 56) + hl 2^(s - 85) + ll 2^(s - 116)
+    if ((hh >> max(118 - s, 0)) != 0) return FX_FAR;
+    const long long d = fx_shift(hh, s - 56) + fx_shift(hl, s - 85) + fx_shift(ll, s - 116);
+    return d & ~(d >> 63);   // the shifts round down
+}
+
+// x^n of 0 <= x <= 1
+__device__ __forceinline__ long long fx_ipow(long long x, int n) {
+    long long r = FX_ONE;
+    for (int k = 0; k < n; ++k) r = k ? (long long)fx_mulhi((unsigned long long)r << 2, (unsigned long long)x << 2) : x;
+    return r;
+}
+
+// exp(-q d) = 2^-(m + k / 256) e^-x from the mathematics of the exponential: q log2(e) d
+// split into integer part m, k and a rest x / ln 2 below 1/256; 2^(-k / 256) from a
+// table, 1 - e^-x by its series to x^5 (the sixth term is below 2^-60).
+struct FXExp {
+    unsigned long long rate;   // q log2(e) 2^(65 - shift), 2^62 to 2^63
+    int shift;
+    long long reach;           // where the value counts as zero (q d = 85, as in float-float)
+};
+constexpr int FX_EXP_K = 256;
+struct FXExpTable {
+    unsigned long long v[FX_EXP_K];   // 2^(63 - k / 256)
+};
+
+// value = v 2^-(63 + m); m = FX_EXP_ZERO: zero
+constexpr int FX_EXP_ZERO = 1 << 20;
+__device__ __forceinline__ unsigned long long fx_exp(long long d, const FXExp& f, const unsigned long long* table, int& m) {
+    if (d > f.reach) {
+        m = FX_EXP_ZERO;
+        return 0;
+    }
+    const unsigned long long t = fx_mulhi((unsigned long long)d << f.shift, f.rate);   // in 2^-55
+    m = int(t >> 55);
+    const unsigned long long tab = table[unsigned(t >> 47) & 255u];
+    const unsigned long long x = fx_mulhi(t << 17, 0xb17217f7d1cf79acull);   // ln 2 times the rest, in 2^-72
+    const unsigned xh = unsigned(x >> 32), xl = unsigned(x);
+    const unsigned long long x2 = ((unsigned long long)xh * xh >> 9) + (__umulhi(xh, xl) >> 8);   // x^2 / 2
+    const unsigned x3 = __umulhi(__umulhi(unsigned(x2 >> 22), xh), 0x55555556u);                  // x^3 / 6, in 2^-58
+    const unsigned x4 = __umulhi(x3, xh);                                                         // x^4 / 6, in 2^-66
+    const unsigned x5 = __umulhi(__umulhi(x4, xh), 53687091u);                                    // x^5 / 120: 2^32 / 80
+    const unsigned long long y = x - x2 + ((unsigned long long)x3 << 14) - ((unsigned long long)x4 << 4) + x5;
+    return tab - (fx_mulhi(tab, y) >> 8);
+}
+
+inline FXExp fx_exp_setup(double q) {
+    const long double rate = (long double)q * 1.4426950408889634073599L;
+    FXExp f{};
+    f.shift = 3 + std::ilogb(rate);
+    f.rate = static_cast<unsigned long long>(std::ldexp(rate, 65 - f.shift));
+    f.reach = static_cast<long long>(std::ldexp(85.0 / q, FX_EXP_UNIT));
+    return f;
+}
+
+// computed once: 0.2 ms where long double is a software type
+inline const FXExpTable& fx_exp_table() {
+    static const FXExpTable table = [] {
+        FXExpTable t;
+        for (int k = 0; k < FX_EXP_K; ++k)
+            t.v[k] = static_cast<unsigned long long>(std::ldexp(std::exp2((long double)-k / FX_EXP_K), 63));
+        return t;
+    }();
+    return table;
+}
+
+// the exponents the fixed-point forms cover: q >= 0.333 keeps q d = 85 below FX_FAR, above 16 the
+// distance's unit counts for more than FP64's rounding
+inline bool fx_supported(const Model& m) {
+    if (m.n != 2) return false;
+    if (m.influence == NLGPU_INFLUENCE_FAST_POLYNOMIAL) return true;
+    if (m.influence == NLGPU_INFLUENCE_POLYNOMIAL) return m.p >= 0 && m.p % 2 == 0 && m.q >= 0.0 && m.q == std::floor(m.q) && m.q <= 16.0;
+    return m.influence == NLGPU_INFLUENCE_EXPONENTIAL && m.p == 2 && m.q >= 0.333 && m.q <= 16.0;
+}
+
 }  // namespace nlgpu

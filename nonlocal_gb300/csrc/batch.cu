@@ -86,7 +86,11 @@ __global__ void k_bt_axpy(i64 n, const double* __restrict__ a, double* __restric
 // pipe spent more on the sums than on the products).  Blocks of stopped
 // instances (done[k] != 0) are skipped.
 // desc: first row (bits 0-31), log2 g (bits 32-34), rows in the block (35-40).
-__global__ void __launch_bounds__(BT_THREADS) k_bt_spmv(i64 nblocks, const unsigned long long* __restrict__ desc,
+// The grid is what the SMs hold, 6 CTAs of 40 registers each: with up to 8 asked for
+// and 5 resident the last wave was nearly empty (six 96 x 96 instances of 130 entries a
+// row: 36.4 -> 28.7 us a product, FP64 pipe 48 -> 60 % busy; 8 CTAs of 32 registers 31.7).
+constexpr int BT_SPMV_CTAS = 6;
+__global__ void __launch_bounds__(BT_THREADS, BT_SPMV_CTAS) k_bt_spmv(i64 nblocks, const unsigned long long* __restrict__ desc,
                                                         const i64* __restrict__ rp, const int4* __restrict__ col4,
                                                         const double2* __restrict__ val2, const double* __restrict__ x,
                                                         double* __restrict__ y, const int32_t* __restrict__ inst,
@@ -97,13 +101,15 @@ __global__ void __launch_bounds__(BT_THREADS) k_bt_spmv(i64 nblocks, const unsig
     const i64 warps = i64(gridDim.x) * (blockDim.x >> 5);
     const double* wv = w ? w : x;
     double acc = 0.0, acc2 = 0.0;
-    int acc_inst = -1;
-    auto flush = [&]() {   // warp-uniform: called by every lane
-        const double a = warp_sum(acc);
-        const double a2 = dot2 ? warp_sum(acc2) : 0.0;
+    int acc_inst = -1, acc_g = 1;
+    auto flush = [&]() {   // warp-uniform: called by every lane; a row's first lane holds its part
+        for (int o = 16; o >= acc_g; o >>= 1) {
+            acc += __shfl_xor_sync(full, acc, o);
+            if (dot2) acc2 += __shfl_xor_sync(full, acc2, o);
+        }
         if (lane == 0 && acc_inst >= 0) {
-            atomicAdd(dot + acc_inst, a);
-            if (dot2) atomicAdd(dot2 + acc_inst, a2);
+            atomicAdd(dot + acc_inst, acc);
+            if (dot2) atomicAdd(dot2 + acc_inst, acc2);
         }
         acc = acc2 = 0.0;
     };
@@ -116,6 +122,7 @@ __global__ void __launch_bounds__(BT_THREADS) k_bt_spmv(i64 nblocks, const unsig
         if (dot && k != acc_inst) {
             flush();
             acc_inst = k;
+            acc_g = 1 << lg;
         }
         const int g = 1 << lg, sub = lane & (g - 1), slot = lane >> lg;
         const i64 r = first + slot;
@@ -139,8 +146,8 @@ __global__ void __launch_bounds__(BT_THREADS) k_bt_spmv(i64 nblocks, const unsig
         if (active && sub == 0) {
             y[r] = s;
             if (dot) {
-                acc += s * wv[r];
-                acc2 += s * s;
+                acc = fma(s, wv[r], acc);
+                if (dot2) acc2 = fma(s, s, acc2);
             }
         }
     }
@@ -354,7 +361,7 @@ void row_blocks(Batch& bt, const Csr& M, dbuf<unsigned long long>& out, i64& cou
 void bt_spmv(Batch& bt, const Csr& M, const double* x, double* y, double* dot, bool skip_done) {
     const bool is_a = &M == &bt.A;
     const i64 nb = is_a ? bt.nblocks_A : bt.nblocks_C;
-    NL_LAUNCH(k_bt_spmv, grid_for(nb * 32, BT_THREADS, 152 * 8), BT_THREADS, 0, bt.stream, nb,
+    NL_LAUNCH(k_bt_spmv, grid_for(nb * 32, BT_THREADS, 152 * BT_SPMV_CTAS), BT_THREADS, 0, bt.stream, nb,
               (is_a ? bt.blocks_A : bt.blocks_C).p, M.rowptr.p, reinterpret_cast<const int4*>(M.col.p),
               reinterpret_cast<const double2*>(M.val.p), x, y, bt.inst_of_row.p,
               (skip_done ? bt.sc.p : bt.sc.p + bt.K * BS_COUNT) + BS_DONE * bt.K, dot, static_cast<const double*>(nullptr),
@@ -874,7 +881,7 @@ std::vector<CgResult> batch_bicgstab(const std::vector<Ctx*>& instances, double 
     NL_CUDA(cudaMemsetAsync(bt.x.p, 0, size_t(N) * sizeof(double), bt.stream));
     NL_CUDA(cudaMemsetAsync(t.p, 0, size_t(N) * sizeof(double), bt.stream));   // A x for x = 0
     auto spmv = [&](const double* in, double* out, double* dot, const double* w, double* dot2) {
-        NL_LAUNCH(k_bt_spmv, grid_for(bt.nblocks_A * 32, BT_THREADS, 152 * 8), BT_THREADS, 0, bt.stream, bt.nblocks_A,
+        NL_LAUNCH(k_bt_spmv, grid_for(bt.nblocks_A * 32, BT_THREADS, 152 * BT_SPMV_CTAS), BT_THREADS, 0, bt.stream, bt.nblocks_A,
                   bt.blocks_A.p, bt.A.rowptr.p, reinterpret_cast<const int4*>(bt.A.col.p),
                   reinterpret_cast<const double2*>(bt.A.val.p), in, out, bt.inst_of_row.p, sc + BB_DONE * K, dot, w,
                   dot2);

@@ -165,25 +165,31 @@ __global__ void k_first_kind_1d(i64 n, const double* __restrict__ bound0, double
 //
 // A row at a time, every pivot cost three CTA barriers and bw^2 / 2 updates with a
 // division each on one SM's FP64 pipe (two lanes a clock): 33 us a pivot,
-// 66.8 ms for 2 001 rows of half bandwidth 102.  Here a block of 16 pivots is one
-// warp's work in registers: it eliminates [A_kk | I], lane j < 16 holding column
-// j of A_kk and lane 16 + j column j of I, which leaves D L^T and L^-1 at no extra
-// instructions; those 216 FP64 instructions of one warp (64 cycles each on its
-// quarter of the SM's FP64 pipe) are the critical path, and everything else is
-// spread over the cluster between two of them:
-//   W = L^-1 A(block, columns after it)                 (all CTAs)
-//   A(i, j) -= sum_k W(k, i) W(k, j) / d_k               (all CTAs but the first)
-//   next diagonal block: the same update, then its elimination   (first CTA)
-// with one cluster barrier after each phase.  The rows keep U = D^-1 W beyond
+// 66.8 ms for 2 001 rows of half bandwidth 102.  Here a block of 16 pivots is the
+// work of four warps in registers: they eliminate [A_kk | I], lane j < 16 holding
+// column j of A_kk and lane 16 + j column j of I, which leaves D L^T and L^-1 at no
+// extra instructions.  A warp's FP64 instruction holds its quarter of the SM's FP64
+// pipe for 64 cycles, so the rows are dealt out over the four quarters: a pivot costs
+// 5 to 8 of them instead of 6 to 21 in one warp.  That is the critical path, and
+// everything else is spread over the cluster between two eliminations:
+//   W = L^-1 A(block, columns after it)                 (the other 15 CTAs)
+//   A(i, j) -= sum_k W(k, i) W(k, j) / d_k               (the other 15 CTAs)
+//   next diagonal block: its own 16 columns of W, the update, the elimination   (first CTA)
+// with a cluster barrier after each phase, of which the first CTA only
+// passes the second one on its way.  The rows keep U = D^-1 W beyond
 // their block; L^-1 and 1 / d are kept per block.  The right-hand side, when there
 // is one, is one more column (its forward substitution comes for free).
-// 2 001 rows of half bandwidth 102: 66.8 -> 2.0 ms, of which the eliminations 1.1.
+// 2 001 rows of half bandwidth 102: 66.8 ms; 2.0 with the elimination in one warp (1.1
+// of it) and W shared by all CTAs; 1.42 now.
 constexpr int BF_NB = 16;
 constexpr int BF_CTAS = 16;
 constexpr int BF_THREADS = 256;
 
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    cluster_arrive();
+    cluster_wait();
 }
 
 struct BandFactor {
@@ -207,34 +213,48 @@ __device__ __forceinline__ double reciprocal(double d) {
     return fma(fma(-d, r, 1.0), r, r);
 }
 
-// eliminates the diagonal block in `a` (rows i of column lane), writes L^-1 and 1 / d
-__device__ __forceinline__ void eliminate_block(double (&a)[BF_NB], double* linv, double* dinv, int* failed) {
+// Warps 0 .. 3 eliminate the diagonal block in `diag` (upper), a warp the rows i = part
+// (mod 4) of [A | I]; writes L^-1 and 1 / d to global memory and to lk, dk.  A pivot's
+// row goes round through shared memory.
+constexpr int BF_PARTS = 4;
+__device__ __forceinline__ void eliminate_block(const double (*diag)[BF_NB + 1], double (*row)[32], double* linv,
+                                                double* dinv, double* lk, double* dk, int* failed, int part) {
+    constexpr int OWN = BF_NB / BF_PARTS;
     const int lane = threadIdx.x & 31;
+    double a[OWN];
+#pragma unroll
+    for (int q = 0; q < OWN; ++q) {
+        const int i = BF_PARTS * q + part;
+        a[q] = lane < BF_NB ? diag[min(i, lane)][max(i, lane)] : (i == lane - BF_NB ? 1.0 : 0.0);
+    }
 #pragma unroll
     for (int k = 0; k < BF_NB; ++k) {
-        // row k is final; by symmetry its lane i holds the multiplier of row i, so the
-        // broadcasts do not wait for the reciprocal
-        const double t = a[k], d = __shfl_sync(0xffffffffu, t, k);
-        double u[BF_NB];
-#pragma unroll
-        for (int i = k + 1; i < BF_NB; ++i) u[i] = __shfl_sync(0xffffffffu, t, i);
-        const double inv = reciprocal(d);
-        if (lane == 0) {
-            dinv[k] = inv;
+        double* pivot = row[k & 1];
+        if (part == k % BF_PARTS) pivot[lane] = a[k / BF_PARTS];
+        asm volatile("bar.sync 1, %0;" ::"n"(BF_PARTS * 32) : "memory");
+        // row k is final; by symmetry its entry i is the multiplier of row i
+        const double t = pivot[lane], d = pivot[k], inv = reciprocal(d);
+        if (part == 0 && lane == 0) {
+            dinv[k] = dk[k] = inv;
             if (d == 0.0) *failed = 1;
         }
         const double s = -t * inv;
 #pragma unroll
-        for (int i = k + 1; i < BF_NB; ++i) a[i] = fma(u[i], s, a[i]);   // row k + 1, the next pivot's, first
+        for (int q = k / BF_PARTS; q < OWN; ++q)   // row k + 1, the next pivot's, is its warp's first
+            if (BF_PARTS * q + part > k) a[q] = fma(pivot[BF_PARTS * q + part], s, a[q]);
     }
     if (lane >= BF_NB)
 #pragma unroll
-        for (int i = 0; i < BF_NB; ++i) linv[i * BF_NB + lane - BF_NB] = a[i];
+        for (int q = 0; q < OWN; ++q) {
+            const int at = (BF_PARTS * q + part) * BF_NB + lane - BF_NB;
+            linv[at] = lk[at] = a[q];
+        }
 }
 
 __global__ void __launch_bounds__(BF_THREADS) k_band_factor(BandFactor p) {
     extern __shared__ double bf_w[];
-    __shared__ double diag[BF_NB][BF_NB + 1], scaled[BF_NB][BF_NB], dk[BF_NB], lk[BF_NB * BF_NB];
+    __shared__ double diag[BF_NB][BF_NB + 1], wn[BF_NB][BF_NB], scaled[BF_NB][BF_NB], dks[2][BF_NB], lk[BF_NB * BF_NB],
+        pivots[2][32];
     const i64 w = p.bw + 1, blocks = (p.n + BF_NB - 1) / BF_NB;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x;
     // entry (i, j >= i) of the matrix, rows past the end an identity
@@ -242,76 +262,89 @@ __global__ void __launch_bounds__(BF_THREADS) k_band_factor(BandFactor p) {
         if (i >= p.n || j >= p.n) return i == j ? 1.0 : 0.0;
         return j - i <= p.bw ? p.band[i * w + (j - i)] : 0.0;
     };
-    auto eliminate = [&](i64 kb) {   // warp 0 of the first CTA, the block in `diag` (upper)
-        double a[BF_NB];
-#pragma unroll
-        for (int i = 0; i < BF_NB; ++i)
-            a[i] = lane < BF_NB ? diag[min(i, lane)][max(i, lane)] : (i == lane - BF_NB ? 1.0 : 0.0);
-        eliminate_block(a, p.linv + kb * BF_NB * BF_NB, p.dinv + kb * BF_NB, p.failed);
+    auto eliminate = [&](i64 kb) {   // the first CTA's warps 0 .. BF_PARTS - 1
+        eliminate_block(diag, pivots, p.linv + kb * BF_NB * BF_NB, p.dinv + kb * BF_NB, lk, dks[kb & 1], p.failed, warp);
     };
     if (rank == 0) {
         diag[tid >> 4][tid & 15] = (tid >> 4) <= (tid & 15) ? entry(tid >> 4, tid & 15) : 0.0;
         __syncthreads();
-        if (warp == 0) eliminate(0);
+        if (warp < BF_PARTS) eliminate(0);
     }
     for (i64 kb = 0; kb < blocks; ++kb) {
         cluster_barrier();
         const i64 k0 = kb * BF_NB, next = k0 + BF_NB;
         const int m = int(max(i64(0), min(p.bw, p.n - next)));   // columns after the block that it reaches
         const int cols = m + (p.f ? 1 : 0);
-        if (tid < BF_NB) dk[tid] = p.dinv[k0 + tid];
-        lk[tid] = p.linv[kb * BF_NB * BF_NB + tid];
-        __syncthreads();
-        for (int t = tid * BF_CTAS + rank; t < BF_NB * cols; t += BF_CTAS * BF_THREADS) {
-            const int r = t / cols, c = t % cols;
-            double v = 0.0, v2 = 0.0;
-#pragma unroll
-            for (int s = 0; s < BF_NB; s += 2) {
-                const double x = c < m ? entry(k0 + s, next + c) : (k0 + s < p.n ? p.f[k0 + s] : 0.0);
-                const double y = c < m ? entry(k0 + s + 1, next + c) : (k0 + s + 1 < p.n ? p.f[k0 + s + 1] : 0.0);
-                if (s <= r) v = fma(lk[r * BF_NB + s], x, v);
-                if (s + 1 <= r) v2 = fma(lk[r * BF_NB + s + 1], y, v2);
-            }
-            p.w[i64(r) * w + c] = v + v2;
-        }
-        cluster_barrier();
-        const double* W = p.w;
-        if (p.in_shared) {
-            for (int t = tid; t < BF_NB * cols; t += BF_THREADS) bf_w[i64(t / cols) * w + t % cols] = p.w[i64(t / cols) * w + t % cols];
-            W = bf_w;
-            __syncthreads();
-        }
+        double* dk = dks[kb & 1];
         if (rank == 0) {
+            // the first CTA takes what the next elimination waits for: the 16 columns of W
+            // over the next diagonal block, that block's update, the elimination
             if (kb + 1 < blocks) {
                 const int r = tid >> 4, c = tid & 15;
-                scaled[r][c] = c < m ? W[r * w + c] * dk[r] : 0.0;
+                double v = 0.0, v2 = 0.0;
+                if (c < m) {
+#pragma unroll
+                    for (int s = 0; s < BF_NB; s += 2) {
+                        const double x = entry(k0 + s, next + c), y = entry(k0 + s + 1, next + c);
+                        if (s <= r) v = fma(lk[r * BF_NB + s], x, v);
+                        if (s + 1 <= r) v2 = fma(lk[r * BF_NB + s + 1], y, v2);
+                    }
+                }
+                wn[r][c] = v + v2;
+                scaled[r][c] = (v + v2) * dk[r];
+            }
+            cluster_arrive();
+            if (kb + 1 < blocks) {
                 __syncthreads();
+                const int r = tid >> 4, c = tid & 15;
                 double v = 0.0;
                 if (r <= c) {
+                    double u = 0.0, u2 = 0.0;
                     v = entry(next + r, next + c);
-                    if (c < m) {
-                        double u = 0.0, u2 = 0.0;
 #pragma unroll
-                        for (int k = 0; k < BF_NB; k += 2) {
-                            u = fma(scaled[k][r], W[k * w + c], u);
-                            u2 = fma(scaled[k + 1][r], W[(k + 1) * w + c], u2);
-                        }
-                        v -= u + u2;
+                    for (int k = 0; k < BF_NB; k += 2) {
+                        u = fma(scaled[k][r], wn[k][c], u);
+                        u2 = fma(scaled[k + 1][r], wn[k + 1][c], u2);
                     }
+                    v -= u + u2;
                 }
                 diag[r][c] = v;
                 __syncthreads();
-                if (warp == 0) eliminate(kb + 1);
+                if (warp < BF_PARTS) eliminate(kb + 1);
             }
+            cluster_wait();   // W is complete
             // the block's rows: U = D^-1 W, and L^-1 f
-            if (warp > 0)
-                for (int t = tid - 32; t < BF_NB * cols; t += BF_THREADS - 32) {
+            if (warp >= BF_PARTS)
+                for (int t = tid - 32 * BF_PARTS; t < BF_NB * cols; t += BF_THREADS - 32 * BF_PARTS) {
                     const int r = t / cols, c = t % cols;
                     if (k0 + r >= p.n) continue;
-                    if (c == m) p.f[k0 + r] = W[r * w + c];
-                    else if (BF_NB + c - r <= p.bw) p.band[(k0 + r) * w + (BF_NB + c - r)] = W[r * w + c] * dk[r];
+                    const double v = p.w[i64(r) * w + c];
+                    if (c == m) p.f[k0 + r] = v;
+                    else if (BF_NB + c - r <= p.bw) p.band[(k0 + r) * w + (BF_NB + c - r)] = v * dk[r];
                 }
         } else {
+            if (tid < BF_NB) dk[tid] = p.dinv[k0 + tid];
+            lk[tid] = p.linv[kb * BF_NB * BF_NB + tid];
+            __syncthreads();
+            for (int t = tid * (BF_CTAS - 1) + rank - 1; t < BF_NB * cols; t += (BF_CTAS - 1) * BF_THREADS) {
+                const int r = t / cols, c = t % cols;
+                double v = 0.0, v2 = 0.0;
+#pragma unroll
+                for (int s = 0; s < BF_NB; s += 2) {
+                    const double x = c < m ? entry(k0 + s, next + c) : (k0 + s < p.n ? p.f[k0 + s] : 0.0);
+                    const double y = c < m ? entry(k0 + s + 1, next + c) : (k0 + s + 1 < p.n ? p.f[k0 + s + 1] : 0.0);
+                    if (s <= r) v = fma(lk[r * BF_NB + s], x, v);
+                    if (s + 1 <= r) v2 = fma(lk[r * BF_NB + s + 1], y, v2);
+                }
+                p.w[i64(r) * w + c] = v + v2;
+            }
+            cluster_barrier();
+            const double* W = p.w;
+            if (p.in_shared) {
+                for (int t = tid; t < BF_NB * cols; t += BF_THREADS) bf_w[i64(t / cols) * w + t % cols] = p.w[i64(t / cols) * w + t % cols];
+                W = bf_w;
+                __syncthreads();
+            }
             // a warp per row a, rows dealt out over the other CTAs
             for (int a = (rank - 1) + (BF_CTAS - 1) * warp; a < m; a += (BF_CTAS - 1) * (BF_THREADS / 32)) {
                 double wa[BF_NB];

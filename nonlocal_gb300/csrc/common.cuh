@@ -30,6 +30,7 @@ struct error : std::runtime_error {
 };
 
 [[noreturn]] inline void cuda_fail(cudaError_t e, const char* what, const char* file, int line) {
+    (void)cudaGetLastError();   // reported here, not by the next launch's check
     const int code = e == cudaErrorMemoryAllocation ? NLGPU_ERR_OUT_OF_MEMORY : NLGPU_ERR_CUDA;
     throw error{code, std::string{what} + ": " + cudaGetErrorString(e) + " (" + file + ":" + std::to_string(line) + ")"};
 }
@@ -44,6 +45,19 @@ struct error : std::runtime_error {
     do {                                                                       \
         if (!(cond)) throw ::nlgpu::error{(code), (msg)};                      \
     } while (0)
+
+// The kernel may use all the shared memory of a block.  The same value on every call:
+// the attribute belongs to the process, and with each call setting its own size one
+// thread's launch could fail on the smaller size another had just set.
+template<class K>
+inline void allow_shared(K* kernel) {
+    int dev = 0, optin = 0;
+    cudaFuncAttributes fa{};
+    NL_CUDA(cudaGetDevice(&dev));
+    NL_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    NL_CUDA(cudaFuncGetAttributes(&fa, kernel));
+    NL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - int(fa.sharedSizeBytes)));
+}
 
 // Kernel launches issued by the library (all host threads).  A launch made
 // while this thread captures a stream into a graph counts into the capture's

@@ -630,7 +630,7 @@ bool upper_to_f32(Ctx& ctx, Csr& A, const Csr& upper) {
     NL_CUDA(cudaStreamSynchronize(ctx.stream));
     const size_t bytes = size_t(std::max(h[1], 1)) * sizeof(float);
     if (h[0] || bytes + 2048 > size_t(std::min(smem_optin, smem_sm))) return false;
-    NL_CUDA(cudaFuncSetAttribute(k_spmv32_up, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+    allow_shared(k_spmv32_up);
     A.up_blocks = blocks;
     A.up_window_max = std::max(h[1], 1);
     return true;

@@ -555,7 +555,7 @@ void band_factor(Ctx& ctx, i64 n, i64 bw, double* band, double* f, BandWork& wor
     const size_t bytes = size_t(BF_NB) * size_t(bw + 1) * sizeof(double);
     p.in_shared = bytes <= 200 * 1024;
     const size_t smem = p.in_shared ? bytes : 0;
-    NL_CUDA(cudaFuncSetAttribute(k_band_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    allow_shared(k_band_factor);
     NL_CUDA(cudaFuncSetAttribute(k_band_factor, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -575,7 +575,7 @@ void band_factor(Ctx& ctx, i64 n, i64 bw, double* band, double* f, BandWork& wor
 void band_solve(Ctx& ctx, i64 n, i64 bw, const double* band, const BandWork& work, double* f, bool forward) {
     const bool in_shared = n <= 24 * 1024;   // the vector in shared memory
     const size_t smem = in_shared ? size_t(n) * sizeof(double) : 0;
-    NL_CUDA(cudaFuncSetAttribute(k_band_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    allow_shared(k_band_solve);
     NL_LAUNCH(k_band_solve, 1, BF_THREADS, smem, ctx.stream, n, bw, band, work.linv.p, work.dinv.p, f, forward, in_shared);
 }
 

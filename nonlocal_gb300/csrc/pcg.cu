@@ -639,7 +639,7 @@ __global__ void k_jacobi_diag64(i64 n, const i64* __restrict__ u_rp, const doubl
 template<bool ILLT>
 void pcg_launch(Ctx& ctx, unsigned grid, size_t smem, PcgArgs& a) {
     auto kernel = k_pcg<ILLT>;
-    NL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    allow_shared(kernel);
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;

@@ -190,7 +190,7 @@ void node_graph(Ctx& ctx, bool local_graph, std::vector<i64>& offsets, std::vect
         a.global_bits = gbits.p;
     }
     auto set_smem = [&](auto kernel) {
-        if (smem > 48 * 1024) NL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        if (smem > 48 * 1024) allow_shared(kernel);
     };
     if (nen == 4) { set_smem(k_node_graph<4, false>); set_smem(k_node_graph<4, true>); }
     else { set_smem(k_node_graph<8, false>); set_smem(k_node_graph<8, true>); }

@@ -51,7 +51,7 @@ def test_threads(T):
 
     def work(seed):
         try:
-            for k, n in enumerate(SIZES[seed:] + SIZES[:seed]):
+            for k, n in enumerate((SIZES[seed:] + SIZES[:seed]) * 6):
                 if not check(T, T.Context(), n, seed + k):
                     bad.append((seed, n))
         except Exception as e:   # reported by the main thread

@@ -303,8 +303,12 @@ __global__ void k_full_map(i64 n, const i64* __restrict__ up_rp, const int32_t* 
             map[k] = upper_entry(up_rp, up_col, full_rp[r], full_col, r, k, symmetric);
 }
 
-// The full rows' values straight from the upper storage, where no map is kept:
-// a search per entry (short rows) ...
+// The full rows' values straight from the upper storage, where no map is kept: a
+// search per entry.  745 million entries of 2 750 a row: 10.3 ms numbered row by row,
+// 37.6 with randomly numbered nodes.  (Moving along the upper rows in tiles of 32
+// columns took 7.7, 1.2 for the rows' upper parts and the clearing of both copies, 3 ms
+// more in all with the FP32 copy; numbered at random, where a tile holds one or two
+// entries, 79.7 + 1.2.)
 __global__ void k_full_search(i64 n, const i64* __restrict__ up_rp, const int32_t* __restrict__ up_col,
                               const double* __restrict__ up_val, const i64* __restrict__ full_rp,
                               const int32_t* __restrict__ full_col, double* __restrict__ full_val,
@@ -320,106 +324,19 @@ __global__ void k_full_search(i64 n, const i64* __restrict__ up_rp, const int32_
         }
 }
 
-// ... or the entries right of the diagonal copied as they lie and the padding after
-// them cleared (a warp per row; without symmetry the whole row) ...
-__global__ void k_full_upper(i64 n, const i64* __restrict__ up_rp, const double* __restrict__ up_val,
-                             const i64* __restrict__ full_rp, const int32_t* __restrict__ full_col, bool symmetric,
-                             double* __restrict__ full_val, float* __restrict__ full32) {
+// the rows of a non-symmetric system copied as they lie, the padding after them
+// cleared (a warp per row)
+__global__ void k_full_copy(i64 n, const i64* __restrict__ up_rp, const double* __restrict__ up_val,
+                            const i64* __restrict__ full_rp, double* __restrict__ full_val, float* __restrict__ full32) {
     const int lane = threadIdx.x & 31;
     const i64 warps = i64(gridDim.x) * (blockDim.x >> 5);
     for (i64 r = (blockIdx.x * i64(blockDim.x) + threadIdx.x) >> 5; r < n; r += warps) {
-        const i64 ub = up_rp[r], fe = full_rp[r + 1];
+        const i64 ub = up_rp[r], fb = full_rp[r], fe = full_rp[r + 1];
         const i64 len = up_rp[r + 1] - ub;
-        i64 lo = full_rp[r];
-        if (symmetric) {   // the diagonal: the first column not left of it
-            i64 hi = fe;
-            while (lo < hi) { const i64 mid = (lo + hi) >> 1; if (full_col[mid] < int32_t(r)) lo = mid + 1; else hi = mid; }
-        }
-        for (i64 k = lane; lo + k < fe; k += 32) {
+        for (i64 k = lane; fb + k < fe; k += 32) {
             const double v = k < len ? up_val[ub + k] : 0.0;
-            full_val[lo + k] = v;
-            if (full32) full32[lo + k] = float(v);
-        }
-    }
-}
-
-// ... and the transposed ones left of it: a warp takes `rows` consecutive rows c of the
-// upper storage and moves along them a tile of 32 columns r at a time, lane r keeping
-// its place in full row r.  A row's entries in the tile are read together
-// (FL_AHEAD rows in flight) and reach their lanes by shuffles; no entry is searched
-// for, a tile costs one search per lane.  A search per entry, a map of 8 bytes each
-// and a gather through it took 15.7 ms on 745 million entries; this takes 8.0 (9.4
-// with four rows in flight, 9.2 through a tile of shared memory written
-// row by row), clearing and k_full_upper 3.  What bounds it is the
-// 8-byte stores, one line each.  Full entries that no upper entry matches stay
-// 0 (the caller has cleared them).
-constexpr int FL_AHEAD = 8;
-__global__ void __launch_bounds__(256) k_full_lower(i64 n, int rows, const i64* __restrict__ up_rp,
-                                                    const int32_t* __restrict__ up_col,
-                                                    const double* __restrict__ up_val, const i64* __restrict__ full_rp,
-                                                    const int32_t* __restrict__ full_col, double* __restrict__ full_val,
-                                                    float* __restrict__ full32) {
-    const unsigned all = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const i64 warps = i64(gridDim.x) * (blockDim.x >> 5);
-    for (i64 c0 = ((blockIdx.x * i64(blockDim.x) + threadIdx.x) >> 5) * rows; c0 < n; c0 += warps * rows) {
-        const i64 base = up_rp[c0];
-        // row c0 + lane: its next entry's place (from `base`), its end, and that entry's column
-        int at = 0, end = 0, next = 0x7fffffff;
-        if (lane < rows && c0 + lane < n) {
-            at = int(up_rp[c0 + lane] - base);
-            end = int(up_rp[c0 + lane + 1] - base);
-            if (at < end && up_col[base + at] == int32_t(c0 + lane)) ++at;   // the diagonal
-            if (at < end) next = up_col[base + at];
-        }
-        for (;;) {
-            const int r0 = __reduce_min_sync(all, next);
-            if (r0 == 0x7fffffff) break;
-            const i64 r = i64(r0) + lane;
-            i64 pos = 0;
-            int32_t cur = 0x7fffffff;
-            if (r < n) {   // the first entry of full row r from column c0 on (c0 < r: left of the diagonal or at it)
-                i64 lo = full_rp[r], hi = full_rp[r + 1];
-                const i64 row_end = hi;
-                while (lo < hi) { const i64 mid = (lo + hi) >> 1; if (full_col[mid] < int32_t(c0)) lo = mid + 1; else hi = mid; }
-                pos = lo;
-                if (lo < row_end) cur = full_col[lo];
-            }
-            for (unsigned todo = __ballot_sync(all, next - r0 < 32); todo;) {
-                int b[FL_AHEAD];
-                int32_t col[FL_AHEAD];
-                double v[FL_AHEAD];
-#pragma unroll
-                for (int u = 0; u < FL_AHEAD; ++u) {
-                    b[u] = todo ? __ffs(todo) - 1 : -1;
-                    todo &= todo - 1;
-                    const int from = __shfl_sync(all, at, b[u] & 31), to = __shfl_sync(all, end, b[u] & 31);
-                    const bool in = b[u] >= 0 && from + lane < to;
-                    col[u] = in ? up_col[base + from + lane] : 0x7fffffff;
-                    v[u] = in ? up_val[base + from + lane] : 0.0;
-                }
-#pragma unroll
-                for (int u = 0; u < FL_AHEAD; ++u) {
-                    if (b[u] < 0) break;
-                    const unsigned present = __reduce_or_sync(all, col[u] - r0 < 32 ? 1u << (col[u] - r0) : 0u);
-                    const int count = __popc(present);
-                    const double mine = __shfl_sync(all, v[u], __popc(present & ((1u << lane) - 1u)) & 31);
-                    if (present >> lane & 1u) {
-                        const int32_t c = int32_t(c0) + b[u];
-                        while (cur < c) cur = full_col[++pos];   // ends at the diagonal at the latest
-                        if (cur == c) {
-                            full_val[pos] = mine;
-                            if (full32) full32[pos] = float(mine);
-                            cur = full_col[++pos];
-                        }
-                    }
-                    const int32_t after = __shfl_sync(all, col[u], count & 31);
-                    if (lane == b[u]) {
-                        at += count;
-                        next = count < 32 ? after : at < end ? up_col[base + at] : 0x7fffffff;
-                    }
-                }
-            }
+            full_val[fb + k] = v;
+            if (full32) full32[fb + k] = float(v);
         }
     }
 }
@@ -434,31 +351,19 @@ void full_map(Ctx& ctx, const Csr& upper, const Csr& full, dbuf<i64>& map, bool 
 
 // The values of the full rows from the upper storage: through the map where one
 // was built (matrices that are filled again and again: radiation, the elasticity
-// systems), straight otherwise; rows of a non-symmetric system are copied.  Below 1024 entries a row on average a search per
-// entry is as fast as the tiles of k_full_lower (200 x 200 4-node, 350 entries: 0.22 ms
-// both; 71 x 53 8-node: 0.10) and faster on the smallest; the rows per warp are
-// as many as leave every SM 32 warps.
+// systems), by a search per entry otherwise; rows of a non-symmetric system are copied.
 void fill_full_from_upper(Ctx& ctx, const Csr& upper, Csr& full, const dbuf<i64>& map, bool symmetric) {
     full.val.resize(size_t(full.nnz));
     float* val32 = full.val32.n == size_t(full.nnz) ? full.val32.p : nullptr;
     const i64 n = full.rows;
-    if (map.n == size_t(full.nnz)) {
+    const unsigned grid = grid_for(n * 32, 256, 152 * 64);
+    if (map.n == size_t(full.nnz))
         gather_full(ctx, full, map, upper.val.p, val32);
-    } else if (!symmetric) {
-        NL_LAUNCH(k_full_upper, grid_for(n * 32, 256, 152 * 64), 256, 0, ctx.stream, n, upper.rowptr.p, upper.val.p,
-                  full.rowptr.p, full.col.p, false, full.val.p, val32);
-    } else if (full.nnz < 1024 * n) {
-        NL_LAUNCH(k_full_search, grid_for(n * 32, 256, 152 * 64), 256, 0, ctx.stream, n, upper.rowptr.p, upper.col.p,
-                  upper.val.p, full.rowptr.p, full.col.p, full.val.p, val32);
-    } else {
-        full.val.zero(ctx.stream);
-        if (val32) full.val32.zero(ctx.stream);
-        NL_LAUNCH(k_full_upper, grid_for(n * 32, 256, 152 * 64), 256, 0, ctx.stream, n, upper.rowptr.p, upper.val.p,
-                  full.rowptr.p, full.col.p, true, full.val.p, val32);
-        const int rows = int(std::max<i64>(1, std::min<i64>(32, n / (152 * 32))));
-        NL_LAUNCH(k_full_lower, grid_for((n + rows - 1) / rows * 32, 256, 152 * 64), 256, 0, ctx.stream, n, rows,
-                  upper.rowptr.p, upper.col.p, upper.val.p, full.rowptr.p, full.col.p, full.val.p, val32);
-    }
+    else if (symmetric)
+        NL_LAUNCH(k_full_search, grid, 256, 0, ctx.stream, n, upper.rowptr.p, upper.col.p, upper.val.p, full.rowptr.p,
+                  full.col.p, full.val.p, val32);
+    else
+        NL_LAUNCH(k_full_copy, grid, 256, 0, ctx.stream, n, upper.rowptr.p, upper.val.p, full.rowptr.p, full.val.p, val32);
 }
 
 void build_patterns(Ctx& ctx, bool local_only, bool symmetric, Csr& inner, Csr* bound, Csr* full,

@@ -123,8 +123,12 @@ __device__ __forceinline__ void load_nodes(const int32_t* __restrict__ elems, in
 // beyond that window are expanded every time).  The set bits are then
 // classified a word at a time against the inner-node bitmap and emitted in
 // increasing order, 32 words per round with a warp scan of the counts: the
-// reference's sorted column list without a sort.  (Writing each lane's own word bit by bit, scattered stores: 300x300
-// 8-node elements, count and fill, 12.6 ms instead of 11.3.)
+// reference's sorted column list without a sort.  Rounds with a word of more than
+// PW_SPARSE bits are written a word at a time with a lane per bit, the others by each
+// lane for its own word.  300x300 8-node elements, the fill pass numbered row by row
+// and at random: words 6.1 and 62.1 ms, lanes 8.3 and 35.9.
+constexpr int PW_SPARSE = 4;
+
 template<int NEN>
 __global__ void __launch_bounds__(PW_WARPS * 32) k_pattern(PatternArgs a) {
     extern __shared__ uint32_t pw_smem[];
@@ -237,18 +241,27 @@ __global__ void __launch_bounds__(PW_WARPS * 32) k_pattern(PatternArgs a) {
                 }
                 const unsigned long long tot = __shfl_sync(full, incl, 31);
                 if (fill) {
-                    // a word at a time, a lane per bit: the stores of a word are contiguous
                     const unsigned long long ex = incl - c;
                     const unsigned long long f21 = (1ull << 21) - 1;
-                    const uint32_t before = (1u << lane) - 1u;
-                    for (unsigned words = __ballot_sync(full, (mi | mb | mf) != 0u); words; words &= words - 1) {
-                        const int s = __ffs(words) - 1;
-                        const uint32_t wi = __shfl_sync(full, mi, s), wb = __shfl_sync(full, mb, s), wf = __shfl_sync(full, mf, s);
-                        const unsigned long long at = __shfl_sync(full, ex, s);
-                        const int32_t node = int32_t(base + i64(w0 + s) * 32 + lane);
-                        if (wi >> lane & 1u) a.col_inner[to_inner + n_inner + i64(at & f21) + __popc(wi & before)] = node;
-                        if (wb >> lane & 1u) a.col_bound[to_bound + n_bound + i64((at >> 21) & f21) + __popc(wb & before)] = node;
-                        if (wf >> lane & 1u) a.col_full[to_full + n_full + i64(at >> 42) + __popc(wf & before)] = node;
+                    if (__reduce_max_sync(full, __popc(mi | mb | mf)) > PW_SPARSE) {
+                        // a word at a time, a lane per bit: the stores of a word are contiguous
+                        const uint32_t before = (1u << lane) - 1u;
+                        for (unsigned words = __ballot_sync(full, (mi | mb | mf) != 0u); words; words &= words - 1) {
+                            const int s = __ffs(words) - 1;
+                            const uint32_t wi = __shfl_sync(full, mi, s), wb = __shfl_sync(full, mb, s), wf = __shfl_sync(full, mf, s);
+                            const unsigned long long at = __shfl_sync(full, ex, s);
+                            const int32_t node = int32_t(base + i64(w0 + s) * 32 + lane);
+                            if (wi >> lane & 1u) a.col_inner[to_inner + n_inner + i64(at & f21) + __popc(wi & before)] = node;
+                            if (wb >> lane & 1u) a.col_bound[to_bound + n_bound + i64((at >> 21) & f21) + __popc(wb & before)] = node;
+                            if (wf >> lane & 1u) a.col_full[to_full + n_full + i64(at >> 42) + __popc(wf & before)] = node;
+                        }
+                    } else {   // each lane the few bits of its own word
+                        i64 pi = to_inner + n_inner + i64(ex & f21);
+                        i64 pb = to_bound + n_bound + i64((ex >> 21) & f21);
+                        i64 pf = to_full + n_full + i64(ex >> 42);
+                        for (uint32_t t = mi; t; t &= t - 1) a.col_inner[pi++] = int32_t(nb + __ffs(t) - 1);
+                        for (uint32_t t = mb; t; t &= t - 1) a.col_bound[pb++] = int32_t(nb + __ffs(t) - 1);
+                        for (uint32_t t = mf; t; t &= t - 1) a.col_full[pf++] = int32_t(nb + __ffs(t) - 1);
                     }
                 }
                 n_inner += i64(tot & ((1ull << 21) - 1));

@@ -34,3 +34,33 @@ def test_one_kernel_fills_the_full_rows(lib):
         pb.conductivity_matrix("FULL")
         launches.append(lib.kernel_launches() - before)
     assert launches[0] == launches[1]
+
+
+@pytest.mark.parametrize("element, nx, ny, radius", [("bilinear", 60, 50, 0.1), ("bilinear", 60, 50, 0.03),
+                                                     ("serendipity", 30, 20, 0.12)])
+def test_pattern_of_scattered_nodes(lib, element, nx, ny, radius):
+    """Words of a few bits and of many in one row: the pattern of randomly numbered nodes, and of nodes of which a
+    half keeps its order, is the permuted pattern of the mesh as numbered row by row."""
+    from nonlocal_gb300.meshgen import relabel_nodes, structured_quad_mesh
+    mesh = structured_quad_mesh(nx, ny, element)
+    n = mesh.n_nodes
+
+    def pairs(m, to_row):
+        pb = problem(m, radius)
+        pb.conductivity_matrix("FULL")
+        out = []
+        for which in ("inner", "bound"):
+            rp, col, _ = pb.matrix(which)
+            row = np.repeat(np.arange(n), np.diff(rp))
+            assert all(np.all(np.diff(col[rp[r]:rp[r + 1]]) > 0) for r in range(n))
+            a, b = to_row[row], to_row[col]
+            out.append(np.unique(np.minimum(a, b) * n + np.maximum(a, b) if which == "inner" else a * n + b))
+        return out
+
+    expected = pairs(mesh, np.arange(n))
+    rng = np.random.default_rng(3)
+    half = np.arange(n)
+    half[n // 2:] = n // 2 + rng.permutation(n - n // 2)
+    for perm in (rng.permutation(n), half):
+        for e, g in zip(expected, pairs(relabel_nodes(mesh, perm), np.argsort(perm))):
+            assert np.array_equal(e, g)

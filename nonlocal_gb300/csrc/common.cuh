@@ -344,6 +344,7 @@ enum { P_PQ = 0, P_RR = 1, P_RZ_A = 2, P_RZ_B = 3, P_BB = 4, P_COUNT = 5 };   //
 struct IncompleteCholesky {
     SweepPlan fwd_plan, bwd_plan;
     i64 n = 0, nnz = 0;
+    double mean_reach = 0.0;     // of a row: its last column minus its own
     dbuf<i64> rp;                // upper pattern (diagonal first)
     dbuf<int32_t> col;
     dbuf<double> a_scaled, u;    // S A S and the factor values

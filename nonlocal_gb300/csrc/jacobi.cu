@@ -25,7 +25,7 @@
 // the float and the step's number, which a reader polls until the number is
 // there: no barrier, no launch between sweeps, and a row waits only for the rows
 // of its band.  k_jacobi32 is one sweep per launch (thread per row), for systems
-// whose sweeps are bound by bandwidth (JA_MAX_ROWS).
+// whose sweeps are bound by bandwidth (JA_MAX_NEAR, JA_MAX_FAR).
 #include "common.cuh"
 
 #include <algorithm>
@@ -95,14 +95,25 @@ __global__ void __launch_bounds__(JB_THREADS) k_jacobi32(i64 n, const i64* __res
 
 // The application in one launch (see the top).  Bound by the 2 k dependent steps,
 // each a store and a load through L2 (a message between SMs of different dies
-// takes about 0.45 us) and the row's sum.  Microseconds an application of twelve
-// sweeps, the kernels of one launch per sweep (without the gaps between them) ->
-// this: 40 401 rows of 4 (200x200 bilinear) 21 -> 16; 163 000 rows of 4 (a dozen
-// systems) 24 -> 23; 56 454 rows of 4 28 -> 18; 271 201 rows of 10 (300x300 8-node)
-// 48 -> 50.
+// takes about 0.45 us) and the row's sum; a gather of a value from far away moves a
+// 32-byte sector past L1 for its 8 bytes, where k_jacobi32 gathers floats through L1.
+// Which form: by the entries of a triangle, with the rows' mean reach against a
+// CTA's rows.  Microseconds an FCG iteration (twelve sweeps and everything else), one launch per
+// sweep -> this:
+//   near columns   bilinear 500x500, 1.0 million entries    109 -> 97
+//                  bilinear 600x600, 1.4                    144 -> 132
+//                  8-node 300x300, 2.0                      140 -> 151
+//   far ones       8-node 170x170, nonlocal cuthill_mckee, 0.64    186 -> 173
+//                  the same numbered at random              357 -> 349
+//                  bilinear 400x400 at random, 0.64         125 -> 124
+//                  8-node 200x200, nonlocal cuthill_mckee, 0.88    324 -> 383
+//                  bilinear 500x500 at random, 1.0          157 -> 170
+//                  8-node 300x300, local cuthill_mckee, 2.0 148 -> 276
 constexpr int JA_THREADS = 1024;
 constexpr int JA_MIN_ROWS = 64;
-constexpr i64 JA_MAX_ROWS = 400000;
+constexpr i64 JA_MAX_NEAR = 1700000, JA_MAX_FAR = 700000;   // entries of a triangle
+constexpr double JA_FAR = 4.0;    // mean reach in CTAs
+constexpr i64 JA_MAX_ROWS = 400000;    // 361 201 measured
 constexpr int JA_MAX_SWEEPS = 32;
 constexpr int JA_BATCH = 4;       // gathers in flight per lane
 constexpr unsigned long long JA_WAIT_LIMIT_NS = 2000000000ull;
@@ -253,13 +264,12 @@ void jacobi_fill(Ctx& ctx, IncompleteCholesky& ic) {
 void jacobi_apply32(Ctx& ctx, IncompleteCholesky& ic, int sweeps, const float* r, float* z, const double* flags) {
     NL_REQUIRE(sweeps >= 1, NLGPU_ERR_ARG, "at least one Jacobi sweep per triangle");
     const i64 n = ic.n;
-    // one launch for the whole application unless bandwidth bounds the sweeps, or a
-    // row's neighbours are too many or too far apart to be worth polling
-    if (n <= JA_MAX_ROWS && sweeps <= JA_MAX_SWEEPS) {
-        int dev = 0, sms = 0;
-        NL_CUDA(cudaGetDevice(&dev));
-        NL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        const i64 rows = std::max<i64>(JA_MIN_ROWS, ((n + sms - 1) / sms + 31) / 32 * 32);
+    int dev = 0, sms = 0;
+    NL_CUDA(cudaGetDevice(&dev));
+    NL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const i64 rows = std::max<i64>(JA_MIN_ROWS, ((n + sms - 1) / sms + 31) / 32 * 32);
+    const bool far = ic.mean_reach > JA_FAR * double(rows);
+    if (n <= JA_MAX_ROWS && ic.nnz - n <= (far ? JA_MAX_FAR : JA_MAX_NEAR) && sweeps <= JA_MAX_SWEEPS) {
         const unsigned grid = unsigned((n + rows - 1) / rows);
         const size_t words = size_t(sweeps + 1) * size_t(n);
         // the CTAs' numbers go on from application to application; another split starts

@@ -227,6 +227,7 @@ __global__ void __launch_bounds__(PW_WARPS * 32) k_pattern(PatternArgs a) {
                     m = bm[w];
                     if (m) iw = a.inner_bits[nb >> 5];
                 }
+                if (!__any_sync(full, m != 0u)) continue;
                 const uint32_t mf = row_inner ? (m & iw) : 0u;
                 const uint32_t mi = a.symmetric ? (mf & mask_from(r, nb)) : mf;
                 const uint32_t mb = m & ~iw & ~bit_of(r, nb);

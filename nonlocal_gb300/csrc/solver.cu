@@ -8,8 +8,10 @@
 //
 // cg_solve runs the persistent kernel of pcg.cu (identity, or the ILLT applied by
 // FP64 Jacobi sweeps).  Here are the ILLT factorisation, the products the other
-// solvers share, and CG with the exact triangular solves, for the factors whose
-// Jacobi sweeps contract too slowly and for NLGPU_OPTION_GLOBAL_SWEEPS:
+// solvers share, and CG with one launch per phase: with the exact triangular solves,
+// for the factors whose Jacobi sweeps contract too slowly and for
+// NLGPU_OPTION_GLOBAL_SWEEPS, and with the identity on large systems
+// (CG_ONE_LAUNCH_ENTRIES):
 //   * SpMV on full-row CSR (both triangles): a group of lanes per row, no atomics;
 //   * all CG scalars stay on the device: reductions write one partial per
 //     block, and every block of the consuming kernel re-adds the partials in a
@@ -38,6 +40,13 @@ namespace {
 
 constexpr int RED_THREADS = 256;
 constexpr int GRAPH_ITERS = 16;
+// Identity-preconditioned CG as one kernel (pcg.cu) up to this many entries, where the
+// product is bound by HBM and a CTA of 16 warps per SM has too few loads in flight;
+// one launch per phase above.  Microseconds an iteration, one kernel / launches:
+// 8-node 110x110 r = 0.05 76 / 97, 130x130 (26 million entries) 129 / 130, bilinear 300x300
+// r = 0.03 (25) 132 / 142, 8-node 150x150 (47) 213 / 184, 8-node 300x300 (745) 2 480 / 1 650,
+// local 2000x2000 (36) 288 / 259.
+constexpr i64 CG_ONE_LAUNCH_ENTRIES = i64(32) << 20;
 constexpr int TRI_THREADS = 1024;
 
 __device__ __forceinline__ double block_sum(double v, double* sh) {
@@ -130,10 +139,10 @@ __global__ void __launch_bounds__(RED_THREADS) k_update_xr(i64 n, double* __rest
     (void)max_iterations;
 }
 
-// converged when |r| <= tol |b| (every block decides the same way)
+// done when |r| <= tol |b|, or r is no longer finite (every block decides the same way)
 __device__ __forceinline__ bool converged(const double* partials, const double* flags, double tol2, double* sh) {
     const double rr = sum_partials(partials + P_RR * RED_BLOCKS, sh);
-    return rr <= tol2 * flags[S_BB];
+    return rr <= tol2 * flags[S_BB] || !isfinite(rr);
 }
 
 // beta = rz_new / rz_old; p = z + beta p; raises the done flag on convergence
@@ -749,19 +758,18 @@ void ilt_apply(Ctx& ctx, const IncompleteCholesky& ic, const double* r, double* 
 
 CgResult cg_solve(Ctx& ctx, const Csr& A, const IncompleteCholesky* M, const double* b, double* x,
                   double tolerance, i64 max_iterations, bool x_is_initial_guess, const CgChunkHook& on_chunk) {
-    if (!(M && ctx.force_global_sweeps)) {
+    if (M ? !ctx.force_global_sweeps : A.nnz <= CG_ONE_LAUNCH_ENTRIES) {
         CgResult r;
         if (pcg_solve(ctx, A, M, b, x, tolerance, max_iterations, x_is_initial_guess, on_chunk, r)) return r;
     }
-    // exact triangular sweeps and the exact factor: asked for, or a factor whose Jacobi
-    // sweeps contract too slowly
-    ilt_make_exact(ctx, const_cast<IncompleteCholesky&>(*M));
-    if (!M->ok) {
-        CgResult r;   // the identity when the exact factorisation breaks down
-        pcg_solve(ctx, A, nullptr, b, x, tolerance, max_iterations, x_is_initial_guess, on_chunk, r);
-        return r;
+    if (M) {
+        // exact triangular sweeps and the exact factor: asked for, or a factor whose Jacobi
+        // sweeps contract too slowly
+        ilt_make_exact(ctx, const_cast<IncompleteCholesky&>(*M));
+        if (!M->ok)   // the identity when the exact factorisation breaks down
+            return cg_solve(ctx, A, nullptr, b, x, tolerance, max_iterations, x_is_initial_guess, on_chunk);
+        ilt_exact_layouts(ctx, const_cast<IncompleteCholesky&>(*M));
     }
-    ilt_exact_layouts(ctx, const_cast<IncompleteCholesky&>(*M));
     const i64 n = A.rows;
     CgWork& w = ctx.cg;
     w.n = n;
@@ -771,6 +779,7 @@ CgResult cg_solve(Ctx& ctx, const Csr& A, const IncompleteCholesky* M, const dou
     if (!x_is_initial_guess) NL_CUDA(cudaMemsetAsync(x, 0, size_t(n) * sizeof(double), ctx.stream));
     double* part = w.partial.p;
     double* flags = w.scalars.p;
+    const double* z = M ? w.z.p : w.r.p;   // M^-1 r
     const double tol2 = tolerance * tolerance;
     CgResult res;
     // |b|^2
@@ -782,9 +791,9 @@ CgResult cg_solve(Ctx& ctx, const Csr& A, const IncompleteCholesky* M, const dou
         // r = b - A x; z = M^-1 r; p = z; rz -> P_RZ_B (the "current" buffer of an even iteration)
         spmv_full(ctx, A, x, w.r.p);
         NL_LAUNCH(k_residual, RED_BLOCKS, RED_THREADS, 0, ctx.stream, n, b, w.r.p, part + P_RR * RED_BLOCKS);
-        precondition(ctx, M, w.r.p, w.z.p, nullptr, nullptr, 0.0);
-        NL_LAUNCH(k_copy, grid_for(n, 256), 256, 0, ctx.stream, n, w.z.p, w.p.p);
-        NL_LAUNCH(k_dot, RED_BLOCKS, RED_THREADS, 0, ctx.stream, n, w.r.p, w.z.p, part + P_RZ_B * RED_BLOCKS,
+        if (M) precondition(ctx, M, w.r.p, w.z.p, nullptr, nullptr, 0.0);
+        NL_LAUNCH(k_copy, grid_for(n, 256), 256, 0, ctx.stream, n, z, w.p.p);
+        NL_LAUNCH(k_dot, RED_BLOCKS, RED_THREADS, 0, ctx.stream, n, w.r.p, z, part + P_RZ_B * RED_BLOCKS,
                   static_cast<const double*>(nullptr));
         double host[8];
         NL_CUDA(cudaMemsetAsync(flags + S_DONE, 0, sizeof(double), ctx.stream));
@@ -806,11 +815,10 @@ CgResult cg_solve(Ctx& ctx, const Csr& A, const IncompleteCholesky* M, const dou
                 NL_LAUNCH(k_dot, RED_BLOCKS, RED_THREADS, 0, ctx.stream, n, w.p.p, w.q.p, part + P_PQ * RED_BLOCKS, flags);
                 NL_LAUNCH(k_update_xr, RED_BLOCKS, RED_THREADS, 0, ctx.stream, n, x, w.r.p, w.p.p, w.q.p, part, parity,
                           flags, max_iterations);
-                precondition(ctx, M, w.r.p, w.z.p, part, flags, tol2);
-                NL_LAUNCH(k_dot, RED_BLOCKS, RED_THREADS, 0, ctx.stream, n, w.r.p, w.z.p,
+                if (M) precondition(ctx, M, w.r.p, w.z.p, part, flags, tol2);
+                NL_LAUNCH(k_dot, RED_BLOCKS, RED_THREADS, 0, ctx.stream, n, w.r.p, z,
                           part + (parity ? P_RZ_B : P_RZ_A) * RED_BLOCKS, flags);
-                NL_LAUNCH(k_update_p, RED_BLOCKS, RED_THREADS, 0, ctx.stream, n, w.p.p, w.z.p, part, parity, flags, tol2,
-                          max_iterations);
+                NL_LAUNCH(k_update_p, RED_BLOCKS, RED_THREADS, 0, ctx.stream, n, w.p.p, z, part, parity, flags, tol2, max_iterations);
             }
             NL_CUDA(cudaMemcpyAsync(host, flags, 8 * sizeof(double), cudaMemcpyDeviceToHost, ctx.stream));
             NL_CUDA(cudaStreamSynchronize(ctx.stream));

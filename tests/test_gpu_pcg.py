@@ -119,3 +119,32 @@ def test_jacobi_application_sizes(ctx, n, band):
     tol = (2 * (band + 4) * np.finfo(np.float32).eps + 2.5 ** -24) * np.abs(exact).max()
     for sweeps in (24, 32, 33):
         assert np.abs(pre.solve_f32(x, sweeps) - exact).max() <= tol, sweeps
+
+
+def test_large_identity_systems_go_by_launches():
+    """34 million entries and more: a launch per phase, so several an iteration; fewer: one kernel for them all."""
+    from nonlocal_gb300 import _lib
+    from nonlocal_gb300 import thermal as T
+    from nonlocal_gb300.meshgen import structured_quad_mesh
+    if _lib.device_count() == 0:
+        pytest.skip("no CUDA device")
+    mesh = structured_quad_mesh(200, 150, "bilinear")
+    for radius, large in ((0.05, False), (0.13, True)):
+        pb = T.Problem2D.from_mesh(mesh)
+        pb.set_model(T.Model2D(influence="fast_polynomial", radius=(radius, radius), local_weight=0.5))
+        pb.add_boundary(T.Boundary(edges=mesh.boundaries["left"], kind="temperature", value=1.0))
+        pb.add_boundary(T.Boundary(edges=mesh.boundaries["right"], kind="flux", value=0.7))
+        pb.find_neighbours()
+        pb.conductivity_matrix("FULL")
+        before = _lib.kernel_launches()
+        x, rep = pb.solve_assembled(tolerance=1e-11, preconditioner="identity")
+        launches = _lib.kernel_launches() - before
+        assert (rep.nnz_solver > 2 ** 25) == large
+        assert launches >= 5 * rep.iterations if large else launches < rep.iterations
+        assert rep.residual <= 1e-11
+        y, ref = pb.solve_assembled(tolerance=1e-11)   # ILLT
+        # both residuals at most 1e-11 |b|; |A^-1| |b| / |x| <= the condition number, below 1e6 here
+        assert np.linalg.norm(x - y) <= 2e-5 * np.linalg.norm(y)
+        with pytest.raises(_lib.NlgpuError) as e:   # the limit of iterations
+            pb.solve_assembled(tolerance=1e-11, preconditioner="identity", max_iterations=1)
+        assert e.value.status == 6

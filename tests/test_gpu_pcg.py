@@ -148,3 +148,67 @@ def test_large_identity_systems_go_by_launches():
         with pytest.raises(_lib.NlgpuError) as e:   # the limit of iterations
             pb.solve_assembled(tolerance=1e-11, preconditioner="identity", max_iterations=1)
         assert e.value.status == 6
+
+
+def arrow(n, dense):
+    """A diagonally dominant arrow: the rows in `dense` hold every column (eigenvalues 1 to 3 times the diagonal's
+    smallest by Gershgorin's circles)."""
+    import scipy.sparse as sp
+    rng = np.random.default_rng(n)
+    rows = [sp.csr_matrix((rng.uniform(-1.0, 1.0, n - 1 - r), (np.full(n - 1 - r, r), np.arange(r + 1, n))), shape=(n, n))
+            for r in dense]
+    U = sum(rows[1:], rows[0])
+    A = (U + U.T).tocsr()
+    d = 2.0 * np.maximum(np.asarray(abs(A).sum(axis=1)).ravel(), 1.0)
+    return (A + sp.diags(d)).tocsr(), (U + sp.diags(d)).tocsr()
+
+
+@pytest.mark.parametrize("n, dense", [(255, [0]), (256, [0]), (257, [0, 3]), (513, [5]), (1025, [0, 1]),
+                                      (5000, [0, 2500, 4000]), (20011, [7])])
+def test_dense_rows(ctx, n, dense):
+    """Rows as long as the matrix: at the lengths where runs are merged, columns and rows of the full matrix."""
+    from nonlocal_gb300 import thermal as T
+    A, U = arrow(n, dense)
+    U.sort_indices()
+    csr = (U.indptr.astype(np.int64), U.indices.astype(np.int64), U.data)
+    b = np.random.default_rng(2).standard_normal(n)
+    x, rep = T.conjugate_gradient(ctx, csr, b, tolerance=1e-12)
+    assert np.linalg.norm(b - A @ x) <= 1.01e-12 * np.linalg.norm(b)
+    again, _ = T.conjugate_gradient(ctx, csr, b, tolerance=1e-12)
+    assert np.array_equal(again, x)
+
+
+def test_a_dense_row_costs_no_more_than_its_entries(ctx):
+    """120 000 columns in one row: the row's sort and its products take milliseconds.  (Ranking the row took 10 s,
+    the host's sort and the products 15 ms.)"""
+    import time
+    from nonlocal_gb300 import thermal as T
+    n = 120000
+    A, U = arrow(n, [0])
+    U.sort_indices()
+    csr = (U.indptr.astype(np.int64), U.indices.astype(np.int64), U.data)
+    b = np.random.default_rng(2).standard_normal(n)
+    T.conjugate_gradient(ctx, csr, b, tolerance=1e-10)
+    t0 = time.perf_counter()
+    x, rep = T.conjugate_gradient(ctx, csr, b, tolerance=1e-10)
+    assert time.perf_counter() - t0 < 1.0
+    assert np.linalg.norm(b - A @ x) <= 1.01e-10 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("n", [40, 700])
+def test_split_entries_are_added_in_one_order(ctx, n):
+    """Entries split into parts of very different size (equal columns in the caller's order): the same bits on every call."""
+    from nonlocal_gb300 import thermal as T
+    rng = np.random.default_rng(n)
+    rp, col, val = [0], [], []
+    for r in range(n):
+        cols = np.sort(rng.integers(r, n, 12))
+        cols[0] = r
+        col += [r] + cols.tolist()
+        val += [60.0] + (rng.standard_normal(12) * 10.0 ** rng.integers(-8, 1, 12)).tolist()
+        rp.append(len(col))
+    csr = (np.array(rp), np.array(col), np.array(val))
+    b = rng.standard_normal(n)
+    first, _ = T.conjugate_gradient(ctx, csr, b, tolerance=1e-12)
+    for _ in range(12):
+        assert np.array_equal(T.conjugate_gradient(ctx, csr, b, tolerance=1e-12)[0], first)

@@ -69,14 +69,19 @@ __global__ void k_cc_place(i64 n, const i64* __restrict__ rp, const i64* __restr
     }
 }
 
-// how many of the entries [b, b + len) come before (c, src)
+// how many of the entries [b, b + len) come before (c, src), one of them; the sources
+// decide only where a column stands twice
 __device__ __forceinline__ i64 rank_among(const int32_t* __restrict__ tcol, const i64* __restrict__ tsrc, i64 b, i64 len,
                                           int32_t c, i64 src) {
     i64 rank = 0;
+    int equal = 0;
     for (i64 j = b; j < b + len; ++j) {
         const int32_t o = __ldg(tcol + j);
-        rank += o < c || (o == c && __ldg(tsrc + j) < src);
+        rank += o < c;
+        equal += o == c;
     }
+    if (equal > 1)
+        for (i64 j = b; j < b + len; ++j) rank += __ldg(tcol + j) == c && __ldg(tsrc + j) < src;
     return rank;
 }
 
@@ -172,8 +177,8 @@ __global__ void __launch_bounds__(CC_RUN) k_cc_finish(i64 total, const i64* __re
     }
 }
 
-// the rows of more than CC_RUN entries, up to `longest`
-void sort_long_rows(Ctx& ctx, const Csr& A, const dbuf<i64>& count, i64 longest, dbuf<int32_t>& tcol, dbuf<i64>& tsrc,
+// the rows of more than CC_RUN entries
+void sort_long_rows(Ctx& ctx, const Csr& A, const dbuf<i64>& count, dbuf<int32_t>& tcol, dbuf<i64>& tsrc,
                     const dbuf<double>& values) {
     const i64 n = A.rows;
     cudaStream_t s = ctx.stream;
@@ -196,7 +201,7 @@ void sort_long_rows(Ctx& ctx, const Csr& A, const dbuf<i64>& count, i64 longest,
         std::swap(tsrc, osrc);
     };
     pass(0);
-    for (i64 width = CC_RUN; width < longest; width *= 2) pass(width);
+    for (i64 width = CC_RUN; width < A.longest; width *= 2) pass(width);
     NL_LAUNCH(k_cc_finish, grid, CC_RUN, 0, s, total, runs.p, row.p, A.rowptr.p, count.p, tcol.p, tsrc.p, values.p, A.col.p,
               A.val.p);
     NL_CUDA(cudaStreamSynchronize(s));   // the scratch buffers are freed on return
@@ -238,12 +243,13 @@ void full_rows_from_caller(Ctx& ctx, i64 n, const int64_t* rowptr, const int64_t
     exclusive_scan(ctx, A.rowptr.p, A.rowptr.p, n + 1, &total);   // synchronises
     NL_REQUIRE(h[0] == 0, NLGPU_ERR_ARG, "A must be the upper triangle with columns in range");
     A.nnz = total;
+    A.longest = i64(h[1]);
     const size_t nnz = size_t(std::max<i64>(total, 1));
     A.col.resize(nnz); A.val.resize(nnz);
     tcol.resize(nnz); tsrc.resize(nnz);
     NL_LAUNCH(k_cc_place, grid, CC_THREADS, 0, s, n, rp.p, dcol.p, first, A.rowptr.p, cursor.p, tcol.p, tsrc.p);
     NL_LAUNCH(k_cc_sort, grid, CC_THREADS, 0, s, n, A.rowptr.p, count.p, tcol.p, tsrc.p, dval.p, A.col.p, A.val.p);
-    if (i64(h[1]) > CC_RUN) sort_long_rows(ctx, A, count, i64(h[1]), tcol, tsrc, dval);
+    if (A.longest > CC_RUN) sort_long_rows(ctx, A, count, tcol, tsrc, dval);
     NL_CUDA(cudaStreamSynchronize(s));   // the scratch buffers are freed on return
 }
 

@@ -238,6 +238,7 @@ Model make_model(const nlgpu_model_2d& m);
 // CSR on the device: int64 row pointers, int32 columns.
 struct Csr {
     i64 rows = 0, nnz = 0;
+    i64 longest = 0;             // entries of the longest row of a caller's matrix (0: an assembled one)
     dbuf<i64> rowptr;
     dbuf<int32_t> col;
     dbuf<double> val;
@@ -758,6 +759,15 @@ __device__ __forceinline__ double row_part(const int32_t* __restrict__ col, cons
     }
     for (; k < end; k += g) s = fma(__ldg(val + k), x[__ldg(col + k)], s);
     return s + s2;
+}
+
+// A row far longer than the others, by a whole warp.  Every lane gets the sum.
+constexpr int LONG_ROW = 256;   // entries per lane from which on a row is taken so
+__device__ __forceinline__ double dense_row(const int32_t* __restrict__ col, const double* __restrict__ val,
+                                            const double* x, i64 begin, i64 end) {
+    double s = row_part(col, val, x, begin + (threadIdx.x & 31), end, 32);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
 }
 
 // log2 of the lanes per row of an FP64 product with rows of `mean` entries: about

@@ -256,18 +256,23 @@ __device__ __forceinline__ bool all_sync(const PcgArgs& a, Cta& c) {
 }
 
 // own q = (A v) on the CTA's rows, 2^lg lanes per row; neighbouring lanes take
-// neighbouring entries, so a gather reads runs of columns
+// neighbouring entries, so a gather reads runs of columns.  DENSE: rows of LONG_ROW << lg
+// entries and more (of a caller's matrix) take the whole warp; a variant of its own,
+// since the test alone cost the others 2.5 % of an iteration.
+template<bool DENSE>
 __device__ __forceinline__ void pcg_spmv(const PcgArgs& a, const Cta& c, const double* v) {
     const int lane = threadIdx.x & 31, g = 1 << a.lg, sub = lane & (g - 1), per = 32 >> a.lg;
     for (int i0 = int(threadIdx.x >> 5) * per; i0 < c.rows; i0 += PCG_WARPS * per) {
         const int i = i0 + (lane >> a.lg);
         double s = 0.0, s2 = 0.0;
+        bool dense = false;
         if (i < c.rows) {
             const i64 b = c.first ? c.entry0 + c.first[i] : a.rp[c.r0 + i];
             const int len = c.first ? c.first[i + 1] - c.first[i] : int(a.rp[c.r0 + i + 1] - b);
+            if constexpr (DENSE) dense = len >= LONG_ROW << a.lg;
             const int32_t* col = a.col + b;
             const double* val = a.val + b;
-            int k = sub;
+            int k = dense ? len : sub;
             for (; k + 3 * g < len; k += 4 * g) {
                 const int32_t j0 = __ldg(col + k), j1 = __ldg(col + k + g), j2 = __ldg(col + k + 2 * g),
                               j3 = __ldg(col + k + 3 * g);
@@ -283,6 +288,12 @@ __device__ __forceinline__ void pcg_spmv(const PcgArgs& a, const Cta& c, const d
         }
         for (int o = g >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (i < c.rows && sub == 0) c.v(OV_Q)[i] = s;
+        if constexpr (DENSE)
+            for (unsigned rows = __ballot_sync(0xffffffffu, dense && sub == 0); rows; rows &= rows - 1) {
+                const int d = i0 + ((__ffs(rows) - 1) >> a.lg);
+                const double t = dense_row(a.col, a.val, v, a.rp[c.r0 + d], a.rp[c.r0 + d + 1]);
+                if (lane == 0) c.v(OV_Q)[d] = t;
+            }
     }
     __syncthreads();
 }
@@ -356,7 +367,7 @@ __device__ __forceinline__ double2 pcg_sweep(const PcgArgs& a, const Cta& c, boo
     return acc;
 }
 
-template<bool ILLT>
+template<bool ILLT, bool DENSE>
 __global__ void __launch_bounds__(PCG_THREADS, 1) k_pcg(PcgArgs a) {
     extern __shared__ __align__(16) unsigned char pcg_smem[];
     __shared__ double sh[4 * PCG_WARPS];
@@ -504,7 +515,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_pcg(PcgArgs a) {
         if (fresh) {
             // r = b - A x, z = M^-1 r, p = z
             const bool zero = a.x_zero && restart == 0;
-            if (!zero) pcg_spmv(a, c, a.x);
+            if (!zero) pcg_spmv<DENSE>(a, c, a.x);
             double s[2] = {0.0, 0.0};
             each([&](int i, i64 row) {
                 const double bi = a.b[row], ri = zero ? bi : bi - c.v(OV_Q)[i];
@@ -540,7 +551,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_pcg(PcgArgs a) {
         }
         fresh = true;
         while (!stop && here < a.iterations_here) {
-            pcg_spmv(a, c, a.p);
+            pcg_spmv<DENSE>(a, c, a.p);
             double pq[1] = {0.0};
             each([&](int i, i64) { pq[0] = fma(c.v(OV_P)[i], c.v(OV_Q)[i], pq[0]); });
             if (!all_sum(a, c, pq, has_rows, row_warps, [&](const double* t) { alpha = rz / t[0]; })) return;
@@ -586,7 +597,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_pcg(PcgArgs a) {
         // the true residual decides
         each([&](int i, i64 row) { a.x[row] = c.v(OV_X)[i]; });
         if (!all_sync(a, c)) return;
-        pcg_spmv(a, c, a.x);
+        pcg_spmv<DENSE>(a, c, a.x);
         double s[1] = {0.0};
         each([&](int i, i64 row) {
             const double d = a.b[row] - c.v(OV_Q)[i];
@@ -636,9 +647,9 @@ __global__ void k_jacobi_diag64(i64 n, const i64* __restrict__ u_rp, const doubl
     }
 }
 
-template<bool ILLT>
+template<bool ILLT, bool DENSE>
 void pcg_launch(Ctx& ctx, unsigned grid, size_t smem, PcgArgs& a) {
-    auto kernel = k_pcg<ILLT>;
+    auto kernel = k_pcg<ILLT, DENSE>;
     allow_shared(kernel);
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
@@ -717,6 +728,7 @@ bool pcg_solve(Ctx& ctx, const Csr& A, const IncompleteCholesky* Mc, const doubl
                             std::ceil(warps / PCG_WARPS) * (40.0 * per_lane + 62.0 * lg + 600.0);
         if (lg == 0 || cost < best) { best = cost; a.lg = lg; }
     }
+    const bool dense = A.longest >= i64(LONG_ROW) << a.lg;
     w.r.reserve(size_t(n));
     w.p.reserve(size_t(n));
     a.rp = A.rowptr.p;
@@ -737,8 +749,8 @@ bool pcg_solve(Ctx& ctx, const Csr& A, const IncompleteCholesky* Mc, const doubl
     NL_CUDA(cudaMemsetAsync(w.sync.p, 0, (sums + PS_COUNT + 1) * sizeof(double), ctx.stream));
     double h[PS_COUNT + 1];
     for (;;) {
-        if (M) pcg_launch<true>(ctx, grid, smem, a);
-        else pcg_launch<false>(ctx, grid, smem, a);
+        if (dense) M ? pcg_launch<true, true>(ctx, grid, smem, a) : pcg_launch<false, true>(ctx, grid, smem, a);
+        else M ? pcg_launch<true, false>(ctx, grid, smem, a) : pcg_launch<false, false>(ctx, grid, smem, a);
         NL_CUDA(cudaMemcpyAsync(h, a.state, sizeof h, cudaMemcpyDeviceToHost, ctx.stream));
         NL_CUDA(cudaStreamSynchronize(ctx.stream));
         int error = 0;

@@ -73,10 +73,12 @@ __device__ __forceinline__ double sum_partials(const double* part, double* sh) {
     return s;
 }
 
-// y = A x on padded full rows, 2^lg lanes per row.  Bound by HBM for large
+// y = A x on padded full rows, 2^lg lanes per row; DENSE: a row far longer than the
+// others by the whole warp.  Bound by HBM for large
 // systems: 300x300 8-node elements, 8.94 GB, 1.60 ms (1.74 with a warp per row and
 // 16-byte loads of four neighbouring entries per lane); a dozen 64..160-edge
 // bilinear systems, 234 -> 175 us.
+template<bool DENSE>
 __global__ void __launch_bounds__(RED_THREADS) k_spmv(i64 n, const i64* __restrict__ rp, const int32_t* __restrict__ col,
                                                       const double* __restrict__ val, int lg, const double* __restrict__ x,
                                                       double* __restrict__ y, const double* __restrict__ flags) {
@@ -85,9 +87,16 @@ __global__ void __launch_bounds__(RED_THREADS) k_spmv(i64 n, const i64* __restri
     const i64 per = 32 >> lg, step = i64(gridDim.x) * (blockDim.x >> 5) * per;
     for (i64 base = ((blockIdx.x * i64(blockDim.x) + threadIdx.x) >> 5) * per; base < n; base += step) {
         const i64 r = base + (lane >> lg);
-        double s = r < n ? row_part(col, val, x, rp[r] + sub, rp[r + 1], g) : 0.0;
+        const bool dense = DENSE && r < n && rp[r + 1] - rp[r] >= i64(LONG_ROW) << lg;
+        double s = r < n && !dense ? row_part(col, val, x, rp[r] + sub, rp[r + 1], g) : 0.0;
         for (int o = g >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (r < n && sub == 0) y[r] = s;
+        if constexpr (DENSE)
+            for (unsigned rows = __ballot_sync(0xffffffffu, dense && sub == 0); rows; rows &= rows - 1) {
+                const i64 d = base + ((__ffs(rows) - 1) >> lg);
+                const double t = dense_row(col, val, x, rp[d], rp[d + 1]);
+                if (lane == 0) y[d] = t;
+            }
     }
 }
 
@@ -593,7 +602,8 @@ void precondition(Ctx& ctx, const IncompleteCholesky* M, const double* r, double
 // ------------------------------------------------------------------ API
 static void launch_spmv(Ctx& ctx, const Csr& A, const double* x, double* y, const double* flags) {
     const int lg = spmv_lanes(double(A.nnz) / double(A.rows), double(A.rows), 152.0 * 2048.0);
-    NL_LAUNCH(k_spmv, grid_for(A.rows << lg, RED_THREADS, 152 * 8), RED_THREADS, 0, ctx.stream, A.rows, A.rowptr.p, A.col.p,
+    auto kernel = A.longest >= i64(LONG_ROW) << lg ? k_spmv<true> : k_spmv<false>;
+    NL_LAUNCH(kernel, grid_for(A.rows << lg, RED_THREADS, 152 * 8), RED_THREADS, 0, ctx.stream, A.rows, A.rowptr.p, A.col.p,
               A.val.p, lg, x, y, flags);
 }
 

@@ -576,9 +576,13 @@ int nlgpu_nonstationary_1d_temperature(nlgpu_ctx* ctx, double* temperature);
  * assembly: 16 or 32, or 0 (default) to time both on a sample of elements at
  * the first such assembly of each (element type, influence kind, pair mode)
  * and keep the faster (32 without timing below 9 728 elements);
- * nlgpu_assembly_tuning reports the choice. */
+ * nlgpu_assembly_tuning reports the choice.
+ * NLGPU_OPTION_WAIT_LIMIT: microseconds (default 2 000 000) after which the CTAs
+ * of the one-launch FP32 ILLT application stop waiting for one another's values;
+ * the call then returns NLGPU_ERR_TIMEOUT.  0: at once, to see that status.  A
+ * batch takes the smallest of its instances'. */
 enum { NLGPU_OPTION_GLOBAL_SWEEPS = 0, NLGPU_OPTION_ORDERED_PAIRS = 1, NLGPU_OPTION_ASSEMBLY_PRECISION = 2,
-       NLGPU_OPTION_FP32_SYMMETRIC = 3, NLGPU_OPTION_ASSEMBLY_WARPS = 4 };
+       NLGPU_OPTION_FP32_SYMMETRIC = 3, NLGPU_OPTION_ASSEMBLY_WARPS = 4, NLGPU_OPTION_WAIT_LIMIT = 5 };
 enum { NLGPU_ASSEMBLY_AUTO = 0, NLGPU_ASSEMBLY_FF = 1, NLGPU_ASSEMBLY_FP64 = 2 };
 int nlgpu_set_option(nlgpu_ctx* ctx, int option, int value);
 /* Warps per CTA of the last float-float pair assembly (0 before any) and the

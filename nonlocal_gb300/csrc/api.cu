@@ -277,12 +277,7 @@ CgResult solve_system(Ctx& c, const nlgpu_solve_options& o, nlgpu_solve_report* 
         r = cg_solve(c, c.full, M, b, c.temperature.p, o.tolerance, o.max_iterations, false);
     }
     if (rep) rep->seconds_solve = seconds(t0);
-    if (M && c.sweep_error.n) {
-        int err = 0;
-        NL_CUDA(cudaMemcpyAsync(&err, c.sweep_error.p, sizeof err, cudaMemcpyDeviceToHost, c.stream));
-        NL_CUDA(cudaStreamSynchronize(c.stream));
-        NL_REQUIRE(err == 0, NLGPU_ERR_TIMEOUT, "a triangular sweep stage wait gave up");
-    }
+    if (M) check_sweeps(c);
     fill_report(c, rep, r);
     return r;
 }
@@ -975,10 +970,8 @@ int nlgpu_illt_solve(nlgpu_ctx* ctx, int64_t n, const double* x, double* y) {
         c.sweep_error.zero(c.stream);
         ilt_apply(c, c.plugin_ilt, dx.p, dy.p);
         dy.download(y, size_t(n), c.stream);
-        int err = 0;
-        c.sweep_error.download(&err, 1, c.stream);
         NL_CUDA(cudaStreamSynchronize(c.stream));
-        NL_REQUIRE(err == 0, NLGPU_ERR_TIMEOUT, "a triangular sweep gave up waiting for its data");
+        check_sweeps(c);
     });
 }
 
@@ -994,10 +987,8 @@ int nlgpu_illt_solve_f32(nlgpu_ctx* ctx, int64_t n, int sweeps, const float* x, 
         c.sweep_error.zero(c.stream);
         ilt_apply32(c, c.plugin_ilt, dx.p, dy.p, std::max(sweeps, 0));
         dy.download(y, size_t(n), c.stream);
-        int err = 0;
-        c.sweep_error.download(&err, 1, c.stream);
         NL_CUDA(cudaStreamSynchronize(c.stream));
-        NL_REQUIRE(err == 0, NLGPU_ERR_TIMEOUT, "a triangular sweep gave up waiting for its data");
+        check_sweeps(c);
     });
 }
 
@@ -1422,6 +1413,11 @@ int nlgpu_set_option(nlgpu_ctx* ctx, int option, int value) {
     if (option == NLGPU_OPTION_ASSEMBLY_WARPS) {
         if (value != 0 && value != 16 && value != 32) return NLGPU_ERR_ARG;
         ctx->ff_warps_option = value;
+        return NLGPU_OK;
+    }
+    if (option == NLGPU_OPTION_WAIT_LIMIT) {
+        if (value < 0) return NLGPU_ERR_ARG;
+        ctx->wait_limit_us = value;
         return NLGPU_OK;
     }
     if (option == NLGPU_OPTION_ASSEMBLY_PRECISION) {

@@ -309,6 +309,12 @@ struct Batch {
 
 namespace {
 
+// the smallest wait limit of the instances
+void batch_wait_limit(Batch& bt) {
+    bt.solver.wait_limit_us = bt.inst[0]->wait_limit_us;
+    for (const Ctx* c : bt.inst) bt.solver.wait_limit_us = std::min(bt.solver.wait_limit_us, c->wait_limit_us);
+}
+
 // concatenates one matrix of every instance (sel picks it) into `out`
 template<class Sel>
 void concat(Batch& bt, Csr& out, Sel sel, bool with_inst) {
@@ -455,6 +461,7 @@ void batch_prepare_mixed(Batch& bt) {
         return local[k];
     }, false);
     NL_CUDA(cudaStreamSynchronize(bt.stream));   // the local matrices go back to their instances
+    batch_wait_limit(bt);
     bt.solver.stream = bt.stream;
     bt.solver.n_nodes = bt.N;
     // the exact IC(0): factored once for every step (the fixed-point factor,
@@ -493,6 +500,7 @@ i64 batch_solve_mixed(Batch& bt, double tolerance, i64 max_iterations, i64* iter
     if (!r.converged) r = cg_solve(bt.solver, bt.A, &bt.ic, bt.b.p, bt.x.p, tol_g, max_iterations, true);
     bt.last_inner = r.iterations;
     bt.last_outer = r.outer_iterations;
+    check_sweeps(bt.solver);
     NL_REQUIRE(r.converged, NLGPU_ERR_NO_CONVERGENCE, "the batched step did not converge");
     if (iterations) for (i64 k = 0; k < K; ++k) iterations[k] = r.iterations;
     return r.iterations;
@@ -844,6 +852,7 @@ std::vector<CgResult> batch_bicgstab(const std::vector<Ctx*>& instances, double 
         NL_CUDA(cudaStreamSynchronize(bt.stream));   // the local matrices go back to their instances
         bt.solver.stream = bt.stream;
         bt.solver.n_nodes = N;
+        batch_wait_limit(bt);
         ilt_build(bt.solver, bt.M, bt.ic, false, IC_SWEEPS_FP32);
         illt = bt.ic.ok;   // the diagonal otherwise (as the reference)
         timer.mark("local matrices, ILLT");
@@ -957,6 +966,7 @@ std::vector<CgResult> batch_bicgstab(const std::vector<Ctx*>& instances, double 
                                 cudaMemcpyDeviceToDevice, bt.stream));
     }
     NL_CUDA(cudaStreamSynchronize(bt.stream));
+    if (illt) check_sweeps(bt.solver);
     return out;
 }
 

@@ -542,6 +542,7 @@ struct Ctx {
     double time_step = 0.0;
     dbuf<double> temperature;
     bool nonstationary_ready = false;
+    int wait_limit_us = 2000000;        // of k_jacobi_all's waits
     dbuf<int> sweep_error;
     bool force_global_sweeps = false;   // use the global-memory sweeps (for comparison)
     int ilt_sweeps = NLGPU_DEFAULT_TRIANGULAR_SWEEPS;   // FP32 ILLT: Jacobi sweeps per triangle (0: exact)
@@ -672,6 +673,9 @@ void ilt_levels_gpu(Ctx& ctx, IncompleteCholesky& ic);
 // jacobi.cu: the factor applied by Jacobi sweeps on its two triangles
 void jacobi_fill(Ctx& ctx, IncompleteCholesky& ic);
 void jacobi_apply32(Ctx& ctx, IncompleteCholesky& ic, int sweeps, const float* r, float* z, const double* flags);
+// waits for the stream; NLGPU_ERR_TIMEOUT when a wait of a factor's application (exact
+// sweeps, k_jacobi_all) has given up since the factor was built or this was last called
+void check_sweeps(Ctx& ctx);
 // mixed.cu
 // FP32 copy of the solver matrix A (full rows) for the mixed solve; with the
 // upper storage of a symmetric A given, only its strictly upper part is copied

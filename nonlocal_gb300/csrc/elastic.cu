@@ -481,12 +481,7 @@ CgResult elastic_solve(Ctx& ctx, const nlgpu_solve_options& o, nlgpu_solve_repor
     } else {
         r = cg_solve(ctx, el.full, M, el.rhs.p, el.displacement.p, o.tolerance, o.max_iterations, false);
     }
-    if (M && ctx.sweep_error.n) {
-        int err = 0;
-        NL_CUDA(cudaMemcpyAsync(&err, ctx.sweep_error.p, sizeof err, cudaMemcpyDeviceToHost, ctx.stream));
-        NL_CUDA(cudaStreamSynchronize(ctx.stream));
-        NL_REQUIRE(err == 0, NLGPU_ERR_TIMEOUT, "a triangular sweep stage wait gave up");
-    }
+    if (M) check_sweeps(ctx);
     if (rep) {
         rep->iterations = r.iterations;
         rep->residual = r.residual;

@@ -116,7 +116,7 @@ constexpr double JA_FAR = 4.0;    // mean reach in CTAs
 constexpr i64 JA_MAX_ROWS = 400000;    // 361 201 measured
 constexpr int JA_MAX_SWEEPS = 32;
 constexpr int JA_BATCH = 4;       // gathers in flight per lane
-constexpr unsigned long long JA_WAIT_LIMIT_NS = 2000000000ull;
+constexpr int JA_POLLS = 4096;
 
 __device__ __forceinline__ unsigned long long ja_globaltimer() {
     unsigned long long t;
@@ -137,11 +137,11 @@ __device__ __forceinline__ unsigned long long ja_get(const unsigned long long* p
 
 // a wait that runs out marks the CTA, which then waits no more; the host sees *error
 __device__ __noinline__ unsigned long long ja_wait_long(const unsigned long long* p, unsigned tag, volatile int* gave_up,
-                                                        int* error) {
+                                                        int* error, unsigned long long limit_ns) {
     const unsigned long long t0 = ja_globaltimer();
     unsigned long long w = ja_get(p);
     while (unsigned(w >> 32) != tag && !*gave_up) {
-        if (ja_globaltimer() - t0 > JA_WAIT_LIMIT_NS) {
+        if (ja_globaltimer() - t0 > limit_ns) {
             atomicExch(error, 1);
             *gave_up = 1;
         }
@@ -162,8 +162,12 @@ struct JacobiAll {
     unsigned long long* steps;   // [sweeps + 1][n]
     unsigned* tags;              // [gridDim.x] last number each CTA used
     int* error;
+    unsigned long long limit_ns;
 };
 
+// POLLS: of a value before the clock is read (a variant of its own for a wait limit of 0:
+// with the number in a register a batch of 163 000 rows took 14 % longer)
+template<int POLLS>
 __global__ void __launch_bounds__(JA_THREADS) k_jacobi_all(JacobiAll a, const double* __restrict__ flags) {
     extern __shared__ float ja_base[];
     __shared__ int gave_up;
@@ -216,8 +220,8 @@ __global__ void __launch_bounds__(JA_THREADS) k_jacobi_all(JacobiAll a, const do
                     for (int u = 0; u < JA_BATCH; ++u)
                         if (k + u * g < w) {
                             for (int tries = 0; unsigned(y[u] >> 32) != tag; ++tries) {
-                                if (tries == 4096) {
-                                    y[u] = ja_wait_long(in + j[u], tag, &gave_up, a.error);
+                                if (tries == POLLS) {
+                                    y[u] = ja_wait_long(in + j[u], tag, &gave_up, a.error, a.limit_ns);
                                     break;
                                 }
                                 y[u] = ja_get(in + j[u]);
@@ -261,6 +265,16 @@ void jacobi_fill(Ctx& ctx, IncompleteCholesky& ic) {
     NL_LAUNCH(k_jacobi_diag, grid_for(n, 256), 256, 0, ctx.stream, n, ic.rp.p, ic.u.p, ic.scale.p, ic.jc.p, ic.jdinv.p);
 }
 
+void check_sweeps(Ctx& ctx) {
+    if (!ctx.sweep_error.n) return;
+    int err = 0;
+    ctx.sweep_error.download(&err, 1, ctx.stream);
+    NL_CUDA(cudaStreamSynchronize(ctx.stream));
+    if (err == 0) return;
+    ctx.sweep_error.zero(ctx.stream);
+    throw error{NLGPU_ERR_TIMEOUT, "a triangular sweep gave up waiting for its data"};
+}
+
 void jacobi_apply32(Ctx& ctx, IncompleteCholesky& ic, int sweeps, const float* r, float* z, const double* flags) {
     NL_REQUIRE(sweeps >= 1, NLGPU_ERR_ARG, "at least one Jacobi sweep per triangle");
     const i64 n = ic.n;
@@ -290,6 +304,7 @@ void jacobi_apply32(Ctx& ctx, IncompleteCholesky& ic, int sweeps, const float* r
         a.sup = ic.jup.slice.p; a.cup = ic.jup.col.p; a.vup = ic.jup.val.p;
         a.r = r; a.c = ic.jc.p; a.dinv = ic.jdinv.p; a.scale = ic.scale32.p; a.z = z;
         a.steps = ic.jsteps.p; a.tags = ic.jtags.p; a.error = ctx.sweep_error.p;
+        a.limit_ns = static_cast<unsigned long long>(ctx.wait_limit_us) * 1000ull;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeCooperative;
         at[0].val.cooperative = 1;
@@ -300,7 +315,7 @@ void jacobi_apply32(Ctx& ctx, IncompleteCholesky& ic, int sweeps, const float* r
         cfg.stream = ctx.stream;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        NL_CUDA(cudaLaunchKernelEx(&cfg, k_jacobi_all, a, flags));
+        NL_CUDA(cudaLaunchKernelEx(&cfg, ctx.wait_limit_us > 0 ? k_jacobi_all<JA_POLLS> : k_jacobi_all<0>, a, flags));
         count_launch();
         return;
     }

@@ -593,6 +593,7 @@ void mpnn_train(Ctx& ctx, const Csr& A, IncompleteCholesky& M, const double* b_g
         m.use = true;
         const CgResult with = timed(true, out.validation_seconds_learned);
         const CgResult without = timed(false, out.validation_seconds_illt);
+        mpnn_check(ctx);
         out.validation_iterations_learned = with.iterations;
         out.validation_iterations_illt = without.iterations;
         m.use = with.converged && !with.learned_fallback && out.validation_seconds_learned < out.validation_seconds_illt;
@@ -607,6 +608,7 @@ void mpnn_check(Ctx& ctx) {
     ctx.mp.error.download(&err, 1, ctx.stream);
     NL_CUDA(cudaStreamSynchronize(ctx.stream));
     NL_REQUIRE(err == 0, NLGPU_ERR_TIMEOUT, "a tensor-core GEMM gave up waiting for its MMAs");
+    check_sweeps(ctx);
 }
 
 }  // namespace nlgpu

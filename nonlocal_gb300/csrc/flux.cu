@@ -15,7 +15,8 @@
 // nq x nq influence evaluations): one warp per element eL, the lanes spread
 // over the (eNL, qNL) points of its neighbour list, each accumulating the
 // contributions to all of eL's quadrature points in registers, then a warp
-// reduction; float-float for the influence kinds that have it, FP64 otherwise.
+// reduction; float-float for the influence kinds that have it unless
+// NLGPU_ASSEMBLY_FP64 is set, FP64 otherwise.
 #include "common.cuh"
 #include "influence.cuh"
 #include "influence_ff.cuh"
@@ -300,8 +301,8 @@ void calc_flux(Ctx& ctx, const double* temperature, double* flux_x, double* flux
     if (ctx.model.nonlocal()) {
         fx.resize(size_t(E * nq)); fy.resize(size_t(E * nq));
         // float-float where the influence has a float-float form and every term is finite
-        // (the FP64 kernel then returns at once), FP64 otherwise
-        const bool in_ff = ff_supported(ctx.model);
+        // (the FP64 kernel then returns at once), FP64 otherwise and where it is asked for
+        const bool in_ff = ff_supported(ctx.model) && ctx.assembly_precision != NLGPU_ASSEMBLY_FP64;
         if (in_ff) {
             load.resize(size_t(E * nq));
             largest.resize(1);

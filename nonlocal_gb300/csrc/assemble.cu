@@ -275,11 +275,6 @@ struct FFArgs {
     FXExp fx_exp;
 };
 
-__device__ __forceinline__ int fx_exponent(const unsigned long long* extent) {
-    const double x = __longlong_as_double((long long)*extent);
-    return x >= 8.0 ? ilogb(x) : 2;
-}
-
 // the largest finite |coordinate| in units of the radii
 __global__ void k_fx_extent(i64 n, const double* __restrict__ qcoord, double ix, double iy,
                             unsigned long long* __restrict__ extent) {

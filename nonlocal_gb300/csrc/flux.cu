@@ -15,8 +15,9 @@
 // nq x nq influence evaluations): one warp per element eL, the lanes spread
 // over the (eNL, qNL) points of its neighbour list, each accumulating the
 // contributions to all of eL's quadrature points in registers, then a warp
-// reduction; float-float for the influence kinds that have it unless
-// NLGPU_ASSEMBLY_FP64 is set, FP64 otherwise.
+// reduction.  The loads and their sums are FP64; the influence values come from the
+// integer pipes where the fixed-point form covers the model (influence_ff.cuh) unless
+// NLGPU_ASSEMBLY_FP64 is set, from the FP64 pipe otherwise.
 #include "common.cuh"
 #include "influence.cuh"
 #include "influence_ff.cuh"
@@ -59,14 +60,10 @@ __global__ void k_flux_local(i64 E, int nen, int nq, const int32_t* __restrict__
     }
 }
 
-// float-float covers sums whose terms are finite; the power of two that brings the
-// largest to [1, 2)
-__device__ __forceinline__ bool flux_in_range(const unsigned long long* largest) {
-    return (*largest >> 52) < 0x7ff;
-}
-__device__ __forceinline__ double flux_power(const unsigned long long* largest, int sign) {
-    const long long e = min(1022ll, max(-1022ll, static_cast<long long>(*largest >> 52) - 1023));
-    return __longlong_as_double((1023 + sign * e) << 52);
+// what the fixed-point form needs: finite loads, and coordinates below 2^21 radii (their
+// unit is 2^-58 of the largest one's power of two); found: the bits of the largest of each
+__device__ __forceinline__ bool flux_in_range(const unsigned long long* found) {
+    return (found[0] >> 52) < 0x7ff && (found[1] >> 52) <= 1023 + FX_MAX_EXPONENT;
 }
 
 template<int NQ, int INF>
@@ -76,8 +73,8 @@ __global__ void __launch_bounds__(FX_THREADS) k_flux_nonlocal(i64 E, const doubl
                                                               const double* __restrict__ lx,
                                                               const double* __restrict__ ly, double* __restrict__ fx,
                                                               double* __restrict__ fy,
-                                                              const unsigned long long* __restrict__ largest) {
-    if (largest && flux_in_range(largest)) return;   // done in float-float
+                                                              const unsigned long long* __restrict__ found) {
+    if (found && flux_in_range(found)) return;   // k_flux_nonlocal_fx does it
     const int lane = threadIdx.x & 31;
     const i64 warps = i64(gridDim.x) * (blockDim.x >> 5);
     for (i64 eL = (blockIdx.x * i64(blockDim.x) + threadIdx.x) >> 5; eL < E; eL += warps) {
@@ -121,92 +118,104 @@ __global__ void __launch_bounds__(FX_THREADS) k_flux_nonlocal(i64 E, const doubl
     }
 }
 
-// largest magnitude of w_q |J| norm times the local flux (as the bits of a double:
-// non-negative doubles order like their bits, and NaN above infinity)
-__global__ void k_flux_scale(i64 count, int nq, const double* __restrict__ jac, Model m, Basis b,
-                             const double* __restrict__ lx, const double* __restrict__ ly,
-                             unsigned long long* __restrict__ largest) {
-    unsigned long long top = 0;
+// the largest magnitude of the loads w_q |J| norm (local flux) and of the coordinates in
+// units of the radii, as the bits of a double: non-negative doubles order like their
+// bits, and NaN above infinity
+__global__ void k_flux_range(i64 count, int nq, const double* __restrict__ qcoord, const double* __restrict__ jac, Model m,
+                             Basis b, const double* __restrict__ lx, const double* __restrict__ ly,
+                             unsigned long long* __restrict__ found) {
+    auto bits = [](double x) { return static_cast<unsigned long long>(__double_as_longlong(fabs(x))); };
+    unsigned long long load = 0, at = 0;
     for (i64 t = blockIdx.x * i64(blockDim.x) + threadIdx.x; t < count; t += i64(gridDim.x) * blockDim.x) {
         const double w = b.w[t % nq] * jac[t] * m.norm;
-        top = max(top, static_cast<unsigned long long>(__double_as_longlong(fabs(w * lx[t]))));
-        top = max(top, static_cast<unsigned long long>(__double_as_longlong(fabs(w * ly[t]))));
+        load = max(load, max(bits(w * lx[t]), bits(w * ly[t])));
+        at = max(at, max(bits(qcoord[2 * t] * m.inv_r[0]), bits(qcoord[2 * t + 1] * m.inv_r[1])));
     }
-    for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(largest, top);
-}
-
-// w_q |J| norm times the local flux in float-float, scaled
-__global__ void k_flux_stage(i64 count, int nq, const double* __restrict__ jac, Model m, Basis b,
-                             const double* __restrict__ lx, const double* __restrict__ ly,
-                             const unsigned long long* __restrict__ largest, float4* __restrict__ load) {
-    const double scale = flux_power(largest, -1);
-    for (i64 t = blockIdx.x * i64(blockDim.x) + threadIdx.x; t < count; t += i64(gridDim.x) * blockDim.x) {
-        const double w = b.w[t % nq] * jac[t] * m.norm;
-        const ff vx = ff_from(w * lx[t] * scale), vy = ff_from(w * ly[t] * scale);
-        load[t] = make_float4(vx.h, vx.l, vy.h, vy.l);
+    for (int o = 16; o > 0; o >>= 1) {
+        load = max(load, __shfl_xor_sync(0xffffffffu, load, o));
+        at = max(at, __shfl_xor_sync(0xffffffffu, at, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(found, load);
+        atomicMax(found + 1, at);
     }
 }
 
-// The nonlocal average as in k_flux_nonlocal with the influence values and the sums
-// in float-float on the FP32 pipes: about 140 FP32 instructions per pair of points
-// against 27 on the FP64 pipe, whose two lanes a clock bound that kernel (120x90
-// 8-node, exponential: 8.38 ms, here 1.00; the error against 64-bit sums is no
-// larger).  A source's coordinates are taken relative to the element's first point
-// in FP64 (two subtractions and two products), so that float-float holds the
-// distances, not the mesh coordinates; a lane's sums are compensated.
+// the loads, and the coordinates in fixed point
+__global__ void k_flux_stage(i64 count, int nq, const double* __restrict__ qcoord, const double* __restrict__ jac, Model m,
+                             Basis b, const double* __restrict__ lx, const double* __restrict__ ly,
+                             const unsigned long long* __restrict__ found, int4* __restrict__ at,
+                             double2* __restrict__ load) {
+    if (!flux_in_range(found)) return;
+    const int ex = fx_exponent(found + 1);
+    for (i64 t = blockIdx.x * i64(blockDim.x) + threadIdx.x; t < count; t += i64(gridDim.x) * blockDim.x) {
+        const double w = b.w[t % nq] * jac[t] * m.norm;
+        const int2 x = fx_coordinate(qcoord[2 * t], m.inv_r[0], ex), y = fx_coordinate(qcoord[2 * t + 1], m.inv_r[1], ex);
+        at[t] = make_int4(x.x, x.y, y.x, y.y);
+        load[t] = make_double2(w * lx[t], w * ly[t]);
+    }
+}
+
+// The nonlocal average as in k_flux_nonlocal with the influence values in fixed point
+// on the integer pipes: of the 27 FP64 operations a pair of points takes there, two
+// remain, the multiply-adds of the load.  That kernel is bound by the FP64 pipe's two
+// lanes a clock, this one by issue: 120x90 8-node elements, exponential, the whole call
+// 8.75 and 1.05 ms.  Against extended precision the error is that kernel's (rms 2.1e-16
+// of the terms' magnitudes for its 2.0e-16 there; 9.6e-17 for 1.0e-16 with 17 000
+// terms); with values and sums in float-float, as fast, it was 6.2e-16 and 8.4e-15.
 template<int NQ, int INF>
-__global__ void __launch_bounds__(FX_THREADS, 2) k_flux_nonlocal_ff(i64 E, const double2* __restrict__ at,
-                                                                 const float4* __restrict__ load,
-                                                                 const i64* __restrict__ noff,
-                                                                 const int32_t* __restrict__ nlist, Model m,
-                                                                 FFExpTable table,
-                                                                 const unsigned long long* __restrict__ largest,
-                                                                 const double* __restrict__ lx,
-                                                                 const double* __restrict__ ly, double* __restrict__ fx,
-                                                                 double* __restrict__ fy) {
-    __shared__ ff etab[2 * FF_EXP_K + 1];
-    if (!flux_in_range(largest)) return;   // k_flux_nonlocal does it
-    for (int t = threadIdx.x; t < 2 * FF_EXP_K + 1; t += FX_THREADS) etab[t] = ff{table.v[t].x, table.v[t].y};
-    __syncthreads();
-    const ff qf = ff_from(m.q);
-    const double back = flux_power(largest, 1);
+__global__ void __launch_bounds__(FX_THREADS, 2) k_flux_nonlocal_fx(i64 E, const int4* __restrict__ at,
+                                                                    const double2* __restrict__ load,
+                                                                    const i64* __restrict__ noff,
+                                                                    const int32_t* __restrict__ nlist, Model m, FXExp fexp,
+                                                                    FXExpTable table,
+                                                                    const unsigned long long* __restrict__ found,
+                                                                    const double* __restrict__ lx,
+                                                                    const double* __restrict__ ly, double* __restrict__ fx,
+                                                                    double* __restrict__ fy) {
+    constexpr bool EXP = INF == NLGPU_INFLUENCE_EXPONENTIAL;
+    __shared__ unsigned long long tab[EXP ? FX_EXP_K : 1];
+    __shared__ int4 own[FX_THREADS / 32][NQ];
+    if (!flux_in_range(found)) return;   // k_flux_nonlocal does it
+    if constexpr (EXP) {
+        for (int t = threadIdx.x; t < FX_EXP_K; t += FX_THREADS) tab[t] = table.v[t];
+        __syncthreads();
+    }
+    const int ex = fx_exponent(found + 1);
     const int lane = threadIdx.x & 31;
+    int4* xq = own[threadIdx.x >> 5];
     const i64 warps = i64(gridDim.x) * (blockDim.x >> 5);
     for (i64 eL = (blockIdx.x * i64(blockDim.x) + threadIdx.x) >> 5; eL < E; eL += warps) {
-        const double2 origin = at[eL * NQ];
-        ff xq[NQ], yq[NQ];
-        ffdot ax[NQ], ay[NQ];
+        __syncwarp();
+        if (lane < NQ) xq[lane] = at[eL * NQ + lane];
+        __syncwarp();
+        double ax[NQ], ay[NQ];
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const double2 p = at[eL * NQ + q];
-            xq[q] = ff_split((p.x - origin.x) * m.inv_r[0]);
-            yq[q] = ff_split((p.y - origin.y) * m.inv_r[1]);
-        }
-        const i64 kb = noff[eL], items = (noff[eL + 1] - kb) * NQ;
-        for (i64 it = lane; it < items; it += 32) {
+        for (int q = 0; q < NQ; ++q) ax[q] = ay[q] = 0.0;
+        const i64 kb = noff[eL];
+        const int items = int(noff[eL + 1] - kb) * NQ;
+        for (int it = lane; it < items; it += 32) {
             const i64 s = i64(nlist[kb + it / NQ]) * NQ + it % NQ;
-            const double2 p = at[s];
-            const float4 v = load[s];
-            const ff xs = ff_split((p.x - origin.x) * m.inv_r[0]), ys = ff_split((p.y - origin.y) * m.inv_r[1]);
+            const int4 p = at[s];
+            const double2 v = load[s];
 #pragma unroll
             for (int q = 0; q < NQ; ++q) {
-                const ff w = shape_ff<INF>(m, ff_sub(xq[q], xs), ff_sub(yq[q], ys), qf, etab);
-                ffdot_add(ax[q], w, ff{v.x, v.y});
-                ffdot_add(ay[q], w, ff{v.z, v.w});
+                const double w = fx_value(fx_shape<INF>(m, xq[q], p, ex, fexp, tab));
+                ax[q] = fma(w, v.x, ax[q]);
+                ay[q] = fma(w, v.y, ay[q]);
             }
         }
         double sx = 0.0, sy = 0.0;
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {
-            const double tx = warp_sum(ff_to(ffdot_value(ax[q]))), ty = warp_sum(ff_to(ffdot_value(ay[q])));
+            const double tx = warp_sum(ax[q]), ty = warp_sum(ay[q]);
             if (q == lane) { sx = tx; sy = ty; }
         }
         if (lane < NQ) {
             const i64 t = eL * NQ + lane;
             const double nw = 1.0 - m.p1;
-            fx[t] = lx[t] * m.p1 + sx * back * nw;
-            fy[t] = ly[t] * m.p1 + sy * back * nw;
+            fx[t] = lx[t] * m.p1 + sx * nw;
+            fy[t] = ly[t] * m.p1 + sy * nw;
         }
     }
 }
@@ -243,44 +252,45 @@ __global__ void k_flux_nodes(i64 n, const i64* __restrict__ ne_off, const int32_
 
 template<int NQ>
 void launch_nonlocal(Ctx& ctx, const double* lx, const double* ly, double* fx, double* fy,
-                     const unsigned long long* largest) {
+                     const unsigned long long* found) {
     const i64 E = ctx.n_elems;
     const unsigned grid = grid_for(E * 32, FX_THREADS, 152 * 64);
     switch (ctx.model.influence) {
     case NLGPU_INFLUENCE_FAST_POLYNOMIAL:
         NL_LAUNCH((k_flux_nonlocal<NQ, NLGPU_INFLUENCE_FAST_POLYNOMIAL>), grid, FX_THREADS, 0, ctx.stream, E,
-                  ctx.qcoord.p, ctx.jac.p, ctx.noff.p, ctx.nlist.p, ctx.model, ctx.basis, lx, ly, fx, fy, largest);
+                  ctx.qcoord.p, ctx.jac.p, ctx.noff.p, ctx.nlist.p, ctx.model, ctx.basis, lx, ly, fx, fy, found);
         break;
     case NLGPU_INFLUENCE_POLYNOMIAL:
         NL_LAUNCH((k_flux_nonlocal<NQ, NLGPU_INFLUENCE_POLYNOMIAL>), grid, FX_THREADS, 0, ctx.stream, E,
-                  ctx.qcoord.p, ctx.jac.p, ctx.noff.p, ctx.nlist.p, ctx.model, ctx.basis, lx, ly, fx, fy, largest);
+                  ctx.qcoord.p, ctx.jac.p, ctx.noff.p, ctx.nlist.p, ctx.model, ctx.basis, lx, ly, fx, fy, found);
         break;
     case NLGPU_INFLUENCE_EXPONENTIAL:
         NL_LAUNCH((k_flux_nonlocal<NQ, NLGPU_INFLUENCE_EXPONENTIAL>), grid, FX_THREADS, 0, ctx.stream, E,
-                  ctx.qcoord.p, ctx.jac.p, ctx.noff.p, ctx.nlist.p, ctx.model, ctx.basis, lx, ly, fx, fy, largest);
+                  ctx.qcoord.p, ctx.jac.p, ctx.noff.p, ctx.nlist.p, ctx.model, ctx.basis, lx, ly, fx, fy, found);
         break;
     default:
         NL_LAUNCH((k_flux_nonlocal<NQ, NLGPU_INFLUENCE_CONSTANT>), grid, FX_THREADS, 0, ctx.stream, E,
-                  ctx.qcoord.p, ctx.jac.p, ctx.noff.p, ctx.nlist.p, ctx.model, ctx.basis, lx, ly, fx, fy, largest);
+                  ctx.qcoord.p, ctx.jac.p, ctx.noff.p, ctx.nlist.p, ctx.model, ctx.basis, lx, ly, fx, fy, found);
         break;
     }
 }
 
 template<int NQ>
-void launch_nonlocal_ff(Ctx& ctx, const float4* load, const unsigned long long* largest, const double* lx, const double* ly,
-                        double* fx, double* fy) {
+void launch_nonlocal_fx(Ctx& ctx, const int4* at, const double2* load, const unsigned long long* found, const double* lx,
+                        const double* ly, double* fx, double* fy) {
     const i64 E = ctx.n_elems;
     const unsigned grid = grid_for(E * 32, FX_THREADS, 152 * 64);
-    FFExpTable table;
-    fill_exp_table(table);
+    const bool exponential = ctx.model.influence == NLGPU_INFLUENCE_EXPONENTIAL;
+    const FXExp fexp = exponential ? fx_exp_setup(ctx.model.q) : FXExp{};
     auto launch = [&](auto kernel) {
-        NL_LAUNCH(kernel, grid, FX_THREADS, 0, ctx.stream, E, reinterpret_cast<const double2*>(ctx.qcoord.p), load, ctx.noff.p,
-                  ctx.nlist.p, ctx.model, table, largest, lx, ly, fx, fy);
+        NL_LAUNCH(kernel, grid, FX_THREADS, 0, ctx.stream, E, at, load, ctx.noff.p, ctx.nlist.p, ctx.model, fexp,
+                  fx_exp_table(), found, lx, ly, fx, fy);
     };
-    switch (ctx.model.influence) {
-    case NLGPU_INFLUENCE_FAST_POLYNOMIAL: launch(k_flux_nonlocal_ff<NQ, NLGPU_INFLUENCE_FAST_POLYNOMIAL>); break;
-    case NLGPU_INFLUENCE_POLYNOMIAL: launch(k_flux_nonlocal_ff<NQ, NLGPU_INFLUENCE_POLYNOMIAL>); break;
-    default: launch(k_flux_nonlocal_ff<NQ, NLGPU_INFLUENCE_EXPONENTIAL>); break;
+    const bool linear = ctx.model.influence == NLGPU_INFLUENCE_POLYNOMIAL && ctx.model.p == 2 && ctx.model.q == 1.0;   // 1 - d
+    switch (linear ? NLGPU_INFLUENCE_FAST_POLYNOMIAL : ctx.model.influence) {
+    case NLGPU_INFLUENCE_FAST_POLYNOMIAL: launch(k_flux_nonlocal_fx<NQ, NLGPU_INFLUENCE_FAST_POLYNOMIAL>); break;
+    case NLGPU_INFLUENCE_POLYNOMIAL: launch(k_flux_nonlocal_fx<NQ, NLGPU_INFLUENCE_POLYNOMIAL>); break;
+    default: launch(k_flux_nonlocal_fx<NQ, NLGPU_INFLUENCE_EXPONENTIAL>); break;
     }
 }
 
@@ -290,8 +300,9 @@ void calc_flux(Ctx& ctx, const double* temperature, double* flux_x, double* flux
     const i64 E = ctx.n_elems, n = ctx.n_nodes;
     const int nen = ctx.basis.nen, nq = ctx.basis.nq;
     dbuf<double> lx, ly, fx, fy, area;
-    dbuf<float4> load;
-    dbuf<unsigned long long> largest;
+    dbuf<int4> at;
+    dbuf<double2> load;
+    dbuf<unsigned long long> found;
     lx.resize(size_t(E * nq)); ly.resize(size_t(E * nq));
     area.resize(size_t(E));
     NL_LAUNCH(k_flux_local, grid_for(E * nq, FX_THREADS), FX_THREADS, 0, ctx.stream, E, nen, nq, ctx.elems.p,
@@ -300,22 +311,23 @@ void calc_flux(Ctx& ctx, const double* temperature, double* flux_x, double* flux
     const double* qy = ly.p;
     if (ctx.model.nonlocal()) {
         fx.resize(size_t(E * nq)); fy.resize(size_t(E * nq));
-        // float-float where the influence has a float-float form and every term is finite
-        // (the FP64 kernel then returns at once), FP64 otherwise and where it is asked for
-        const bool in_ff = ff_supported(ctx.model) && ctx.assembly_precision != NLGPU_ASSEMBLY_FP64;
-        if (in_ff) {
+        // in fixed point where it covers the model and the values are in its range (the FP64
+        // kernel then returns at once)
+        const bool fixed = fx_supported(ctx.model) && ctx.assembly_precision != NLGPU_ASSEMBLY_FP64;
+        if (fixed) {
+            at.resize(size_t(E * nq));
             load.resize(size_t(E * nq));
-            largest.resize(1);
-            largest.zero(ctx.stream);
-            NL_LAUNCH(k_flux_scale, grid_for(E * nq, FX_THREADS, 152 * 8), FX_THREADS, 0, ctx.stream, E * nq, nq, ctx.jac.p,
-                      ctx.model, ctx.basis, lx.p, ly.p, largest.p);
-            NL_LAUNCH(k_flux_stage, grid_for(E * nq, FX_THREADS), FX_THREADS, 0, ctx.stream, E * nq, nq, ctx.jac.p,
-                      ctx.model, ctx.basis, lx.p, ly.p, largest.p, load.p);
-            if (nq == 4) launch_nonlocal_ff<4>(ctx, load.p, largest.p, lx.p, ly.p, fx.p, fy.p);
-            else launch_nonlocal_ff<9>(ctx, load.p, largest.p, lx.p, ly.p, fx.p, fy.p);
+            found.resize(2);
+            found.zero(ctx.stream);
+            NL_LAUNCH(k_flux_range, grid_for(E * nq, FX_THREADS, 152 * 8), FX_THREADS, 0, ctx.stream, E * nq, nq,
+                      ctx.qcoord.p, ctx.jac.p, ctx.model, ctx.basis, lx.p, ly.p, found.p);
+            NL_LAUNCH(k_flux_stage, grid_for(E * nq, FX_THREADS), FX_THREADS, 0, ctx.stream, E * nq, nq, ctx.qcoord.p,
+                      ctx.jac.p, ctx.model, ctx.basis, lx.p, ly.p, found.p, at.p, load.p);
+            if (nq == 4) launch_nonlocal_fx<4>(ctx, at.p, load.p, found.p, lx.p, ly.p, fx.p, fy.p);
+            else launch_nonlocal_fx<9>(ctx, at.p, load.p, found.p, lx.p, ly.p, fx.p, fy.p);
         }
-        if (nq == 4) launch_nonlocal<4>(ctx, lx.p, ly.p, fx.p, fy.p, in_ff ? largest.p : nullptr);
-        else launch_nonlocal<9>(ctx, lx.p, ly.p, fx.p, fy.p, in_ff ? largest.p : nullptr);
+        if (nq == 4) launch_nonlocal<4>(ctx, lx.p, ly.p, fx.p, fy.p, fixed ? found.p : nullptr);
+        else launch_nonlocal<9>(ctx, lx.p, ly.p, fx.p, fy.p, fixed ? found.p : nullptr);
         qx = fx.p;
         qy = fy.p;
     }

@@ -93,6 +93,13 @@ __device__ __forceinline__ long long fx_distance(int4 a, int4 b, int ex) {
     return d & ~(d >> 63);   // the shifts round down
 }
 
+// the exponent of the coordinates' unit: of the largest one, given by its bits
+constexpr int FX_MAX_EXPONENT = 20;   // below that the unit of the high words, 2^-8 radii, is far smaller than the radii
+__device__ __forceinline__ int fx_exponent(const unsigned long long* extent) {
+    const double x = __longlong_as_double((long long)*extent);
+    return x >= 8.0 ? ilogb(x) : 2;
+}
+
 // x^n of 0 <= x <= 1
 __device__ __forceinline__ long long fx_ipow(long long x, int n) {
     long long r = FX_ONE;
@@ -131,6 +138,51 @@ __device__ __forceinline__ unsigned long long fx_exp(long long d, const FXExp& f
     const unsigned x5 = __umulhi(__umulhi(x4, xh), 53687091u);                                    // x^5 / 120: 2^32 / 80
     const unsigned long long y = x - x2 + ((unsigned long long)x3 << 14) - ((unsigned long long)x4 << 4) + x5;
     return tab - (fx_mulhi(tab, y) >> 8);
+}
+
+// A value as v 2^-(63 + m) with v from 2^62 up to 2^63 (m = FX_EXP_ZERO: zero).  Kept so, an
+// influence has as many bits near the horizon, where it is small, as elsewhere.
+struct FXValue {
+    unsigned long long v;
+    int m;
+};
+
+// of x 2^-60, 0 <= x <= 2^60
+__device__ __forceinline__ FXValue fx_normalised(long long x) {
+    const int z = max(__clzll(x), 1);
+    return x > 0 ? FXValue{(unsigned long long)x << (z - 1), z - 4} : FXValue{0, FX_EXP_ZERO};
+}
+
+__device__ __forceinline__ FXValue fx_power(FXValue x, int n) {
+    if (n == 1 || (n > 0 && x.m == FX_EXP_ZERO)) return x;
+    FXValue r{1ull << 63, 0};
+    for (int k = 0; k < n; ++k) {   // 2^60 <= high product < 2^62
+        const unsigned long long h = fx_mulhi(r.v, x.v);
+        const int s = h >> 61 ? 1 : 2;
+        r = FXValue{h << s, r.m + x.m + s - 1};
+    }
+    return r;
+}
+
+// shape<INF> of two points (n = 2 and the exponents that fx_supported names)
+template<int INF>
+__device__ __forceinline__ FXValue fx_shape(const Model& m, int4 a, int4 b, int ex, const FXExp& f,
+                                            const unsigned long long* table) {
+    if constexpr (INF == NLGPU_INFLUENCE_EXPONENTIAL) {
+        FXValue r;
+        r.v = fx_exp(fx_distance<FX_EXP_UNIT>(a, b, ex), f, table, r.m);
+        return r;
+    } else {
+        const long long d = fx_distance<60>(a, b, ex);
+        if constexpr (INF == NLGPU_INFLUENCE_FAST_POLYNOMIAL) return fx_normalised(FX_ONE - d);
+        else return d < FX_ONE ? fx_power(fx_normalised(FX_ONE - fx_ipow(d, m.p / 2)), int(m.q)) : FXValue{0, FX_EXP_ZERO};
+    }
+}
+
+// the double (its 53 bits rounded from 62 or 63)
+__device__ __forceinline__ double fx_value(FXValue x) {
+    const unsigned long long h = (x.v + 512) >> 10;   // 2^52 .. 2^53
+    return x.m == FX_EXP_ZERO ? 0.0 : __longlong_as_double((long long)(((unsigned long long)(1021 - x.m) << 52) + h));
 }
 
 inline FXExp fx_exp_setup(double q) {

@@ -1,4 +1,5 @@
-"""The float-float nodal flux: scale invariance over the whole exponent range, and non-finite temperatures."""
+"""The nodal flux in fixed point: scale invariance over the whole exponent range, non-finite temperatures, and the
+rounding of the FP64 kernel."""
 import numpy as np
 import pytest
 
@@ -33,3 +34,47 @@ def test_flux_scaling_and_non_finite_temperatures(element, influence, p):
     for a, b in zip(pb.calc_flux(u), f0):
         assert not np.isfinite(a[corner])
         assert np.abs(a[far] - b[far]).max() <= 819 * 4 * np.finfo(float).eps * scale
+
+
+@pytest.mark.parametrize("element, nx, ny, influence, radius, p, q", [
+    ("bilinear", 5, 3, "fast_polynomial", 0.5, 2, 1.0),
+    ("bilinear", 40, 30, "fast_polynomial", 0.9, 2, 1.0),      # thousands of terms a lane
+    ("bilinear", 100, 100, "fast_polynomial", 0.7, 2, 1.0),    # (30 000 an element: float-float lost 2e-14 of them)
+    ("serendipity", 12, 10, "polynomial", 0.6, 2, 1.0),
+    ("serendipity", 12, 10, "polynomial", 0.6, 8, 3.0),
+    ("bilinear", 20, 15, "polynomial", 0.4, 2, 16.0),          # the steepest covered
+    ("serendipity", 16, 12, "exponential", 0.4, 2, 0.5),
+    ("serendipity", 16, 12, "exponential", 0.2, 2, 0.333),     # the ends of the covered range,
+    ("serendipity", 16, 12, "exponential", 0.2, 2, 16.0),
+    ("serendipity", 16, 12, "exponential", 0.2, 2, 17.0),      # outside,
+    ("bilinear", 16, 12, "exponential", 0.005, 40, 2.0),       # d^(p / n) beyond single precision
+    ("bilinear", 16, 12, "exponential", 1e-7, 2, 0.5),         # coordinates of millions of radii
+])
+@pytest.mark.parametrize("waves", [False, True])
+def test_flux_rounds_as_the_fp64_kernel(element, nx, ny, influence, radius, p, q, waves):
+    """Against the option's FP64 kernel: each of the two rounds the squared distance, the value, the weight and the sums
+    to an eps or two; the waves cancel in the sums."""
+    from nonlocal_gb300 import _lib
+    from nonlocal_gb300 import thermal as T
+    from nonlocal_gb300.meshgen import structured_quad_mesh
+    if _lib.device_count() == 0:
+        pytest.skip("no CUDA device")
+    mesh = structured_quad_mesh(nx, ny, element, jitter=0.15, seed=2)
+    x, y = mesh.nodes.T
+    t = np.sin(31.0 * x) * np.cos(29.0 * y) if waves else 3.0 * x + y * y
+    flux = []
+    for kind in ("auto", "fp64"):
+        pb = T.Problem2D.from_mesh(mesh)
+        pb.set_model(T.Model2D(influence=influence, radius=(radius, radius), local_weight=0.0, p=p, q=q))
+        pb.set_assembly_precision(kind)
+        flux.append(np.array(pb.calc_flux(t)))
+    assert np.isfinite(flux[1]).all()
+    # what a relative change of d does to the value: q (p / n) d^(p / n) e^(-q d^(p / n)) <= p / n / e for the
+    # exponential, p q / n at most for the polynomials
+    eps = np.finfo(float).eps
+    steep = p * q / 2.0 if influence != "exponential" else p / 2.0
+    grad = 45.0 if waves else 4.0   # the largest |grad t|, and the quadrature's part of it
+    # the normalisation makes the influence's integral 1 over the plane, at most 1 over the mesh; radii far below
+    # an element's size see one point, whose share is bounded by the flux itself
+    size = max(np.abs(flux[1]).max(), 1.1 * grad)
+    assert np.abs(flux[0] - flux[1]).max() <= (4.0 * steep + 8.0) * eps * size

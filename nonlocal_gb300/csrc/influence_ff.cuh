@@ -1,5 +1,5 @@
-// Influence functions in float-float, shared by the pair assembly and the flux
-// post-processing.
+// Influence functions in float-float (the pair assembly of mixed-precision solves) and in
+// fixed point (the pair assembly and the flux post-processing).
 #pragma once
 
 #include <cmath>
@@ -21,7 +21,12 @@ __device__ __forceinline__ ff shape_ff(const Model& m, ff z0, ff z1, ff q, const
     if constexpr (INF == NLGPU_INFLUENCE_FAST_POLYNOMIAL) {
         return ff_lt(d, 1.0f) ? ff_sub(ff_make(1.0f), d) : ff_make(0.0f);
     } else {
-        const ff dp = ff_ipow(d, m.p / m.n);
+        ff dp = d;
+        if (m.p != m.n) {
+            dp = ff_ipow(d, m.p / m.n);
+            // beyond single precision the exponential is 0
+            if (INF == NLGPU_INFLUENCE_EXPONENTIAL && !(dp.h <= 1e30f) && d.h <= 3.4e38f) dp = ff_make(1e30f);
+        }
         if constexpr (INF == NLGPU_INFLUENCE_POLYNOMIAL)
             return ff_lt(d, 1.0f) ? ff_ipow(ff_sub(ff_make(1.0f), dp), int(m.q)) : ff_make(0.0f);
         else
@@ -37,8 +42,8 @@ inline void fill_exp_table(FFExpTable& t) {
     }
 }
 
-// float-float covers the continuous influence kinds with an integral power
-// p / n and constant conductivity; the rest runs the FP64 kernel
+// float-float covers the continuous influence kinds with an integral power p / n; the
+// rest runs the FP64 kernel
 inline bool ff_supported(const Model& m) {
     if (m.n < 1) return false;
     if (m.influence == NLGPU_INFLUENCE_FAST_POLYNOMIAL) return true;

@@ -75,3 +75,15 @@ def test_non_finite_field_reaches_its_rows(T):
     # beyond the influence of the element nothing changes, to the order of the sums
     far = np.isfinite(fp[0])
     assert far.any() and np.abs(ff[0] - clean)[far].max() <= 1e-14 * np.abs(clean).max()
+
+
+def test_powers_beyond_single_precision(T):
+    """Elements several radii wide and a steep exponential: d^(p / n) overflows a float, where the value is 0."""
+    from nonlocal_gb300.meshgen import structured_quad_mesh
+    mesh = structured_quad_mesh(16, 12, "bilinear", jitter=0.15, seed=2)
+    model = T.Model2D(influence="exponential", radius=(0.005, 0.005), local_weight=0.3, p=40, q=2.0)
+    _, (ff, _, fp) = matrices(T, mesh, model)
+    scale = np.abs(fp[0]).max()
+    assert np.isfinite(fp[0]).all()
+    for a, b in zip(ff, fp):   # values of 48 bits whose exponent is good to p / n times that
+        assert np.abs(a - b).max(initial=0.0) <= 1e-12 * scale

@@ -38,6 +38,42 @@ namespace {
 constexpr int AS_THREADS = 256;
 constexpr int AS_WARPS = AS_THREADS / 32;
 
+// What the fixed-point form of the pair blocks (below) depends on over the whole mesh.  An
+// element's x and y gradients share an exponent, so the smaller component has fewer bits;
+// that matters where an element with |w_x| << |w_y| meets one with |g_x| >> |g_y|, whose
+// products are then as large as the others'.  A power of two moved from one component's
+// g to its w (ff_shift) leaves every product as it is and evens out what all elements
+// have in common (a stretched mesh whose conductivity makes up for it); what remains is the
+// loss.  FP64 solves allow 4 bits (58 - 4 against 53), mixed-precision ones 10 (48, as the
+// influence values); meshes beyond that, and for fixed-point values coordinates of
+// 2^(FX_MAX_EXPONENT + 1) radii, take the FP64 kernel: each of the two kernels looks and one returns at once.
+constexpr int FF_NONE = 1 << 12;   // the four below are the largest difference of exponents + FF_NONE; 0: no element
+struct FFRange {
+    unsigned long long extent;     // the bits of the largest finite |coordinate| in units of the radii
+    int wx, wy, gx, gy;            // of w_x over w_y, w_y over w_x, g_x over g_y, g_y over g_x in an element
+};
+struct FFGate {
+    const FFRange* range;          // null: no condition
+    int max_loss;
+    bool fixed;                    // fixed-point values
+};
+
+__device__ __forceinline__ void ff_losses(const FFRange* r, int& x, int& y) {   // before the shift
+    x = r->wx == 0 || r->gy == 0 ? -FF_NONE : min(r->wx, r->gy) - FF_NONE;
+    y = r->wy == 0 || r->gx == 0 ? -FF_NONE : min(r->wy, r->gx) - FF_NONE;
+}
+__device__ __forceinline__ int ff_shift(const FFRange* r) {   // w_x 2^shift, g_x 2^-shift
+    int x, y;
+    ff_losses(r, x, y);
+    return min(256, max(-256, (y - x) >> 1));
+}
+__device__ __forceinline__ bool ff_in_range(const FFGate& g) {
+    int x, y;
+    ff_losses(g.range, x, y);
+    const int s = ff_shift(g.range);
+    return max(x + s, y - s) <= g.max_loss && (!g.fixed || int(g.range->extent >> 52) <= 1023 + FX_MAX_EXPONENT);
+}
+
 struct AssembleArgs {
     i64 E;
     i64 e0;                   // first element (the float-float kernel's tuning samples start later)
@@ -55,6 +91,7 @@ struct AssembleArgs {
     bool symmetric;
     int cap;                  // accumulator entries in shared memory
     int* error;               // set when an entry is missing from its pattern
+    FFGate gate;              // the fixed-point kernel's range: the FP64 kernel runs beyond it
 };
 
 __device__ __forceinline__ i64 find_col(const int32_t* col, i64 lo, i64 hi, int32_t c) {
@@ -90,6 +127,7 @@ __global__ void __launch_bounds__(AS_THREADS) k_assemble_pairs(AssembleArgs a, M
     __shared__ i64 row_start[NEN];
     __shared__ int row_len[NEN], row_off[NEN + 1];
     __shared__ int use_smem;
+    if (a.gate.range && ff_in_range(a.gate)) return;   // k_assemble_pairs_ff did it
 
     auto* pairs = reinterpret_cast<PairSmem<NEN, NQ>*>(smem_raw);
     double* acc = reinterpret_cast<double*>(smem_raw + sizeof(PairSmem<NEN, NQ>) * AS_WARPS);
@@ -236,16 +274,16 @@ __global__ void __launch_bounds__(AS_THREADS) k_assemble_pairs(AssembleArgs a, M
 // The same pair blocks off the FP64 pipe: the influence values in fixed point
 // (influence_ff.cuh, 60 bits) or float-float (ff.cuh, about 48 bits, for exponents that
 // the former does not cover), both contractions in fixed point on the integer
-// multipliers.  Everything a block multiplies lies within a few binary orders of its
-// largest factor, so eNL's gradients carry one exponent per element and the
-// exponential's values one per pair; a number is then up to 61 bits in two signed
+// multipliers.  Both elements' gradients carry one exponent each (FFRange says where that
+// is not enough) and the exponential's values one per pair; a number is then up to 61 bits in two signed
 // words (hi 2^30 + lo), a multiply-add three 32 x 32 + 64-bit ones (hi hi, and
 // hi lo + lo hi into a second accumulator; lo lo lies below the result's last bit),
 // and the sums are exact.  Against the compensated float-float dot product (12
 // FP32 instructions a term, errors of order 2^-48) that is a quarter of the
 // instructions and half the pipe time (64 lanes a clock against 128); the gradients'
-// 58 bits leave an error below FP64's (against extended precision, entries' median
-// 2.4e-14 for the FP64 kernel's 3.4e-14 on 8-node meshes, with cancellation).
+// 58 bits leave an error below FP64's (against extended precision and the root of the
+// diagonal entries' product, rms, 12 x 14 bilinear and 6 x 8 8-node meshes, exponential:
+// 3.3e-16 and 9.7e-16 for the FP64 kernel's 5.2e-16 and 1.3e-15).
 // Weights, Lambda and the constant factors are folded into the two staged copies
 // of the gradients (k_ff_stage), the pairs this element owns are listed once per
 // element, and a pair whose influence is zero everywhere ends there.
@@ -264,7 +302,7 @@ constexpr int FF_LIST = 1024;     // candidates listed at a time
 
 struct FFArgs {
     const int4* qcoord;     // [e][q]: coordinates in units of the radii, (x/r0 .h, .l, y/r1 .h, .l) or fixed point
-    const unsigned long long* extent;   // fixed point: the largest |coordinate|, as the bits of a double
+    const FFRange* range;
     const int2* g;          // [e][q][x, y][j]: w_q norm (1 - p1) [lambda_q] Lambda G_j 2^(57 - exps.x) as hi 2^30 + lo
     const int4* w;          // [e][i][q]: w_q G_i 2^(57 - exps.y), (x hi, lo, y hi, lo)
     const int2* exps;       // [e]: the exponents of the largest |g| and |w|
@@ -275,17 +313,49 @@ struct FFArgs {
     FXExp fx_exp;
 };
 
-// the largest finite |coordinate| in units of the radii
-__global__ void k_fx_extent(i64 n, const double* __restrict__ qcoord, double ix, double iy,
-                            unsigned long long* __restrict__ extent) {
-    unsigned long long m = 0ull;
-    for (i64 t = blockIdx.x * i64(blockDim.x) + threadIdx.x; t < n; t += i64(gridDim.x) * blockDim.x) {
-        const double x = fabs(qcoord[2 * t] * ix), y = fabs(qcoord[2 * t + 1] * iy);
-        if (isfinite(x)) m = max(m, (unsigned long long)__double_as_longlong(x));
-        if (isfinite(y)) m = max(m, (unsigned long long)__double_as_longlong(y));
+// the conductivity times a gradient, as the pair blocks use it
+__device__ __forceinline__ double2 ff_flux(const Model& m, double gx, double gy) {
+    if (m.cond_kind == NLGPU_CONDUCTIVITY_ISOTROPIC) return make_double2(gx, gy);
+    if (m.cond_kind == NLGPU_CONDUCTIVITY_ORTHOTROPIC) return make_double2(m.cond[0] * gx, m.cond[1] * gy);
+    return make_double2(m.cond[0] * gx + m.cond[2] * gy, m.cond[2] * gx + m.cond[1] * gy);
+}
+
+// one warp per element
+__global__ void k_ff_range(i64 E, int nen, int nq, const double* __restrict__ deriv, const double* __restrict__ qcoord, Model m,
+                           FFRange* __restrict__ range) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    unsigned long long extent = 0;
+    int wx = 0, wy = 0, gx = 0, gy = 0;
+    for (i64 e = (blockIdx.x * i64(blockDim.x) + threadIdx.x) / 32; e < E; e += i64(gridDim.x) * blockDim.x / 32) {
+        for (int t = lane; t < 2 * nq; t += 32) {
+            const double x = fabs(qcoord[2 * e * nq + t] * m.inv_r[t & 1]);
+            if (isfinite(x)) extent = max(extent, (unsigned long long)__double_as_longlong(x));
+        }
+        unsigned top[4] = {0u, 0u, 0u, 0u};   // high words of the largest |w_x|, |w_y|, |g_x|, |g_y|
+        auto high = [](double x) { return unsigned(__double2hiint(x)) & 0x7fffffffu; };
+        for (int t = lane; t < nen * nq; t += 32) {
+            const double2 d = reinterpret_cast<const double2*>(deriv)[e * nen * nq + t], g = ff_flux(m, d.x, d.y);
+            top[0] = max(top[0], high(d.x)); top[1] = max(top[1], high(d.y));
+            top[2] = max(top[2], high(g.x)); top[3] = max(top[3], high(g.y));
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) top[k] = __reduce_max_sync(full, top[k]);
+        // a component that is zero everywhere counts as far below the other
+        auto take = [](unsigned a, unsigned b, int& ab, int& ba) {
+            if (a >= 0x7ff00000u || b >= 0x7ff00000u || (a | b) == 0u) return;
+            const int d = (a ? int(a >> 20) : -1500) - (b ? int(b >> 20) : -1500);
+            ab = max(ab, FF_NONE + d);
+            ba = max(ba, FF_NONE - d);
+        };
+        take(top[0], top[1], wx, wy);
+        take(top[2], top[3], gx, gy);
     }
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(extent, m);
+    for (int o = 16; o > 0; o >>= 1) extent = max(extent, __shfl_xor_sync(full, extent, o));
+    if (lane == 0) {
+        atomicMax(&range->extent, extent);
+        atomicMax(&range->wx, wx); atomicMax(&range->wy, wy); atomicMax(&range->gx, gx); atomicMax(&range->gy, gy);
+    }
 }
 
 // x 2^(57 - e), |x| < 2^(e + 1), by integer operations (the FP64 pipe's conversions made the staging 0.19 ms
@@ -303,24 +373,22 @@ __device__ __forceinline__ int2 ff_fixed(double x, int e) {
 __global__ void k_ff_stage(i64 E, int nen, int nq, const int32_t* __restrict__ elems, const uint8_t* __restrict__ is_inner,
                            const double* __restrict__ deriv, const double* __restrict__ qcoord,
                            const double* __restrict__ cond_field, Model m, Basis b,
-                           const unsigned long long* __restrict__ extent, int4* __restrict__ qff,
+                           const FFRange* __restrict__ range, bool fixed, int4* __restrict__ qff,
                            int2* __restrict__ g, int4* __restrict__ w, int2* __restrict__ exps,
                            int32_t* __restrict__ nodes) {
     const double cnl = m.norm * (1.0 - m.p1);
     const bool iso = m.cond_kind == NLGPU_CONDUCTIVITY_ISOTROPIC;
     const int lane = threadIdx.x & 31;
+    const int shift = ff_shift(range);
+    const double up = scalbn(1.0, shift), down = scalbn(1.0, -shift);
     auto values = [&](i64 e, int t, double (&v)[4]) {   // (Lambda G scaled, w G) of (i, q) = (t / nq, t % nq)
         const double gx = deriv[2 * (e * nen * nq + t)], gy = deriv[2 * (e * nen * nq + t) + 1];
         const int q = t % nq;
         const double lam = cond_field ? cond_field[e * nq + q] : m.cond[0];
         const double c = b.w[q] * cnl * (iso ? lam : 1.0);
-        v[0] = c * gx; v[1] = c * gy;
-        if (m.cond_kind == NLGPU_CONDUCTIVITY_ORTHOTROPIC) { v[0] *= m.cond[0]; v[1] *= m.cond[1]; }
-        else if (!iso) {
-            v[0] = c * (m.cond[0] * gx + m.cond[2] * gy);
-            v[1] = c * (m.cond[2] * gx + m.cond[1] * gy);
-        }
-        v[2] = b.w[q] * gx; v[3] = b.w[q] * gy;
+        const double2 g = ff_flux(m, gx, gy);
+        v[0] = c * g.x * down; v[1] = c * g.y;
+        v[2] = b.w[q] * gx * up; v[3] = b.w[q] * gy;
     };
     for (i64 e = (blockIdx.x * i64(blockDim.x) + threadIdx.x) / 32; e < E; e += i64(gridDim.x) * blockDim.x / 32) {
         // the high words of the largest magnitudes
@@ -337,9 +405,9 @@ __global__ void k_ff_stage(i64 E, int nen, int nq, const int32_t* __restrict__ e
         bool bad_g = mg >= 0x7ff00000u, bad_w = mw >= 0x7ff00000u;
         if (lane < nq) {
             const double x = qcoord[2 * (e * nq + lane)], y = qcoord[2 * (e * nq + lane) + 1];
-            if (extent) {   // fixed point has no NaN: the element's blocks become one
+            if (fixed) {   // fixed point has no NaN: the element's blocks become one
                 const bool finite = isfinite(x * m.inv_r[0]) && isfinite(y * m.inv_r[1]);
-                const int ex = fx_exponent(extent);
+                const int ex = fx_exponent(&range->extent);
                 const int2 fx = fx_coordinate(finite ? x : 0.0, m.inv_r[0], ex);
                 const int2 fy = fx_coordinate(finite ? y : 0.0, m.inv_r[1], ex);
                 qff[e * nq + lane] = make_int4(fx.x, fx.y, fy.x, fy.y);
@@ -408,7 +476,8 @@ __global__ void __launch_bounds__(WARPS * 32) k_assemble_pairs_ff(AssembleArgs a
         for (int t = threadIdx.x; t < 2 * FF_EXP_K + 1; t += blockDim.x) etab[t] = ff{f.ff_table.v[t].x, f.ff_table.v[t].y};
     if constexpr (EXP && FIX)
         for (int t = threadIdx.x; t < FX_EXP_K; t += blockDim.x) xtab[t] = f.fx_table.v[t];
-    const int ex = FIX ? fx_exponent(f.extent) : 0;
+    if (!ff_in_range(a.gate)) return;   // k_assemble_pairs does it
+    const int ex = FIX ? fx_exponent(&f.range->extent) : 0;
 
     auto* pairs = reinterpret_cast<PairFF<NEN, NQ>*>(smem_raw);
     double* acc = reinterpret_cast<double*>(smem_raw + sizeof(PairFF<NEN, NQ>) * WARPS * GROUPS);
@@ -730,7 +799,7 @@ template<int NEN, int NQ, int INF>
 void launch_pairs(Ctx& ctx, const AssembleArgs& a, bool sym) {
     const size_t fixed = sizeof(PairSmem<NEN, NQ>) * AS_WARPS;
     const size_t dyn = fixed + size_t(a.cap) * (sizeof(double) + sizeof(int32_t));
-    const unsigned grid = unsigned(std::min<i64>(a.E, 152 * 16));
+    const unsigned grid = unsigned(std::min<i64>(a.E, a.gate.range ? 152 * 2 : 152 * 16));   // mostly to return
     if (sym) {
         auto kernel = k_assemble_pairs<NEN, NQ, INF, true>;
         NL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
@@ -754,10 +823,10 @@ void dispatch_influence(Ctx& ctx, const AssembleArgs& a, bool sym) {
 
 template<int NEN, int NQ, int INF, int WARPS>
 void launch_pairs_ff_w(Ctx& ctx, AssembleArgs a, const FFArgs& f, bool sym) {
-    auto kernel = f.extent ? (sym ? k_assemble_pairs_ff<NEN, NQ, INF, true, WARPS, true>
-                                  : k_assemble_pairs_ff<NEN, NQ, INF, false, WARPS, true>)
-                           : (sym ? k_assemble_pairs_ff<NEN, NQ, INF, true, WARPS, false>
-                                  : k_assemble_pairs_ff<NEN, NQ, INF, false, WARPS, false>);
+    auto kernel = a.gate.fixed ? (sym ? k_assemble_pairs_ff<NEN, NQ, INF, true, WARPS, true>
+                                      : k_assemble_pairs_ff<NEN, NQ, INF, false, WARPS, true>)
+                               : (sym ? k_assemble_pairs_ff<NEN, NQ, INF, true, WARPS, false>
+                                      : k_assemble_pairs_ff<NEN, NQ, INF, false, WARPS, false>);
     // the row accumulators take what shared memory the per-warp blocks leave
     int dev = 0, optin = 0;
     NL_CUDA(cudaGetDevice(&dev));
@@ -783,7 +852,7 @@ void launch_pairs_ff(Ctx& ctx, AssembleArgs a, const FFArgs& f, bool sym) {
     int warps = ctx.ff_warps_option;
     if (warps == 0 && a.E < 152 * 64) warps = 32;   // the four samples would cost as much as the assembly
     if (warps == 0) {
-        const int key = NEN * 1000 + INF * 10 + (sym ? 1 : 0) + (f.extent ? 2 : 0);
+        const int key = NEN * 1000 + INF * 10 + (sym ? 1 : 0) + (a.gate.fixed ? 2 : 0);
         auto it = ctx.ff_warps_tuned.find(key);
         if (it != ctx.ff_warps_tuned.end()) {
             warps = it->second;
@@ -854,7 +923,7 @@ void assemble_full(Ctx& ctx) {
     err.resize(1);
     err.zero(ctx.stream);
     a.error = err.p;
-    dbuf<unsigned long long> extent;
+    dbuf<FFRange> range;
     // unordered pairs need a symmetric influence and constant conductivity
     const bool sym = ctx.symmetric && !ctx.cond_field.n && !ctx.ordered_pairs;
     // The pair blocks in fixed point: the FP64 kernel's accuracy at a quarter of its
@@ -872,16 +941,15 @@ void assemble_full(Ctx& ctx) {
         ctx.ff_w.reserve(size_t(ctx.n_elems * nen * nq));
         ctx.ff_exps.reserve(size_t(ctx.n_elems));
         ctx.ff_nodes.reserve(size_t(ctx.n_elems * nen));
-        if (fixed) {
-            extent.resize(1);
-            extent.zero(ctx.stream);
-            NL_LAUNCH(k_fx_extent, grid_for(ctx.n_elems * nq, 256, 152 * 4), 256, 0, ctx.stream, ctx.n_elems * nq,
-                      ctx.qcoord.p, ctx.model.inv_r[0], ctx.model.inv_r[1], extent.p);
-        }
+        range.resize(1);
+        range.zero(ctx.stream);
+        a.gate = {range.p, ctx.ff_assembly ? 10 : 4, fixed};
+        NL_LAUNCH(k_ff_range, grid_for(ctx.n_elems * 32, 256, 152 * 8), 256, 0, ctx.stream, ctx.n_elems, nen, nq, ctx.deriv.p,
+                  ctx.qcoord.p, ctx.model, range.p);
         NL_LAUNCH(k_ff_stage, grid_for(ctx.n_elems * 32, 256), 256, 0, ctx.stream, ctx.n_elems, nen, nq, ctx.elems.p,
-                  ctx.is_inner.p, ctx.deriv.p, ctx.qcoord.p, a.cond_field, ctx.model, ctx.basis, extent.p,
+                  ctx.is_inner.p, ctx.deriv.p, ctx.qcoord.p, a.cond_field, ctx.model, ctx.basis, range.p, fixed,
                   ctx.ff_qcoord.p, ctx.ff_g.p, ctx.ff_w.p, ctx.ff_exps.p, ctx.ff_nodes.p);
-        FFArgs f{ctx.ff_qcoord.p, extent.p, ctx.ff_g.p, ctx.ff_w.p, ctx.ff_exps.p, ctx.ff_nodes.p, {}, {}, {}};
+        FFArgs f{ctx.ff_qcoord.p, range.p, ctx.ff_g.p, ctx.ff_w.p, ctx.ff_exps.p, ctx.ff_nodes.p, {}, {}, {}};
         if (ctx.model.influence == NLGPU_INFLUENCE_EXPONENTIAL && fixed) {
             f.fx_table = fx_exp_table();
             f.fx_exp = fx_exp_setup(ctx.model.q);
@@ -890,7 +958,8 @@ void assemble_full(Ctx& ctx) {
         }
         if (nen == 4) dispatch_influence_ff<4, 4>(ctx, a, f, sym);
         else dispatch_influence_ff<8, 9>(ctx, a, f, sym);
-    } else if (ctx.basis.nen == 4) {
+    }
+    if (ctx.basis.nen == 4) {
         a.cap = int((200 * 1024 - sizeof(PairSmem<4, 4>) * AS_WARPS) / 12);
         dispatch_influence<4, 4>(ctx, a, sym);
     } else {

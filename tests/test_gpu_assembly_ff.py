@@ -87,3 +87,89 @@ def test_powers_beyond_single_precision(T):
     assert np.isfinite(fp[0]).all()
     for a, b in zip(ff, fp):   # values of 48 bits whose exponent is good to p / n times that
         assert np.abs(a - b).max(initial=0.0) <= 1e-12 * scale
+
+
+def exact_inner(mesh, pb, model):
+    """The inner matrix by pairs of elements in extended precision (polynomial influence, without its normalisation),
+    and beside it the sums of its terms' magnitudes."""
+    L = np.longdouble
+    qc, jac, der = (v.astype(L) for v in pb.quadrature())
+    w = pb.basis()["basis_weights"].astype(L)
+    off, lst = pb.neighbours()
+    lam = np.array(model.conductivity * (2 if len(model.conductivity) == 1 else 1), dtype=L)
+    K, M = (np.zeros((mesh.n_nodes, mesh.n_nodes), dtype=L) for _ in range(2))
+    power = 1 if model.influence == "fast_polynomial" else int(model.q)
+    for e in range(mesh.n_elements):
+        for f in lst[off[e]:off[e + 1]]:
+            d = (((qc[e][:, None] - qc[f][None]) / np.array(model.radius, dtype=L)) ** 2).sum(-1)
+            phi = np.where(d < 1, 1 - d, 0) ** power * w[:, None] * w[None]
+            g = der[f] * lam
+            at = np.ix_(mesh.elements[e], mesh.elements[f])
+            K[at] += sum(der[e][:, :, k] @ phi @ g[:, :, k].T for k in (0, 1))
+            M[at] += sum(abs(der[e][:, :, k]) @ phi @ abs(g[:, :, k]).T for k in (0, 1))
+    return K, M
+
+
+def errors(T, mesh, model, fixed):
+    """Per assembly precision: the largest error of an entry against its terms' sum, and against the root of its
+    diagonal entries' product."""
+    pb = T.Problem2D.from_mesh(mesh)
+    pb.set_model(model)
+    pb.add_boundary(T.Boundary(edges=fixed, kind="temperature", value=1.0))
+    pb.find_neighbours()
+    K, M = exact_inner(mesh, pb, model)
+    diag = np.sqrt(np.abs(K.diagonal()))
+    out = {}
+    for kind in ("ff", "auto", "fp64"):
+        pb.set_assembly_precision(kind)
+        pb.conductivity_matrix("FULL")
+        rp, col, val = pb.matrix("inner")
+        row = np.repeat(np.arange(mesh.n_nodes), np.diff(rp))
+        free = ~np.isin(row, fixed) & ~np.isin(col, fixed)
+        row, col, val = row[free], col[free], val[free]
+        ref, mag = K[row, col], M[row, col]
+        err = np.abs(val / ((val * ref).sum() / (ref * ref).sum()) - ref)   # up to the influence's normalisation
+        out[kind] = (float((err / np.where(mag > 0, mag, 1)).max()), float((err / (diag[row] * diag[col])).max()))
+    return out
+
+
+@pytest.mark.parametrize("aspect, conductivity", [
+    ("x", (1e6, 1.0)),        # stretched elements, the conductivity makes up for it: a common power of two
+    ("x", (1.0,)),
+    ("x", (1.0, 0.0)),        # nothing in one direction
+    ("both", (1.0,)),         # elements stretched one way beside ones stretched the other: FP64 for FP64 solves
+])
+def test_stretched_elements(T, aspect, conductivity):
+    """As accurate as the FP64 kernel, whose entries are sums of at most 81 pairs of 16 products: 8 eps of the diagonal
+    (of the terms where the entries' scales differ by powers of the stretch)."""
+    from nonlocal_gb300.meshgen import BILINEAR, QuadMesh
+    rng = np.random.default_rng(5)
+    if aspect == "x":
+        xs, ys, radius, move = np.arange(7) * 1000.0, np.arange(6) * 1.0, (2100.0, 2.1), (200.0, 0.2)
+    else:
+        xs = np.concatenate([[0.0], np.cumsum([1000.0] * 3 + [1.0] * 3)])
+        ys = np.concatenate([[0.0], np.cumsum([1.0, 1.0, 30.0, 1000.0, 1000.0])])
+        radius, move = (2100.0, 2100.0), (0.2, 0.2)
+    X, Y = np.meshgrid(xs, ys)
+    nodes = np.stack([X.ravel(), Y.ravel()], 1) + rng.uniform(-1.0, 1.0, (42, 2)) * np.array(move)
+    el = np.array([[j * 7 + i, j * 7 + i + 1, (j + 1) * 7 + i + 1, (j + 1) * 7 + i] for j in range(5) for i in range(6)])
+    model = T.Model2D(influence="fast_polynomial", radius=radius, local_weight=0.0, conductivity=conductivity)
+    e = errors(T, QuadMesh(BILINEAR, nodes, el.astype(np.int64), {}), model, np.array([[0, 7]]))
+    which = 1 if aspect == "x" else 0
+    eps = np.finfo(float).eps
+    assert e["fp64"][which] <= 8 * eps
+    assert e["auto"][which] <= 8 * eps
+    assert e["ff"][which] <= 1e-12
+
+
+def test_coordinates_of_a_billion_radii(T):
+    """Fixed-point coordinates have a unit of 2^-58 of the largest: far from the origin the FP64 kernel takes over."""
+    from nonlocal_gb300.meshgen import structured_quad_mesh
+    mesh = structured_quad_mesh(6, 5, "bilinear", width=6.0, height=5.0)
+    mesh.nodes += 2.0 ** 31
+    model = T.Model2D(influence="fast_polynomial", radius=(2.25, 2.25), local_weight=0.3)
+    _, (ff, auto, fp) = matrices(T, mesh, model)
+    scale = np.abs(fp[0]).max()
+    for a, x, b in zip(ff, auto, fp):
+        assert np.abs(x - b).max(initial=0.0) <= 32 * 2.0 ** -53 * 20 * scale
+        assert np.abs(a - b).max(initial=0.0) <= 32 * 2.0 ** -53 * 20 * scale

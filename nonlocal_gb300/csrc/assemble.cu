@@ -275,15 +275,17 @@ __global__ void __launch_bounds__(AS_THREADS) k_assemble_pairs(AssembleArgs a, M
 // (influence_ff.cuh, 60 bits) or float-float (ff.cuh, about 48 bits, for exponents that
 // the former does not cover), both contractions in fixed point on the integer
 // multipliers.  Both elements' gradients carry one exponent each (FFRange says where that
-// is not enough) and the exponential's values one per pair; a number is then up to 61 bits in two signed
+// is not enough) and the influence values one per pair, so that the entries at the
+// horizon's edge, where they are small, keep their digits; a number is up to 61 bits in two signed
 // words (hi 2^30 + lo), a multiply-add three 32 x 32 + 64-bit ones (hi hi, and
 // hi lo + lo hi into a second accumulator; lo lo lies below the result's last bit),
 // and the sums are exact.  Against the compensated float-float dot product (12
 // FP32 instructions a term, errors of order 2^-48) that is a quarter of the
 // instructions and half the pipe time (64 lanes a clock against 128); the gradients'
 // 58 bits leave an error below FP64's (against extended precision and the root of the
-// diagonal entries' product, rms, 12 x 14 bilinear and 6 x 8 8-node meshes, exponential:
-// 3.3e-16 and 9.7e-16 for the FP64 kernel's 5.2e-16 and 1.3e-15).
+// diagonal entries' product, rms, 12 x 14 bilinear and 6 x 8 8-node meshes: exponential
+// 3.3e-16 and 9.7e-16 for the FP64 kernel's 5.2e-16 and 1.3e-15, 1 - d 1.2e-16 and 3.8e-16 for
+// 1.8e-16 and 4.9e-16).
 // Weights, Lambda and the constant factors are folded into the two staged copies
 // of the gradients (k_ff_stage), the pairs this element owns are listed once per
 // element, and a pair whose influence is zero everywhere ends there.
@@ -446,7 +448,7 @@ template<int NEN, int NQ>
 struct PairFF {
     static constexpr int PS = (NQ + 1) / 2 * 2;   // influence values per row, padded to whole 16 bytes
     int4 q[NQ];           // eNL's points
-    int2 phi[NQ * PS];    // shape(qL, qNL) 2^(60 - e_p), e_p an exponent of the pair
+    int2 phi[NQ * PS];    // shape(qL, qNL) 2^(60 - e_p), e_p an exponent of the pair's largest
     int4 h[NQ * NEN];     // H(qL, j): (x hi, lo, y hi, lo)
     int32_t nodes[NEN];
 };
@@ -568,13 +570,14 @@ __global__ void __launch_bounds__(WARPS * 32) k_assemble_pairs_ff(AssembleArgs a
                 bool finite = !bad;
                 if constexpr (FIX) {
                     long long v[PR];
-                    if constexpr (EXP) {
+                    if constexpr (INF != NLGPU_INFLUENCE_FAST_POLYNOMIAL) {
                         int mv[PR], smallest = FX_EXP_ZERO;
 #pragma unroll
                         for (int rnd = 0; rnd < PR; ++rnd) {
                             const int t = min(gl + LANES * rnd, NQ * NQ - 1);
-                            v[rnd] = (long long)(fx_exp(fx_distance<FX_EXP_UNIT>(eq[t / NQ], ps.q[t % NQ], ex), f.fx_exp, xtab,
-                                                    mv[rnd]) >> 3);
+                            const FXValue x = fx_shape<INF>(m, eq[t / NQ], ps.q[t % NQ], ex, f.fx_exp, xtab);
+                            v[rnd] = (long long)(x.v >> 3);
+                            mv[rnd] = x.m;
                             smallest = min(smallest, mv[rnd]);
                         }
 #pragma unroll
@@ -584,19 +587,22 @@ __global__ void __launch_bounds__(WARPS * 32) k_assemble_pairs_ff(AssembleArgs a
 #pragma unroll
                         for (int rnd = 0; rnd < PR; ++rnd) v[rnd] >>= min(mv[rnd] - smallest, 63);
                     } else {
-                        bool some = false;
+                        unsigned top = 0;   // the values' bits above 2^32, one more where there are none
 #pragma unroll
                         for (int rnd = 0; rnd < PR; ++rnd) {
                             const int t = min(gl + LANES * rnd, NQ * NQ - 1);
                             const long long d = fx_distance<60>(eq[t / NQ], ps.q[t % NQ], ex);
-                            if constexpr (INF == NLGPU_INFLUENCE_POLYNOMIAL)
-                                v[rnd] = d < FX_ONE ? fx_ipow(FX_ONE - fx_ipow(d, m.p / 2), int(m.q)) : 0;
-                            else
-                                v[rnd] = d < FX_ONE ? FX_ONE - d : 0;
-                            some = some || v[rnd] != 0;
+                            v[rnd] = d < FX_ONE ? FX_ONE - d : 0;
+                            top = max(top, unsigned(v[rnd] >> 32) | unsigned(v[rnd] != 0));
                         }
-                        const unsigned any = __ballot_sync(0xffffffffu, some) >> (LANES * group) & (0xffffffffu >> (32 - LANES));
-                        active = active && (any != 0 || self || bad);
+#pragma unroll
+                        for (int o = LANES / 2; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+                        active = active && (top != 0 || self || bad);
+                        // a pair at the horizon's edge: its small values moved up
+                        const int s = max(__clz(int(top)) - 4, 0);
+                        e_p = -s;
+#pragma unroll
+                        for (int rnd = 0; rnd < PR; ++rnd) v[rnd] <<= s;
                     }
                     if (!__any_sync(0xffffffffu, active)) continue;
 #pragma unroll
@@ -893,7 +899,9 @@ void launch_pairs_ff(Ctx& ctx, AssembleArgs a, const FFArgs& f, bool sym) {
 
 template<int NEN, int NQ>
 void dispatch_influence_ff(Ctx& ctx, const AssembleArgs& a, const FFArgs& f, bool sym) {
-    switch (ctx.model.influence) {
+    // the polynomial 1 - d is the fast one
+    const bool linear = a.gate.fixed && ctx.model.influence == NLGPU_INFLUENCE_POLYNOMIAL && ctx.model.p == 2 && ctx.model.q == 1.0;
+    switch (linear ? NLGPU_INFLUENCE_FAST_POLYNOMIAL : ctx.model.influence) {
     case NLGPU_INFLUENCE_FAST_POLYNOMIAL: launch_pairs_ff<NEN, NQ, NLGPU_INFLUENCE_FAST_POLYNOMIAL>(ctx, a, f, sym); break;
     case NLGPU_INFLUENCE_POLYNOMIAL: launch_pairs_ff<NEN, NQ, NLGPU_INFLUENCE_POLYNOMIAL>(ctx, a, f, sym); break;
     default: launch_pairs_ff<NEN, NQ, NLGPU_INFLUENCE_EXPONENTIAL>(ctx, a, f, sym); break;

@@ -55,9 +55,10 @@ inline bool ff_supported(const Model& m) {
 // ---------------------------------------------------------------- fixed point
 // The influence functions of the usual exponents (n = 2) in 64-bit integers, for the
 // pair assembly, whose contractions want fixed-point operands.  Coordinates in
-// units of the radii are 59-bit integers with one exponent per mesh, values have 60
-// bits: as accurate as FP64 (whose squared distance and exponential round to 53 bits
-// each), on pipes that have 32 times the FP64 rate.
+// units of the radii are 59-bit integers with one exponent per mesh; 1 - d has an error of
+// 2^-60 and its powers 60 bits, the exponential 54 (the units of q d log2(e), 2^-55, and of the two
+// that fx_mulhi drops): as accurate as FP64, whose squared distance and exponential
+// round to 53 bits each, on pipes that have 32 times the FP64 rate.
 
 // floor-like a b 2^-64 of unsigned numbers, up to 2 below (the low halves' product is left out)
 __device__ __forceinline__ unsigned long long fx_mulhi(unsigned long long a, unsigned long long b) {

@@ -162,6 +162,22 @@ def test_stretched_elements(T, aspect, conductivity):
     assert e["ff"][which] <= 1e-12
 
 
+@pytest.mark.parametrize("influence, q", [("fast_polynomial", 1.0), ("polynomial", 1.0), ("polynomial", 3.0),
+                                          ("polynomial", 16.0)])
+@pytest.mark.parametrize("element, nx, ny, radius", [("bilinear", 14, 12, 0.25), ("serendipity", 8, 6, 0.35)])
+def test_entries_at_the_edge_of_the_influence(T, influence, q, element, nx, ny, radius):
+    """Entries that only pairs at the horizon make, however small, keep their digits: a pair's values are good to 2^-52
+    of its largest one, of which an entry's own terms are 2^-17 or more in a block of 64 on a jittered mesh."""
+    from nonlocal_gb300.meshgen import structured_quad_mesh
+    mesh = structured_quad_mesh(nx, ny, element, jitter=0.2, seed=1)
+    model = T.Model2D(influence=influence, radius=(radius, radius), local_weight=0.0, q=q, conductivity=(2.0, 1.0))
+    e = errors(T, mesh, model, mesh.boundaries["left"])
+    assert e["auto"][0] <= 2.0 ** -35
+    assert e["ff"][0] <= 2.0 ** -35
+    # against the diagonal: the FP64 kernel's bound as for the stretched elements, q times for the power
+    assert e["auto"][1] <= 32 * q ** 0.5 * np.finfo(float).eps
+
+
 def test_coordinates_of_a_billion_radii(T):
     """Fixed-point coordinates have a unit of 2^-58 of the largest: far from the origin the FP64 kernel takes over."""
     from nonlocal_gb300.meshgen import structured_quad_mesh

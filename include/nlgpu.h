@@ -566,7 +566,7 @@ int nlgpu_nonstationary_1d_temperature(nlgpu_ctx* ctx, double* temperature);
  * NLGPU_ASSEMBLY_FP64 always in FP64 operations.  Float-float (about 48
  * significant bits) covers the fast-polynomial, polynomial and exponential
  * influence with integral p / n, fixed point those with n = 2 (polynomials of
- * even p and q <= 16, exponentials of p = 2 and 0.333 <= q <= 16); other models
+ * even p and q <= 16, exponentials of p = 2 and 0.333 <= q <= 2); other models
  * use FP64.  The nodal flux's nonlocal average is in float-float where that
  * covers the model, in FP64 otherwise and with NLGPU_ASSEMBLY_FP64.
  * NLGPU_OPTION_FP32_SYMMETRIC = 1 makes the mixed solve's FP32 SpMV read only

@@ -204,9 +204,10 @@ struct BandFactor {
 };
 
 // 1 / d by two Newton steps from the hardware's approximation, without the
-// division's special cases (the chain of pivots waits for it).  0 gives a
-// non-finite value, as the division.
+// division's special cases (the chain of pivots waits for it), where d and 1 / d are
+// normal numbers.
 __device__ __forceinline__ double reciprocal(double d) {
+    if ((unsigned(__double2hiint(d)) >> 20 & 0x7ffu) - 2u >= 2042u) return 1.0 / d;
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
     r = fma(fma(-d, r, 1.0), r, r);

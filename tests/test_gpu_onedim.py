@@ -114,3 +114,13 @@ def test_band_factor_sizes(elements, radius, p1, order):
     rhs[-1] += 1e-3 * 0.7
     bound = 64 * n * np.finfo(float).eps * (np.abs(A) @ np.abs(u[1:]) + np.abs(rhs))
     assert u[0] == 0.3 and np.all(np.abs(A @ u[1:] - rhs) <= bound.max())
+
+
+@pytest.mark.parametrize("k", [0, 1019, 1021, 1022, 1023, -1018, -1021, -1022])
+def test_pivots_at_the_ends_of_the_range(lib, k):
+    """One local linear element of conductivity 2^k: its pivot's reciprocal is normal, subnormal, or the pivot the
+    smallest normal number."""
+    from nonlocal_gb300 import thermal as T
+    t = T.stationary_heat_equation_solver_1d(None, 1, 1, 1.0, 0.1, 1.0, conductivity=2.0 ** k, t_left=1.0,
+                                             q_right=2.0 ** (k - 1) if k > -1022 else 2.0 ** k, sin_source=False)
+    assert np.array_equal(t, [1.0, 1.5 if k > -1022 else 2.0])

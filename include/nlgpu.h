@@ -581,9 +581,12 @@ int nlgpu_nonstationary_1d_temperature(nlgpu_ctx* ctx, double* temperature);
  * NLGPU_OPTION_WAIT_LIMIT: microseconds (default 2 000 000) after which the CTAs
  * of the one-launch FP32 ILLT application stop waiting for one another's values;
  * the call then returns NLGPU_ERR_TIMEOUT.  0: at once, to see that status.  A
- * batch takes the smallest of its instances'. */
+ * batch takes the smallest of its instances'.
+ * NLGPU_OPTION_BAND_CTAS: CTAs of the 1D factorisation's cluster, 0 (default) 16
+ * where the device has room for such a cluster and 8 elsewhere, or 8. */
 enum { NLGPU_OPTION_GLOBAL_SWEEPS = 0, NLGPU_OPTION_ORDERED_PAIRS = 1, NLGPU_OPTION_ASSEMBLY_PRECISION = 2,
-       NLGPU_OPTION_FP32_SYMMETRIC = 3, NLGPU_OPTION_ASSEMBLY_WARPS = 4, NLGPU_OPTION_WAIT_LIMIT = 5 };
+       NLGPU_OPTION_FP32_SYMMETRIC = 3, NLGPU_OPTION_ASSEMBLY_WARPS = 4, NLGPU_OPTION_WAIT_LIMIT = 5,
+       NLGPU_OPTION_BAND_CTAS = 6 };
 enum { NLGPU_ASSEMBLY_AUTO = 0, NLGPU_ASSEMBLY_FF = 1, NLGPU_ASSEMBLY_FP64 = 2 };
 int nlgpu_set_option(nlgpu_ctx* ctx, int option, int value);
 /* Warps per CTA of the last float-float pair assembly (0 before any) and the

@@ -33,7 +33,7 @@ MATRIX_INNER, MATRIX_BOUND, MATRIX_LOCAL = 0, 1, 2
 PRECONDITIONER = {"identity": 0, "illt": 1, "illt_learned": 2}
 PRECISION = {"fp64": 0, "mixed": 1}
 OPTION_GLOBAL_SWEEPS, OPTION_ORDERED_PAIRS, OPTION_ASSEMBLY_PRECISION, OPTION_FP32_SYMMETRIC = 0, 1, 2, 3
-OPTION_ASSEMBLY_WARPS, OPTION_WAIT_LIMIT = 4, 5
+OPTION_ASSEMBLY_WARPS, OPTION_WAIT_LIMIT, OPTION_BAND_CTAS = 4, 5, 6
 BATCH_METHOD = {"identity_fp64": 0, "mixed_illt": 1}
 ASSEMBLY = {"auto": 0, "ff": 1, "fp64": 2}
 

@@ -1415,6 +1415,11 @@ int nlgpu_set_option(nlgpu_ctx* ctx, int option, int value) {
         ctx->ff_warps_option = value;
         return NLGPU_OK;
     }
+    if (option == NLGPU_OPTION_BAND_CTAS) {
+        if (value != 0 && value != 8) return NLGPU_ERR_ARG;
+        ctx->band_ctas = value;
+        return NLGPU_OK;
+    }
     if (option == NLGPU_OPTION_WAIT_LIMIT) {
         if (value < 0) return NLGPU_ERR_ARG;
         ctx->wait_limit_us = value;

@@ -543,6 +543,7 @@ struct Ctx {
     dbuf<double> temperature;
     bool nonstationary_ready = false;
     int wait_limit_us = 2000000;        // of k_jacobi_all's waits
+    int band_ctas = 0;                  // of the 1D factorisation's cluster (0: 16 where they fit, else 8)
     dbuf<int> sweep_error;
     bool force_global_sweeps = false;   // use the global-memory sweeps (for comparison)
     int ilt_sweeps = NLGPU_DEFAULT_TRIANGULAR_SWEEPS;   // FP32 ILLT: Jacobi sweeps per triangle (0: exact)

@@ -160,7 +160,7 @@ __global__ void k_first_kind_1d(i64 n, const double* __restrict__ bound0, double
     }
 }
 
-// Band LDL^T in blocks of BF_NB rows, one cluster of BF_CTAS CTAs (upper band:
+// Band LDL^T in blocks of BF_NB rows, one cluster of CTAS CTAs (upper band:
 // band[i * (bw + 1) + (j - i)]).
 //
 // A row at a time, every pivot cost three CTA barriers and bw^2 / 2 updates with a
@@ -182,7 +182,6 @@ __global__ void k_first_kind_1d(i64 n, const double* __restrict__ bound0, double
 // 2 001 rows of half bandwidth 102: 66.8 ms; 2.0 with the elimination in one warp (1.1
 // of it) and W shared by all CTAs; 1.42 now.
 constexpr int BF_NB = 16;
-constexpr int BF_CTAS = 16;
 constexpr int BF_THREADS = 256;
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
@@ -252,6 +251,8 @@ __device__ __forceinline__ void eliminate_block(const double (*diag)[BF_NB + 1],
         }
 }
 
+// CTAS: 16, or 8 (the largest portable cluster) where no 16 fit
+template<int CTAS>
 __global__ void __launch_bounds__(BF_THREADS) k_band_factor(BandFactor p) {
     extern __shared__ double bf_w[];
     __shared__ double diag[BF_NB][BF_NB + 1], wn[BF_NB][BF_NB], scaled[BF_NB][BF_NB], dks[2][BF_NB], lk[BF_NB * BF_NB],
@@ -327,7 +328,7 @@ __global__ void __launch_bounds__(BF_THREADS) k_band_factor(BandFactor p) {
             if (tid < BF_NB) dk[tid] = p.dinv[k0 + tid];
             lk[tid] = p.linv[kb * BF_NB * BF_NB + tid];
             __syncthreads();
-            for (int t = tid * (BF_CTAS - 1) + rank - 1; t < BF_NB * cols; t += (BF_CTAS - 1) * BF_THREADS) {
+            for (int t = tid * (CTAS - 1) + rank - 1; t < BF_NB * cols; t += (CTAS - 1) * BF_THREADS) {
                 const int r = t / cols, c = t % cols;
                 double v = 0.0, v2 = 0.0;
 #pragma unroll
@@ -347,7 +348,7 @@ __global__ void __launch_bounds__(BF_THREADS) k_band_factor(BandFactor p) {
                 __syncthreads();
             }
             // a warp per row a, rows dealt out over the other CTAs
-            for (int a = (rank - 1) + (BF_CTAS - 1) * warp; a < m; a += (BF_CTAS - 1) * (BF_THREADS / 32)) {
+            for (int a = (rank - 1) + (CTAS - 1) * warp; a < m; a += (CTAS - 1) * (BF_THREADS / 32)) {
                 double wa[BF_NB];
 #pragma unroll
                 for (int k = 0; k < BF_NB; ++k) wa[k] = W[k * w + a] * dk[k];
@@ -550,27 +551,42 @@ struct BandWork {
     }
 };
 
+template<int CTAS>
+bool launch_band_factor(Ctx& ctx, const BandFactor& p, size_t smem) {
+    auto kernel = k_band_factor<CTAS>;
+    allow_shared(kernel);
+    if (CTAS > 8) NL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = CTAS;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(CTAS);
+    cfg.blockDim = dim3(BF_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx.stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (CTAS > 8) {   // a part of a GPU may have no 16 SMs that one cluster can span
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) {
+            (void)cudaGetLastError();
+            return false;
+        }
+    }
+    NL_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
+    count_launch();
+    return true;
+}
+
+// 2 001 rows of half bandwidth 102, the whole solve: 1.75 ms with 16 CTAs, 2.28 with 8
 void band_factor(Ctx& ctx, i64 n, i64 bw, double* band, double* f, BandWork& work, int* failed) {
     work.resize(n, bw);
     BandFactor p{n, bw, band, f, work.linv.p, work.dinv.p, work.w.p, failed, 0};
     const size_t bytes = size_t(BF_NB) * size_t(bw + 1) * sizeof(double);
     p.in_shared = bytes <= 200 * 1024;
     const size_t smem = p.in_shared ? bytes : 0;
-    allow_shared(k_band_factor);
-    NL_CUDA(cudaFuncSetAttribute(k_band_factor, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = BF_CTAS;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(BF_CTAS);
-    cfg.blockDim = dim3(BF_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = ctx.stream;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    NL_CUDA(cudaLaunchKernelEx(&cfg, k_band_factor, p));
-    count_launch();
+    if (ctx.band_ctas == 8 || !launch_band_factor<16>(ctx, p, smem)) launch_band_factor<8>(ctx, p, smem);
 }
 
 void band_solve(Ctx& ctx, i64 n, i64 bw, const double* band, const BandWork& work, double* f, bool forward) {

@@ -124,3 +124,20 @@ def test_pivots_at_the_ends_of_the_range(lib, k):
     t = T.stationary_heat_equation_solver_1d(None, 1, 1, 1.0, 0.1, 1.0, conductivity=2.0 ** k, t_left=1.0,
                                              q_right=2.0 ** (k - 1) if k > -1022 else 2.0 ** k, sin_source=False)
     assert np.array_equal(t, [1.0, 1.5 if k > -1022 else 2.0])
+
+
+@pytest.mark.parametrize("elements, radius, p1, order", [(1, 0.1, 1.0, 1), (33, 0.06, 0.4, 2), (120, 0.9, 0.5, 1),
+                                                         (500, 0.3, 0.5, 2)])
+def test_cluster_of_eight(lib, monkeypatch, elements, radius, p1, order):
+    """The factorisation's form for devices without room for a cluster of 16."""
+    from nonlocal_gb300 import thermal as T
+
+    class Eight(T.Context):
+        def __init__(self, *args):
+            super().__init__(*args)
+            lib.check(self._lib.nlgpu_set_option(self.handle, lib.OPTION_BAND_CTAS, 8))
+
+    monkeypatch.setattr(T, "Context", Eight)
+    test_band_factor_sizes(elements, radius, p1, order)
+    c = Eight()
+    assert c._lib.nlgpu_set_option(c.handle, lib.OPTION_BAND_CTAS, 4) == 1

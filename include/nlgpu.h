@@ -146,6 +146,12 @@ int nlgpu_set_device(int device);
  * on, or NULL for a stream the context creates and owns. */
 int nlgpu_create(nlgpu_ctx** ctx, void* stream);
 int nlgpu_destroy(nlgpu_ctx* ctx);
+/* Buffers that calls have done with stay with their contexts for the next calls
+ * (at most 1 GiB each), and those of destroyed contexts with the process (at most
+ * 1 GiB a device), together at most 4 GiB a device.  They go back when an
+ * allocation fails; this gives those of the current device back to other
+ * libraries at once (it waits for the device). */
+int nlgpu_release_idle_memory(void);
 int nlgpu_synchronize(nlgpu_ctx* ctx);
 
 /* ---- mesh: mesh_2d<T, I>::mesh_2d + init (libraries/mesh/mesh_2d/mesh_2d.hpp:83-108)

@@ -98,6 +98,7 @@ SIGNATURES = {
     "nlgpu_set_device": (c_int, [c_int]),
     "nlgpu_create": (c_int, [ctypes.POINTER(c_p), c_p]),
     "nlgpu_destroy": (c_int, [c_p]),
+    "nlgpu_release_idle_memory": (c_int, []),
     "nlgpu_synchronize": (c_int, [c_p]),
     "nlgpu_mesh_2d": (c_int, [c_p, c_int, c_i64, c_p, c_i64, c_p]),
     "nlgpu_get_quadrature": (c_int, [c_p, c_p, c_p, c_p]),

@@ -424,6 +424,10 @@ int nlgpu_destroy(nlgpu_ctx* ctx) {
     });
 }
 
+int nlgpu_release_idle_memory(void) {
+    return guarded([&] { release_idle_memory(); });
+}
+
 int nlgpu_synchronize(nlgpu_ctx* ctx) {
     if (!ctx) return NLGPU_ERR_ARG;
     return guarded(ctx, [&] { NL_CUDA(cudaStreamSynchronize(ctx->stream)); });

@@ -118,7 +118,7 @@ inline unsigned grid_for(i64 n, int block, i64 cap = 152 * 32) {
 // order makes that safe without the device-wide wait of cudaFree.  When the arena
 // ends -- its stream has been waited for -- its blocks go to a pool that the process
 // shares.  Both are bounded (util.cu), and all idle blocks go back when an
-// allocation fails.  A solve makes 20 to 180 buffers, 10 to 20 us each with
+// allocation fails or the caller asks (nlgpu_release_idle_memory).  A solve makes 20 to 180 buffers, 10 to 20 us each with
 // cudaMalloc and cudaFree: a caller's 2 852-row CG took 2.48 ms, 1.78 with the
 // arena; the flux of 120 x 90 8-node elements 1.40 and 1.12; a classical
 // 151 x 97 solve 6.7 and 5.5; six 96 x 96 conductivity fields 25.2 and 23.3.
@@ -135,6 +135,8 @@ private:
     std::unique_ptr<Blocks> blocks;
     int device = 0;
 };
+
+void release_idle_memory();   // of the current device: every arena's and the pool's
 
 // the arena that this thread's allocations come from (none: cudaMalloc, cudaFree)
 extern thread_local std::shared_ptr<Arena> t_arena;

@@ -13,18 +13,21 @@ thread_local std::shared_ptr<Arena> t_arena;
 namespace {
 
 // What is kept idle: an arena BLOCK_MAX a block and IDLE_MAX in all, the pool of a
-// device POOL_MAX; anything above is freed at once, as it would be without them.
+// device POOL_MAX, all arenas and the pool of a device together DEVICE_MAX (1.4 % of its
+// memory); anything above is freed at once, as it would be without them.
 // (A problem whose matrices exceed BLOCK_MAX runs for tens of milliseconds, beside
 // which its few large frees, 1 to 5 ms each, matter little; the small ones matter.)
 constexpr size_t BLOCK_MAX = size_t(256) << 20;
 constexpr size_t IDLE_MAX = size_t(1) << 30;
 constexpr size_t POOL_MAX = size_t(1) << 30;
+constexpr size_t DEVICE_MAX = size_t(4) << 30;
 
 // idle blocks by size
 struct IdleBlocks {
     std::mutex mutex;
     std::multimap<size_t, void*> blocks;
     size_t bytes = 0;
+    std::atomic<size_t>* device_bytes = nullptr;   // idle on the device in all
     // the smallest block that holds `need` without wasting more than an eighth of
     // it (64 KB for small requests)
     void* get(size_t need, size_t* capacity) {
@@ -34,13 +37,23 @@ struct IdleBlocks {
         void* p = it->second;
         *capacity = it->first;
         bytes -= it->first;
+        *device_bytes -= it->first;
         blocks.erase(it);
         return p;
     }
     bool put(void* p, size_t capacity, size_t limit) {
         std::lock_guard<std::mutex> lock{mutex};
         if (capacity > BLOCK_MAX || bytes + capacity > limit) return false;
-        blocks.emplace(capacity, p);
+        if ((*device_bytes += capacity) > DEVICE_MAX) {
+            *device_bytes -= capacity;
+            return false;
+        }
+        try {
+            blocks.emplace(capacity, p);
+        } catch (...) {
+            *device_bytes -= capacity;
+            throw;
+        }
         bytes += capacity;
         return true;
     }
@@ -49,6 +62,7 @@ struct IdleBlocks {
         std::lock_guard<std::mutex> lock{mutex};
         for (const auto& b : blocks) cudaFree(b.second);
         blocks.clear();
+        *device_bytes -= bytes;
         bytes = 0;
     }
 };
@@ -63,15 +77,20 @@ namespace {
 // gone when static objects end)
 struct Memory {
     std::mutex mutex;
-    std::map<int, IdleBlocks> pools;
+    struct Device {
+        std::atomic<size_t> idle{0};
+        IdleBlocks pool;
+        Device() { pool.device_bytes = &idle; }
+    };
+    std::map<int, Device> devices;
     std::map<IdleBlocks*, int> arenas;   // with their devices
     IdleBlocks& pool(int device) {
         std::lock_guard<std::mutex> lock{mutex};
-        return pools[device];
+        return devices[device].pool;
     }
     void give_back(int device) {
         std::lock_guard<std::mutex> lock{mutex};
-        pools[device].give_back();
+        devices[device].pool.give_back();
         for (const auto& [blocks, d] : arenas)
             if (d == device) blocks->give_back();
     }
@@ -95,6 +114,7 @@ int current_device() {
 Arena::Arena() : blocks{std::make_unique<Blocks>()}, device{current_device()} {
     Memory& m = memory();
     std::lock_guard<std::mutex> lock{m.mutex};
+    blocks->device_bytes = &m.devices[device].idle;
     m.arenas.emplace(blocks.get(), device);
 }
 
@@ -105,6 +125,7 @@ Arena::~Arena() {
         m.arenas.erase(blocks.get());
     }
     IdleBlocks& pool = m.pool(device);
+    *blocks->device_bytes -= blocks->bytes;
     for (const auto& [size, p] : blocks->blocks) {
         bool kept = false;
         try {
@@ -114,6 +135,8 @@ Arena::~Arena() {
         if (!kept) cudaFree(p);
     }
 }
+
+void release_idle_memory() { memory().give_back(current_device()); }
 
 void* Arena::get(size_t bytes, size_t* capacity) {
     bytes = (bytes + 511) / 512 * 512;

@@ -151,6 +151,12 @@ def read_su2(path: str) -> Su2Mesh:
     return Su2Mesh(element, nodes, elements, groups)
 
 
+def release_idle_memory() -> None:
+    """Gives the device memory that finished calls left with their contexts, and destroyed contexts with the process,
+    back to other libraries (it is bounded, and also goes back when one of this library's allocations fails)."""
+    L.check(L.load().nlgpu_release_idle_memory())
+
+
 def cuthill_mckee(problem: "Problem2D", only_local: bool = False, reverse: bool = False) -> np.ndarray:
     """mesh::utils::cuthill_mckee(mesh, only_local, reverse) (cuthill_mckee.hpp:166-171)."""
     return problem.cuthill_mckee(only_local, reverse)

@@ -63,3 +63,31 @@ def test_threads(T):
     for t in threads:
         t.join()
     assert not bad
+
+
+def test_idle_memory_is_bounded_and_given_back(T):
+    """Sixteen contexts whose last call left several hundred megabytes each: at most 4 GiB stay idle, and go back when
+    asked for, with the contexts alive and after them; the contexts work on."""
+    import torch
+    free = lambda: torch.cuda.mem_get_info()[0]
+    torch.cuda.init()
+    contexts = [T.Context() for _ in range(16)]
+    T.release_idle_memory()
+    n = 1500000
+    csr = (np.append(np.arange(0, 2 * n, 2), 2 * n - 1), np.empty(2 * n - 1, dtype=np.int64), np.empty(2 * n - 1))
+    csr[1][0::2], csr[1][1::2] = np.arange(n), np.arange(1, n)
+    csr[2][0::2], csr[2][1::2] = 5.0, -1.0
+    b = np.ones(n)
+    x = [T.conjugate_gradient(c, csr, b, preconditioner_csr=csr, tolerance=1e-10)[0] for c in contexts]
+    held = free()
+    T.release_idle_memory()
+    idle = free() - held
+    # blocks of 4 n bytes and more, of which the driver's pages of 2 MiB take up to a third more
+    assert (1 << 30) < idle <= (4 << 30) * 4 // 3
+    assert all(np.array_equal(v, x[0]) for v in x)
+    assert np.array_equal(T.conjugate_gradient(contexts[0], csr, b, preconditioner_csr=csr, tolerance=1e-10)[0], x[0])
+    for c in contexts:
+        c.close()
+    held = free()
+    T.release_idle_memory()
+    assert 0 <= free() - held <= (1 << 30) * 4 // 3

@@ -46,7 +46,8 @@ constexpr int AS_WARPS = AS_THREADS / 32;
 // have in common (a stretched mesh whose conductivity makes up for it); what remains is the
 // loss.  FP64 solves allow 4 bits (58 - 4 against 53), mixed-precision ones 10 (48, as the
 // influence values); meshes beyond that, and for fixed-point values coordinates of
-// 2^(FX_MAX_EXPONENT + 1) radii, take the FP64 kernel: each of the two kernels looks and one returns at once.
+// 2^(FX_MAX_EXPONENT + 1) radii, take the FP64 kernel: this form's returns at once and
+// leaves a word that the host reads with the assembly's errors.
 constexpr int FF_NONE = 1 << 12;   // the four below are the largest difference of exponents + FF_NONE; 0: no element
 struct FFRange {
     unsigned long long extent;     // the bits of the largest finite |coordinate| in units of the radii
@@ -91,7 +92,7 @@ struct AssembleArgs {
     bool symmetric;
     int cap;                  // accumulator entries in shared memory
     int* error;               // set when an entry is missing from its pattern
-    FFGate gate;              // the fixed-point kernel's range: the FP64 kernel runs beyond it
+    FFGate gate;              // the fixed-point form's range; beyond it error[1] is set and nothing done
 };
 
 __device__ __forceinline__ i64 find_col(const int32_t* col, i64 lo, i64 hi, int32_t c) {
@@ -127,7 +128,6 @@ __global__ void __launch_bounds__(AS_THREADS) k_assemble_pairs(AssembleArgs a, M
     __shared__ i64 row_start[NEN];
     __shared__ int row_len[NEN], row_off[NEN + 1];
     __shared__ int use_smem;
-    if (a.gate.range && ff_in_range(a.gate)) return;   // k_assemble_pairs_ff did it
 
     auto* pairs = reinterpret_cast<PairSmem<NEN, NQ>*>(smem_raw);
     double* acc = reinterpret_cast<double*>(smem_raw + sizeof(PairSmem<NEN, NQ>) * AS_WARPS);
@@ -478,7 +478,10 @@ __global__ void __launch_bounds__(WARPS * 32) k_assemble_pairs_ff(AssembleArgs a
         for (int t = threadIdx.x; t < 2 * FF_EXP_K + 1; t += blockDim.x) etab[t] = ff{f.ff_table.v[t].x, f.ff_table.v[t].y};
     if constexpr (EXP && FIX)
         for (int t = threadIdx.x; t < FX_EXP_K; t += blockDim.x) xtab[t] = f.fx_table.v[t];
-    if (!ff_in_range(a.gate)) return;   // k_assemble_pairs does it
+    if (!ff_in_range(a.gate)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) a.error[1] = 1;
+        return;
+    }
     const int ex = FIX ? fx_exponent(&f.range->extent) : 0;
 
     auto* pairs = reinterpret_cast<PairFF<NEN, NQ>*>(smem_raw);
@@ -805,7 +808,7 @@ template<int NEN, int NQ, int INF>
 void launch_pairs(Ctx& ctx, const AssembleArgs& a, bool sym) {
     const size_t fixed = sizeof(PairSmem<NEN, NQ>) * AS_WARPS;
     const size_t dyn = fixed + size_t(a.cap) * (sizeof(double) + sizeof(int32_t));
-    const unsigned grid = unsigned(std::min<i64>(a.E, a.gate.range ? 152 * 2 : 152 * 16));   // mostly to return
+    const unsigned grid = unsigned(std::min<i64>(a.E, 152 * 16));
     if (sym) {
         auto kernel = k_assemble_pairs<NEN, NQ, INF, true>;
         NL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn)));
@@ -928,7 +931,7 @@ void assemble_full(Ctx& ctx) {
     a.bd_rp = ctx.bound.rowptr.p; a.bd_col = ctx.bound.col.p; a.bd_val = ctx.bound.val.p;
     a.symmetric = ctx.symmetric;
     dbuf<int> err;
-    err.resize(1);
+    err.resize(2);   // [an entry outside the pattern, beyond the fixed-point form's range]
     err.zero(ctx.stream);
     a.error = err.p;
     dbuf<FFRange> range;
@@ -941,8 +944,8 @@ void assemble_full(Ctx& ctx) {
     // enough for it; polynomials are as fast in fixed point (16.3 and 16.0).
     const bool fx = fx_supported(ctx.model);
     const bool fixed = fx && (ctx.ff_assembly ? ctx.model.influence != NLGPU_INFLUENCE_EXPONENTIAL : ctx.fx_assembly);
-    ctx.ff_assembled = ctx.ff_assembly && ff_supported(ctx.model);
-    if (ctx.ff_assembled || fixed) {
+    const bool staged = fixed || (ctx.ff_assembly && ff_supported(ctx.model));
+    if (staged) {
         const int nen = ctx.basis.nen, nq = ctx.basis.nq;
         ctx.ff_qcoord.reserve(size_t(ctx.n_elems * nq));
         ctx.ff_g.reserve(size_t(ctx.n_elems * nen * nq * 2));
@@ -967,18 +970,28 @@ void assemble_full(Ctx& ctx) {
         if (nen == 4) dispatch_influence_ff<4, 4>(ctx, a, f, sym);
         else dispatch_influence_ff<8, 9>(ctx, a, f, sym);
     }
-    if (ctx.basis.nen == 4) {
-        a.cap = int((200 * 1024 - sizeof(PairSmem<4, 4>) * AS_WARPS) / 12);
-        dispatch_influence<4, 4>(ctx, a, sym);
-    } else {
-        a.cap = int((200 * 1024 - sizeof(PairSmem<8, 9>) * AS_WARPS) / 12);
-        dispatch_influence<8, 9>(ctx, a, sym);
+    auto in_fp64 = [&] {
+        if (ctx.basis.nen == 4) {
+            a.cap = int((200 * 1024 - sizeof(PairSmem<4, 4>) * AS_WARPS) / 12);
+            dispatch_influence<4, 4>(ctx, a, sym);
+        } else {
+            a.cap = int((200 * 1024 - sizeof(PairSmem<8, 9>) * AS_WARPS) / 12);
+            dispatch_influence<8, 9>(ctx, a, sym);
+        }
+    };
+    int herr[2] = {0, 0};
+    auto finish = [&] {
+        set_dirichlet_diagonal(ctx, ctx.inner, 1.0);
+        err.download(herr, 2, ctx.stream);
+        NL_CUDA(cudaStreamSynchronize(ctx.stream));
+    };
+    if (!staged) in_fp64();
+    finish();
+    if (herr[1]) {
+        in_fp64();
+        finish();
     }
-    set_dirichlet_diagonal(ctx, ctx.inner, 1.0);
-    int herr = 0;
-    NL_CUDA(cudaMemcpyAsync(&herr, err.p, sizeof herr, cudaMemcpyDeviceToHost, ctx.stream));
-    NL_CUDA(cudaStreamSynchronize(ctx.stream));
-    NL_REQUIRE(herr == 0, NLGPU_ERR_STATE, "assembly met an entry outside the sparsity pattern");
+    NL_REQUIRE(herr[0] == 0, NLGPU_ERR_STATE, "assembly met an entry outside the sparsity pattern");
 }
 
 void assemble_local(Ctx& ctx, Csr& mtx, double weight, int integrand) {

@@ -553,7 +553,6 @@ struct Ctx {
     bool fp32_symmetric = false;        // FP32 SpMV from the strictly upper part (for comparison)
     int assembly_precision = NLGPU_ASSEMBLY_AUTO;
     bool ff_assembly = false;           // pair blocks in float-float on the FP32 pipes (mixed precision)
-    bool ff_assembled = false;          // the last assembly ran in float-float
     bool fx_assembly = true;            // else: pair blocks in fixed point instead of FP64 (where it covers the model)
     int ff_warps_option = 0;            // warps per CTA of the float-float pair assembly (0: tuned)
     int ff_warps_used = 0;              // ... of its last launch

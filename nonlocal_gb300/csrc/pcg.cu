@@ -669,13 +669,21 @@ void pcg_launch(Ctx& ctx, unsigned grid, size_t smem, PcgArgs& a) {
 
 // A x = b by CG with the ILLT (M, applied by FP64 Jacobi sweeps) or the identity
 // (M null).  Returns false, x as the caller left it, when the factor needs the
-// exact triangular solves.
+// exact triangular solves or the sweeps' values do not fit the device's memory.
 bool pcg_solve(Ctx& ctx, const Csr& A, const IncompleteCholesky* Mc, const double* b, double* x, double tolerance,
                i64 max_iterations, bool x_is_initial_guess, const CgChunkHook& on_chunk, CgResult& res) {
     const i64 n = A.rows;
     CgWork& w = ctx.cg;
     auto* M = const_cast<IncompleteCholesky*>(Mc);
     w.n = n;
+    if (M) {   // 400 bytes a row, more than a classical matrix: where they do not fit, the exact solves
+        try {
+            w.steps.reserve(size_t(PCG_MAX_SWEEPS + 1) * size_t(n) * 2);
+        } catch (const error& e) {
+            if (e.code != NLGPU_ERR_OUT_OF_MEMORY) throw;
+            return false;
+        }
+    }
     if (M && !M->j64_ready) {
         M->jlo.val64.resize(M->jlo.val.n);
         M->jup.val64.resize(M->jup.val.n);
@@ -708,7 +716,6 @@ bool pcg_solve(Ctx& ctx, const Csr& A, const IncompleteCholesky* Mc, const doubl
         a.wlo = M->jlo.max_width; a.wup = M->jup.max_width;
         const size_t bytes = size_t(rows) * (size_t(a.wlo + a.wup) * (sizeof(double) + sizeof(int32_t)) + 2 * sizeof(int32_t));
         if (smem + bytes <= room) { a.staged = 1; smem += bytes; }
-        w.steps.reserve(size_t(PCG_MAX_SWEEPS + 1) * size_t(n) * 2);
         NL_CUDA(cudaMemsetAsync(w.steps.p, 0, size_t(PCG_MAX_SWEEPS + 1) * size_t(n) * 16, ctx.stream));
         a.steps = reinterpret_cast<ulonglong2*>(w.steps.p);
         a.lo = {M->jlo.slice.p, M->jlo.col.p, M->jlo.val64.p};

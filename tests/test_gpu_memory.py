@@ -91,3 +91,40 @@ def test_idle_memory_is_bounded_and_given_back(T):
     held = free()
     T.release_idle_memory()
     assert 0 <= free() - held <= (1 << 30) * 4 // 3
+
+
+def test_sweep_values_that_do_not_fit(T):
+    """The FP64 CG's sweep values take 400 bytes a row: with room for the exact triangular solves' memory alone, the
+    solve takes those."""
+    import scipy.sparse as sp
+    import torch
+    n = 1200000
+    offs = [40000]   # few dependency levels
+    U = sp.diags([np.full(n, 8.0)] + [np.full(n - o, -1.0) for o in offs], [0] + offs, shape=(n, n)).tocsr()
+    csr = (U.indptr.astype(np.int64), U.indices.astype(np.int64), U.data)
+    A, b = U + sp.triu(U, 1).T, np.random.default_rng(0).standard_normal(n)
+
+    def solve(ctx):
+        x = T.conjugate_gradient(ctx, csr, b, preconditioner_csr=csr, tolerance=1e-10)[0]
+        assert np.linalg.norm(b - A @ x) <= 1.01e-10 * np.linalg.norm(b)
+
+    T.release_idle_memory()
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    ctx = T.Context()
+    T.L.check(ctx._lib.nlgpu_set_option(ctx.handle, T.L.OPTION_GLOBAL_SWEEPS, 1))
+    solve(ctx)   # its blocks are below 256 MiB and stay with the context
+    need = before - torch.cuda.mem_get_info()[0]
+    ctx.close()
+    T.release_idle_memory()
+    assert need < 1 << 30
+    room = need + (160 << 20)   # the sweep values are 480 MB, more than what only the exact solves need
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - room, dtype=torch.uint8, device="cuda")
+    try:
+        ctx = T.Context()
+        solve(ctx)
+        ctx.close()
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+        T.release_idle_memory()

@@ -859,7 +859,9 @@ void launch_pairs_ff_w(Ctx& ctx, AssembleArgs a, const FFArgs& f, bool sym) {
 template<int NEN, int NQ, int INF>
 void launch_pairs_ff(Ctx& ctx, AssembleArgs a, const FFArgs& f, bool sym) {
     int warps = ctx.ff_warps_option;
-    if (warps == 0 && a.E < 152 * 64) warps = 32;   // the four samples would cost as much as the assembly
+    // 32 was the choice on every workload measured; below this the four samples (12 elements an SM, a
+    // fifth of the assembly at the limit) and the clearing of the matrices cost more than a choice gives
+    if (warps == 0 && a.E < 152 * 64) warps = 32;
     if (warps == 0) {
         const int key = NEN * 1000 + INF * 10 + (sym ? 1 : 0) + (a.gate.fixed ? 2 : 0);
         auto it = ctx.ff_warps_tuned.find(key);

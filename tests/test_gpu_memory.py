@@ -128,3 +128,82 @@ def test_sweep_values_that_do_not_fit(T):
         del filler
         torch.cuda.empty_cache()
         T.release_idle_memory()
+
+
+def problem(T, n, stream=None, field=False, **model):
+    from nonlocal_gb300.meshgen import structured_quad_mesh
+    mesh = structured_quad_mesh(n, n - 3, "bilinear")
+    pb = T.Problem2D.from_mesh(mesh, stream=stream)
+    pb.set_model(T.Model2D(**dict(dict(influence="fast_polynomial", radius=(0.08, 0.08), local_weight=0.5), **model)))
+    if field:
+        pb.set_conductivity_field(np.random.default_rng(1).uniform(0.5, 2.0, mesh.n_elements * 4))
+    pb.add_boundary(T.Boundary(edges=mesh.boundaries["left"], kind="temperature", value=1.0))
+    pb.add_boundary(T.Boundary(edges=mesh.boundaries["right"], kind="flux", value=0.7))
+    pb.find_neighbours()
+    return pb
+
+
+def close(a, b):
+    # residuals of 1e-11 |b| and condition numbers below 1e4
+    return np.linalg.norm(a - b) <= 2e-7 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("options", [{}, dict(precision="mixed"), dict(precision="mixed", coarse_aggregates=64)])
+def test_callers_stream(T, options):
+    import torch
+    s = torch.cuda.Stream()
+    ref = problem(T, 40).stationary(tolerance=1e-11, **options)[0]
+    for _ in range(4):
+        with torch.cuda.stream(s):   # work before the call, on memory that the allocators may exchange
+            torch.randn(1 << 22, device="cuda")
+        assert close(problem(T, 40, s.cuda_stream).stationary(tolerance=1e-11, **options)[0], ref)
+
+
+def test_batches_in_turn(T):
+    """Batches made and destroyed while their instances live on and are assembled again."""
+    solvers = [T.NonstationaryHeatEquationSolver2D(problem(T, n), 1e-3) for n in (20, 31, 44)]
+    ref = {}
+    for k in range(6):
+        for s in solvers:
+            s.compute(np.zeros(s.problem.n_nodes))
+        batch = T.BatchNonstationary(solvers)
+        batch.set_method("mixed_illt" if k % 2 else "identity_fp64")
+        for _ in range(3):
+            batch.step(1.0, tolerance=1e-12)
+        t = np.concatenate([batch.temperature(i) for i in range(3)])
+        assert close(t, ref.setdefault(0, t))
+        if k % 3 == 0:
+            batch.close()
+    fields = [problem(T, 30, field=True) for _ in range(3)]
+    for k in range(4):
+        for p in fields:
+            p.conductivity_matrix("FULL")
+        x = np.concatenate(T.solve_assembled_batch(fields, tolerance=1e-11, precision="mixed" if k % 2 else "fp64")[0])
+        assert close(x, ref.setdefault(1, x))
+
+
+def test_threads_of_every_solver(T):
+    jobs = [lambda: problem(T, 45).stationary(tolerance=1e-11, precision="mixed")[0],
+            lambda: problem(T, 40).stationary(tolerance=1e-11, precision="mixed", coarse_aggregates=100)[0],
+            lambda: problem(T, 33, influence="exponential").stationary(tolerance=1e-11)[0],
+            lambda: problem(T, 30, field=True).stationary(tolerance=1e-11, precision="mixed")[0],
+            lambda: problem(T, 60, radius=(0.05, 0.05)).stationary(tolerance=1e-11, preconditioner="identity")[0],
+            lambda: T.stationary_heat_equation_solver_1d(None, 500, 2, 1.0, 0.05, 0.5)]
+    ref = [job() for job in jobs]
+    bad = []
+
+    def work(seed):
+        for i in range(12):
+            k = (5 * i + seed) % len(jobs)
+            try:
+                if not close(jobs[k](), ref[k]):
+                    bad.append(k)
+            except Exception as e:   # reported by the main thread
+                bad.append((k, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad

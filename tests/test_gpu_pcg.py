@@ -212,3 +212,21 @@ def test_split_entries_are_added_in_one_order(ctx, n):
     first, _ = T.conjugate_gradient(ctx, csr, b, tolerance=1e-12)
     for _ in range(12):
         assert np.array_equal(T.conjugate_gradient(ctx, csr, b, tolerance=1e-12)[0], first)
+
+
+@pytest.mark.parametrize("blocks", [1, 50, 5000])
+def test_pivots_that_fail_take_the_exact_factor(ctx, blocks):
+    """Kershaw's matrix, positive definite, whose IC(0) has a negative pivot: the fixed-point sweeps fail, and the exact
+    factorisation retries with its diagonal shifts."""
+    import scipy.sparse as sp
+    from nonlocal_gb300 import thermal as T
+    K = np.array([[3.0, -2, 0, 2], [-2, 3, -2, 0], [0, -2, 3, -2], [2, 0, -2, 3]])
+    A = sp.kron(sp.identity(blocks), K).tocsr()
+    U = sp.triu(A).tocsr()
+    U.eliminate_zeros()
+    U.sort_indices()
+    csr = (U.indptr.astype(np.int64), U.indices.astype(np.int64), U.data)
+    b = np.random.default_rng(0).standard_normal(4 * blocks)
+    x, rep = T.conjugate_gradient(ctx, csr, b, preconditioner_csr=csr, tolerance=1e-11)
+    assert rep.preconditioner_ok and rep.preconditioner_shifts >= 1
+    assert np.linalg.norm(b - A @ x) <= 1.01e-11 * np.linalg.norm(b)

@@ -322,42 +322,68 @@ __device__ __forceinline__ double2 ff_flux(const Model& m, double gx, double gy)
     return make_double2(m.cond[0] * gx + m.cond[2] * gy, m.cond[2] * gx + m.cond[1] * gy);
 }
 
-// one warp per element
+// One warp per element, on exponents: with an isotropic or orthotropic Lambda those of
+// g are those of w moved by the two conductivities' (to one bit), so that the loops hold no
+// FP64 operation.
 __global__ void k_ff_range(i64 E, int nen, int nq, const double* __restrict__ deriv, const double* __restrict__ qcoord, Model m,
                            FFRange* __restrict__ range) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    unsigned long long extent = 0;
+    const bool aniso = m.cond_kind != NLGPU_CONDUCTIVITY_ISOTROPIC && m.cond_kind != NLGPU_CONDUCTIVITY_ORTHOTROPIC;
+    auto high = [](double x) { return unsigned(__double2hiint(x)) & 0x7fffffffu; };
+    auto exponent = [](unsigned high) { return high ? int(high >> 20) : -1500; };   // zero counts as far below
+    const unsigned lx = m.cond_kind == NLGPU_CONDUCTIVITY_ORTHOTROPIC ? high(m.cond[0]) : 1u;
+    const unsigned ly = m.cond_kind == NLGPU_CONDUCTIVITY_ORTHOTROPIC ? high(m.cond[1]) : 1u;
+    const int lambda = exponent(lx) - exponent(ly);
+    unsigned long long at = 0;   // the largest finite |coordinate| of the lane's axis, as bits
     int wx = 0, wy = 0, gx = 0, gy = 0;
     for (i64 e = (blockIdx.x * i64(blockDim.x) + threadIdx.x) / 32; e < E; e += i64(gridDim.x) * blockDim.x / 32) {
         for (int t = lane; t < 2 * nq; t += 32) {
-            const double x = fabs(qcoord[2 * e * nq + t] * m.inv_r[t & 1]);
-            if (isfinite(x)) extent = max(extent, (unsigned long long)__double_as_longlong(x));
+            const unsigned long long x = (unsigned long long)__double_as_longlong(qcoord[2 * e * nq + t]) << 1 >> 1;
+            if (x < 0x7ffull << 52) at = max(at, x);
         }
         unsigned top[4] = {0u, 0u, 0u, 0u};   // high words of the largest |w_x|, |w_y|, |g_x|, |g_y|
-        auto high = [](double x) { return unsigned(__double2hiint(x)) & 0x7fffffffu; };
         for (int t = lane; t < nen * nq; t += 32) {
-            const double2 d = reinterpret_cast<const double2*>(deriv)[e * nen * nq + t], g = ff_flux(m, d.x, d.y);
+            const double2 d = reinterpret_cast<const double2*>(deriv)[e * nen * nq + t];
             top[0] = max(top[0], high(d.x)); top[1] = max(top[1], high(d.y));
-            top[2] = max(top[2], high(g.x)); top[3] = max(top[3], high(g.y));
+            if (aniso) {
+                const double2 g = ff_flux(m, d.x, d.y);
+                top[2] = max(top[2], high(g.x)); top[3] = max(top[3], high(g.y));
+            }
         }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) top[k] = __reduce_max_sync(full, top[k]);
-        // a component that is zero everywhere counts as far below the other
-        auto take = [](unsigned a, unsigned b, int& ab, int& ba) {
-            if (a >= 0x7ff00000u || b >= 0x7ff00000u || (a | b) == 0u) return;
-            const int d = (a ? int(a >> 20) : -1500) - (b ? int(b >> 20) : -1500);
+        top[0] = __reduce_max_sync(full, top[0]);
+        top[1] = __reduce_max_sync(full, top[1]);
+        if (aniso) {
+            top[2] = __reduce_max_sync(full, top[2]);
+            top[3] = __reduce_max_sync(full, top[3]);
+        }
+        auto take = [](int d, int& ab, int& ba) {
             ab = max(ab, FF_NONE + d);
             ba = max(ba, FF_NONE - d);
         };
-        take(top[0], top[1], wx, wy);
-        take(top[2], top[3], gx, gy);
+        const int d = exponent(top[0]) - exponent(top[1]);
+        if (max(top[0], top[1]) >= 0x7ff00000u || (top[0] | top[1]) == 0u) continue;
+        take(d, wx, wy);
+        if (!aniso && lx && ly) take(d + lambda, gx, gy);
+        else if (!aniso && (lx || ly)) take(lx && top[0] ? 3000 : ly && top[1] ? -3000 : 0, gx, gy);
+        else if (aniso && max(top[2], top[3]) < 0x7ff00000u && (top[2] | top[3])) take(exponent(top[2]) - exponent(top[3]), gx, gy);
     }
-    for (int o = 16; o > 0; o >>= 1) extent = max(extent, __shfl_xor_sync(full, extent, o));
-    if (lane == 0) {
-        atomicMax(&range->extent, extent);
-        atomicMax(&range->wx, wx); atomicMax(&range->wy, wy); atomicMax(&range->gx, gx); atomicMax(&range->gy, gy);
-    }
+    // the lanes of one axis, in units of its radius (2 nq and 32 are even: a lane keeps its axis)
+    for (int o = 16; o > 1; o >>= 1) at = max(at, __shfl_xor_sync(full, at, o));
+    unsigned long long extent =
+        (unsigned long long)__double_as_longlong(fabs(__longlong_as_double((long long)at) * m.inv_r[lane & 1]));
+    extent = max(extent, __shfl_xor_sync(full, extent, 1));
+    // a CTA's first (200 x 200 elements, every warp's atomics on five words: 40 us)
+    __shared__ FFRange cta;
+    if (threadIdx.x == 0) cta = FFRange{0ull, 0, 0, 0, 0};
+    __syncthreads();
+    auto raise = [&](FFRange* r, unsigned long long x, int a, int b, int c, int d) {
+        atomicMax(&r->extent, x);
+        atomicMax(&r->wx, a); atomicMax(&r->wy, b); atomicMax(&r->gx, c); atomicMax(&r->gy, d);
+    };
+    if (lane == 0) raise(&cta, extent, wx, wy, gx, gy);
+    __syncthreads();
+    if (threadIdx.x == 0) raise(range, cta.extent, cta.wx, cta.wy, cta.gx, cta.gy);
 }
 
 // x 2^(57 - e), |x| < 2^(e + 1), by integer operations (the FP64 pipe's conversions made the staging 0.19 ms
@@ -957,7 +983,7 @@ void assemble_full(Ctx& ctx) {
         range.resize(1);
         range.zero(ctx.stream);
         a.gate = {range.p, ctx.ff_assembly ? 10 : 4, fixed};
-        NL_LAUNCH(k_ff_range, grid_for(ctx.n_elems * 32, 256, 152 * 8), 256, 0, ctx.stream, ctx.n_elems, nen, nq, ctx.deriv.p,
+        NL_LAUNCH(k_ff_range, grid_for(ctx.n_elems * 32, 256, 152 * 4), 256, 0, ctx.stream, ctx.n_elems, nen, nq, ctx.deriv.p,
                   ctx.qcoord.p, ctx.model, range.p);
         NL_LAUNCH(k_ff_stage, grid_for(ctx.n_elems * 32, 256), 256, 0, ctx.stream, ctx.n_elems, nen, nq, ctx.elems.p,
                   ctx.is_inner.p, ctx.deriv.p, ctx.qcoord.p, a.cond_field, ctx.model, ctx.basis, range.p, fixed,

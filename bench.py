@@ -417,8 +417,11 @@ def run_gpu(args, w, mesh, world, rank, local, dist):
                               (6, "illt_jacobi32", 20), (1, "pair_assembly", 2), (7, "pair_assembly_ff", 2),
                               (8, "flux", 2)]:
         v = ctypes.c_double()
+        before = L.kernel_launches()
         L.check(lib.nlgpu_time_stage(h, stage, reps, ctypes.byref(v)))
         stage_ms[name] = v.value
+        if stage == 6:   # one launch an application, or one a sweep
+            jacobi_kernel = "k_jacobi_all" if L.kernel_launches() - before < 2 * (reps + 1) else "k_jacobi32"
     n = pb.n_nodes
     nnz_solver = rep_plain.nnz_solver
     spmv_bytes = nnz_solver * (8 + 4) + (n + 1) * 8 + 2 * n * 8
@@ -461,9 +464,10 @@ def run_gpu(args, w, mesh, world, rank, local, dist):
         k = L.DEFAULT_TRIANGULAR_SWEEPS
         jac_bytes = k * (factor_offdiag_entries(lib, h, n) * 8 + 2 * n * 16)
         achieved = jac_bytes / (stage_ms["illt_jacobi32"] * 1e-3) / 1e9
-        roof = {"kernel": "k_jacobi_all", "bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"],
+        roof = {"kernel": jacobi_kernel, "bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"],
                 "peak_kind": pk_kind, "unit": "GB/s", "frac": achieved / pk["hbm_gbs"],
-                "traffic": traffic.get(("k_jacobi32", args.workload)), "sweeps_per_application": 2 * k}
+                "traffic": traffic.get((jacobi_kernel, args.workload)), "launches_per_application":
+                    1 if jacobi_kernel == "k_jacobi_all" else 2 * k, "sweeps_per_application": 2 * k}
     roof["algorithmic_per_launch"] = {"spmv_bytes": spmv_bytes, "spmv32_bytes": spmv32_bytes,
                                       "pair_assembly_flops": ff_flops}
     roof["per_solve_ms"] = per_solve_ms
@@ -531,7 +535,7 @@ def run_gpu(args, w, mesh, world, rank, local, dist):
                                          "residual": rep_plain_same.residual, "tolerance": stop_tol},
         "speedup_vs_plain_fp64": plain_ms / mean_ms,
         "speedup_vs_plain_fp64_at_stop_tolerance": plain_same_ms / mean_ms,
-        # heat_equation_solution_2d::calc_flux of the solution (FP64): local flux, the
+        # heat_equation_solution_2d::calc_flux of the solution: local flux, the
         # nonlocal average over every ordered neighbour pair's nq x nq quadrature points
         "post_processing": {"flux_ms": stage_ms["flux"],
                             "flux_pair_quadrature_evaluations_per_s":

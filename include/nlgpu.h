@@ -573,8 +573,10 @@ int nlgpu_nonstationary_1d_temperature(nlgpu_ctx* ctx, double* temperature);
  * significant bits) covers the fast-polynomial, polynomial and exponential
  * influence with integral p / n, fixed point those with n = 2 (polynomials of
  * even p and q <= 16, exponentials of p = 2 and 0.333 <= q <= 2); other models
- * use FP64.  The nodal flux's nonlocal average is in float-float where that
- * covers the model, in FP64 otherwise and with NLGPU_ASSEMBLY_FP64.
+ * use FP64, and so do meshes on which the fixed-point form would be less accurate
+ * (elements stretched in different directions, coordinates beyond 2^21 radii).
+ * The nodal flux takes its influence values in fixed point in the same cases, its
+ * loads and sums are FP64; with NLGPU_ASSEMBLY_FP64 all of it is.
  * NLGPU_OPTION_FP32_SYMMETRIC = 1 makes the mixed solve's FP32 SpMV read only
  * the strictly upper part of a symmetric solver matrix (half the entries,
  * transposed contributions added with shared-memory atomics) instead of its

@@ -347,7 +347,7 @@ enum { P_PQ = 0, P_RR = 1, P_RZ_A = 2, P_RZ_B = 3, P_BB = 4, P_COUNT = 5 };   //
 struct IncompleteCholesky {
     SweepPlan fwd_plan, bwd_plan;
     i64 n = 0, nnz = 0;
-    double mean_reach = 0.0;     // of a row: its last column minus its own
+    double far_share = 0.0;      // of the entries: those more than two CTAs of k_jacobi_all from the diagonal
     dbuf<i64> rp;                // upper pattern (diagonal first)
     dbuf<int32_t> col;
     dbuf<double> a_scaled, u;    // S A S and the factor values
@@ -678,6 +678,7 @@ void jacobi_apply32(Ctx& ctx, IncompleteCholesky& ic, int sweeps, const float* r
 // waits for the stream; NLGPU_ERR_TIMEOUT when a wait of a factor's application (exact
 // sweeps, k_jacobi_all) has given up since the factor was built or this was last called
 void check_sweeps(Ctx& ctx);
+i64 jacobi_cta_rows(i64 n);   // rows of a CTA of the one-launch application (k_jacobi_all)
 // mixed.cu
 // FP32 copy of the solver matrix A (full rows) for the mixed solve; with the
 // upper storage of a symmetric A given, only its strictly upper part is copied

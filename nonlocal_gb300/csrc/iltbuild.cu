@@ -24,16 +24,16 @@ constexpr int IB_THREADS = 256;
 constexpr int IB_LEVEL_THREADS = 1024;
 
 // every row of the upper pattern starts with its diagonal
-// also the rows' reaches (last column minus the diagonal's) added up
-__global__ void k_check_diag_first(i64 n, const i64* __restrict__ rp, const int32_t* __restrict__ col,
-                                   int* __restrict__ bad, unsigned long long* __restrict__ reach) {
+// also how many entries lie more than `near` columns from the diagonal
+__global__ void k_check_diag_first(i64 n, const i64* __restrict__ rp, const int32_t* __restrict__ col, i64 near,
+                                   int* __restrict__ bad, unsigned long long* __restrict__ far) {
     unsigned long long sum = 0;
     for (i64 r = blockIdx.x * i64(blockDim.x) + threadIdx.x; r < n; r += i64(gridDim.x) * blockDim.x) {
         if (rp[r + 1] <= rp[r] || col[rp[r]] != int32_t(r)) *bad = 1;
-        else sum += max(col[rp[r + 1] - 1] - int32_t(r), 0);
+        for (i64 k = rp[r]; k < rp[r + 1]; ++k) sum += col[k] - r > near;
     }
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(reach, sum);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(far, sum);
 }
 
 __global__ void k_col_count(i64 nnz, const int32_t* __restrict__ col, unsigned long long* __restrict__ cnt) {
@@ -200,12 +200,12 @@ void ilt_levels_gpu(Ctx& ctx, IncompleteCholesky& ic) {
 // Jacobi layouts, all on the device
 void ilt_structure_gpu(Ctx& ctx, const Csr& upper, IncompleteCholesky& ic, bool levels) {
     const i64 n = upper.rows, nnz = upper.nnz;
-    dbuf<unsigned long long> found;   // [a bad row, the reaches]
+    dbuf<unsigned long long> found;   // [a bad row, far entries]
     found.resize(2);
     found.zero(ctx.stream);
     int* flag = reinterpret_cast<int*>(found.p);
     NL_LAUNCH(k_check_diag_first, grid_for(n, IB_THREADS), IB_THREADS, 0, ctx.stream, n, upper.rowptr.p, upper.col.p,
-              flag, found.p + 1);
+              2 * jacobi_cta_rows(n), flag, found.p + 1);
     ic.rp.resize(size_t(n + 1));
     ic.col.resize(size_t(nnz));
     NL_CUDA(cudaMemcpyAsync(ic.rp.p, upper.rowptr.p, size_t(n + 1) * sizeof(i64), cudaMemcpyDeviceToDevice, ctx.stream));
@@ -228,7 +228,7 @@ void ilt_structure_gpu(Ctx& ctx, const Csr& upper, IncompleteCholesky& ic, bool 
     found.download(h, 2, ctx.stream);
     NL_CUDA(cudaStreamSynchronize(ctx.stream));
     NL_REQUIRE(!h[0], NLGPU_ERR_ARG, "every row of the preconditioner matrix needs its diagonal first");
-    ic.mean_reach = double(h[1]) / double(n);
+    ic.far_share = double(h[1]) / double(std::max<i64>(nnz - n, 1));
     ic.ic_levels = 0;
     if (levels) ilt_levels_gpu(ctx, ic);
     // Jacobi layouts of U^T (values u[l_to_u]) and U

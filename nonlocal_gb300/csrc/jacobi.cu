@@ -97,22 +97,28 @@ __global__ void __launch_bounds__(JB_THREADS) k_jacobi32(i64 n, const i64* __res
 // each a store and a load through L2 (a message between SMs of different dies
 // takes about 0.45 us) and the row's sum; a gather of a value from far away moves a
 // 32-byte sector past L1 for its 8 bytes, where k_jacobi32 gathers floats through L1.
-// Which form: by the entries of a triangle, with the rows' mean reach against a
-// CTA's rows.  Microseconds an FCG iteration (twelve sweeps and everything else), one launch per
-// sweep -> this:
+// Which form: by the entries of a triangle, and by the share of them whose columns lie more
+// than two CTAs away: 0 for rows numbered along the mesh, 0 to 1.2 % after cuthill_mckee of
+// the local graph, 4.8 to 8.1 % after that of the nonlocal graph, 97 % at random.  (The mean
+// reach of the rows is below a CTA after the nonlocal cuthill_mckee, and says nothing.)  At
+// 250x250 8-node, nonlocal cuthill_mckee, an application takes 72 million instructions and
+// 10 million L2 requests, by rows 28 and 3.4.
+// Microseconds an FCG iteration (twelve sweeps and everything else), one launch per sweep -> this:
 //   near columns   bilinear 500x500, 1.0 million entries    109 -> 97
 //                  bilinear 600x600, 1.4                    144 -> 132
+//                  8-node 200x200, local cuthill_mckee, 0.88    100 -> 88
 //                  8-node 300x300, 2.0                      140 -> 151
+//                  8-node 300x300, local cuthill_mckee, 2.0 148 -> 276
 //   far ones       8-node 170x170, nonlocal cuthill_mckee, 0.64    186 -> 173
 //                  the same numbered at random              357 -> 349
 //                  bilinear 400x400 at random, 0.64         125 -> 124
-//                  8-node 200x200, nonlocal cuthill_mckee, 0.88    324 -> 383
+//                  8-node 200x200, nonlocal cuthill_mckee, 0.88    313 -> 391
 //                  bilinear 500x500 at random, 1.0          157 -> 170
-//                  8-node 300x300, local cuthill_mckee, 2.0 148 -> 276
+//                  8-node 250x250, nonlocal cuthill_mckee, 1.4     603 -> 919
 constexpr int JA_THREADS = 1024;
 constexpr int JA_MIN_ROWS = 64;
 constexpr i64 JA_MAX_NEAR = 1700000, JA_MAX_FAR = 700000;   // entries of a triangle
-constexpr double JA_FAR = 4.0;    // mean reach in CTAs
+constexpr double JA_FAR_SHARE = 0.03;
 constexpr i64 JA_MAX_ROWS = 400000;    // 361 201 measured
 constexpr int JA_MAX_SWEEPS = 32;
 constexpr int JA_BATCH = 4;       // gathers in flight per lane
@@ -265,6 +271,13 @@ void jacobi_fill(Ctx& ctx, IncompleteCholesky& ic) {
     NL_LAUNCH(k_jacobi_diag, grid_for(n, 256), 256, 0, ctx.stream, n, ic.rp.p, ic.u.p, ic.scale.p, ic.jc.p, ic.jdinv.p);
 }
 
+i64 jacobi_cta_rows(i64 n) {
+    int dev = 0, sms = 0;
+    NL_CUDA(cudaGetDevice(&dev));
+    NL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    return std::max<i64>(JA_MIN_ROWS, ((n + sms - 1) / sms + 31) / 32 * 32);
+}
+
 void check_sweeps(Ctx& ctx) {
     if (!ctx.sweep_error.n) return;
     int err = 0;
@@ -278,19 +291,16 @@ void check_sweeps(Ctx& ctx) {
 void jacobi_apply32(Ctx& ctx, IncompleteCholesky& ic, int sweeps, const float* r, float* z, const double* flags) {
     NL_REQUIRE(sweeps >= 1, NLGPU_ERR_ARG, "at least one Jacobi sweep per triangle");
     const i64 n = ic.n;
-    int dev = 0, sms = 0;
-    NL_CUDA(cudaGetDevice(&dev));
-    NL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const i64 rows = std::max<i64>(JA_MIN_ROWS, ((n + sms - 1) / sms + 31) / 32 * 32);
-    const bool far = ic.mean_reach > JA_FAR * double(rows);
-    if (n <= JA_MAX_ROWS && ic.nnz - n <= (far ? JA_MAX_FAR : JA_MAX_NEAR) && sweeps <= JA_MAX_SWEEPS) {
+    const i64 rows = jacobi_cta_rows(n);
+    const i64 most = ic.far_share > JA_FAR_SHARE ? JA_MAX_FAR : JA_MAX_NEAR;
+    if (n <= JA_MAX_ROWS && ic.nnz - n <= most && sweeps <= JA_MAX_SWEEPS) {
         const unsigned grid = unsigned((n + rows - 1) / rows);
         const size_t words = size_t(sweeps + 1) * size_t(n);
         // the CTAs' numbers go on from application to application; another split starts
         // afresh (outside any capture: a solve's first application is eager)
         if (ic.jsteps.n < words || ic.jsplit_n != n || ic.jsplit_rows != rows) {
             ic.jsteps.reserve(words);
-            ic.jtags.reserve(size_t(sms));
+            ic.jtags.reserve(grid);
             ic.jsteps.zero(ctx.stream);
             ic.jtags.zero(ctx.stream);
             ic.jsplit_n = n;

@@ -87,3 +87,30 @@ def test_sweeps_by_the_reach_of_the_columns(lib, step, one_launch):
     # vector or less, and FP32 a few 1e-7
     ref = pre.solve(x.astype(np.float64))
     assert np.linalg.norm(y - ref) <= 3e-4 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("every, one_launch", [(0, True), (20, True), (5, False)])
+def test_sweeps_by_the_share_of_far_columns(lib, every, one_launch):
+    """160 000 rows of five near entries, and one 20 000 columns away on none of them, on every 20th (0.9 %
+    of the entries) and on every 5th (3.4 %): a mean reach below four CTAs in all three; both forms give M^-1 x."""
+    import scipy.sparse as sp
+    from nonlocal_gb300 import thermal as T
+    n, k, away = 160000, 5, 20000
+    offs = [100 * j for j in range(1, k + 1)]
+    U = sp.diags([np.full(n, 4.0 * (k + 1))] + [np.full(n - o, -1.0) for o in offs], [0] + offs, shape=(n, n))
+    if every:
+        rows = np.arange(0, n - away, every)
+        U = U + sp.coo_matrix((np.full(rows.size, -1.0), (rows, rows + away)), shape=(n, n))
+    U = U.tocsr()
+    U.sort_indices()
+    pre = T.EigenILLTPreconditioner()
+    assert pre.compute((U.indptr, U.indices, U.data)).computation_info() == pre.SUCCESS
+    x = np.random.default_rng(0).standard_normal(n).astype(np.float32)
+    pre.solve_f32(x)
+    before = lib.kernel_launches()
+    y = pre.solve_f32(x, 6)
+    launches = lib.kernel_launches() - before
+    assert launches == 1 if one_launch else launches >= 12
+    # a row's off-diagonal sum is at most 6 / 24 of its diagonal, as above
+    ref = pre.solve(x.astype(np.float64))
+    assert np.linalg.norm(y - ref) <= 3e-4 * np.linalg.norm(ref)

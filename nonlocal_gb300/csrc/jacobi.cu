@@ -104,8 +104,13 @@ __global__ void __launch_bounds__(JB_THREADS) k_jacobi32(i64 n, const i64* __res
 // 250x250 8-node, nonlocal cuthill_mckee, an application takes 72 million instructions and
 // 10 million L2 requests, by rows 28 and 3.4.
 // Microseconds an FCG iteration (twelve sweeps and everything else), one launch per sweep -> this:
-//   near columns   bilinear 500x500, 1.0 million entries    109 -> 97
-//                  bilinear 600x600, 1.4                    144 -> 132
+// (a nonlocal matrix passes through L2 between two applications, a local one leaves the factor there):
+//   short rows     bilinear 500x500, 1.0 million entries    109 -> 97, nonlocal 246 -> 239
+//                  bilinear 600x600, 1.4                    140 -> 140, nonlocal 305 -> 293
+//   longer ones    8-node 200x200, 0.88                     101 -> 83, nonlocal 301 -> 286
+//                  8-node 225x225, 1.1                      nonlocal 394 -> 384
+//                  8-node 250x250, 1.4                      115 -> 117, nonlocal 526 -> 558
+//                  the same with a radius of 0.02           227 -> 255
 //                  8-node 200x200, local cuthill_mckee, 0.88    100 -> 88
 //                  8-node 300x300, 2.0                      140 -> 151
 //                  8-node 300x300, local cuthill_mckee, 2.0 148 -> 276
@@ -117,7 +122,8 @@ __global__ void __launch_bounds__(JB_THREADS) k_jacobi32(i64 n, const i64* __res
 //                  8-node 250x250, nonlocal cuthill_mckee, 1.4     603 -> 919
 constexpr int JA_THREADS = 1024;
 constexpr int JA_MIN_ROWS = 64;
-constexpr i64 JA_MAX_NEAR = 1700000, JA_MAX_FAR = 700000;   // entries of a triangle
+constexpr i64 JA_MAX_NEAR = 1700000, JA_MAX_LONG = 1200000, JA_MAX_FAR = 700000;   // entries of a triangle
+constexpr i64 JA_LONG_ROW = 5;    // a row's mean entries: 4 on bilinear meshes, 7 on 8-node ones
 constexpr double JA_FAR_SHARE = 0.03;
 constexpr i64 JA_MAX_ROWS = 400000;    // 361 201 measured
 constexpr int JA_MAX_SWEEPS = 32;
@@ -292,8 +298,9 @@ void jacobi_apply32(Ctx& ctx, IncompleteCholesky& ic, int sweeps, const float* r
     NL_REQUIRE(sweeps >= 1, NLGPU_ERR_ARG, "at least one Jacobi sweep per triangle");
     const i64 n = ic.n;
     const i64 rows = jacobi_cta_rows(n);
-    const i64 most = ic.far_share > JA_FAR_SHARE ? JA_MAX_FAR : JA_MAX_NEAR;
-    if (n <= JA_MAX_ROWS && ic.nnz - n <= most && sweeps <= JA_MAX_SWEEPS) {
+    const i64 entries = ic.nnz - n;
+    const i64 most = ic.far_share > JA_FAR_SHARE ? JA_MAX_FAR : entries > JA_LONG_ROW * n ? JA_MAX_LONG : JA_MAX_NEAR;
+    if (n <= JA_MAX_ROWS && entries <= most && sweeps <= JA_MAX_SWEEPS) {
         const unsigned grid = unsigned((n + rows - 1) / rows);
         const size_t words = size_t(sweeps + 1) * size_t(n);
         // the CTAs' numbers go on from application to application; another split starts

@@ -114,3 +114,24 @@ def test_sweeps_by_the_share_of_far_columns(lib, every, one_launch):
     # a row's off-diagonal sum is at most 6 / 24 of its diagonal, as above
     ref = pre.solve(x.astype(np.float64))
     assert np.linalg.norm(y - ref) <= 3e-4 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("n, k, one_launch", [(150000, 7, True), (190000, 7, False), (290000, 5, True)])
+def test_sweeps_by_the_length_of_the_rows(lib, n, k, one_launch):
+    """Near columns: 1.05 million entries of seven a row take the one-launch application, 1.33 million do not, and
+    of five a row 1.45 million do; both forms give M^-1 x."""
+    import scipy.sparse as sp
+    from nonlocal_gb300 import thermal as T
+    offs = [100 * j for j in range(1, k + 1)]
+    U = sp.diags([np.full(n, 4.0 * k)] + [np.full(n - o, -1.0) for o in offs], [0] + offs, shape=(n, n)).tocsr()
+    pre = T.EigenILLTPreconditioner()
+    assert pre.compute((U.indptr, U.indices, U.data)).computation_info() == pre.SUCCESS
+    x = np.random.default_rng(0).standard_normal(n).astype(np.float32)
+    pre.solve_f32(x)
+    before = lib.kernel_launches()
+    y = pre.solve_f32(x, 6)
+    launches = lib.kernel_launches() - before
+    assert launches == 1 if one_launch else launches >= 12
+    # a row's off-diagonal sum is at most a quarter of its diagonal, as above
+    ref = pre.solve(x.astype(np.float64))
+    assert np.linalg.norm(y - ref) <= 3e-4 * np.linalg.norm(ref)

@@ -105,12 +105,12 @@ __global__ void __launch_bounds__(JB_THREADS) k_jacobi32(i64 n, const i64* __res
 // 10 million L2 requests, by rows 28 and 3.4.
 // Microseconds an FCG iteration (twelve sweeps and everything else), one launch per sweep -> this:
 // (a nonlocal matrix passes through L2 between two applications, a local one leaves the factor there):
-//   short rows     bilinear 500x500, 1.0 million entries    109 -> 97, nonlocal 246 -> 239
-//                  bilinear 600x600, 1.4                    140 -> 140, nonlocal 305 -> 293
-//   longer ones    8-node 200x200, 0.88                     101 -> 83, nonlocal 301 -> 286
-//                  8-node 225x225, 1.1                      nonlocal 394 -> 384
-//                  8-node 250x250, 1.4                      115 -> 117, nonlocal 526 -> 558
-//                  the same with a radius of 0.02           227 -> 255
+//   short rows     bilinear 500x500, 1.0 million entries    109 -> 97, nonlocal 247 -> 240
+//                  bilinear 600x600, 1.4                    139 -> 138, nonlocal 306 -> 293
+//   longer ones    8-node 200x200, 0.88                     97 -> 79, nonlocal 300 -> 286
+//                  8-node 225x225, 1.1                      nonlocal 389 -> 383
+//                  8-node 250x250, 1.4                      114 -> 118, nonlocal 519 -> 556
+//                  the same with a radius of 0.02           227 -> 262
 //                  8-node 200x200, local cuthill_mckee, 0.88    100 -> 88
 //                  8-node 300x300, 2.0                      140 -> 151
 //                  8-node 300x300, local cuthill_mckee, 2.0 148 -> 276

@@ -121,6 +121,38 @@ __device__ __forceinline__ bool mx_reduce_last(double (&v)[N], double* part, uns
     return true;
 }
 
+// The same for one sum of which only lane 0 of each warp holds a part, with 72 bytes of
+// shared memory: k_spmv32 gathers through L1, and what its eight CTAs an SM hold as shared
+// memory is taken from there (2 KB each: 8-node 200x200 at random 316 -> 322 ms a solve, 250x250 743 -> 757).
+// Only thread 0 of the last block gets the total.
+__device__ __forceinline__ bool mx_dot_last(double& v, double* part, unsigned* ticket, double* sh) {
+    constexpr int WARPS = MX_THREADS / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) sh[warp] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) s += sh[w];
+        part[blockIdx.x] = s;
+        __threadfence();
+        sh[WARPS] = atomicAdd(ticket, 1u) == gridDim.x - 1 ? 1.0 : 0.0;
+    }
+    __syncthreads();
+    if (sh[WARPS] == 0.0) return false;
+    double s = 0.0;
+    for (unsigned k = threadIdx.x; k < gridDim.x; k += blockDim.x) s += __ldcg(part + k);
+    s = warp_sum(s);
+    if (lane == 0) sh[warp] = s;
+    __syncthreads();
+    if (threadIdx.x != 0) return false;
+    v = 0.0;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) v += sh[w];
+    *ticket = 0u;
+    return true;
+}
+
 // q = A32 p (FP32 values, FP32 accumulation), warp per padded full row, in
 // difference form  y_i = sum_j a_ij (x_j - x_i) + s_i x_i  with s_i the row sum
 // of the FP64 matrix: the rows of the conductivity matrix sum to (nearly) zero,
@@ -140,7 +172,7 @@ __global__ void __launch_bounds__(MX_THREADS) k_spmv32(i64 n, const i64* __restr
                                                        const float* __restrict__ rowsum, const float* __restrict__ x,
                                                        float* __restrict__ y, double* __restrict__ dot_partial,
                                                        double* __restrict__ flags, i64 ring, unsigned* ticket) {
-    __shared__ double sh[MX_THREADS + 1];
+    __shared__ double sh[MX_THREADS / 32 + 1];
     if (flags && flags[S_DONE] != 0.0) return;
     i64 slot = 0;
     if (ring) {   // direction slot of the current iteration in the rings of x and y
@@ -171,10 +203,10 @@ __global__ void __launch_bounds__(MX_THREADS) k_spmv32(i64 n, const i64* __restr
         }
     }
     if (dot_partial) {   // p_j.q_j: the last block stores it and alpha = (p_j.r) / (p_j.q_j)
-        double v[1] = {double(dot)};
-        if (mx_reduce_last<1>(v, dot_partial, ticket, sh) && threadIdx.x == 0) {
-            flags[S_PQ + slot] = v[0];
-            flags[S_ALPHA] = flags[S_PR] / v[0];
+        double v = double(dot);
+        if (mx_dot_last(v, dot_partial, ticket, sh)) {
+            flags[S_PQ + slot] = v;
+            flags[S_ALPHA] = flags[S_PR] / v;
         }
     }
 }
